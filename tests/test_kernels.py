@@ -125,6 +125,31 @@ def test_float32_matrix_product(ops, m, n, k):
         ops.linear(x.to(DEV), rand((n, k + 1), torch.float32, 7).to(DEV))
 
 
+@pytest.mark.parametrize("m, n, k", [(1, 128, 4), (16, 127, 36), (17, 129, 256), (33, 256, 2048), (65, 260, 300), (129, 2048, 1028),
+                                     (300, 514, 2052), (150, 19000, 260), (700, 2048, 2048), (1030, 7000, 544)])
+def test_float32_matrix_product_on_split_operands(ops, m, n, k):
+    """Sizes around the tiles of the tensor-core product: K in one segment and several, in turn and side by side."""
+    x, w = rand((m, k), torch.float32, 5).to(DEV), rand((n, k), torch.float32, 6).to(DEV)
+    got = ops.linear(x, w)
+    # a product of split operands lacks up to 2^-21 of itself, each of a block's 12 MMAs cuts up to 2^-22 of its sum, and
+    # the blocks' and segments' sums are added with 2^-24 each
+    bound = (2.0 ** -21 + 12 * 2.0 ** -22 + (k / 32 + 16) * 2.0 ** -24) * (x.double().abs() @ w.double().abs().T)
+    assert bool(((got.double() - x.double() @ w.double().T).abs() <= bound + 1e-30).all())
+    for a, b in ((0, 1), (m // 2, m), (m // 3, m // 3 + 17)):              # whatever rows stand beside them
+        assert torch.equal(ops.linear(x[a:b].contiguous(), w), got[a:b])
+    torch.cuda.synchronize()
+    ops.check_device_errors()
+
+
+def test_float32_matrix_product_keeps_infinities_and_nans(ops):
+    x, w = rand((40, 512), torch.float32, 5), rand((300, 512), torch.float32, 6)
+    x[3, 5], x[9, 7], w[11, 100], w[12, 100] = math.inf, math.nan, -math.inf, 3e38
+    x[20, 100] = -3e38                                                       # an overflow beside w[12, 100]
+    got, want = ops.linear(x.to(DEV), w.to(DEV)).cpu(), (x.double() @ w.double().T).float()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[got.isinf()], want[want.isinf()])
+
+
 @pytest.mark.parametrize("m, n, k", [(1, 48, 64), (9, 1000, 192), (300, 250, 520)])
 def test_bfloat16_matrix_product(ops, m, n, k):
     x, w = rand((m, k), torch.bfloat16, 5), rand((n, k), torch.bfloat16, 6)

@@ -18,62 +18,15 @@
 //
 // Every wait on an mbarrier gives up after about two seconds, records where in an error word the
 // host can read, and the CTA goes on to free its tensor memory and return.
-#include <cuda.h>
-
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace {
 
 constexpr int BM = 128, BK = 64, UMMA_K = 16;
 constexpr int EPI_WARPS = 8, THREADS = 64 + 32 * EPI_WARPS;     // two epilogue warps for each quarter of the accumulator's lanes
 constexpr int A_BYTES = BM * BK * 2;
-constexpr long long WAIT_CYCLES = 4000000000ll;     // about two seconds at 2 GHz
 
 enum { EPI_STORE = 0, EPI_SWIGLU = 1 };
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-// false: the wait ran out of time (the error word says which one)
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* error, int code) {
-    const long long start = clock64();
-    uint32_t done = 0;
-    while (true) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-        if (done) return true;
-        if (clock64() - start > WAIT_CYCLES) {
-            atomicExch(error, code);
-            return false;
-        }
-    }
-}
-
-__device__ __forceinline__ void tma_load_2d(void* smem, const CUtensorMap* map, uint64_t* bar, int x, int y) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(smem_u32(smem)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y) : "memory");
-}
-
-// Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes (64 bfloat16) with
-// the 128-byte swizzle: start address, stride between groups of 8 rows (1024 bytes), sm_100 version.
-__device__ __forceinline__ uint64_t smem_desc(const void* tile) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_u32(tile) & 0x3FFFF) >> 4);          // bits 0..13: start address / 16
-    d |= (uint64_t)1 << 16;                                      // bits 16..29: leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;                            // bits 32..45: stride byte offset / 16
-    d |= (uint64_t)1 << 46;                                      // bits 46..47: descriptor version of sm_100
-    d |= (uint64_t)2 << 61;                                      // bits 61..63: 128-byte swizzle
-    return d;
-}
 
 // Instruction descriptor: bfloat16 x bfloat16 -> float32, both operands K-major, tile M x N.
 __device__ __forceinline__ uint32_t instr_desc(int m, int n) {
@@ -91,9 +44,6 @@ __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t a_desc, uint64_t 
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {      // r: 32 registers (indices known at compile time)
     asm volatile(
@@ -545,35 +495,9 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_pair_kernel(const __grid
     }
 }
 
-typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiled encode_tiled() {
-    static EncodeTiled fn = nullptr;
-    if (!fn) {
-        void* sym = nullptr;
-        cudaDriverEntryPointQueryResult result;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &result) == cudaSuccess &&
-            result == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiled>(sym);
-    }
-    return fn;
-}
-
 // A [rows, cols] row-major bfloat16 matrix, boxes of box_rows x 64 columns, 128-byte swizzle.
 int make_map(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld, int box_rows) {
-    EncodeTiled encode = encode_tiled();
-    if (!encode) return ts_fail("gemm_tcgen05: the driver does not export cuTensorMapEncodeTiled");
-    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
-    const cuuint32_t elem[2] = {1, 1};
-    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return ts_fail("gemm_tcgen05: cuTensorMapEncodeTiled failed with %d", (int)r);
-    return 0;
+    return make_tile_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, rows, cols, ld, box_rows, "gemm_tcgen05");
 }
 
 bool g_pairing = true;

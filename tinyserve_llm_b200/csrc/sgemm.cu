@@ -1,5 +1,6 @@
-// float32 matrix product C[M, N] = A[M, K] . B[N, K]^T with FFMA and float32 accumulation: the
-// engine's true 32-bit projection (no tensor-core mode that rounds its inputs).  Each output element
+// float32 matrix product C[M, N] = A[M, K] . B[N, K]^T: the engine's true 32-bit projection (no tensor-core mode that
+// rounds its inputs).  A single product whose rows TMA takes runs in sgemm_tcgen05.cu, to the same accuracy; this file's
+// kernel, FFMA with float32 accumulation, takes the others and batches of products.  Each output element
 // sums over k in ascending order, so a row's result does not depend on what else is in the batch.
 // Any M, N, K; rows of A and B are K-contiguous (the checkpoint's [out_features, in_features]).
 // A batched form runs one such product per blockIdx.z.
@@ -61,11 +62,27 @@ sgemm_nt_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
     }
 }
 
+bool sgemm_tcgen05_supported(const float* x, const float* w, int K, long long ldx, long long ldw);
+long long sgemm_tcgen05_scratch_floats(int M, int N, int K);
+int sgemm_tcgen05(const float* x, const float* w, float* y, int M, int N, int K, long long ldx, long long ldw, long long ldy,
+                  float* scratch, int* error, cudaStream_t stream);
+
+// Floats of scratch `ts_sgemm_nt` may use (sgemm_tcgen05.cu).
+TS_API long long ts_sgemm_nt_scratch_floats(int M, int N, int K) {
+    return M > 0 && N > 0 && K > 0 ? sgemm_tcgen05_scratch_floats(M, N, K) : 0;
+}
+
+// On the tensor cores where TMA takes rows and addresses, whatever M is (a row's result must not depend on what else is in
+// the batch); else by multiply-adds.  `error`: an int the host can read, for waits that run out.
 TS_API int ts_sgemm_nt(const float* A, const float* B, float* C, int M, int N, int K, long long lda, long long ldb,
-                       long long ldc, cudaStream_t stream) {
+                       long long ldc, float* scratch, long long scratch_floats, int* error, cudaStream_t stream) {
     TS_REQUIRE(M >= 0 && N > 0 && K > 0, "sgemm: bad sizes M=%d N=%d K=%d", M, N, K);
     TS_REQUIRE(lda >= K && ldb >= K && ldc >= N, "sgemm: row strides smaller than the rows");
     if (M == 0) return 0;
+    if (error && sgemm_tcgen05_supported(A, B, K, lda, ldb)) {
+        TS_REQUIRE(scratch_floats >= sgemm_tcgen05_scratch_floats(M, N, K), "sgemm: %lld floats of scratch are too few", scratch_floats);
+        return sgemm_tcgen05(A, B, C, M, N, K, lda, ldb, ldc, scratch, error, stream);
+    }
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     TS_REQUIRE(grid.y <= 65535, "sgemm: M=%d needs more than 65535 row tiles", M);
     sgemm_nt_kernel<<<grid, 256, 0, stream>>>(A, B, C, M, N, K, lda, ldb, ldc, 0, 0, 0);

@@ -1,0 +1,383 @@
+// float32 matrix product y[M, N] = x[M, K] . W[N, K]^T on the fifth-generation tensor cores, to float32's own accuracy.
+//
+// Every operand enters as the sum of two TF32 numbers, v = hi + lo (hi is v to the nearest of 11 significant bits, lo the rest,
+// of which the tensor cores drop the last bit: 2^-23 of v), and W x = W_hi x_hi + W_hi x_lo + W_lo x_hi in tcgen05.mma kind::tf32
+// with float32 accumulators; the small terms go first.  The tensor cores cut what an accumulator cannot hold, so they add up 32
+// terms of k only: a block's sum leaves tensor memory and is added to the running sum in registers by an ordinary rounded
+// addition.  Measured against 64-bit products: 1.9e-7 (2,048 terms) and 1.8e-7 (8,192), where the multiply-add chain of sgemm.cu is
+// 8.0e-7 and 1.6e-6 off; 1.3e-7 against 1.5e-7 at 64 terms.  An element that comes out infinite or NaN (infinite inputs, for
+// which hi + lo does not stand, or an overflow) is worked out again by that chain, so such elements are what plain arithmetic gives.
+//
+// A row's result does not depend on what else is in the batch: the blocks of k, the segments k is cut into and the order
+// they are added up in follow from N and K alone, and the rows' tile (the MMA's N side) does not enter an element's sum.
+//
+// One CTA: 128 rows of W (the MMA's 128 lanes) against BX rows of x.  Warp 0 issues TMA loads into a ring of raw tiles, warp 1 the
+// MMAs, warps 2..9 split (two teams, a block each): a thread puts its row of W into tensor memory as hi and lo (the MMA's A
+// operand, so that neither passes through shared memory again) and its share of x into two swizzled tiles; the warps from 10
+// on add the blocks' sums up.
+// mbarriers: `raw_full` / `raw_empty` TMA <-> split, `ready` / `free` split <-> MMA, `sum_full` / `sum_empty` MMA <-> adders.
+// K is cut into segments, enough of them that the tiles of W times the segments fill the SMs.  Where there are rows of x enough
+// to fill them anyway a CTA takes the segments one after another and adds each one's sum to y; else each segment is a CTA's
+// work, its sums go to scratch, and a second kernel adds them up in the same order.
+// Measured on a B200, products with cold weights one after another, us, before (sgemm.cu) and now:
+//   rows of x             1          8         100        300      512
+//   16,384 x 2,048      192 / 53   192 / 53   306 / 68
+//   2,048 x 8,192                  677 / 29   636 / 40      - / 100
+//   3,072 x 2,048                                                 241 / 70
+// What bounds it: a block of k costs 0.75 to 0.93 us whatever BX is.  An MMA of 8 numbers of k takes some 107 cycles with up to 64
+// rows of x and 137 with 128 (67 by the tensor cores' rate); with one of the twelve MMAs issued (timing only) the first column
+// is 34 us, and loads alone stream W at 4.4 TB/s.
+//
+// Every wait on an mbarrier gives up after about two seconds and records where in an error word the host reads.
+#include "tcgen05.cuh"
+
+namespace {
+
+constexpr int BW = 128, BK = 32;                     // rows of W a tile; k a block: 128 bytes, one swizzled row
+constexpr int SPLIT_WARPS = 4, ADDERS_FROM = 2 + 2 * SPLIT_WARPS;    // two teams of split warps
+// Blocks of k the tensor cores add up before the sum goes to the registers.  2: 3 to 7 % faster, twice the error (3.8e-7 against
+// 1.9e-7 at 2,048 terms).
+constexpr int SUM_BLOCKS = 1;
+__host__ __device__ constexpr int share_of(int bx) { return bx >= 64 ? 4 : 2; }           // adder warps a quarter of the lanes
+__host__ __device__ constexpr int threads_of(int bx) { return 32 * (ADDERS_FROM + 4 * share_of(bx)); }
+constexpr int W_BYTES = BW * BK * 4;
+constexpr int SMS = 148;
+constexpr long long MAX_SCRATCH = 64ll << 20;        // floats: more than that and the segments are taken in turn
+constexpr int MIN_SEGMENT = 8;                       // blocks of k a segment has at least (256 terms)
+
+struct SgemmParams {
+    float* y;                                        // output, or the segments' sums [segments][M][N]
+    const float* x;
+    const float* w;
+    int M, N, K;
+    long long ldx, ldw, ldy, segment_stride;
+    int blocks, per_segment, in_turn;                // blocks of k in all, and a segment; 1: a CTA takes all segments in turn
+    int items;                                       // tiles, times segments unless in turn
+    int* error;
+};
+
+// A from tensor memory (its 128 lanes the rows, a column a number of K), B from shared memory
+__device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr), "f"(r[0]), "f"(r[1]), "f"(r[2]), "f"(r[3]), "f"(r[4]), "f"(r[5]), "f"(r[6]), "f"(r[7]), "f"(r[8]), "f"(r[9]),
+          "f"(r[10]), "f"(r[11]), "f"(r[12]), "f"(r[13]), "f"(r[14]), "f"(r[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr) : "memory");
+}
+
+// v to the nearest number of 11 significant bits.  The rest, v - hi, has at most 12, of which the tensor cores drop the last; past
+// the largest number hi is infinite and the rest NaN, and for a NaN the rest is one, so the sum never hides either.
+__device__ __forceinline__ float to_tf32(float v) { return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u); }
+
+struct Item { int n0, m0, segment, first, count; };    // a CTA's piece of work: a tile and the blocks of k it takes
+__device__ __forceinline__ Item item_of(const SgemmParams& p, int item, int bx) {
+    const int n_tiles = (p.N + BW - 1) / BW, m_tiles = (p.M + bx - 1) / bx;
+    Item it;
+    it.n0 = item % n_tiles * BW;
+    it.m0 = item / n_tiles % m_tiles * bx;
+    it.segment = item / n_tiles / m_tiles;
+    it.first = it.segment * p.per_segment;
+    it.count = p.in_turn ? p.blocks : min(p.per_segment, p.blocks - it.first);
+    return it;
+}
+
+// A persistent CTA an SM: the four kinds of warps walk over the same items, each counting blocks (g) over all of them, so that
+// the loads and MMAs of an item run under the sums of the one before.
+template <int BX, int RING, int PAIRS, int SUMS>
+__global__ void __launch_bounds__(threads_of(BX), 1)
+sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, SgemmParams p) {
+    constexpr int X_BYTES = BX * BK * 4, RAW_BYTES = W_BYTES + X_BYTES;               // ring of [W | x]; PAIRS of [x hi | x lo]
+    constexpr int A_COLS = SUMS * BX, TMEM_USED = A_COLS + PAIRS * 2 * BK;            // PAIRS of [W hi | W lo]
+    constexpr int TMEM_COLS = TMEM_USED <= 256 ? 256 : 512;
+    static_assert(TMEM_USED <= 512, "tensor memory has 512 columns");
+    // a slot's barrier is waited on by one team only: the other could come to it a round early, where the parity it waits
+    // for stands for the round before the first
+    static_assert(RING % 2 == 0 && PAIRS % 2 == 0, "a ring slot and a pair of operand tiles belong to one team");
+    constexpr int OWN = BX / share_of(BX);           // columns of an adder
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t raw_full_bar[RING], raw_empty_bar[RING], ready_bar[PAIRS], free_bar[PAIRS], sum_full_bar[SUMS], sum_empty_bar[SUMS];
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ int failed;
+    unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    unsigned char* split = ring + RING * RAW_BYTES;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < RING; ++s) {
+            mbar_init(&raw_full_bar[s], 1);
+            mbar_init(&raw_empty_bar[s], SPLIT_WARPS);
+        }
+        for (int b = 0; b < PAIRS; ++b) {
+            mbar_init(&ready_bar[b], SPLIT_WARPS);
+            mbar_init(&free_bar[b], 1);
+        }
+        for (int b = 0; b < SUMS; ++b) {
+            mbar_init(&sum_full_bar[b], 1);
+            mbar_init(&sum_empty_bar[b], 4 * share_of(BX));
+        }
+        failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)),
+                     "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = tmem_base_slot;
+    chain_wait();
+    chain_release();
+
+    if (warp == 0 && lane == 0) {
+        int g = 0;
+        for (int at = blockIdx.x; at < p.items && !failed; at += gridDim.x) {
+            const Item it = item_of(p, at, BX);
+            for (int i = 0; i < it.count; ++i, ++g) {
+                const int s = g % RING;
+                if (!mbar_wait(&raw_empty_bar[s], ((g / RING) & 1) ^ 1, p.error, 21)) { failed = 1; break; }
+                mbar_expect_tx(&raw_full_bar[s], RAW_BYTES);
+                tma_load_2d(ring + s * RAW_BYTES, &map_w, &raw_full_bar[s], (it.first + i) * BK, it.n0);
+                tma_load_2d(ring + s * RAW_BYTES + W_BYTES, &map_x, &raw_full_bar[s], (it.first + i) * BK, it.m0);
+            }
+        }
+    } else if (warp == 1 && lane == 0) {
+        // float32 accumulator, TF32 operands, B K-major, 128 x BX
+        const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(BX >> 3) << 17) | ((uint32_t)(BW >> 4) << 24);
+        int g = 0, sums = 0;
+        for (int at = blockIdx.x; at < p.items && !failed; at += gridDim.x) {
+            const Item it = item_of(p, at, BX);
+            for (int i = 0, j = 0; i < it.count; ++i, ++g) {                          // j: the block's place in its segment
+                const int a = g % PAIRS, b = sums % SUMS;
+                const bool more = j % SUM_BLOCKS != 0;                                // the sum is begun already
+                if (!more && !mbar_wait(&sum_empty_bar[b], ((sums / SUMS) & 1) ^ 1, p.error, 24)) { failed = 1; break; }
+                if (!mbar_wait(&ready_bar[a], (g / PAIRS) & 1, p.error, 23)) { failed = 1; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t w_hi = tmem_base + A_COLS + a * 2 * BK, w_lo = w_hi + BK, d = tmem_base + b * BX;
+                const uint64_t x_hi = smem_desc(split + a * 2 * X_BYTES), x_lo = smem_desc(split + a * 2 * X_BYTES + X_BYTES);
+#pragma unroll
+                for (int k = 0; k < BK / 8; ++k) umma_tf32(d, w_hi + 8 * k, x_lo + 2 * k, idesc, k != 0 || more);   // 8 numbers of K: 8 columns, 32 bytes
+#pragma unroll
+                for (int k = 0; k < BK / 8; ++k) umma_tf32(d, w_lo + 8 * k, x_hi + 2 * k, idesc, 1);
+#pragma unroll
+                for (int k = 0; k < BK / 8; ++k) umma_tf32(d, w_hi + 8 * k, x_hi + 2 * k, idesc, 1);
+                umma_commit(&free_bar[a]);
+                j = j + 1 == p.per_segment ? 0 : j + 1;
+                if (j % SUM_BLOCKS == 0 || i + 1 == it.count) {
+                    umma_commit(&sum_full_bar[b]);
+                    ++sums;
+                }
+            }
+        }
+    } else if (warp >= 2 && warp < ADDERS_FROM) {
+        // blocks in turn between the teams: a block's split is a chain of waits, loads and stores, and two run side by side
+        const int team = (warp - 2) / SPLIT_WARPS, quarter = warp & 3, row = quarter * 32 + lane;   // a warp reaches the quarter of the lanes its number gives
+        const uint32_t lane_addr = tmem_base + A_COLS + ((uint32_t)(quarter * 32) << 16);
+        int total = 0;
+        for (int at = blockIdx.x; at < p.items; at += gridDim.x) total += item_of(p, at, BX).count;
+        for (int g = team; g < total; g += 2) {
+            const int s = g % RING, a = g % PAIRS;
+            if (!mbar_wait(&raw_full_bar[s], (g / RING) & 1, p.error, 22) || failed) { failed = 1; break; }
+            if (!mbar_wait(&free_bar[a], ((g / PAIRS) & 1) ^ 1, p.error, 26)) { failed = 1; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const unsigned char* w_row = ring + s * RAW_BYTES + row * 128;            // 16-byte piece c lies at c ^ (row % 8)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                float hi[16], lo[16];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const float4 v = *reinterpret_cast<const float4*>(w_row + (((4 * half + c) ^ (row & 7)) << 4));
+                    const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        hi[4 * c + j] = to_tf32(e[j]);
+                        lo[4 * c + j] = e[j] - hi[4 * c + j];
+                    }
+                }
+                tmem_st16(lane_addr + a * 2 * BK + 16 * half, hi);
+                tmem_st16(lane_addr + a * 2 * BK + BK + 16 * half, lo);
+            }
+            const float4* raw = reinterpret_cast<const float4*>(ring + s * RAW_BYTES + W_BYTES);
+            float4* x_hi = reinterpret_cast<float4*>(split + a * 2 * X_BYTES);
+            float4* x_lo = reinterpret_cast<float4*>(split + a * 2 * X_BYTES + X_BYTES);
+#pragma unroll 4
+            for (int e = quarter * 32 + lane; e < X_BYTES / 16; e += 32 * SPLIT_WARPS) {
+                const float4 v = raw[e];
+                const float4 h = make_float4(to_tf32(v.x), to_tf32(v.y), to_tf32(v.z), to_tf32(v.w));
+                x_lo[e] = make_float4(v.x - h.x, v.y - h.y, v.z - h.z, v.w - h.w);
+                x_hi[e] = h;
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");              // the MMAs read x through the async proxy
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&ready_bar[a]);
+                mbar_arrive(&raw_empty_bar[s]);
+            }
+        }
+    } else if (warp >= ADDERS_FROM) {
+        const int quarter = warp & 3, side = (warp - ADDERS_FROM) >> 2;
+        const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + side * OWN;
+        float sum[OWN];
+#pragma unroll
+        for (int j = 0; j < OWN; ++j) sum[j] = 0.f;
+        int sums = 0;
+        for (int at = blockIdx.x; at < p.items && !failed; at += gridDim.x) {
+            const Item it = item_of(p, at, BX);
+            const int n = it.n0 + quarter * 32 + lane, m_first = it.m0 + side * OWN;
+            for (int from = 0; from < it.count && !failed; from += p.per_segment) {   // a segment
+                const int blocks = min(p.per_segment, it.count - from);
+                for (int i = 0; i < blocks; i += SUM_BLOCKS, ++sums) {
+                    const int b = sums % SUMS;
+                    if (!mbar_wait(&sum_full_bar[b], (sums / SUMS) & 1, p.error, 25) || failed) { failed = 1; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    uint32_t v[OWN];
+#pragma unroll
+                    for (int j = 0; j < OWN; j += 8) tmem_ld8(lane_addr + b * BX + j, v + j);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");  // read: the accumulator goes back before the additions
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sum_empty_bar[b]);
+#pragma unroll
+                    for (int j = 0; j < OWN; ++j) sum[j] += __uint_as_float(v[j]);
+                }
+                if (failed) break;
+                float* y = p.y + it.segment * p.segment_stride + (long long)m_first * p.ldy + n;
+                const int k0 = (it.first + from) * BK, k1 = min(p.K, k0 + blocks * BK);
+#pragma unroll
+                for (int j = 0; j < OWN; ++j) {
+                    if (n < p.N && m_first + j < p.M) {
+                        float v = sum[j];
+                        if (!isfinite(v)) {          // hi + lo does not stand for infinite or the largest numbers
+                            v = 0.f;
+                            for (int k = k0; k < k1; ++k) v = fmaf(p.x[(m_first + j) * p.ldx + k], p.w[n * p.ldw + k], v);
+                        }
+                        y[j * p.ldy] = from ? y[j * p.ldy] + v : v;
+                    }
+                    sum[j] = 0.f;
+                }
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    }
+}
+
+// y[m, n] = the segments' sums in order; four neighbours a thread where rows allow
+template <int V>
+__global__ void __launch_bounds__(256) add_segments_kernel(const float* __restrict__ parts, float* __restrict__ y, int segments,
+                                                           long long segment_stride, int M, int N, long long ldy) {
+    chain_wait();
+    chain_release();
+    const long long e = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * V;
+    if (e >= (long long)M * N) return;
+    float sum[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) sum[j] = parts[e + j];
+#pragma unroll 4
+    for (int s = 1; s < segments; ++s) {
+        float next[V];
+        if (V == 4) *reinterpret_cast<float4*>(next) = *reinterpret_cast<const float4*>(parts + s * segment_stride + e);
+        else next[0] = parts[s * segment_stride + e];
+#pragma unroll
+        for (int j = 0; j < V; ++j) sum[j] += next[j];
+    }
+    float* out = y + e / N * ldy + e % N;
+    if (V == 4) *reinterpret_cast<float4*>(out) = *reinterpret_cast<float4*>(sum);
+    else out[0] = sum[0];
+}
+
+// How K is cut, from N and K alone: enough segments that the tiles of W fill the SMs once, none shorter than MIN_SEGMENT blocks.
+void cut(int N, int K, int* blocks, int* per_segment, int* segments) {
+    *blocks = (K + BK - 1) / BK;
+    const int tiles = (N + BW - 1) / BW;
+    int s = SMS / tiles;
+    if (s > *blocks / MIN_SEGMENT) s = *blocks / MIN_SEGMENT;
+    if (s < 1) s = 1;
+    *per_segment = (*blocks + s - 1) / s;
+    *segments = (*blocks + *per_segment - 1) / *per_segment;
+}
+
+template <int BX, int RING, int PAIRS, int SUMS>
+int launch(SgemmParams p, int segments, cudaStream_t stream) {
+    CUtensorMap map_w, map_x;
+    if (make_tile_map(&map_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.w, p.N, p.K, p.ldw, BW, "sgemm_tcgen05")) return 1;
+    if (make_tile_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.x, p.M, p.K, p.ldx, BX, "sgemm_tcgen05")) return 1;
+    constexpr size_t smem = (size_t)RING * (W_BYTES + BX * BK * 4) + PAIRS * 2 * BX * BK * 4 + 1024;
+    auto kernel = sgemm_tcgen05_kernel<BX, RING, PAIRS, SUMS>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    p.items = ((p.N + BW - 1) / BW) * ((p.M + BX - 1) / BX) * (p.in_turn ? 1 : segments);
+    TS_CHAINED_CHECK("sgemm_tcgen05", launch_chained(kernel, dim3(p.items < SMS ? p.items : SMS), dim3(threads_of(BX)), smem, stream,
+                                                     map_w, map_x, p));
+    return 0;
+}
+
+// Rows of x a CTA, and whether it takes the segments in turn.  Neither enters an element's sum.
+struct Shape { int bx, in_turn; };
+Shape choose(int M, int N, int blocks, int per_segment, int segments) {
+    static const struct { int bx; double ns; } kinds[4] = {{16, 750}, {32, 770}, {64, 820}, {128, 930}};   // of a block of k, as measured
+    Shape best{128, segments > 1};
+    double least = 1e30;
+    for (const auto& kind : kinds)
+        for (int in_turn = 0; in_turn < (segments > 1 ? 2 : 1); ++in_turn) {
+            if (segments > 1 && !in_turn && (long long)segments * M * N > MAX_SCRATCH) continue;
+            const long long items = (long long)((N + BW - 1) / BW) * ((M + kind.bx - 1) / kind.bx) * (in_turn ? 1 : segments);
+            double ns = (double)((items + SMS - 1) / SMS) * (500.0 + (in_turn ? blocks : per_segment) * kind.ns);
+            if (segments > 1 && !in_turn) ns += 2500.0 + (double)segments * M * N * 8.0 / 5000.0;     // the second kernel
+            if (ns < least) {
+                least = ns;
+                best = Shape{kind.bx, in_turn};
+            }
+        }
+    return best;
+}
+
+}  // namespace
+
+// 1 if TMA takes the sizes and addresses: 16-byte aligned bases and rows.
+bool sgemm_tcgen05_supported(const float* x, const float* w, int K, long long ldx, long long ldw) {
+    return K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0;
+}
+
+// Floats of scratch a product of these sizes needs (0: none).
+long long sgemm_tcgen05_scratch_floats(int M, int N, int K) {
+    int blocks, per, segments;
+    cut(N, K, &blocks, &per, &segments);
+    return segments > 1 && !choose(M, N, blocks, per, segments).in_turn ? (long long)segments * M * N : 0;
+}
+
+int sgemm_tcgen05(const float* x, const float* w, float* y, int M, int N, int K, long long ldx, long long ldw, long long ldy,
+                  float* scratch, int* error, cudaStream_t stream) {
+    int blocks, per, segments;
+    cut(N, K, &blocks, &per, &segments);
+    const Shape shape = choose(M, N, blocks, per, segments);
+    const bool parts = segments > 1 && !shape.in_turn;
+    SgemmParams p{parts ? scratch : y, x, w, M, N, K, ldx, ldw, parts ? N : ldy, parts ? (long long)M * N : 0, blocks, per,
+                  shape.in_turn, 0, error};
+    const int failed = shape.bx == 16 ? launch<16, 8, 4, 4>(p, segments, stream) : shape.bx == 32 ? launch<32, 8, 4, 4>(p, segments, stream)
+                     : shape.bx == 64 ? launch<64, 6, 4, 4>(p, segments, stream) : launch<128, 4, 2, 3>(p, segments, stream);
+    if (failed || !parts) return failed;
+    const bool vec = N % 4 == 0 && ldy % 4 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)scratch % 16 == 0;
+    const long long items = (long long)M * N / (vec ? 4 : 1);
+    auto kernel = vec ? add_segments_kernel<4> : add_segments_kernel<1>;
+    TS_CHAINED_CHECK("sgemm_tcgen05 (segments)",
+                     launch_chained(kernel, dim3((unsigned)((items + 255) / 256)), dim3(256), 0, stream, (const float*)scratch, y,
+                                    segments, (long long)M * N, M, N, ldy));
+    return 0;
+}

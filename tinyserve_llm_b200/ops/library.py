@@ -51,7 +51,8 @@ _SIGNATURES = {
     "ts_rope_store": ("int", "ppppiipipplliiiiiiiip"),
     "ts_sample_scratch_words": ("int", "ii"),
     "ts_sample": ("int", "plpppiipip"),
-    "ts_sgemm_nt": ("int", "pppiiilllp"),
+    "ts_sgemm_nt": ("int", "pppiiilllplpp"),
+    "ts_sgemm_nt_scratch_floats": ("long long", "iii"),
     "ts_skinny_linear_max_rows": ("int", ""),
     "ts_skinny_linear": ("int", "pppiiilliip"),
     "ts_skinny_qkv_rope_store": ("int", "pppiilpppiipipplliiiiiip"),
@@ -115,6 +116,12 @@ _WAIT_CODES: dict[int, tuple[str, str]] = {
     15: ("attention_tcgen05", "softmax waiting for scores"),
     16: ("attention_tcgen05", "epilogue waiting for the last product"),
     17: ("attention_tcgen05", "softmax waiting for the previous product before rescaling"),
+    21: ("sgemm_tcgen05", "TMA producer waiting for a free ring slot"),
+    22: ("sgemm_tcgen05", "split warps waiting for operands"),
+    23: ("sgemm_tcgen05", "MMA issuer waiting for split operands"),
+    24: ("sgemm_tcgen05", "MMA issuer waiting for a drained accumulator"),
+    25: ("sgemm_tcgen05", "adders waiting for a block's sums"),
+    26: ("sgemm_tcgen05", "split warps waiting for free operand tiles"),
 }
 
 
@@ -1488,7 +1495,7 @@ class Ops:
     def linear(self, x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None = None,
                out: torch.Tensor | None = None) -> torch.Tensor:
         """
-        x [M, K] . weight[N, K]^T.  float32: the engine's FFMA kernel.  bfloat16: up to 32 rows of x on
+        x [M, K] . weight[N, K]^T.  float32: the engine's own kernels, on split TF32 operands or FFMA.  bfloat16: up to 32 rows of x on
         the engine's weight-streaming kernel, more on the library product (cuBLAS through torch.mm).
         `out` (contiguous [M, N] of the output dtype) receives the product instead of a new tensor.
         """
@@ -1506,9 +1513,11 @@ class Ops:
             if tuple(out.shape) != (x.shape[0], weight.shape[0]):
                 raise KernelError(f"linear: out is {tuple(out.shape)}, the product {(x.shape[0], weight.shape[0])}")
         if x.dtype == torch.float32:
-            self._call("ts_sgemm_nt", _ptr(x), _ptr(weight), _ptr(out), x.shape[0], weight.shape[0],
-                       x.shape[1], x.shape[1], weight.shape[1],
-                       weight.shape[0], _stream())
+            (M, K), N = x.shape, weight.shape[0]
+            floats = int(self.lib.ts_sgemm_nt_scratch_floats(M, N, K))
+            scratch = torch.empty((floats,), dtype=torch.float32, device=x.device) if floats else None
+            self._call("ts_sgemm_nt", _ptr(x), _ptr(weight), _ptr(out), M, N, K, K, K, N, _ptr(scratch), floats,
+                       self.error_word().data_ptr(), _stream())
             return out
         if self._skinny(x, weight):
             self._call("ts_skinny_linear", _ptr(weight), _ptr(x), _ptr(out), x.shape[0], weight.shape[0],

@@ -2,9 +2,9 @@
 Bias-free projection y = x . W^T with W stored [out_features, in_features] (the checkpoint layout).
 
 bfloat16: the library matrix product (cuBLAS through torch.mm), as the reference does through
-nn.Linear (model/llama.py:200-201, :220-221).  float32: the engine's own FFMA kernel, so that no
-reduced-precision matrix mode can slip in and the reduction order of a row does not depend on what
-else is in the batch.
+nn.Linear (model/llama.py:200-201, :220-221).  float32: the engine's own kernels (every operand as two TF32 numbers on the tensor
+cores, or FFMA), so that no reduced-precision matrix mode can slip in and the reduction order of a
+row does not depend on what else is in the batch.
 """
 
 from __future__ import annotations
