@@ -294,6 +294,36 @@ def test_paged_attention(ops, dtype, generic, nh, nkv, hd, page, window):
     torch.testing.assert_close(got, plain.rnd(want, act_of(dtype)), **tol(dtype, 2))
 
 
+@pytest.mark.parametrize("nh, nkv, hd, page, window", [(8, 2, 64, 64, 0), (6, 2, 32, 16, 0), (5, 1, 48, 32, 0), (12, 4, 128, 256, 0),
+                                                       (3, 1, 80, 8, 0), (32, 2, 64, 64, 0), (4, 4, 16, 4, 30), (6, 3, 128, 64, 100)])
+def test_float32_attention_tiles_do_not_depend_on_the_cut(ops, nh, nkv, hd, page, window):
+    """A request of 203 tokens whole, in portions and with its last tokens alone: the same bits; a later key's NaN reaches no earlier row."""
+    n, width = 203, (nh + 2 * nkv) * hd
+    pages = -(-n // page)
+    binding = make_binding(2 * pages, 1, nkv, page, hd, torch.float32, [list(range(pages))[::-1], list(range(pages, 2 * pages))])
+    keys, values = rand((n, nkv, hd), torch.float32, 20), rand((n, nkv, hd), torch.float32, 30)
+    for s in range(2):
+        fill_cache(binding, s, keys, values)
+    qkv = rand((n, width), torch.float32, 11, 2.0).to(DEV)
+    scale = hd ** -0.5
+
+    def run(lens, ends):
+        rows = torch.cat([qkv[c - q:c] for q, c in zip(lens, ends)])
+        return ops.paged_attention(rows, make_ctx(lens, ends), binding, nh, nkv, hd, scale, window)
+
+    whole = run([n, n], [n, n])
+    assert torch.equal(whole[:n], whole[n:])
+    want = plain_paged_attention(qkv.cpu()[:, :nh * hd].double().view(n, nh, hd), [keys], [values], [n], [n], scale, window)
+    torch.testing.assert_close(whole[:n].cpu().double().view(n, nh, hd), want, **tol(torch.float32, 2))
+    for lens, ends in (([70, 133], [70, n]), ([1, 64], [150, 64]), ([1, 1], [n, 128]), ([65, 1], [129, 64])):
+        got, at = run(lens, ends), 0
+        for q, c in zip(lens, ends):
+            assert torch.equal(got[at:at + q], whole[c - q:c]), (lens, ends)
+            at += q
+    binding.v_pool[binding.block_table[0, 150 // page], 0, :, 150 % page] = math.nan
+    assert torch.equal(run([n], [n])[:150], whole[:150])
+
+
 @pytest.mark.parametrize("hd, g", [(64, 4), (128, 3)])
 def test_tensor_core_attention_on_long_batches(ops, hd, g):
     """Decode over many splits (contexts up to 2,300 keys), prompts of several tiles, and a decode-only batch."""

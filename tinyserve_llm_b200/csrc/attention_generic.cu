@@ -250,15 +250,28 @@ TS_API int ts_paged_attention_split(const void* q, long long q_stride, void* out
                                      nullptr, 0, 0.f, 0, 0, 0, -INFINITY, stream);
 }
 
-// Queries, keys and values of one head size in the columns [q | k | v] of one projection's output.
+bool paged_attention_f32_supported(const void* q, long long q_stride, const void* out, const void* k_pool, const void* v_pool,
+                                   const KVGeometry& geo, int nh, int nkv, int hd);
+int paged_attention_f32(const float* q, long long q_stride, float* out, const float* k_pool, const float* v_pool, KVGeometry geo,
+                        const int* block_table, int table_width, const int* positions, const int* cu_q, int num_seqs,
+                        int num_tokens, int max_q_len, int nh, int nkv, int hd, float scale, int window, cudaStream_t stream);
+
+// Queries, keys and values of one head size in the columns [q | k | v] of one projection's output.  With `cu_q` (the requests'
+// first tokens, [num_seqs + 1]) float32 goes to attention_f32.cu where it takes the sizes; `max_q_len`: the longest portion.
 TS_API int ts_paged_attention_generic(const void* qkv, void* out, const void* k_pool, const void* v_pool,
                                       long long page_stride, long long entry_offset, int page_tokens, int num_pages,
                                       const int* block_table, int table_width, const int* positions,
-                                      const int* seq_of_token, int num_tokens, int nh, int nkv, int hd, float scale,
-                                      int window, int dtype, cudaStream_t stream) {
+                                      const int* seq_of_token, const int* cu_q, int num_seqs, int max_q_len, int num_tokens, int nh,
+                                      int nkv, int hd, float scale, int window, int dtype, cudaStream_t stream) {
     TS_REQUIRE(hd > 0 && hd % 16 == 0 && hd <= 256,
                "paged_attention: head_dim %d is not supported (multiples of 16 up to 256)", hd);
-    return ts_paged_attention_split(qkv, (long long)(nh + 2 * nkv) * hd, out, k_pool, v_pool, page_stride, entry_offset,
+    const long long q_stride = (long long)(nh + 2 * nkv) * hd;
+    const KVGeometry geo{page_stride, entry_offset, page_tokens, num_pages};
+    if (cu_q && num_seqs > 0 && dtype == TS_F32 && num_tokens > 0 && nkv > 0 && nh > 0 && nh % nkv == 0 && page_tokens > 0 && table_width > 0 && window >= 0 &&
+        paged_attention_f32_supported(qkv, q_stride, out, k_pool, v_pool, geo, nh, nkv, hd))
+        return paged_attention_f32((const float*)qkv, q_stride, (float*)out, (const float*)k_pool, (const float*)v_pool, geo, block_table,
+                                   table_width, positions, cu_q, num_seqs, num_tokens, max_q_len, nh, nkv, hd, scale, window, stream);
+    return ts_paged_attention_split(qkv, q_stride, out, k_pool, v_pool, page_stride, entry_offset,
                                     page_stride, entry_offset, page_tokens, num_pages, block_table, table_width,
                                     positions, seq_of_token, num_tokens, nh, nkv, hd, hd, scale, window, dtype, stream);
 }

@@ -29,7 +29,7 @@ _SIGNATURES = {
     "ts_attention_bf16_scratch_floats": ("long long", "iiii"),
     "ts_attention_bf16_supported": ("int", "iiii"),
     "ts_paged_attention_bf16": ("int", "pppplliipippiiiiiiifiplpip"),
-    "ts_paged_attention_generic": ("int", "pppplliipippiiiifiip"),
+    "ts_paged_attention_generic": ("int", "pppplliipipp" "pii" "iiiifiip"),
     "ts_paged_attention_bf16_sigmoid": ("int", "pl" "ppp" "lliipippiiiiiiifiplpi" "pppl" "p"),
     "ts_paged_attention_bf16_masked": ("int", "pl" "ppp" "lllliipippiiiiiiifiifi" "plpi" "fp"),
     "ts_attention_tcgen05_supported": ("int", "iiiii"),
@@ -413,8 +413,8 @@ class Ops:
                         window: int, generic: bool = False) -> torch.Tensor:
         """
         [T, nh * hd].  bfloat16 with head size 64 or 128 and pages of a multiple of 64 tokens runs on
-        the tensor-core kernels (prefill tiles and split-key decode); everything else, and
-        `generic=True`, on the generic kernel.
+        the tensor-core kernels (prefill tiles and split-key decode), float32 on tiles of multiply-adds where the
+        step's context says which tokens are whose; everything else, and `generic=True`, on the generic kernel.
         """
         self._check(qkv, "qkv", tuple(_DTYPE_CODE), 2)
         out = torch.empty((qkv.shape[0], nh * hd), dtype=qkv.dtype, device=qkv.device)
@@ -458,10 +458,12 @@ class Ops:
             if ctx.min_q_len <= 1:
                 self.launches += 1 if max_q_len <= 1 else 2          # decode + combine (+ prefill) in one call
             return out
+        cu_q = None if generic else getattr(ctx, "cu_q", None)
         self._call("ts_paged_attention_generic", _ptr(qkv), _ptr(out), _ptr(binding.k_pool), _ptr(binding.v_pool),
                    binding.page_stride, binding.entry_offset, binding.page_tokens,
                    binding.num_pages, _ptr(binding.block_table), binding.table_width,
-                   _ptr(ctx.positions), _ptr(ctx.seq_of_token), qkv.shape[0], nh, nkv, hd,
+                   _ptr(ctx.positions), _ptr(ctx.seq_of_token), _ptr(cu_q),
+                   cu_q.shape[0] - 1 if cu_q is not None else 0, int(getattr(ctx, "max_q_len", 2)), qkv.shape[0], nh, nkv, hd,
                    scale, window, _DTYPE_CODE[qkv.dtype], _stream())
         return out
 
