@@ -356,12 +356,13 @@ TS_API int ts_recurrence_scan(const float* qk, int qk_group, const float* decay,
     return ts_fail("recurrence_scan: unknown dtype code %d", v_dtype);
 }
 
+// `singles` 1: only requests that feed one token are walked (prompt portions: recurrence_tiles.cu).
 TS_API int ts_linear_recurrence(const void* q, const void* k, const void* v, long long q_stride, long long k_stride,
                                 long long v_stride, const float* z, long long z_stride, const float* bias,
                                 const float* head_decay, float inv_tau, float q_scale, float k_scale, const float* freq,
                                 int rot_dims, const int* positions, const int* cu_q, const int* slots, int num_seqs,
                                 float* state, long long slot_stride, float* out, int heads, int dim, int vdim,
-                                int num_tokens, float* prepared, int dtype, cudaStream_t stream) {
+                                int num_tokens, float* prepared, int singles, int dtype, cudaStream_t stream) {
     TS_REQUIRE(heads > 0 && dim > 0 && vdim > 0 && num_seqs >= 0 && num_tokens >= 0, "linear_recurrence: bad sizes");
     TS_REQUIRE(dim <= 16 * LR_ROWGROUPS, "linear_recurrence: %d key channels a head are not supported (up to %d)", dim,
                16 * LR_ROWGROUPS);
@@ -386,7 +387,7 @@ TS_API int ts_linear_recurrence(const void* q, const void* k, const void* v, lon
         return ts_fail("linear_recurrence: unknown dtype code %d", dtype);
     TS_LAUNCH_CHECK("linear_recurrence (prepare)");
     RecurrenceArgs p{prepared, total, 1, prepared + 2 * total, v, v_stride, vdim, nullptr, cu_q, slots, state, slot_stride, out,
-                     heads, dim, vdim, 0};
+                     heads, dim, vdim, singles};
     if (dtype == TS_F32) return launch_recurrence<float>(p, LR_PLAIN, num_seqs, stream);
     return launch_recurrence<__nv_bfloat16>(p, LR_PLAIN, num_seqs, stream);
 }

@@ -14,10 +14,18 @@
 //   o_t = sum_i r_(t,i) d_(t-1,i) S_0[i] + sum_{j<t} P[t][j] v_j + bonus_t v_t,
 //   P[t][j] = sum_i r_(t,i) k_(j,i) a_(j+1,i) ... a_(t-1,i),   S_B = d_B S_0 + sum_j (k_j a_(j+1) ... a_B) v_j^T
 //
+// Plain recurrence (gated linear attention, retention): the same with the token's own write in its read-out,
+//   o_t = sum_i q_(t,i) d_(t,i) S_0[i] + sum_{j<=t} P[t][j] v_j,   P[t][j] = sum_i q_(t,i) k_(j,i) a_(j+1,i) ... a_(t,i)
+//
+// Delta rule with decays per channel: with G[t][j]_i = a_(j+1,i) ... a_(t,i),
+//   u_t = b_t (v_t - (d_t k_t)^T S_0 - sum_{j<t} (sum_i k_(t,i) k_(j,i) G[t][j]_i) u_j),
+//   o_t = (d_t q_t)^T S_0 + sum_{j<=t} (sum_i q_(t,i) k_(j,i) G[t][j]_i) u_j,   S_B = d_B S_0 + sum_j (G[B][j] k_j) u_j^T,
+// the system of the first line solved as above; its k side has two sets of rows, those that read S_0 and those that update it.
+//
 // No decay is ever divided by another: products of decays are taken as they are needed.
 //
 // A first kernel works out, per tile and q/k head (time mixing: head), what all columns of the state share: the
-// "pack" (16 rows for the q side, 16 for the k side, one with the channels' decays over the tile) and the coefficients
+// "pack" (16 rows for the q side, 16 or 32 for the k side, one with the channels' decays over the tile) and the coefficients
 // (W = M diag(b); P W, so that O = diag(c) S_0^T Q + (P W) (V - diag(c) R) does not wait for U; c; G[B]).  The second
 // kernel walks the tiles: a CTA owns one request, one head and 16 columns of the state and does three small
 // products a tile on tensor cores,
@@ -43,10 +51,12 @@ constexpr int WARPS = 4, THREADS = WARPS * 32;   // of the scan
 constexpr int CP = 20;             // pitch of a coefficient matrix: a warp's fragment loads fall into different banks
 constexpr int COEF = 2 * B * CP + 2 * B;   // W [16][20], P W (time mixing: P) [16][20], c [16], g [16]
 constexpr int RP = 24;             // pitch of the partial sums and of U: likewise
-// A pack: 33 rows (16 q-side, 16 k-side, the channels' decays) of `rows` floats and a pad that does the same for it.
+// A pack: 16 rows of the q side, `sets` times 16 of the k side, one with the channels' decays, each of `rows` floats and a pad
+// that does the same for it.
 __host__ __device__ constexpr int pack_pitch(int rows) { return rows + 8; }
-__host__ __device__ constexpr int pack_floats(int rows) { return (2 * B + 1) * pack_pitch(rows); }
-enum { DELTA = 0, MIX = 1 };
+__host__ __device__ constexpr int pack_floats(int rows, int sets) { return ((1 + sets) * B + 1) * pack_pitch(rows); }
+enum { DELTA = 0, MIX = 1, CHANNEL = 2 };           // delta rule, a decay a head; time mixing and plain; delta rule, a decay a channel
+__host__ __device__ constexpr int sets_of(int mode) { return mode == CHANNEL ? 2 : 1; }
 
 __device__ __forceinline__ float softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
 
@@ -96,7 +106,7 @@ __global__ void __launch_bounds__(128) delta_tile_prepare_kernel(PrepareArgs p) 
     }
     __syncthreads();
     const long long slot = tile_slot(seq, begin, tile);
-    float* pack = p.pack + (slot * p.kv_heads + g) * pack_floats(p.rows);
+    float* pack = p.pack + (slot * p.kv_heads + g) * pack_floats(p.rows, 1);
     for (int e = threadIdx.x; e < B * p.rows; e += 128) {
         const int t = e / p.rows, i = e % p.rows;
         pack[t * pack_pitch(p.rows) + i] = qs[t * pitch + i];
@@ -171,7 +181,7 @@ __global__ void __launch_bounds__(128) mix_tile_prepare_kernel(PrepareArgs p) {
     float* ks = rs + B * pitch;
     float* as = ks + B * pitch;
     const long long slot = tile_slot(seq, begin, tile);
-    float* pack = p.pack + (slot * p.heads + h) * pack_floats(p.rows);
+    float* pack = p.pack + (slot * p.heads + h) * pack_floats(p.rows, 1);
     const long long width = (long long)p.heads * p.dim, hc = (long long)h * p.dim;
     for (int e = threadIdx.x; e < B * p.rows; e += 128) {
         const int t = e / p.rows, i = e % p.rows;
@@ -229,6 +239,223 @@ __global__ void __launch_bounds__(128) mix_tile_prepare_kernel(PrepareArgs p) {
     }
 }
 
+struct PlainArgs {
+    const void* q; const void* k; long long q_stride, k_stride;
+    const float* z; long long z_stride; const float* bias;   // decay logits a channel (a = sigmoid(z + bias)^inv_tau), or
+    const float* head_decay;                                 // one decay a head
+    float inv_tau, q_scale, k_scale;
+    const float* freq; int rot_dims; const int* positions;   // rotation by halves over the first rot_dims channels
+    const int* cu_q; const int* prefill_seqs;
+    float* pack; float* coef;
+    int heads, dim, rows;
+};
+
+// The plain recurrence's pack and P.  grid (tiles, heads, portions), 128 threads.  Bound by its own arithmetic (a decay and,
+// with rotation, a sine and a cosine an element, then the running products); it takes the place of a kernel that wrote q, k and the
+// decays of every token to memory.
+template <typename T>
+__global__ void __launch_bounds__(128) plain_tile_prepare_kernel(PlainArgs p) {
+    extern __shared__ float smem[];
+    const int seq = p.prefill_seqs[blockIdx.z], tile = blockIdx.x, h = blockIdx.y;
+    if (seq < 0) return;
+    const int begin = p.cu_q[seq], n = p.cu_q[seq + 1] - begin;
+    if (n <= 1 || tile * B >= n) return;
+    const int t0 = begin + tile * B, m = min(B, n - tile * B);
+    const int pitch = p.rows + 1;
+    float* qs = smem;                                    // [16][pitch]
+    float* ks = qs + B * pitch;
+    float* as = ks + B * pitch;
+    const int half = p.rot_dims / 2;
+    for (int e = threadIdx.x; e < B * p.rows; e += 128) {
+        const int t = e / p.rows, i = e % p.rows;
+        float qv = 0.f, kv = 0.f, av = 1.f;              // a token past the portion's end changes nothing
+        if (t < m && i < p.dim) {
+            const T* qr = (const T*)p.q + (long long)(t0 + t) * p.q_stride + (long long)h * p.dim;
+            const T* kr = (const T*)p.k + (long long)(t0 + t) * p.k_stride + (long long)h * p.dim;
+            qv = to_float<T>(qr[i]);
+            kv = to_float<T>(kr[i]);
+            if (i < p.rot_dims) {
+                const int f = i < half ? i : i - half, other = i < half ? i + half : i - half;
+                float sn, cs;
+                sincosf((float)p.positions[t0 + t] * p.freq[f], &sn, &cs);
+                const float qo = to_float<T>(qr[other]), ko = to_float<T>(kr[other]);
+                qv = i < half ? qv * cs - qo * sn : qv * cs + qo * sn;
+                kv = i < half ? kv * cs - ko * sn : kv * cs + ko * sn;
+            }
+            qv *= p.q_scale;
+            kv *= p.k_scale;
+            if (p.z) {
+                const float x = p.z[(long long)(t0 + t) * p.z_stride + (long long)h * p.dim + i] + (p.bias ? p.bias[h * p.dim + i] : 0.f);
+                av = expf((fminf(x, 0.f) - log1pf(expf(-fabsf(x)))) * p.inv_tau);
+            } else {
+                av = p.head_decay[h];
+            }
+        }
+        qs[t * pitch + i] = qv;
+        ks[t * pitch + i] = kv;
+        as[t * pitch + i] = av;
+    }
+    __syncthreads();
+    const long long slot = tile_slot(seq, begin, tile);
+    {   // P[t][j], t >= j: thread j = tid / 8 walks t with the running product of its channels
+        const int j = threadIdx.x >> 3, part = threadIdx.x & 7;
+        float sum[B];
+#pragma unroll
+        for (int t = 0; t < B; ++t) sum[t] = 0.f;
+        for (int i = part; i < p.dim; i += 8) {
+            float run = ks[j * pitch + i];
+#pragma unroll
+            for (int t = 0; t < B; ++t) {
+                if (t > j) run *= as[t * pitch + i];
+                if (t >= j) sum[t] = fmaf(qs[t * pitch + i], run, sum[t]);
+            }
+        }
+        float* out = p.coef + (slot * p.heads + h) * COEF + B * CP;
+#pragma unroll
+        for (int t = 0; t < B; ++t) {
+            float s = sum[t];
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (part == 0) out[t * CP + j] = s;                                         // 0 where t < j
+        }
+    }
+    float* pack = p.pack + (slot * p.heads + h) * pack_floats(p.rows, 1);
+    for (int i = threadIdx.x; i < p.rows; i += 128) {    // a thread a channel: products from the left and from the right
+        const int pp = pack_pitch(p.rows);
+        float left = 1.f, right = 1.f;
+        for (int t = 0; t < B; ++t) {
+            left *= as[t * pitch + i];
+            pack[t * pp + i] = qs[t * pitch + i] * left;
+        }
+        for (int t = B - 1; t >= 0; --t) {
+            pack[(B + t) * pp + i] = ks[t * pitch + i] * right;
+            right *= as[t * pitch + i];
+        }
+        pack[2 * B * pp + i] = left;
+    }
+}
+
+struct ChannelArgs {
+    const float* q; const float* k; long long qk_stride;     // after the convolution
+    const float* z;                                          // [tokens, heads * dim] decay logits
+    const void* b; long long b_stride;                       // [tokens, heads] step sizes' logits
+    const float* bias; const float* rate;                    // dt_bias [heads * dim], A_log [heads]
+    const int* cu_q; const int* prefill_seqs;
+    float* pack; float* coef;
+    int heads, kv_heads, dim, rows;
+    float unit_eps, q_scale;
+};
+
+// The pack and the coefficients of the delta rule with decays per channel.  grid (tiles, value heads, portions), 128 threads.
+template <typename T>
+__global__ void __launch_bounds__(128) channel_tile_prepare_kernel(ChannelArgs p) {
+    extern __shared__ float smem[];
+    const int seq = p.prefill_seqs[blockIdx.z], tile = blockIdx.x, h = blockIdx.y, g = h / (p.heads / p.kv_heads);
+    if (seq < 0) return;
+    const int begin = p.cu_q[seq], n = p.cu_q[seq + 1] - begin;
+    if (n <= 1 || tile * B >= n) return;
+    const int t0 = begin + tile * B, m = min(B, n - tile * B);
+    const int pitch = p.rows + 1;
+    float* qs = smem;                                    // [16][pitch]
+    float* ks = qs + B * pitch;
+    float* as = ks + B * pitch;
+    float* kk = as + B * pitch;                          // [16][17]: sum_i k_t k_j G[t][j]
+    float* qk = kk + B * (B + 1);                        // sum_i q_t k_j G[t][j]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float rate = expf(p.rate[h]);
+    for (int t = warp; t < B; t += 4) {
+        const float* qr = p.q + (long long)(t0 + t) * p.qk_stride + (long long)g * p.dim;
+        const float* kr = p.k + (long long)(t0 + t) * p.qk_stride + (long long)g * p.dim;
+        const float* zr = p.z + ((long long)(t0 + t) * p.heads + h) * p.dim;
+        float sq = 0.f, sk = 0.f;
+        for (int i = lane; i < p.rows; i += 32) {
+            const bool ok = t < m && i < p.dim;          // a token past the portion's end changes nothing
+            const float qv = ok ? qr[i] : 0.f, kv = ok ? kr[i] : 0.f;
+            qs[t * pitch + i] = qv;
+            ks[t * pitch + i] = kv;
+            as[t * pitch + i] = ok ? expf(-rate * softplus(zr[i] + p.bias[h * p.dim + i])) : 1.f;
+            sq += qv * qv;
+            sk += kv * kv;
+        }
+        const float iq = p.q_scale / sqrtf(warp_sum(sq) + p.unit_eps), ik = 1.f / sqrtf(warp_sum(sk) + p.unit_eps);
+        for (int i = lane; i < p.rows; i += 32) { qs[t * pitch + i] *= iq; ks[t * pitch + i] *= ik; }   // the lane's own elements
+    }
+    __syncthreads();
+    {   // t >= j: thread j = tid / 8 walks t with the running product of its channels
+        const int j = threadIdx.x >> 3, part = threadIdx.x & 7;
+        float sum_k[B], sum_q[B];
+#pragma unroll
+        for (int t = 0; t < B; ++t) sum_k[t] = sum_q[t] = 0.f;
+        for (int i = part; i < p.dim; i += 8) {
+            float run = ks[j * pitch + i];
+#pragma unroll
+            for (int t = 0; t < B; ++t) {
+                if (t > j) run *= as[t * pitch + i];
+                if (t >= j) {
+                    sum_k[t] = fmaf(ks[t * pitch + i], run, sum_k[t]);
+                    sum_q[t] = fmaf(qs[t * pitch + i], run, sum_q[t]);
+                }
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < B; ++t) {
+            float a = sum_k[t], b = sum_q[t];
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) {
+                a += __shfl_xor_sync(0xffffffffu, a, o);
+                b += __shfl_xor_sync(0xffffffffu, b, o);
+            }
+            if (part == 0) {
+                kk[t * (B + 1) + j] = a;
+                qk[t * (B + 1) + j] = b;
+            }
+        }
+    }
+    __syncthreads();
+    const long long slot = tile_slot(seq, begin, tile);
+    float* pack = p.pack + (slot * p.heads + h) * pack_floats(p.rows, 2);
+    for (int i = threadIdx.x; i < p.rows; i += 128) {    // a thread a channel: products from the left and from the right
+        const int pp = pack_pitch(p.rows);
+        float left = 1.f, right = 1.f;
+        for (int t = 0; t < B; ++t) {
+            left *= as[t * pitch + i];
+            pack[t * pp + i] = qs[t * pitch + i] * left;
+            pack[(B + t) * pp + i] = ks[t * pitch + i] * left;
+        }
+        for (int t = B - 1; t >= 0; --t) {
+            pack[(2 * B + t) * pp + i] = ks[t * pitch + i] * right;
+            right *= as[t * pitch + i];
+        }
+        pack[3 * B * pp + i] = left;
+    }
+    if (warp) return;
+    // lane j holds column j (lanes 16..31 mirror lanes 0..15 and store nothing)
+    const int j = lane & (B - 1);
+    const float b = j < m ? 1.f / (1.f + expf(-to_float<T>(((const T*)p.b)[(long long)(t0 + j) * p.b_stride + h]))) : 0.f;
+    float* out = p.coef + (slot * p.heads + h) * COEF;
+    float M[B];
+#pragma unroll
+    for (int t = 0; t < B; ++t) {
+        const float bt = __shfl_sync(0xffffffffu, b, t);
+        const float A = t > j ? bt * kk[t * (B + 1) + j] : 0.f;
+        float row = t == j ? 1.f : 0.f;                  // M[t][j] = delta - sum_s A[t][s] M[s][j]
+#pragma unroll
+        for (int s = 0; s < t; ++s) row = fmaf(-__shfl_sync(0xffffffffu, A, s), M[s], row);
+        M[t] = row;
+    }
+#pragma unroll
+    for (int t = 0; t < B; ++t) {
+        const float P = t >= j ? qk[t * (B + 1) + j] : 0.f;
+        float pw = 0.f;
+#pragma unroll
+        for (int s = 0; s <= t; ++s) pw = fmaf(__shfl_sync(0xffffffffu, P, s), M[s] * b, pw);
+        if (lane < B) {
+            out[t * CP + j] = M[t] * b;
+            out[B * CP + t * CP + j] = pw;
+        }
+    }
+}
+
 struct ScanArgs {
     const float* pack; const float* coef;
     const void* v; long long v_stride;                   // elements between tokens; a head's values start at h * vdim
@@ -277,8 +504,8 @@ template <typename T, int NT, int MODE>
 __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
     constexpr int WROWS = 8 * NT, ROWS = WARPS * WROWS;  // rows of a warp; rows of the state
     constexpr int PP = pack_pitch(ROWS);
-    constexpr int PACK = pack_floats(ROWS), STAGE = PACK + COEF;
-    constexpr int TQ = MODE == DELTA ? 2 * B : B;        // rows of the pack that meet S_0
+    constexpr int SETS = sets_of(MODE), PACK = pack_floats(ROWS, SETS), STAGE = PACK + COEF;
+    constexpr int TQ = MODE == MIX ? B : 2 * B;          // rows of the pack that meet S_0
     extern __shared__ __align__(16) float smem[];
     float* red = smem + 2 * STAGE;                       // [WARPS][TQ][RP]
     float* G_s = red + WARPS * TQ * RP;                  // [B][RP]: what the state's update takes, G[B] U or V
@@ -375,18 +602,18 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 x[k] = to_float<T>(vnow[k]);
-                if (MODE == DELTA) {
+                if (MODE != MIX) {
                     float sum = 0.f;
 #pragma unroll
                     for (int w = 0; w < WARPS; ++w) sum += red[(w * TQ + B + c + 4 * k) * RP + col];
-                    x[k] = fmaf(-coef[2 * B * CP + c + 4 * k], sum, x[k]);
+                    x[k] = MODE == DELTA ? fmaf(-coef[2 * B * CP + c + 4 * k], sum, x[k]) : x[k] - sum;
                 }
             }
             if (MODE == MIX && !makes_o) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) G_s[(c + 4 * k) * RP + col] = x[k];
             }
-            if (MODE == DELTA || makes_o) {
+            if (MODE != MIX || makes_o) {
                 const float* m = coef + (makes_o ? B * CP : 0);
                 float big[4] = {}, small[4] = {};
 #pragma unroll
@@ -399,7 +626,7 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
                     const int t = r + 8 * half;
                     float y0 = big[2 * half] + small[2 * half], y1 = big[2 * half + 1] + small[2 * half + 1];
                     if (!makes_o) {
-                        const float g = coef[2 * B * CP + B + t];
+                        const float g = MODE == DELTA ? coef[2 * B * CP + B + t] : 1.f;
                         *reinterpret_cast<float2*>(G_s + t * RP + 8 * nt_uo + 2 * c) = make_float2(g * y0, g * y1);
                     } else {
                         float q0 = 0.f, q1 = 0.f;
@@ -435,12 +662,12 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
                 float big[4] = {}, small[4] = {};
-                const float* k = pack + (B + c) * PP + warp * WROWS + 8 * nt + r;
+                const float* k = pack + (SETS * B + c) * PP + warp * WROWS + 8 * nt + r;
 #pragma unroll
                 for (int ks = 0; ks < 2; ++ks)
                     mma_split(big, small, a[ks], split_tf32(k[8 * ks * PP]), split_tf32(k[(8 * ks + 4) * PP]));
                 float2 d = make_float2(cB, cB);
-                if (MODE == MIX) d = *reinterpret_cast<const float2*>(pack + 2 * B * PP + warp * WROWS + 8 * nt + 2 * c);
+                if (MODE != DELTA) d = *reinterpret_cast<const float2*>(pack + (1 + SETS) * B * PP + warp * WROWS + 8 * nt + 2 * c);
                 S[nt][0] = fmaf(d.x, S[nt][0], big[0] + small[0]);
                 S[nt][1] = fmaf(d.y, S[nt][1], big[1] + small[1]);
                 S[nt][2] = fmaf(d.x, S[nt][2], big[2] + small[2]);
@@ -466,8 +693,8 @@ int launch_scan(const ScanArgs& p, int portions, cudaStream_t stream) {
     const dim3 grid((p.vdim + COLS - 1) / COLS, p.heads, portions);
 #define TS_TILES(NT)                                                                                                 \
     do {                                                                                                             \
-        constexpr int TQ = MODE == DELTA ? 2 * B : B;                                                                \
-        const size_t smem = sizeof(float) * (2 * (pack_floats(WARPS * 8 * NT) + COEF) + (WARPS * TQ + B) * RP);      \
+        constexpr int TQ = MODE == MIX ? B : 2 * B;                                                                  \
+        const size_t smem = sizeof(float) * (2 * (pack_floats(WARPS * 8 * NT, sets_of(MODE)) + COEF) + (WARPS * TQ + B) * RP); \
         auto kernel = recurrence_tiles_kernel<T, NT, MODE>;                                                          \
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                        \
         kernel<<<grid, THREADS, smem, stream>>>(p);                                                                  \
@@ -484,8 +711,9 @@ int launch_scan(const ScanArgs& p, int portions, cudaStream_t stream) {
 }  // namespace
 
 // Floats of the two buffers the tile kernels need: packs (`heads`: the q/k heads) and coefficients (`heads`: the value heads).
-TS_API long long ts_recurrence_tiles_pack_floats(int num_tokens, int num_seqs, int heads, int dim) {
-    return ((long long)num_tokens / B + num_seqs + 1) * heads * pack_floats(padded_rows(dim));
+// `sets`: k-side sets of rows (2: delta rule with decays per channel).
+TS_API long long ts_recurrence_tiles_pack_floats(int num_tokens, int num_seqs, int heads, int dim, int sets) {
+    return ((long long)num_tokens / B + num_seqs + 1) * heads * pack_floats(padded_rows(dim), sets);
 }
 TS_API long long ts_recurrence_tiles_coef_floats(int num_tokens, int num_seqs, int heads) {
     return ((long long)num_tokens / B + num_seqs + 1) * heads * COEF;
@@ -540,4 +768,67 @@ TS_API int ts_mix_tiles(const void* r, const void* k, long long rk_stride, const
         return launch_scan<__nv_bfloat16, MIX>(s, portions, stream);
     }
     return ts_fail("mix_tiles: unknown dtype code %d", dtype);
+}
+
+// The plain recurrence over a step's prompt portions: q, k, v as `ts_linear_recurrence` takes them.
+TS_API int ts_plain_tiles(const void* q, const void* k, const void* v, long long q_stride, long long k_stride, long long v_stride,
+                          const float* z, long long z_stride, const float* bias, const float* head_decay, float inv_tau,
+                          float q_scale, float k_scale, const float* freq, int rot_dims, const int* positions, const int* cu_q,
+                          const int* slots, const int* prefill_seqs, int portions, int max_q_len, float* state,
+                          long long slot_stride, float* pack, float* coef, float* out, int heads, int dim, int vdim, int dtype,
+                          cudaStream_t stream) {
+    TS_REQUIRE(heads > 0 && dim > 0 && dim <= 256 && vdim > 0, "plain_tiles: %d heads of %d channels", heads, dim);
+    TS_REQUIRE(rot_dims >= 0 && rot_dims <= dim && rot_dims % 2 == 0, "plain_tiles: rotation over %d of %d channels", rot_dims, dim);
+    TS_REQUIRE((z != nullptr) != (head_decay != nullptr), "plain_tiles: either decay logits or one decay per head");
+    TS_REQUIRE(slot_stride >= (long long)heads * dim * vdim, "plain_tiles: a state slot is too small");
+    TS_REQUIRE(portions >= 0 && portions <= 65535 && heads <= 65535, "plain_tiles: grid too large");
+    if (portions == 0 || max_q_len <= 1) return 0;
+    const PlainArgs a{q, k, q_stride, k_stride, z, z_stride, bias, head_decay, inv_tau, q_scale, k_scale, freq, freq ? rot_dims : 0,
+                      positions, cu_q, prefill_seqs, pack, coef, heads, dim, padded_rows(dim)};
+    const size_t smem = sizeof(float) * (3 * B * (a.rows + 1));
+    const dim3 grid((max_q_len + B - 1) / B, heads, portions);
+    const ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, vdim};
+    if (dtype == TS_F32) {
+        cudaFuncSetAttribute(plain_tile_prepare_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        plain_tile_prepare_kernel<float><<<grid, 128, smem, stream>>>(a);
+        TS_LAUNCH_CHECK("plain_tiles (prepare)");
+        return launch_scan<float, MIX>(s, portions, stream);
+    }
+    if (dtype == TS_BF16) {
+        cudaFuncSetAttribute(plain_tile_prepare_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        plain_tile_prepare_kernel<__nv_bfloat16><<<grid, 128, smem, stream>>>(a);
+        TS_LAUNCH_CHECK("plain_tiles (prepare)");
+        return launch_scan<__nv_bfloat16, MIX>(s, portions, stream);
+    }
+    return ts_fail("plain_tiles: unknown dtype code %d", dtype);
+}
+
+// The delta rule with decays per channel over a step's prompt portions: q, k float32 [tokens, kv_heads * dim] stretches after the
+// convolution, v float32 [tokens, heads * vdim], z float32 [tokens, heads * dim], b [tokens, heads] logits of dtype `b_dtype`.
+TS_API int ts_channel_tiles(const float* q, const float* k, long long qk_stride, const float* z, const void* b, long long b_stride,
+                            int b_dtype, const float* dt_bias, const float* a_log, const float* v, long long v_stride,
+                            const int* cu_q, const int* slots, const int* prefill_seqs, int portions, int max_q_len, float* state,
+                            long long slot_stride, float* pack, float* coef, float* out, int heads, int kv_heads, int dim,
+                            int vdim, float unit_eps, float q_scale, cudaStream_t stream) {
+    TS_REQUIRE(heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && dim > 0 && dim <= 256 && vdim > 0,
+               "channel_tiles: %d heads over %d q/k heads of %d channels", heads, kv_heads, dim);
+    TS_REQUIRE(slot_stride >= (long long)heads * dim * vdim, "channel_tiles: a state slot is too small");
+    TS_REQUIRE(portions >= 0 && portions <= 65535 && heads <= 65535, "channel_tiles: grid too large");
+    if (portions == 0 || max_q_len <= 1) return 0;
+    const ChannelArgs a{q, k, qk_stride, z, b, b_stride, dt_bias, a_log, cu_q, prefill_seqs, pack, coef, heads, kv_heads, dim,
+                        padded_rows(dim), unit_eps, q_scale};
+    const size_t smem = sizeof(float) * (3 * B * (a.rows + 1) + 2 * B * (B + 1));
+    const dim3 grid((max_q_len + B - 1) / B, heads, portions);
+    if (b_dtype == TS_F32) {
+        cudaFuncSetAttribute(channel_tile_prepare_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        channel_tile_prepare_kernel<float><<<grid, 128, smem, stream>>>(a);
+    } else if (b_dtype == TS_BF16) {
+        cudaFuncSetAttribute(channel_tile_prepare_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        channel_tile_prepare_kernel<__nv_bfloat16><<<grid, 128, smem, stream>>>(a);
+    } else {
+        return ts_fail("channel_tiles: unknown dtype code %d", b_dtype);
+    }
+    TS_LAUNCH_CHECK("channel_tiles (prepare)");
+    const ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, vdim};
+    return launch_scan<float, CHANNEL>(s, portions, stream);
 }

@@ -61,7 +61,7 @@ _SIGNATURES = {
     "ts_skinny_linear_groups": ("int", "pppiiiillllip"),
     "ts_gemm_tcgen05_gated": ("int", "pppiiilliffpp"),
     "ts_stream_norm": ("int", "ppppppiifppifiippp" "pppff" "ppppill" "p"),
-    "ts_linear_recurrence": ("int", "ppplllplppfffpipppiplpiiiipip"),
+    "ts_linear_recurrence": ("int", "ppplllplppfffpipppiplpiiiipiip"),
     "ts_head_norm_gate": ("int", "piplpippliiififip"),
     "ts_latent_prepare": ("int", "pliiippfp" "f" "pppplliipiiiip"),
     "ts_latent_attention": ("int", "pllpliip" "fp" "plliipipppiiiifiiplip"),
@@ -90,10 +90,12 @@ _SIGNATURES = {
     "ts_delta_prepare_head": ("int", "pplpppppp" "iiiiffppp"),
     "ts_token_shift": ("int", "pppppplp" "iiiip"),
     "ts_time_mix_prepare": ("int", "pplppppp" "iiipippiplipip"),
-    "ts_recurrence_tiles_pack_floats": ("long long", "iiii"),
+    "ts_recurrence_tiles_pack_floats": ("long long", "iiiii"),
     "ts_recurrence_tiles_coef_floats": ("long long", "iii"),
     "ts_delta_tiles": ("int", "pplppppl" "pppii" "plppp" "iiiiffp"),
     "ts_mix_tiles": ("int", "pplppppl" "pppii" "plppp" "iiip"),
+    "ts_plain_tiles": ("int", "ppplll" "plpp" "fffpip" "pppii" "plppp" "iiiip"),
+    "ts_channel_tiles": ("int", "pplpplipp" "pl" "pppii" "plppp" "iiiiffp"),
     "ts_delta_prepare": ("int", "pplppppl" "ppiiiiffip"),
     "ts_mlstm_prepare": ("int", "ppllpplppffppiplpppiiiip"),
     "ts_row_scaled_activation": ("int", "ppppiiiip"),
@@ -598,12 +600,23 @@ class Ops:
         if position is not None:
             freq, rot = position.frequencies, position.dims
         out = torch.empty((T, heads * vdim), dtype=torch.float32, device=q.device)
+        tiles = self.portions_by_tiles(ctx)
+        if tiles:                                            # prompt portions sixteen tokens at a time
+            pack, coef = self._tile_buffers(ctx, T, heads, heads, dim, q.device)
+            self._call("ts_plain_tiles", _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(z),
+                       z.stride(0) if z is not None else 0, _ptr(bias), _ptr(head_decays), inv_tau, q_scale, k_scale, _ptr(freq),
+                       rot, _ptr(ctx.positions), _ptr(ctx.cu_q), _ptr(binding.state_slots), _ptr(ctx.prefill_seqs),
+                       ctx.prefill_seqs.shape[0], ctx.max_q_len, state.data_ptr(), state.stride(0) // 4, _ptr(pack), _ptr(coef),
+                       _ptr(out), heads, dim, vdim, _DTYPE_CODE[q.dtype], _stream())
+            self.launches += 1                               # what the columns of a tile share, then the scan
+            if ctx.min_q_len > 1:
+                return out
         prepared = torch.empty((3, T, heads * dim), dtype=torch.float32, device=q.device)   # q, k, decays as they enter the scan
         self._call("ts_linear_recurrence", _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(z),
                    z.stride(0) if z is not None else 0, _ptr(bias), _ptr(head_decays), inv_tau, q_scale, k_scale,
                    _ptr(freq), rot, _ptr(ctx.positions), _ptr(ctx.cu_q), _ptr(binding.state_slots),
                    binding.state_slots.shape[0], state.data_ptr(), state.stride(0) // 4, _ptr(out), heads, dim, vdim,
-                   T, _ptr(prepared), _DTYPE_CODE[q.dtype], _stream())
+                   T, _ptr(prepared), 1 if tiles else 0, _DTYPE_CODE[q.dtype], _stream())
         self.launches += 1                                   # the kernel that prepares the scan's inputs
         return out
 
@@ -1088,12 +1101,12 @@ class Ops:
 
     def portions_by_tiles(self, ctx) -> bool:
         """Whether the step holds prompt portions that the kernels of `delta_tiles` and `mix_tiles` take (a bare context may not list them)."""
-        return bool(self.recurrence_tiles and ctx.max_q_len > 1 and getattr(ctx, "prefill_seqs", None) is not None
+        return bool(self.recurrence_tiles and getattr(ctx, "max_q_len", 0) > 1 and getattr(ctx, "prefill_seqs", None) is not None
                     and ctx.prefill_seqs.shape[0] > 0)
 
-    def _tile_buffers(self, ctx, T: int, qk_heads: int, heads: int, dim: int, device) -> tuple[torch.Tensor, torch.Tensor]:
+    def _tile_buffers(self, ctx, T: int, qk_heads: int, heads: int, dim: int, device, sets: int = 1) -> tuple[torch.Tensor, torch.Tensor]:
         seqs = ctx.cu_q.shape[0] - 1
-        floats = (int(self.lib.ts_recurrence_tiles_pack_floats(T, seqs, qk_heads, dim)),
+        floats = (int(self.lib.ts_recurrence_tiles_pack_floats(T, seqs, qk_heads, dim, sets)),
                   int(self.lib.ts_recurrence_tiles_coef_floats(T, seqs, heads)))
         return tuple(torch.empty((n,), dtype=torch.float32, device=device) for n in floats)
 
@@ -1118,6 +1131,33 @@ class Ops:
         self._call("ts_delta_tiles", _ptr(q), _ptr(k), q.stride(0), _ptr(gates), _ptr(dt_bias), _ptr(a_log), _ptr(v), v.stride(0),
                    _ptr(ctx.cu_q), _ptr(binding.state_slots), _ptr(ctx.prefill_seqs), ctx.prefill_seqs.shape[0], ctx.max_q_len,
                    state.data_ptr(), stride, _ptr(pack), _ptr(coef), _ptr(out), heads, kv_heads, dim, vdim, unit_eps, q_scale, _stream())
+        self.launches += 1                                   # what the columns of a tile share, then the scan
+        return out
+
+    def channel_tiles(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tensor, b: torch.Tensor, dt_bias: torch.Tensor,
+                      a_log: torch.Tensor, ctx, binding, *, heads: int, kv_heads: int, dim: int, vdim: int, unit_eps: float,
+                      q_scale: float) -> torch.Tensor:
+        """
+        `delta_prepare` and its scan for the step's prompt portions, sixteen tokens at a time: float32 [T, heads * vdim], of
+        which the rows of requests that feed one token are left unwritten.  q, k, v float32 stretches after the convolution,
+        z float32 [T, heads * dim] and b [T, heads] the logits of the decays and the step sizes.
+        """
+        T = q.shape[0]
+        for t, name, cols in ((q, "q", kv_heads * dim), (k, "k", kv_heads * dim), (v, "v", heads * vdim)):
+            if t.dtype != torch.float32 or t.stride(1) != 1 or tuple(t.shape) != (T, cols) or (name == "k" and t.stride(0) != q.stride(0)):
+                raise KernelError(f"channel_tiles: {name} must be a float32 [T, {cols}] stretch (q and k of one row stride)")
+        self._check(z, "decay logits", torch.float32, 2)
+        if tuple(z.shape) != (T, heads * dim) or b.dtype not in _DTYPE_CODE or b.stride(1) != 1 or tuple(b.shape) != (T, heads):
+            raise KernelError("channel_tiles: decay logits [T, heads * dim] and beta logits [T, heads] are needed")
+        if dt_bias.numel() != heads * dim or a_log.numel() != heads:
+            raise KernelError("channel_tiles: a bias a channel and a rate a head are needed")
+        state, stride = self._state_floats(binding, heads * dim * vdim, "channel_tiles")
+        pack, coef = self._tile_buffers(ctx, T, heads, heads, dim, q.device, sets=2)
+        out = torch.empty((T, heads * vdim), dtype=torch.float32, device=q.device)
+        self._call("ts_channel_tiles", _ptr(q), _ptr(k), q.stride(0), _ptr(z), _ptr(b), b.stride(0), _DTYPE_CODE[b.dtype], _ptr(dt_bias),
+                   _ptr(a_log), _ptr(v), v.stride(0), _ptr(ctx.cu_q), _ptr(binding.state_slots), _ptr(ctx.prefill_seqs),
+                   ctx.prefill_seqs.shape[0], ctx.max_q_len, state.data_ptr(), stride, _ptr(pack), _ptr(coef), _ptr(out), heads,
+                   kv_heads, dim, vdim, unit_eps, q_scale, _stream())
         self.launches += 1                                   # what the columns of a tile share, then the scan
         return out
 

@@ -134,8 +134,12 @@ class GatedDeltaRule(Mixer):
                                         qk_group=H // G, singles=tiles, out=o)
         else:
             z = self.decay_up(y[:, C:C + self.decay_rank].contiguous(), out_dtype=torch.float32)  # decay logits, float32 from here on
-            prepared, beta = ops.delta_prepare(q, k, z, self.dt_bias, self.a_log, b, **sizes)
-            o = ops.recurrence_scan(prepared, v, ctx, matrices, heads=H, dim=D, vdim=V, beta=beta)
+            o, tiles = None, ops.portions_by_tiles(ctx)
+            if tiles:
+                o = ops.channel_tiles(q, k, v, z, b, self.dt_bias, self.a_log, ctx, matrices, vdim=V, **sizes)
+            if not tiles or ctx.min_q_len <= 1:
+                prepared, beta = ops.delta_prepare(q, k, z, self.dt_bias, self.a_log, b, **sizes)
+                o = ops.recurrence_scan(prepared, v, ctx, matrices, heads=H, dim=D, vdim=V, beta=beta, singles=tiles, out=o)
         return ops.head_norm_gate(o, gate, self.norm_weight, H, V, s.out_norm_eps, x.dtype,
                                   gate_kind="silu" if self.full_gate else "sigmoid", scale=scale, out=out)
 
