@@ -425,6 +425,60 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, int o_head, c
     }
 }
 
+// The same for heads of 128 or 256 value channels in rows that 16-byte loads take: a lane holds CH runs of four channels, each of its
+// inputs read once, all at the start (2,048 tokens x 8 heads of 256, bfloat16: 15.6 us, and 8.7 here; 5 by the bytes).
+template <typename T, int CH>
+__global__ void __launch_bounds__(128)
+head_norm_gate_vec_kernel(const float* __restrict__ o, const T* __restrict__ gate, long long gate_stride, const float* __restrict__ weight,
+                          int weight_stride, T* __restrict__ out, long long out_stride, long long items, int heads, float eps,
+                          int gate_kind, float scale) {
+    constexpr int V = 128 * CH;
+    const long long item = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (item >= items) return;
+    const int lane = threadIdx.x & 31, h = (int)(item % heads);
+    const long long t = item / heads;
+    float4 x[CH], w[CH];
+    __align__(16) T g[CH][4];
+#pragma unroll
+    for (int k = 0; k < CH; ++k) {
+        const int j = 128 * k + 4 * lane;
+        x[k] = *reinterpret_cast<const float4*>(o + item * V + j);
+        if (sizeof(T) == 4) *reinterpret_cast<uint4*>(g[k]) = *reinterpret_cast<const uint4*>(gate + t * gate_stride + (long long)h * V + j);
+        else *reinterpret_cast<uint2*>(g[k]) = *reinterpret_cast<const uint2*>(gate + t * gate_stride + (long long)h * V + j);
+        w[k] = weight ? *reinterpret_cast<const float4*>(weight + (long long)h * weight_stride + j) : make_float4(1.f, 1.f, 1.f, 1.f);
+    }
+    float acc = 0.f;
+#pragma unroll
+    for (int k = 0; k < CH; ++k) acc += x[k].x * x[k].x + x[k].y * x[k].y + x[k].z * x[k].z + x[k].w * x[k].w;
+    const float inv = 1.f / sqrtf(warp_sum(acc) / (float)V + eps);
+#pragma unroll
+    for (int k = 0; k < CH; ++k) {
+        const float xs[4] = {x[k].x, x[k].y, x[k].z, x[k].w}, ws[4] = {w[k].x, w[k].y, w[k].z, w[k].w};
+        __align__(16) T y[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float a = to_float<T>(g[k][e]), sig = 1.f / (1.f + expf(-a));
+            y[e] = from_float<T>(xs[e] * inv * ws[e] * (gate_kind == 1 ? sig : a * sig) * scale);
+        }
+        T* dst = out + t * out_stride + (long long)h * V + 128 * k + 4 * lane;
+        if (sizeof(T) == 4) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(y);
+        else *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(y);
+    }
+}
+
+template <typename T>
+static bool head_norm_gate_vec(const float* o, int o_head, const void* gate, long long gate_stride, const float* weight, int weight_stride,
+                               const float* log_max, void* out, long long out_stride, long long items, int heads, int vdim, float eps,
+                               int gate_kind, float scale, cudaStream_t stream) {
+    if ((vdim != 128 && vdim != 256) || o_head != vdim || log_max || gate_stride % 4 || out_stride % 4 || weight_stride % 4 ||
+        ((uintptr_t)o | (uintptr_t)weight) % 16 || ((uintptr_t)gate | (uintptr_t)out) % (4 * sizeof(T)))
+        return false;
+    auto kernel = vdim == 128 ? head_norm_gate_vec_kernel<T, 1> : head_norm_gate_vec_kernel<T, 2>;
+    kernel<<<(unsigned)((items + 3) / 4), 128, 0, stream>>>(o, (const T*)gate, gate_stride, weight, weight_stride, (T*)out, out_stride, items,
+                                                            heads, eps, gate_kind, scale);
+    return true;
+}
+
 TS_API int ts_head_norm_gate(const float* o, int o_head, const void* gate, long long gate_stride, const float* weight,
                              int weight_stride, const float* log_max, void* out, long long out_stride, int num_tokens,
                              int heads, int vdim, float eps, int gate_kind, float scale, int dtype, cudaStream_t stream) {
@@ -433,6 +487,13 @@ TS_API int ts_head_norm_gate(const float* o, int o_head, const void* gate, long 
     if (num_tokens == 0) return 0;
     const long long items = (long long)num_tokens * heads;
     const unsigned blocks = (unsigned)((items + 3) / 4);
+    if (dtype == TS_F32 ? head_norm_gate_vec<float>(o, o_head, gate, gate_stride, weight, weight_stride, log_max, out, out_stride, items,
+                                                    heads, vdim, eps, gate_kind, scale, stream)
+                        : dtype == TS_BF16 && head_norm_gate_vec<__nv_bfloat16>(o, o_head, gate, gate_stride, weight, weight_stride, log_max, out,
+                                                                                out_stride, items, heads, vdim, eps, gate_kind, scale, stream)) {
+        TS_LAUNCH_CHECK("head_norm_gate");
+        return 0;
+    }
     if (dtype == TS_F32)
         head_norm_gate_kernel<float><<<blocks, 128, 0, stream>>>(o, o_head, (const float*)gate, gate_stride, weight,
             weight_stride, log_max, (float*)out, out_stride, items, heads, vdim, eps, gate_kind, scale);
