@@ -247,13 +247,14 @@ struct PlainArgs {
     const float* freq; int rot_dims; const int* positions;   // rotation by halves over the first rot_dims channels
     const int* cu_q; const int* prefill_seqs;
     float* pack; float* coef;
-    int heads, dim, rows;
+    int heads, dim;
 };
 
 // The plain recurrence's pack and P.  grid (tiles, heads, portions), 128 threads.  Bound by its own arithmetic (a decay and,
 // with rotation, a sine and a cosine an element, then the running products); it takes the place of a kernel that wrote q, k and the
-// decays of every token to memory.
-template <typename T>
+// decays of every token to memory.  2,048 tokens, 8 heads of 128: 27 us (34 before ROWS was a constant and the warps skipped the t
+// ahead of their j); the scan behind it 133 us where the walk token by token took 262.
+template <typename T, int ROWS>
 __global__ void __launch_bounds__(128) plain_tile_prepare_kernel(PlainArgs p) {
     extern __shared__ float smem[];
     const int seq = p.prefill_seqs[blockIdx.z], tile = blockIdx.x, h = blockIdx.y;
@@ -261,13 +262,14 @@ __global__ void __launch_bounds__(128) plain_tile_prepare_kernel(PlainArgs p) {
     const int begin = p.cu_q[seq], n = p.cu_q[seq + 1] - begin;
     if (n <= 1 || tile * B >= n) return;
     const int t0 = begin + tile * B, m = min(B, n - tile * B);
-    const int pitch = p.rows + 1;
+    const int pitch = ROWS + 1;
     float* qs = smem;                                    // [16][pitch]
     float* ks = qs + B * pitch;
     float* as = ks + B * pitch;
     const int half = p.rot_dims / 2;
-    for (int e = threadIdx.x; e < B * p.rows; e += 128) {
-        const int t = e / p.rows, i = e % p.rows;
+#pragma unroll 4
+    for (int e = threadIdx.x; e < B * ROWS; e += 128) {
+        const int t = e / ROWS, i = e % ROWS;
         float qv = 0.f, kv = 0.f, av = 1.f;              // a token past the portion's end changes nothing
         if (t < m && i < p.dim) {
             const T* qr = (const T*)p.q + (long long)(t0 + t) * p.q_stride + (long long)h * p.dim;
@@ -306,6 +308,7 @@ __global__ void __launch_bounds__(128) plain_tile_prepare_kernel(PlainArgs p) {
             float run = ks[j * pitch + i];
 #pragma unroll
             for (int t = 0; t < B; ++t) {
+                if (t < (int)(threadIdx.x >> 5) * 4) continue;                          // the warp's four j begin here
                 if (t > j) run *= as[t * pitch + i];
                 if (t >= j) sum[t] = fmaf(qs[t * pitch + i], run, sum[t]);
             }
@@ -319,14 +322,16 @@ __global__ void __launch_bounds__(128) plain_tile_prepare_kernel(PlainArgs p) {
             if (part == 0) out[t * CP + j] = s;                                         // 0 where t < j
         }
     }
-    float* pack = p.pack + (slot * p.heads + h) * pack_floats(p.rows, 1);
-    for (int i = threadIdx.x; i < p.rows; i += 128) {    // a thread a channel: products from the left and from the right
-        const int pp = pack_pitch(p.rows);
+    float* pack = p.pack + (slot * p.heads + h) * pack_floats(ROWS, 1);
+    for (int i = threadIdx.x; i < ROWS; i += 128) {    // a thread a channel: products from the left and from the right
+        const int pp = pack_pitch(ROWS);
         float left = 1.f, right = 1.f;
+#pragma unroll
         for (int t = 0; t < B; ++t) {
             left *= as[t * pitch + i];
             pack[t * pp + i] = qs[t * pitch + i] * left;
         }
+#pragma unroll
         for (int t = B - 1; t >= 0; --t) {
             pack[(B + t) * pp + i] = ks[t * pitch + i] * right;
             right *= as[t * pitch + i];
@@ -342,12 +347,13 @@ struct ChannelArgs {
     const float* bias; const float* rate;                    // dt_bias [heads * dim], A_log [heads]
     const int* cu_q; const int* prefill_seqs;
     float* pack; float* coef;
-    int heads, kv_heads, dim, rows;
+    int heads, kv_heads, dim;
     float unit_eps, q_scale;
 };
 
 // The pack and the coefficients of the delta rule with decays per channel.  grid (tiles, value heads, portions), 128 threads.
-template <typename T>
+// Three portions of 1,001, 667 and 333 tokens, 8 heads of 128: 32 us; the scan behind it 94 us, token by token 300.
+template <typename T, int ROWS>
 __global__ void __launch_bounds__(128) channel_tile_prepare_kernel(ChannelArgs p) {
     extern __shared__ float smem[];
     const int seq = p.prefill_seqs[blockIdx.z], tile = blockIdx.x, h = blockIdx.y, g = h / (p.heads / p.kv_heads);
@@ -355,7 +361,7 @@ __global__ void __launch_bounds__(128) channel_tile_prepare_kernel(ChannelArgs p
     const int begin = p.cu_q[seq], n = p.cu_q[seq + 1] - begin;
     if (n <= 1 || tile * B >= n) return;
     const int t0 = begin + tile * B, m = min(B, n - tile * B);
-    const int pitch = p.rows + 1;
+    const int pitch = ROWS + 1;
     float* qs = smem;                                    // [16][pitch]
     float* ks = qs + B * pitch;
     float* as = ks + B * pitch;
@@ -368,7 +374,8 @@ __global__ void __launch_bounds__(128) channel_tile_prepare_kernel(ChannelArgs p
         const float* kr = p.k + (long long)(t0 + t) * p.qk_stride + (long long)g * p.dim;
         const float* zr = p.z + ((long long)(t0 + t) * p.heads + h) * p.dim;
         float sq = 0.f, sk = 0.f;
-        for (int i = lane; i < p.rows; i += 32) {
+#pragma unroll
+        for (int i = lane; i < ROWS; i += 32) {
             const bool ok = t < m && i < p.dim;          // a token past the portion's end changes nothing
             const float qv = ok ? qr[i] : 0.f, kv = ok ? kr[i] : 0.f;
             qs[t * pitch + i] = qv;
@@ -378,7 +385,7 @@ __global__ void __launch_bounds__(128) channel_tile_prepare_kernel(ChannelArgs p
             sk += kv * kv;
         }
         const float iq = p.q_scale / sqrtf(warp_sum(sq) + p.unit_eps), ik = 1.f / sqrtf(warp_sum(sk) + p.unit_eps);
-        for (int i = lane; i < p.rows; i += 32) { qs[t * pitch + i] *= iq; ks[t * pitch + i] *= ik; }   // the lane's own elements
+        for (int i = lane; i < ROWS; i += 32) { qs[t * pitch + i] *= iq; ks[t * pitch + i] *= ik; }   // the lane's own elements
     }
     __syncthreads();
     {   // t >= j: thread j = tid / 8 walks t with the running product of its channels
@@ -390,6 +397,7 @@ __global__ void __launch_bounds__(128) channel_tile_prepare_kernel(ChannelArgs p
             float run = ks[j * pitch + i];
 #pragma unroll
             for (int t = 0; t < B; ++t) {
+                if (t < warp * 4) continue;                                             // the warp's four j begin here
                 if (t > j) run *= as[t * pitch + i];
                 if (t >= j) {
                     sum_k[t] = fmaf(ks[t * pitch + i], run, sum_k[t]);
@@ -413,15 +421,17 @@ __global__ void __launch_bounds__(128) channel_tile_prepare_kernel(ChannelArgs p
     }
     __syncthreads();
     const long long slot = tile_slot(seq, begin, tile);
-    float* pack = p.pack + (slot * p.heads + h) * pack_floats(p.rows, 2);
-    for (int i = threadIdx.x; i < p.rows; i += 128) {    // a thread a channel: products from the left and from the right
-        const int pp = pack_pitch(p.rows);
+    float* pack = p.pack + (slot * p.heads + h) * pack_floats(ROWS, 2);
+    for (int i = threadIdx.x; i < ROWS; i += 128) {    // a thread a channel: products from the left and from the right
+        const int pp = pack_pitch(ROWS);
         float left = 1.f, right = 1.f;
+#pragma unroll
         for (int t = 0; t < B; ++t) {
             left *= as[t * pitch + i];
             pack[t * pp + i] = qs[t * pitch + i] * left;
             pack[(B + t) * pp + i] = ks[t * pitch + i] * left;
         }
+#pragma unroll
         for (int t = B - 1; t >= 0; --t) {
             pack[(2 * B + t) * pp + i] = ks[t * pitch + i] * right;
             right *= as[t * pitch + i];
@@ -569,6 +579,10 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
         }
         const float* pack = smem + (tile & 1) * STAGE;
         const float* coef = pack + PACK;
+        if (MODE == MIX && !makes_o) {                   // what the update takes is there from the start
+#pragma unroll
+            for (int k = 0; k < 4; ++k) G_s[(c + 4 * k) * RP + col] = to_float<T>(vnow[k]);
+        }
         // product 1: the pack's rows against this warp's rows of S
         {
             float big[TQ / B][2][4] = {}, small[TQ / B][2][4] = {};
@@ -609,10 +623,6 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
                     x[k] = MODE == DELTA ? fmaf(-coef[2 * B * CP + c + 4 * k], sum, x[k]) : x[k] - sum;
                 }
             }
-            if (MODE == MIX && !makes_o) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) G_s[(c + 4 * k) * RP + col] = x[k];
-            }
             if (MODE != MIX || makes_o) {
                 const float* m = coef + (makes_o ? B * CP : 0);
                 float big[4] = {}, small[4] = {};
@@ -649,7 +659,7 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
                 }
             }
         }
-        __syncthreads();                                 // what the update takes is in
+        if (MODE != MIX) __syncthreads();                // what the update takes is in
         // product 3, S^T <- decay S^T + G^T K, and the state after the tile
         {
             SplitA a[2];
@@ -784,22 +794,28 @@ TS_API int ts_plain_tiles(const void* q, const void* k, const void* v, long long
     TS_REQUIRE(portions >= 0 && portions <= 65535 && heads <= 65535, "plain_tiles: grid too large");
     if (portions == 0 || max_q_len <= 1) return 0;
     const PlainArgs a{q, k, q_stride, k_stride, z, z_stride, bias, head_decay, inv_tau, q_scale, k_scale, freq, freq ? rot_dims : 0,
-                      positions, cu_q, prefill_seqs, pack, coef, heads, dim, padded_rows(dim)};
-    const size_t smem = sizeof(float) * (3 * B * (a.rows + 1));
+                      positions, cu_q, prefill_seqs, pack, coef, heads, dim};
+    const int rows = padded_rows(dim);
+    const size_t smem = sizeof(float) * (3 * B * (rows + 1));
     const dim3 grid((max_q_len + B - 1) / B, heads, portions);
     const ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, vdim};
+#define TS_PLAIN_PREPARE(T)                                                                                                    \
+    do {                                                                                                                       \
+        auto kernel = rows == 64 ? plain_tile_prepare_kernel<T, 64> : rows == 128 ? plain_tile_prepare_kernel<T, 128>          \
+                                                                                  : plain_tile_prepare_kernel<T, 256>;         \
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                                  \
+        kernel<<<grid, 128, smem, stream>>>(a);                                                                                \
+        TS_LAUNCH_CHECK("plain_tiles (prepare)");                                                                              \
+    } while (0)
     if (dtype == TS_F32) {
-        cudaFuncSetAttribute(plain_tile_prepare_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        plain_tile_prepare_kernel<float><<<grid, 128, smem, stream>>>(a);
-        TS_LAUNCH_CHECK("plain_tiles (prepare)");
+        TS_PLAIN_PREPARE(float);
         return launch_scan<float, MIX>(s, portions, stream);
     }
     if (dtype == TS_BF16) {
-        cudaFuncSetAttribute(plain_tile_prepare_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        plain_tile_prepare_kernel<__nv_bfloat16><<<grid, 128, smem, stream>>>(a);
-        TS_LAUNCH_CHECK("plain_tiles (prepare)");
+        TS_PLAIN_PREPARE(__nv_bfloat16);
         return launch_scan<__nv_bfloat16, MIX>(s, portions, stream);
     }
+#undef TS_PLAIN_PREPARE
     return ts_fail("plain_tiles: unknown dtype code %d", dtype);
 }
 
@@ -816,18 +832,21 @@ TS_API int ts_channel_tiles(const float* q, const float* k, long long qk_stride,
     TS_REQUIRE(portions >= 0 && portions <= 65535 && heads <= 65535, "channel_tiles: grid too large");
     if (portions == 0 || max_q_len <= 1) return 0;
     const ChannelArgs a{q, k, qk_stride, z, b, b_stride, dt_bias, a_log, cu_q, prefill_seqs, pack, coef, heads, kv_heads, dim,
-                        padded_rows(dim), unit_eps, q_scale};
-    const size_t smem = sizeof(float) * (3 * B * (a.rows + 1) + 2 * B * (B + 1));
+                        unit_eps, q_scale};
+    const int rows = padded_rows(dim);
+    const size_t smem = sizeof(float) * (3 * B * (rows + 1) + 2 * B * (B + 1));
     const dim3 grid((max_q_len + B - 1) / B, heads, portions);
-    if (b_dtype == TS_F32) {
-        cudaFuncSetAttribute(channel_tile_prepare_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        channel_tile_prepare_kernel<float><<<grid, 128, smem, stream>>>(a);
-    } else if (b_dtype == TS_BF16) {
-        cudaFuncSetAttribute(channel_tile_prepare_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        channel_tile_prepare_kernel<__nv_bfloat16><<<grid, 128, smem, stream>>>(a);
-    } else {
-        return ts_fail("channel_tiles: unknown dtype code %d", b_dtype);
-    }
+    TS_REQUIRE(b_dtype == TS_F32 || b_dtype == TS_BF16, "channel_tiles: unknown dtype code %d", b_dtype);
+#define TS_CHANNEL_PREPARE(T)                                                                                                  \
+    do {                                                                                                                       \
+        auto kernel = rows == 64 ? channel_tile_prepare_kernel<T, 64> : rows == 128 ? channel_tile_prepare_kernel<T, 128>      \
+                                                                                    : channel_tile_prepare_kernel<T, 256>;     \
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                                  \
+        kernel<<<grid, 128, smem, stream>>>(a);                                                                                \
+    } while (0)
+    if (b_dtype == TS_F32) TS_CHANNEL_PREPARE(float);
+    else TS_CHANNEL_PREPARE(__nv_bfloat16);
+#undef TS_CHANNEL_PREPARE
     TS_LAUNCH_CHECK("channel_tiles (prepare)");
     const ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, vdim};
     return launch_scan<float, CHANNEL>(s, portions, stream);
