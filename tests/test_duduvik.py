@@ -553,3 +553,60 @@ def test_greedy_generation_through_the_entry_point(folders, name):
               CacheConfig(block_size=16), dtype="float32", num_blocks=24, seed=0)
     done = llm.generate(prompts, SamplingParams(max_tokens=new, temperature=0.0, ignore_eos=True))
     assert [c.token_ids[0] for c in done] == want
+
+
+@pytest.mark.parametrize("heads, rank, rot, page, window, lens, before, sink", [
+    (16, 512, 64, 64, 1024, [301], [0], False), (16, 512, 64, 256, 0, [240, 75], [40, 0], False), (3, 128, 16, 16, 37, [303, 2, 66], [0, 9, 100], True),
+    (19, 256, 32, 64, 2, [181], [5], False), (16, 384, 0, 32, 64, [330], [64], True), (33, 128, 64, 64, 0, [100, 1, 33, 1], [3, 200, 0, 7], False)])
+def test_latent_attention_of_portions_four_tokens_a_tile(heads, rank, rot, page, window, lens, before, sink):
+    """The kernel of prompt portions against the one of single tokens (a context without `cu_q`) and the sums in 64 bits."""
+    from types import SimpleNamespace
+
+    from gpu_util import i32
+    from tinyserve_llm_b200.cache.storage import EntryBinding
+    from tinyserve_llm_b200.ops import get_ops
+    ops, g, width, dev = get_ops(), torch.Generator().manual_seed(7), rank + rot, "cuda"
+    T, ends = sum(lens), [a + b for a, b in zip(lens, before)]
+    pages = [-(-n // page) for n in ends]
+    order = torch.randperm(sum(pages), generator=g).tolist()
+    pool = torch.full((sum(pages), 1, 1, page, width), float("nan"), dtype=torch.bfloat16, device=dev)
+    table, rows, at = [], [], 0
+    for n, k in zip(ends, pages):
+        table.append(order[at:at + k] + [-1] * (max(pages) - k))
+        at += k
+        rows.append((torch.randn(n, width, generator=g) * 0.5).to(torch.bfloat16))
+        for j in range(n):
+            pool[table[-1][j // page], 0, 0, j % page] = rows[-1][j].to(dev)
+    binding = EntryBinding(pool, None, page * width, 0, page, sum(pages), i32(table), max(pages), True)
+    cu = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    positions = [p for n, b in zip(lens, before) for p in range(b, b + n)]
+    base = dict(positions=i32(positions), seq_of_token=i32([s for s, n in enumerate(lens) for _ in range(n)]), max_ctx_len=max(ends))
+    portions = SimpleNamespace(cu_q=i32(cu), max_q_len=max(lens), **base)
+    q_lat, q = torch.randn(T, heads, rank, generator=g), torch.randn(T, heads * (4 + rot), generator=g).to(torch.bfloat16)
+    freq = torch.tensor([100.0 ** (-2.0 * i / rot) for i in range(rot // 2)], dtype=torch.float32, device=dev) if rot else None
+    sinks = torch.linspace(-3, 3, heads, device=dev) if sink else None
+
+    def run(ctx):
+        return ops.latent_attention(q_lat.to(dev), q.to(dev), ctx, binding, heads, 4 + rot, 4, rank, rot, freq, 0.1, window, sink=sinks)
+
+    got, single = run(portions), run(SimpleNamespace(**base))
+    want = torch.zeros(T, heads, rank, dtype=torch.float64)
+    for t, p in enumerate(positions):
+        keys = rows[base["seq_of_token"][t]][max(0, p - window + 1) if window else 0:p + 1].double()
+        s = torch.einsum("hd,jd->hj", q_lat[t].double(), keys[:, :rank])
+        if rot:
+            part = q[t].double().view(heads, 4 + rot)[:, 4:]
+            s += torch.einsum("hr,jr->hj", plain.rotate_half(part[None], torch.tensor([p]), rot, 100.0)[0], keys[:, rank:])
+        s = s * 0.1
+        if sink:
+            want[t] = torch.softmax(torch.cat([s, sinks.cpu().double()[:, None]], 1), -1)[:, :-1] @ keys[:, :rank]
+        else:
+            want[t] = torch.softmax(s, -1) @ keys[:, :rank]
+    off = [((o.cpu().double() - want).norm() / want.norm()).item() for o in (got, single)]
+    assert off[0] <= 1.1 * off[1] and off[0] < 4e-3, off              # the output's own rounding to bfloat16 is 1.6e-3
+    # what a later token of the tile left in the cache reaches no earlier one
+    s = max(range(len(lens)), key=lambda i: lens[i])
+    j = before[s] + 41
+    pool[table[s][j // page], 0, 0, j % page] = float("nan")
+    again = run(portions)
+    assert torch.equal(again[cu[s]:cu[s] + 41], got[cu[s]:cu[s] + 41]) and not bool(torch.isfinite(again[cu[s] + 41]).any())

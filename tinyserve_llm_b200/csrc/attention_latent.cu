@@ -312,6 +312,20 @@ static int launch_latent(const float* q_lat, long long ql_t, long long ql_h, con
     return 0;
 }
 
+bool ts_latent_tokens_supported(int rank, int rot);
+int ts_latent_attention_tokens_launch(const float* q_lat, long long ql_t, long long ql_h, const void* q, long long q_stride,
+                                      int q_head_width, int q_rot_offset, const float* freq, float magnitude, const float* sink,
+                                      const void* k_pool, KVGeometry geo, const int* block_table, int table_width,
+                                      const int* positions, const int* cu_q, int num_seqs, void* out, int num_tokens, int heads,
+                                      int rank, int rot, float scale, int window, cudaStream_t stream);
+
+// Whether four tokens a CTA pay.  Such a CTA holds an SM by itself and takes as long as 1.5 rounds of two CTAs of a token each do
+// (183 against 122 us over windows of 1,024 keys), so the rounds decide.
+static bool tokens_pay(int num_tokens, int num_seqs, int heads) {
+    const long long groups = (heads + 15) / 16, tiles = ((long long)num_tokens / 4 + num_seqs) * groups, singles = num_tokens * groups;
+    return 3 * ((tiles + 147) / 148) < 2 * ((singles + 295) / 296);
+}
+
 // How many floats of scratch a call with these sizes needs (0: the step is large enough to run without splits).
 TS_API long long ts_latent_attention_scratch_floats(int num_tokens, int heads, int rank, int max_keys) {
     const int groups = (heads + LA_WARPS - 1) / LA_WARPS;
@@ -324,9 +338,9 @@ TS_API int ts_latent_attention(const float* q_lat, long long ql_token_stride, lo
                                long long q_stride, int q_head_width, int q_rot_offset, const float* freq,
                                float magnitude, const float* sink, const void* k_pool, long long page_stride, long long entry_offset, int page_tokens,
                                int num_pages, const int* block_table, int table_width, const int* positions,
-                               const int* seq_of_token, void* out, int num_tokens, int heads, int rank, int rot,
-                               float scale, int window, int max_keys, float* scratch, long long scratch_floats, int dtype,
-                               cudaStream_t stream) {
+                               const int* seq_of_token, const int* cu_q, int num_seqs, int max_q_len, void* out, int num_tokens,
+                               int heads, int rank, int rot, float scale, int window, int max_keys, float* scratch,
+                               long long scratch_floats, int dtype, cudaStream_t stream) {
     TS_REQUIRE(num_tokens >= 0 && heads > 0 && rank > 0 && rot >= 0 && rot % 2 == 0, "latent_attention: bad sizes");
     TS_REQUIRE(rank <= 512, "latent_attention: a latent of %d channels is not supported (up to 512)", rank);
     TS_REQUIRE(rank + rot <= 1024, "latent_attention: cache rows of %d channels are not supported", rank + rot);
@@ -347,6 +361,12 @@ TS_API int ts_latent_attention(const float* q_lat, long long ql_token_stride, lo
     }
     if (dtype == TS_BF16 && ts_latent_mma_supported(rank, rot) && page_stride % 8 == 0 && entry_offset % 8 == 0 &&
         (uintptr_t)k_pool % 16 == 0) {
+        // prompt portions, where the context says which tokens are whose: four tokens a CTA
+        if (need == 0 && cu_q && num_seqs > 0 && max_q_len > 1 && num_tokens <= 1 << 24 && heads <= 65535 &&
+            tokens_pay(num_tokens, num_seqs, heads) && ts_latent_tokens_supported(rank, rot))
+            return ts_latent_attention_tokens_launch(q_lat, ql_token_stride, ql_head_stride, q, q_stride, q_head_width, q_rot_offset, freq,
+                                                     magnitude, sink, k_pool, geo, block_table, table_width, positions, cu_q, num_seqs,
+                                                     out, num_tokens, heads, rank, rot, scale, window, stream);
         // bfloat16 with sizes the tensor-core kernel takes: heads as the rows of mma.sync products
         if (ts_latent_attention_mma_launch(q_lat, ql_token_stride, ql_head_stride, q, q_stride, q_head_width, q_rot_offset,
                                            freq, magnitude, sink, k_pool, geo, block_table, table_width, positions, seq_of_token, out,

@@ -64,7 +64,7 @@ _SIGNATURES = {
     "ts_linear_recurrence": ("int", "ppplllplppfffpipppiplpiiiipiip"),
     "ts_head_norm_gate": ("int", "piplpippliiififip"),
     "ts_latent_prepare": ("int", "pliiippfp" "f" "pppplliipiiiip"),
-    "ts_latent_attention": ("int", "pllpliip" "fp" "plliipipppiiiifiiplip"),
+    "ts_latent_attention": ("int", "pllpliip" "fp" "plliipipp" "pii" "piiiifiiplip"),
     "ts_latent_attention_scratch_floats": ("long long", "iiii"),
     "ts_set_latent_mma": ("void", "i"),
     "ts_moe_route": ("int", "ppppppiiiip"),
@@ -1384,10 +1384,12 @@ class Ops:
                 scratch = torch.empty((floats,), dtype=torch.float32, device=q.device)
                 if store is not None:
                     store[key] = scratch
+        cu_q = getattr(ctx, "cu_q", None)                    # a bare context may not say which tokens are whose
         self._call("ts_latent_attention", _ptr(q_lat), q_lat.stride(0), q_lat.stride(1), _ptr(q), q.stride(0), q_head_width,
                    q_rot_offset, _ptr(freq), float(magnitude), _ptr(sink), _ptr(binding.k_pool), binding.page_stride, binding.entry_offset,
                    binding.page_tokens, binding.num_pages, _ptr(binding.block_table), binding.table_width,
-                   _ptr(ctx.positions), _ptr(ctx.seq_of_token), _ptr(out), q.shape[0], heads, rank, rot, scale, window,
+                   _ptr(ctx.positions), _ptr(ctx.seq_of_token), _ptr(cu_q), cu_q.shape[0] - 1 if cu_q is not None else 0,
+                   int(getattr(ctx, "max_q_len", 0) or 0), _ptr(out), q.shape[0], heads, rank, rot, scale, window,
                    max_keys, _ptr(scratch), floats, _DTYPE_CODE[q.dtype], _stream())
         if floats:
             self.launches += 1                               # the kernel that merges the splits

@@ -139,6 +139,7 @@ class LatentAttention(Mixer):
         lens = ctx.cu_q[1:] - ctx.cu_q[:-1]
         seqs = ctx.seq_of_token.long().clamp_min(0)
         out = copy.copy(ctx)
+        out.max_q_len = 1
         out.seq_of_token = torch.where((ctx.seq_of_token >= 0) & (lens[seqs] == 1), ctx.seq_of_token, -1).to(torch.int32)
         return out
 
