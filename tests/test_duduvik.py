@@ -506,6 +506,39 @@ def test_router_ties_go_to_the_lower_index_and_shares_are_a_softmax():
     assert sorted(pair_of_row.tolist()) == [0, 1, 2, 3] and [pair_of_row.tolist()[r] for r in row_of_pair.tolist()] == [0, 1, 2, 3]
 
 
+@pytest.mark.parametrize("scoring", ["softmax_chosen", "sigmoid"])
+@pytest.mark.parametrize("tokens,experts,top", [(1, 1, 1), (1, 32, 4), (8, 33, 4), (16, 128, 8), (12, 129, 10), (3, 512, 33), (17, 32, 4), (13, 64, 10),
+                                                (8, 513, 4), (300, 512, 10), (40, 2048, 8)])
+def test_routing_of_few_pairs_is_the_general_routing(tokens, experts, top, scoring):
+    """Steps inside and outside what one CTA routes, and the widths whose scores stay in registers, with ties and padding rows, against the choice spelled out on the CPU."""
+    from types import SimpleNamespace
+    from tinyserve_llm_b200.ops import get_ops
+    ops = get_ops()
+    assert bool(ops.lib.ts_moe_route_few_supported(tokens, experts, top)) == (tokens <= 16 and tokens * top <= 128 and experts <= 512)
+    g = torch.Generator().manual_seed(tokens * 7 + experts)
+    logits = (torch.randn(tokens, experts, generator=g) * 4).round() / 4                 # many ties
+    bias = (torch.randn(experts, generator=g) * 2).round() / 4                           # sums are exact
+    seq = torch.where(torch.arange(tokens) % 5 == 3, -1, 0).to(torch.int32)
+    chosen, share, offsets, pair_of_row, row_of_pair = (t.cpu() for t in ops.moe_route(
+        logits.cuda(), bias.cuda(), SimpleNamespace(seq_of_token=seq.cuda()), top, scoring))
+    scores = logits + bias
+    order = torch.sort(scores, dim=-1, descending=True, stable=True).indices[:, :top]    # the lower index of equal scores
+    real = seq >= 0
+    assert torch.equal(chosen.long(), torch.where(real[:, None], order, -1))
+    picked = scores.gather(1, order).double()
+    want = torch.softmax(picked, -1) if scoring == "softmax_chosen" else torch.sigmoid(picked)
+    torch.testing.assert_close(share[real].double(), want[real], atol=2e-7, rtol=2e-6)
+    counts = torch.bincount(order[real].flatten(), minlength=experts)
+    assert offsets.tolist() == [0] + counts.cumsum(0).tolist()
+    flat, rows = chosen.flatten(), row_of_pair.flatten()
+    assert torch.equal(rows < 0, flat < 0)
+    used = rows[rows >= 0].long()
+    assert sorted(used.tolist()) == list(range(int(counts.sum())))
+    assert torch.equal(pair_of_row[used].long(), (rows >= 0).nonzero().flatten()) and not pair_of_row[int(counts.sum()):].any()
+    e = flat[rows >= 0].long()
+    assert bool(((offsets[e] <= used) & (used < offsets[e + 1])).all())
+
+
 # ---------------------------------------------------------------------------------------------- entry points
 def test_replay_program_on_a_model_folder(folders, tmp_path):
     """bin/trace_run on a Duduvik folder: portions, a decoded tail, two requests side by side, a reused slot."""

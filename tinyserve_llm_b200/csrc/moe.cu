@@ -13,6 +13,7 @@
 //   ts_moe_arrange   (token, choice) pairs sorted by expert: every CTA takes the exclusive scan of the
 //                    counts and places its pairs behind their expert's offset.  Which row of an
 //                    expert's stretch a pair lands in is not fixed; no result depends on it.
+//   ts_moe_route_few both in one launch, for steps of few pairs.
 //   ts_moe_linear    grouped product over the sorted pairs: row i of expert e's stretch times W_e^T,
 //                    W [experts, N, K].  Tiles of 32 pairs x 64 columns, FFMA with float32 sums over k
 //                    in ascending order (a pair's result does not depend on its row or on the batch).
@@ -31,63 +32,6 @@
 
 // the kinds of gated activation are those of common.cuh (ts_gated_activation)
 
-__global__ void moe_route_kernel(const float* __restrict__ logits, const float* __restrict__ bias,
-                                 const int* __restrict__ seq_of_token, int* __restrict__ chosen, float* __restrict__ share,
-                                 int* __restrict__ counts, int num_tokens, int experts, int top, int scoring) {
-    const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (t >= num_tokens) return;
-    const int lane = threadIdx.x & 31;
-    if (seq_of_token && seq_of_token[t] < 0) {            // a padding row takes part in nothing
-        for (int j = lane; j < top; j += 32) chosen[(long long)t * top + j] = -1;
-        return;
-    }
-    const float* z = logits + (long long)t * experts;
-    float first = 0.f, total = 0.f;
-    unsigned long long taken_lo = 0;                       // experts this lane has given away (its e = lane + 32 i, i < 64)
-    for (int j = 0; j < top; ++j) {
-        float best = -INFINITY;
-        int arg = 0x7fffffff;
-        for (int e = lane, i = 0; e < experts; e += 32, ++i) {
-            if (taken_lo >> i & 1) continue;
-            const float x = z[e] + (bias ? bias[e] : 0.f);
-            if (x > best || (x == best && e < arg)) { best = x; arg = e; }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oa = __shfl_xor_sync(0xffffffffu, arg, o);
-            if (ob > best || (ob == best && oa < arg)) { best = ob; arg = oa; }
-        }
-        if (arg != 0x7fffffff && (arg & 31) == lane) taken_lo |= 1ull << (arg >> 5);
-        if (j == 0) first = best;
-        const float w = scoring == 1 ? 1.f / (1.f + expf(-best)) : expf(best - first);   // the first choice is the largest
-        total += w;
-        if (lane == 0) {
-            chosen[(long long)t * top + j] = arg;
-            share[(long long)t * top + j] = w;
-            atomicAdd(counts + arg, 1);
-        }
-    }
-    __syncwarp();
-    if (lane == 0 && scoring == 0)
-        for (int j = 0; j < top; ++j) share[(long long)t * top + j] /= total;
-}
-
-TS_API int ts_moe_route(const float* logits, const float* bias, const int* seq_of_token, int* chosen, float* share,
-                        int* counts, int num_tokens, int experts, int top, int scoring, cudaStream_t stream) {
-    TS_REQUIRE(experts > 0 && top > 0 && top <= experts, "moe_route: %d of %d experts", top, experts);
-    TS_REQUIRE(experts <= 2048, "moe_route: %d experts are not supported (up to 2048)", experts);
-    if (num_tokens <= 0) return 0;
-    moe_route_kernel<<<(num_tokens + 3) / 4, 128, 0, stream>>>(logits, bias, seq_of_token, chosen, share, counts,
-                                                               num_tokens, experts, top, scoring);
-    TS_LAUNCH_CHECK("moe_route");
-    return 0;
-}
-
-// Scores over all router outputs, choice inside the best groups (see the head of this file).  A warp a token.
-// The scores and the choice scores are computed once into the warp's shared memory; every round of a choice
-// (the best group, the best output) is a walk of each lane over its own entries and two warp reductions: the
-// largest value as an ordered integer, then the lowest index among the lanes that hold it.
 __device__ __forceinline__ unsigned ordered_key(float x) {
     const unsigned u = __float_as_uint(x + 0.f);          // -0 becomes +0: equal values, equal keys
     return u & 0x80000000u ? ~u : u | 0x80000000u;
@@ -100,6 +44,172 @@ __device__ __forceinline__ int warp_argmax(float best, int arg) {
     return (int)__reduce_min_sync(0xffffffffu, (unsigned)(key == top ? arg : 0x7fffffff));
 }
 
+// One token's choice, by one warp: `give(j, expert, weight)` on lane 0 for every choice in order; the sum of the weights is returned
+// (scoring 0 divides by it).  REGS scores a lane are read once and stay in registers (experts <= 32 REGS); 0 reads them for every choice.
+template <int REGS, typename Give>
+__device__ __forceinline__ float moe_choose(const float* __restrict__ z, const float* __restrict__ bias, int experts, int top, int scoring,
+                                            int lane, Give give) {
+    float held[REGS > 0 ? REGS : 1];
+    if constexpr (REGS > 0) {
+#pragma unroll
+        for (int i = 0; i < REGS; ++i) {
+            const int e = lane + 32 * i;
+            held[i] = e < experts ? z[e] + (bias ? bias[e] : 0.f) : nanf("");       // compares with nothing: never chosen
+        }
+    }
+    float first = 0.f, total = 0.f;
+    unsigned long long taken = 0;                          // experts this lane has given away (its e = lane + 32 i, i < 64)
+    for (int j = 0; j < top; ++j) {
+        float best = -INFINITY;
+        int arg = 0x7fffffff;
+        auto look = [&](int i, float x) {
+            if (taken >> i & 1) return;
+            const int e = lane + 32 * i;
+            if (x > best || (x == best && e < arg)) { best = x; arg = e; }
+        };
+        if constexpr (REGS > 0) {
+#pragma unroll
+            for (int i = 0; i < REGS; ++i) look(i, held[i]);
+        } else {
+            for (int i = 0; lane + 32 * i < experts; ++i) look(i, z[lane + 32 * i] + (bias ? bias[lane + 32 * i] : 0.f));
+        }
+        arg = warp_argmax(best, arg);
+        best = __shfl_sync(0xffffffffu, best, arg & 31);   // (none left: every lane has -inf)
+        if (arg != 0x7fffffff && (arg & 31) == lane) taken |= 1ull << (arg >> 5);
+        if (j == 0) first = best;
+        const float w = scoring == 1 ? 1.f / (1.f + expf(-best)) : expf(best - first);   // the first choice is the largest
+        total += w;
+        if (lane == 0) give(j, arg < experts ? arg : -1, w);   // -1: no score was left that compares with another
+    }
+    return total;
+}
+
+// start[e] = counts of the experts before e, start[experts] = all; by one warp.
+__device__ __forceinline__ void moe_starts(const int* counts, int* start, int experts, int lane) {
+    int run = 0;
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+        const int own = e0 + lane < experts ? counts[e0 + lane] : 0;
+        int sum = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int ahead = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += ahead;
+        }
+        if (e0 + lane < experts) start[e0 + lane] = run + sum - own;
+        run += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    if (lane == 0) start[experts] = run;
+}
+
+// A warp a token.  The chain of choices bounds it: scores in registers, two reductions a choice, the shares divided by one lane each
+// and the starts added up by a warp (here and in the arrangement) instead of in a row by one thread took routing and arranging
+// 100 tokens, 512 experts, 10 chosen from 39 to 13 us, 2,048 tokens, 128 experts, 8 chosen from 39 to 14.
+template <int REGS>
+__global__ void moe_route_kernel(const float* __restrict__ logits, const float* __restrict__ bias,
+                                 const int* __restrict__ seq_of_token, int* __restrict__ chosen, float* __restrict__ share,
+                                 int* __restrict__ counts, int num_tokens, int experts, int top, int scoring) {
+    const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (t >= num_tokens) return;
+    const int lane = threadIdx.x & 31;
+    if (seq_of_token && seq_of_token[t] < 0) {            // a padding row takes part in nothing
+        for (int j = lane; j < top; j += 32) chosen[(long long)t * top + j] = -1;
+        return;
+    }
+    const float total = moe_choose<REGS>(logits + (long long)t * experts, bias, experts, top, scoring, lane, [&](int j, int e, float w) {
+        chosen[(long long)t * top + j] = e;
+        share[(long long)t * top + j] = w;
+        if (e >= 0) atomicAdd(counts + e, 1);
+    });
+    __syncwarp();
+    if (scoring == 0)
+        for (int j = lane; j < top; j += 32) share[(long long)t * top + j] /= total;
+}
+
+// Routing and arranging in one CTA, for steps of few pairs: the counts and cursors live in shared memory, so there are no counters to
+// clear and no second launch.  Such a step is what its launches cost.  Measured on a B200 (us, captured; three launches / this one):
+// 1 token of 32 experts, 4 chosen 5.6 / 2.6; 16 tokens 5.6 / 3.1; 8 of 128 experts 6.9 / 3.7; 16 of 128, 8 chosen 7.9 / 5.5; 12 of 512,
+// 10 chosen 11.9 / 9.8.  Beyond, one SM is the slower one (32 tokens of 32 experts 7.2 / 7.4; 64 of 128, 8 chosen 19 / 38), so the line is
+// drawn at a warp a token.
+constexpr int ROUTE_WARPS = 16, ROUTE_TOKENS = 16, ROUTE_PAIRS = 128, ROUTE_EXPERTS = 512;
+
+template <int REGS>
+__global__ void __launch_bounds__(ROUTE_WARPS * 32)
+moe_route_few_kernel(const float* __restrict__ logits, const float* __restrict__ bias, const int* __restrict__ seq_of_token,
+                     int* __restrict__ chosen, float* __restrict__ share, int* __restrict__ offsets, int* __restrict__ pair_of_row,
+                     int* __restrict__ row_of_pair, int num_tokens, int experts, int top, int scoring) {
+    __shared__ int counts[ROUTE_EXPERTS], start[ROUTE_EXPERTS + 1], pick[ROUTE_PAIRS];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, pairs = num_tokens * top;
+    for (int e = tid; e < experts; e += blockDim.x) counts[e] = 0;
+    __syncthreads();
+    for (int t = warp; t < num_tokens; t += ROUTE_WARPS) {
+        if (seq_of_token && seq_of_token[t] < 0) {        // a padding row takes part in nothing
+            for (int j = lane; j < top; j += 32) pick[t * top + j] = -1;
+            continue;
+        }
+        const float total = moe_choose<REGS>(logits + (long long)t * experts, bias, experts, top, scoring, lane, [&](int j, int e, float w) {
+            pick[t * top + j] = e;
+            share[t * top + j] = w;
+            if (e >= 0) atomicAdd(counts + e, 1);
+        });
+        __syncwarp();
+        if (scoring == 0)
+            for (int j = lane; j < top; j += 32) share[t * top + j] /= total;
+    }
+    __syncthreads();
+    if (warp == 0) moe_starts(counts, start, experts, lane);
+    __syncthreads();
+    for (int e = tid; e <= experts; e += blockDim.x) offsets[e] = start[e];
+    for (int r = start[experts] + tid; r < pairs; r += blockDim.x) pair_of_row[r] = 0;       // rows no pair takes
+    __syncthreads();                                      // `start` is used up as the cursors
+    for (int p = tid; p < pairs; p += blockDim.x) {
+        const int e = pick[p];
+        chosen[p] = e;
+        const int row = e < 0 ? -1 : atomicAdd(start + e, 1);
+        if (row >= 0) pair_of_row[row] = p;
+        row_of_pair[p] = row;
+    }
+}
+
+// Whether `ts_moe_route_few` takes the sizes.
+TS_API int ts_moe_route_few_supported(int num_tokens, int experts, int top) {
+    return num_tokens > 0 && num_tokens <= ROUTE_TOKENS && top > 0 && (long long)num_tokens * top <= ROUTE_PAIRS && experts > 0 && experts <= ROUTE_EXPERTS;
+}
+
+// `ts_moe_route` and `ts_moe_arrange` in one.
+TS_API int ts_moe_route_few(const float* logits, const float* bias, const int* seq_of_token, int* chosen, float* share, int* offsets,
+                            int* pair_of_row, int* row_of_pair, int num_tokens, int experts, int top, int scoring, cudaStream_t stream) {
+    TS_REQUIRE(top <= experts && ts_moe_route_few_supported(num_tokens, experts, top), "moe_route: %d of %d experts for %d tokens", top, experts, num_tokens);
+    auto go = [&](auto kernel) {
+        kernel<<<1, ROUTE_WARPS * 32, 0, stream>>>(logits, bias, seq_of_token, chosen, share, offsets, pair_of_row, row_of_pair, num_tokens, experts, top,
+                                                   scoring);
+    };
+    if (experts <= 32) go(moe_route_few_kernel<1>);
+    else if (experts <= 128) go(moe_route_few_kernel<4>);
+    else go(moe_route_few_kernel<16>);
+    TS_LAUNCH_CHECK("moe_route (few)");
+    return 0;
+}
+
+TS_API int ts_moe_route(const float* logits, const float* bias, const int* seq_of_token, int* chosen, float* share,
+                        int* counts, int num_tokens, int experts, int top, int scoring, cudaStream_t stream) {
+    TS_REQUIRE(experts > 0 && top > 0 && top <= experts, "moe_route: %d of %d experts", top, experts);
+    TS_REQUIRE(experts <= 2048, "moe_route: %d experts are not supported (up to 2048)", experts);
+    if (num_tokens <= 0) return 0;
+    auto go = [&](auto kernel) {
+        kernel<<<(num_tokens + 3) / 4, 128, 0, stream>>>(logits, bias, seq_of_token, chosen, share, counts, num_tokens, experts, top, scoring);
+    };
+    if (experts <= 32) go(moe_route_kernel<1>);
+    else if (experts <= 128) go(moe_route_kernel<4>);
+    else if (experts <= 512) go(moe_route_kernel<16>);
+    else go(moe_route_kernel<0>);
+    TS_LAUNCH_CHECK("moe_route");
+    return 0;
+}
+
+// Scores over all router outputs, choice inside the best groups (see the head of this file).  A warp a token.
+// The scores and the choice scores are computed once into the warp's shared memory; every round of a choice
+// (the best group, the best output) is a walk of each lane over its own entries and two warp reductions: the
+// largest value as an ordered integer, then the lowest index among the lanes that hold it.
 __global__ void moe_route_grouped_kernel(const float* __restrict__ logits, const float* __restrict__ correction,
                                          const int* __restrict__ seq_of_token, int* __restrict__ chosen,
                                          float* __restrict__ share, int* __restrict__ counts, float* __restrict__ identity_share,
@@ -186,10 +296,8 @@ __global__ void moe_route_grouped_kernel(const float* __restrict__ logits, const
     }
     __syncwarp();
     const float norm = weight_scale / (total + share_eps);
-    if (lane == 0) {
-        for (int j = 0; j < top; ++j) share[(long long)t * top + j] *= norm;
-        if (identity_share) identity_share[t] = identity * norm;
-    }
+    for (int j = lane; j < top; j += 32) share[(long long)t * top + j] *= norm;
+    if (lane == 0 && identity_share) identity_share[t] = identity * norm;
 }
 
 TS_API int ts_moe_route_grouped(const float* logits, const float* correction, const int* seq_of_token, int* chosen,
@@ -218,11 +326,7 @@ __global__ void moe_arrange_kernel(const int* __restrict__ chosen, const int* __
                                    int* __restrict__ offsets, int* __restrict__ pair_of_row, int* __restrict__ row_of_pair,
                                    int pairs, int experts) {
     extern __shared__ int start[];                        // experts + 1
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int e = 0; e < experts; ++e) { start[e] = run; run += counts[e]; }
-        start[experts] = run;
-    }
+    if (threadIdx.x < 32) moe_starts(counts, start, experts, threadIdx.x);
     __syncthreads();
     if (blockIdx.x == 0)
         for (int e = threadIdx.x; e <= experts; e += blockDim.x) offsets[e] = start[e];

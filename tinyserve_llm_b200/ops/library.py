@@ -68,6 +68,8 @@ _SIGNATURES = {
     "ts_latent_attention_scratch_floats": ("long long", "iiii"),
     "ts_set_latent_mma": ("void", "i"),
     "ts_moe_route": ("int", "ppppppiiiip"),
+    "ts_moe_route_few": ("int", "ppppppppiiiip"),
+    "ts_moe_route_few_supported": ("int", "iii"),
     "ts_moe_arrange": ("int", "ppppppiip"),
     "ts_moe_linear": ("int", "plpipipiipiiiffpiip"),
     "ts_moe_combine": ("int", "pppppiiiippp"),
@@ -1424,11 +1426,16 @@ class Ops:
         dev = logits.device
         chosen = torch.empty((T, top), dtype=torch.int32, device=dev)
         share = torch.empty((T, top), dtype=torch.float32, device=dev)
-        counters = torch.zeros((2 * E,), dtype=torch.int32, device=dev)       # per expert: count, then placement cursor
         offsets = torch.empty((E + 1,), dtype=torch.int32, device=dev)
-        pair_of_row = torch.zeros((T * top,), dtype=torch.int32, device=dev)
         row_of_pair = torch.empty((T * top,), dtype=torch.int32, device=dev)
         seq_of_token = getattr(ctx, "seq_of_token", None)
+        if top <= E and self.lib.ts_moe_route_few_supported(T, E, top):       # a step of few pairs: one launch, nothing to clear
+            pair_of_row = torch.empty((T * top,), dtype=torch.int32, device=dev)
+            self._call("ts_moe_route_few", _ptr(logits), _ptr(bias), _ptr(seq_of_token), _ptr(chosen), _ptr(share), _ptr(offsets),
+                       _ptr(pair_of_row), _ptr(row_of_pair), T, E, top, 1 if scoring == "sigmoid" else 0, _stream())
+            return chosen, share, offsets, pair_of_row, row_of_pair
+        counters = torch.zeros((2 * E,), dtype=torch.int32, device=dev)       # per expert: count, then placement cursor
+        pair_of_row = torch.zeros((T * top,), dtype=torch.int32, device=dev)
         self._call("ts_moe_route", _ptr(logits), _ptr(bias), _ptr(seq_of_token), _ptr(chosen), _ptr(share), _ptr(counters),
                    T, E, top, 1 if scoring == "sigmoid" else 0, _stream())
         self._call("ts_moe_arrange", _ptr(chosen), _ptr(counters), counters.data_ptr() + 4 * E, _ptr(offsets),
