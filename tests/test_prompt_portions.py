@@ -1,0 +1,164 @@
+"""Kernels that only prompt portions reach (tiles of sixteen tokens, runs of the convolution, head norms by wide loads), at their edges."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from gpu_util import i32, make_ctx
+from tinyserve_llm_b200.cache.storage import EntryBinding
+from tinyserve_llm_b200.ops import get_ops
+
+pytestmark = pytest.mark.gpu
+
+LENS = [1, 2, 15, 16, 17, 33, 1, 75]                    # single tokens go to the scan, beside tiles that are full, short and one over
+
+
+def _step(state, lens=LENS):
+    ctx = make_ctx(lens, [n + 5 * s for s, n in enumerate(lens)])
+    ctx.prefill_seqs = i32([s for s, n in enumerate(lens) if n > 1])
+    rows = state.shape[0]
+    return ctx, EntryBinding(None, None, 0, 0, 16, 0, state=state.view(torch.uint8).view(rows, -1), state_slots=i32([rows - 1 - s for s in range(len(lens))]))
+
+
+def _close_to_64_bits(got, want, heads):
+    """By head: the worst row and the median of the norm of the difference.  A term of either path carries about 2^-21 of itself; the
+    worst rows are those whose terms cancel."""
+    got, want = (t.reshape(t.shape[0], heads, -1) for t in (got.double().cpu(), want))
+    err = (got - want).norm(dim=-1) / want.norm(dim=-1).clamp_min(1e-30)
+    assert float(err.max()) < 2e-4 and float(err.median()) < 5e-6, f"worst {float(err.max()):.2e}, median {float(err.median()):.2e}"
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("decays", ["channel", "head", "gone"])
+@pytest.mark.parametrize("dim,vdim", [(64, 64), (100, 52), (128, 40), (256, 129)])
+def test_plain_recurrence_of_portions(dim, vdim, decays, dtype):
+    ops, H, tau = get_ops(), 3, 4.0
+    g = torch.Generator().manual_seed(dim + vdim)
+    T = sum(LENS)
+    y = (torch.randn(T, H * (2 * dim + vdim) + 4, generator=g) * 0.5).to(dtype)
+    z = torch.randn(T, H * dim, generator=g) + 5
+    if decays == "gone":                                 # decays that are zero in float32, beside ones near one
+        z[:, ::3] = -1e4
+    per_head = torch.tensor([0.999, 0.7, 1e-30])
+    state = torch.randn(len(LENS) + 3, H * dim * vdim, generator=g)
+    dev, yd = state.cuda(), y.cuda()
+    ctx, binding = _step(dev)
+    cuts = (0, H * dim, 2 * H * dim, H * (2 * dim + vdim))
+    q, k, v = (yd[:, a:b] for a, b in zip(cuts, cuts[1:]))
+    logits = dict(z=None, bias=None, head_decays=per_head.cuda()) if decays == "head" else dict(z=z.cuda(), bias=None, head_decays=None)
+    before = ops.calls.get("ts_plain_tiles", 0)
+    got = ops.linear_recurrence(q, k, v, ctx, binding, heads=H, dim=dim, vdim=vdim, inv_tau=1 / tau, q_scale=0.7, k_scale=1.3, **logits)
+    assert ops.calls.get("ts_plain_tiles", 0) == before + 1
+    qh, kh, vh = (y[:, a:b].double().view(T, H, -1) for a, b in zip(cuts, cuts[1:]))
+    a = per_head.double()[None, :, None].expand(T, H, dim) if decays == "head" else torch.sigmoid(z.double()).pow(1 / tau).view(T, H, dim)
+
+    def walk(q, k, v, left):
+        out, at = torch.empty(T, H, vdim, dtype=torch.float64), 0
+        for s, n in enumerate(LENS):
+            S = left[len(left) - 1 - s]
+            for t in range(at, at + n):
+                S.mul_(a[t][:, :, None]).add_(1.3 * k[t][:, :, None] * v[t][:, None, :])
+                out[t] = 0.7 * torch.einsum("hdv,hd->hv", S, q[t])
+            at += n
+        return out, left
+
+    start = state.double().view(-1, H, dim, vdim)
+    want, left = walk(qh, kh, vh, start.clone())
+    size, left_size = walk(qh.abs(), kh.abs(), vh.abs(), start.abs())                   # what the terms amount to: a head without memory is q . k, which cancels
+    # a product of split operands is within 2^-21, a decay product over up to 75 steps within 75 2^-23; twice their sum
+    for mine, true, terms in ((got, want, size), (dev, left, left_size)):
+        mine, true, terms = (t.double().cpu().reshape(-1, H, true[0, 0].numel()) for t in (mine, true, terms))
+        worst = float(((mine - true).norm(dim=-1) / terms.norm(dim=-1).clamp_min(1e-30)).max())
+        assert worst < 2e-5, f"{worst:.2e} of the terms"
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("decay", [-6.0, 0.0, 30.0])
+@pytest.mark.parametrize("dim,vdim,heads,kv_heads", [(64, 64, 2, 1), (100, 52, 3, 3), (128, 128, 2, 1), (256, 33, 2, 2)])
+def test_channel_decayed_delta_rule_of_portions(dim, vdim, heads, kv_heads, decay, dtype):
+    """From decays near one to decays that are zero in float32, with keys that repeat (the delta rule's corrections are then large)."""
+    ops, H, G = get_ops(), heads, kv_heads
+    g = torch.Generator().manual_seed(dim + vdim)
+    T, C = sum(LENS), 2 * kv_heads * dim + heads * vdim
+    conv = torch.randn(T, C, generator=g)
+    conv[1::2, G * dim:2 * G * dim] = conv[0:T - 1:2, G * dim:2 * G * dim][:conv[1::2].shape[0]]
+    z = torch.randn(T, H * dim, generator=g) + decay
+    b = (torch.randn(T, H, generator=g) * 2).to(dtype)
+    dt_bias, a_log = torch.randn(H * dim, generator=g) * 0.3, torch.randn(H, generator=g) * 0.5
+    state = torch.randn(len(LENS) + 3, H * dim * vdim, generator=g)
+    dev, cd = state.cuda(), conv.cuda()
+    ctx, binding = _step(dev)
+    sizes = dict(heads=H, kv_heads=G, dim=dim, unit_eps=1e-6, q_scale=0.25)
+    parts = cd[:, :G * dim], cd[:, G * dim:2 * G * dim], cd[:, 2 * G * dim:]
+    rest = z.cuda(), b.cuda(), dt_bias.cuda(), a_log.cuda()
+    got = ops.channel_tiles(*parts, *rest, ctx, binding, vdim=vdim, **sizes)
+    prepared, beta = ops.delta_prepare(parts[0], parts[1], rest[0], rest[2], rest[3], rest[1], **sizes)
+    got = ops.recurrence_scan(prepared, parts[2], ctx, binding, heads=H, dim=dim, vdim=vdim, beta=beta, singles=True, out=got)
+    q, k, a = (t.double().cpu().view(T, H, dim) for t in prepared)                      # as the token-by-token walk takes them
+    bt, v = beta.double().cpu(), conv[:, 2 * G * dim:].double().view(T, H, vdim)
+    want, left = torch.empty(T, H, vdim, dtype=torch.float64), state.double().view(-1, H, dim, vdim).clone()
+    at = 0
+    for s, n in enumerate(LENS):
+        S = left[len(left) - 1 - s]
+        for t in range(at, at + n):
+            S.mul_(a[t][:, :, None])
+            S.add_(k[t][:, :, None] * (bt[t][:, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k[t])))[:, None, :])
+            want[t] = torch.einsum("hdv,hd->hv", S, q[t])
+        at += n
+    _close_to_64_bits(got, want, H)
+    _close_to_64_bits(dev, left.view(len(left), -1), H)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lens,channels", [([256], 4), ([1, 2, 3, 4, 5, 250, 7], 516), ([300] + [1] * 13, 1032), ([8] * 33, 128)])
+def test_convolution_by_runs_of_tokens_is_the_convolution(lens, channels, dtype):
+    """The same bits from rows that wide loads take (runs of tokens) and from rows one element further (an element at a time)."""
+    ops = get_ops()
+    g = torch.Generator().manual_seed(channels)
+    T = sum(lens)
+    wide = torch.zeros(T, channels + 8, dtype=dtype, device="cuda")
+    x = torch.randn(T, channels, generator=g).to(dtype).cuda()
+    taps = torch.randn(channels, 4, generator=g).cuda()
+    state = torch.randn(len(lens) + 3, 3 * channels, generator=g).cuda()
+    results = []
+    for offset in (0, 1):
+        held = state.clone()
+        ctx, binding = _step(held, lens)
+        ctx.seq_of_token[-1] = -1 if lens[-1] == 1 else ctx.seq_of_token[-1]                # a padding row
+        wide[:, offset:offset + channels] = x
+        y = ops.short_conv_silu(wide[:, offset:offset + channels], taps, ctx, binding)
+        results.append((y[:T - 1] if lens[-1] == 1 else y, held))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+    n = lens[0]
+    past = state[-1].view(3, channels).double()
+    full = torch.cat([past, x[:n].double()])
+    acc = sum(full[j:j + n] * taps[:, j].double() for j in range(4))
+    torch.testing.assert_close(results[0][0][:n].double(), torch.nn.functional.silu(acc), atol=3e-6, rtol=3e-6)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("tokens,heads,vdim", [(1, 1, 128), (3, 3, 256), (33, 5, 128), (2, 1, 384)])
+@pytest.mark.parametrize("kind,per_head", [("silu", False), ("sigmoid", True), ("silu", None)])
+def test_head_norm_by_wide_loads(tokens, heads, vdim, kind, per_head, dtype):
+    """Columns of wider tensors, on the loads' boundaries and beside them."""
+    ops = get_ops()
+    g = torch.Generator().manual_seed(vdim + tokens)
+    n, eps = heads * vdim, 1e-5
+    o = torch.randn(tokens, n, generator=g) * 3
+    gate = torch.randn(tokens, n, generator=g).to(dtype)
+    weight = None if per_head is None else 1 + torch.randn(n if per_head else vdim, generator=g) * 0.3
+    oh = o.double().view(tokens, heads, vdim)
+    w = 1.0 if weight is None else weight.double().view(-1, vdim)
+    act = torch.nn.functional.silu if kind == "silu" else torch.sigmoid
+    want = (oh / (oh.pow(2).mean(-1, keepdim=True) + eps).sqrt() * w).view(tokens, n) * act(gate.double()) * 0.5
+    # one rounding to the type behind float32 steps
+    tol = dict(atol=2e-6, rtol=4e-6) if dtype == torch.float32 else dict(atol=1e-6, rtol=2.0 ** -8)
+    for offset in (0, 4, 1):
+        wide, into = (torch.zeros(tokens, n + 8, dtype=dtype, device="cuda") for _ in range(2))
+        wide[:, offset:offset + n] = gate.cuda()
+        ops.head_norm_gate(o.cuda(), wide[:, offset:offset + n], None if weight is None else weight.cuda(), heads, vdim, eps, dtype, gate_kind=kind,
+                           weight_per_head=bool(per_head), scale=0.5, out=into[:, offset:offset + n])
+        torch.testing.assert_close(into[:, offset:offset + n].double().cpu(), want, **tol)
+        into[:, offset:offset + n] = 0
+        assert not into.any()
