@@ -1102,7 +1102,7 @@ class Ops:
         return out
 
     def portions_by_tiles(self, ctx) -> bool:
-        """Whether the step holds prompt portions that the kernels of `delta_tiles` and `mix_tiles` take (a bare context may not list them)."""
+        """Whether the step holds prompt portions, which go sixteen tokens at a time (a bare context may not list them)."""
         return bool(self.recurrence_tiles and getattr(ctx, "max_q_len", 0) > 1 and getattr(ctx, "prefill_seqs", None) is not None
                     and ctx.prefill_seqs.shape[0] > 0)
 
