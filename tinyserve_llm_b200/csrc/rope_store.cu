@@ -64,8 +64,11 @@ __global__ void rope_store_kernel(T* qkv, const int* __restrict__ positions, con
     }
 }
 
-// The same with 16-byte accesses: a thread rotates VN dims of the first half against their partners.
-// Needs rot / 2 and hd to be multiples of VN and 16-byte aligned rows.
+// The same with 16-byte accesses: a thread rotates VN dims of the first half against their partners; value heads are cut the
+// same way and copied.  Needs rot / 2 and hd to be multiples of VN and 16-byte aligned rows.
+// Latency bounds it (a chain of load, rotate, store a turn of the loop), so a token's pieces go over as many threads as there are, up
+// to 256 and else in equal turns.  Measured on a B200, bfloat16, with the values in a loop of their own behind 128 or 256 threads, and
+// now: 2,048 tokens, 32:8 heads of 64, 8.6 / 7.4 us (3.9 by the bytes); portions on 32:8 heads of 128 20.9 / 15.9.
 template <typename T, int VN>
 __global__ void rope_store_vec_kernel(T* qkv, const int* __restrict__ positions, const int* __restrict__ seq_of_token,
                                       const float* __restrict__ table, int rot, const int* __restrict__ block_table,
@@ -94,7 +97,7 @@ __global__ void rope_store_vec_kernel(T* qkv, const int* __restrict__ positions,
     const long long head_stride = (long long)geo.page_tokens * hd;
     const int pair_chunks = half / VN, pass_chunks = (hd - rot) / VN;
     const int per_head = pair_chunks + pass_chunks;
-    const int total = (nh + nkv) * per_head;
+    const int total = (nh + 2 * nkv) * per_head, rotated = (nh + nkv) * per_head;
     float c[VN], sn[VN];
     auto load_angles = [&](int i) {
 #pragma unroll
@@ -106,7 +109,7 @@ __global__ void rope_store_vec_kernel(T* qkv, const int* __restrict__ positions,
         }
     };
     bool have_angles = false;
-    if (cs && (int)threadIdx.x < total && (int)threadIdx.x % per_head < pair_chunks) {
+    if (cs && (int)threadIdx.x < rotated && (int)threadIdx.x % per_head < pair_chunks) {
         load_angles(((int)threadIdx.x % per_head) * VN);
         have_angles = true;
     }
@@ -115,6 +118,15 @@ __global__ void rope_store_vec_kernel(T* qkv, const int* __restrict__ positions,
     for (int w = threadIdx.x; w < total; w += blockDim.x) {
         const int head = w / per_head, ch = w % per_head;
         T* h = row + (long long)head * hd;
+        if (w >= rotated) {                                  // a value head
+            if (base < 0) continue;
+            T* dst = v_pool + base + (long long)(head - nh - nkv) * head_stride;
+            const int d = ch < pair_chunks ? ch * VN : rot + (ch - pair_chunks) * VN;
+            const uint4 a = *reinterpret_cast<const uint4*>(h + d);
+            if (ch < pair_chunks) *reinterpret_cast<uint4*>(dst + d + half) = *reinterpret_cast<const uint4*>(h + d + half);
+            *reinterpret_cast<uint4*>(dst + d) = a;
+            continue;
+        }
         const bool is_k = head >= nh;
         T* dst = (is_k && base >= 0) ? k_pool + base + (long long)(head - nh) * head_stride : nullptr;
         if (ch < pair_chunks) {
@@ -149,15 +161,6 @@ __global__ void rope_store_vec_kernel(T* qkv, const int* __restrict__ positions,
             *reinterpret_cast<uint4*>(dst + d) = *reinterpret_cast<const uint4*>(h + d);
         }
     }
-    if (base >= 0) {
-        const T* v = row + (long long)(nh + nkv) * hd;
-        const int chunks_per_head = hd / VN;
-        for (int w = threadIdx.x; w < nkv * chunks_per_head; w += blockDim.x) {
-            const int head = w / chunks_per_head, d = (w % chunks_per_head) * VN;
-            *reinterpret_cast<uint4*>(v_pool + base + (long long)head * head_stride + d) =
-                *reinterpret_cast<const uint4*>(v + (long long)head * hd + d);
-        }
-    }
 }
 
 TS_API int ts_rope_store(void* qkv, const int* positions, const int* seq_of_token, const float* table, int table_rows,
@@ -177,8 +180,8 @@ TS_API int ts_rope_store(void* qkv, const int* positions, const int* seq_of_toke
     const bool aligned = (uintptr_t)qkv % 16 == 0 && (uintptr_t)k_pool % 16 == 0 && (uintptr_t)v_pool % 16 == 0 &&
                          page_stride % vn == 0 && entry_offset % vn == 0 && (uintptr_t)table % 16 == 0;
     if ((dtype == TS_F32 || dtype == TS_BF16) && aligned && hd % vn == 0 && (rot / 2) % vn == 0) {
-        const int work = (nh + nkv) * ((rot / 2 + hd - rot) / vn);
-        const int vthreads = work >= 256 ? 256 : (work >= 128 ? 128 : 64);
+        const int work = (nh + 2 * nkv) * ((rot / 2 + hd - rot) / vn), turns = (work + 255) / 256;
+        const int vthreads = ((work + turns - 1) / turns + 31) / 32 * 32;      // equal turns, at most 256 threads
         if (dtype == TS_F32)
             TS_CHAINED_CHECK("rope_store", launch_chained(rope_store_vec_kernel<float, 4>, dim3(num_tokens), dim3(vthreads),
                                                           0, stream, (float*)qkv, positions, seq_of_token, table, rot,
