@@ -162,3 +162,49 @@ def test_head_norm_by_wide_loads(tokens, heads, vdim, kind, per_head, dtype):
         torch.testing.assert_close(into[:, offset:offset + n].double().cpu(), want, **tol)
         into[:, offset:offset + n] = 0
         assert not into.any()
+
+
+def _portion_of_mode(mode, plant):
+    """One form of the recurrences over the portions of LENS: {input: value} planted in a token's inputs."""
+    ops, H, G, D, V = get_ops(), 2, 1, 64, 64
+    T = sum(LENS)
+    g = torch.Generator().manual_seed(5)
+    heads = G if mode in ("head", "channel") else H
+    inputs = {"q": torch.randn(T, heads * D, generator=g), "k": torch.randn(T, heads * D, generator=g), "v": torch.randn(T, H * V, generator=g),
+              "z": torch.randn(T, H * D, generator=g), "b": torch.randn(T, H, generator=g), "gates": torch.randn(T, 2 * H, generator=g)}
+    for name, (token, column, value) in plant.items():
+        inputs[name][token, column] = value
+    x = {name: t.cuda() for name, t in inputs.items()}
+    state = torch.randn(len(LENS), H * D * V, generator=g).cuda()
+    ctx, binding = _step(state)
+    sizes = dict(heads=H, kv_heads=G, dim=D, vdim=V, unit_eps=1e-6, q_scale=0.25)
+    per_head, per_channel = torch.zeros(H).cuda(), torch.zeros(H * D).cuda()
+    if mode == "plain":
+        out = ops.linear_recurrence(x["q"], x["k"], x["v"], ctx, binding, heads=H, dim=D, vdim=V, z=x["z"], bias=None, head_decays=None, inv_tau=0.1,
+                                    q_scale=0.25, k_scale=1.0)
+    elif mode == "mixing":
+        out = ops.mix_tiles(x["q"], x["k"], x["v"], x["z"], per_channel, per_channel + 0.5, ctx, binding, heads=H, dim=D)
+    elif mode == "channel":
+        out = ops.channel_tiles(x["q"], x["k"], x["v"], x["z"], x["b"], per_channel, per_head, ctx, binding, **sizes)
+    else:
+        out = ops.delta_tiles(x["q"], x["k"], x["v"], x["gates"], per_head, per_head, ctx, binding, **sizes)
+    for s, n in enumerate(LENS):
+        if n == 1:                                       # not written by the tiles
+            out[sum(LENS[:s])] = 0
+    return out.view(T, H, V).cpu()
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf"), 3.401e38])
+@pytest.mark.parametrize("mode,name", [(m, n) for m, names in (("plain", "qkvz"), ("mixing", "qkvz"), ("channel", "qkvzb"), ("head", ["q", "k", "v", "gates"])) for n in names])
+def test_what_is_not_finite_reaches_no_earlier_token(mode, name, value):
+    """A token in the middle of a tile, in the portion of 75 tokens: the rows before it and the other requests' keep their bits."""
+    begin = sum(LENS[:-1])
+    token = begin + 37
+    clean, got = _portion_of_mode(mode, {}), _portion_of_mode(mode, {name: (token, 1, value)})
+    assert torch.equal(got[:token], clean[:token])
+    if name == "v":                                      # head 0, column 1, from the token on; everything else stands
+        assert not torch.equal(got[token:, 0, 1], clean[token:, 0, 1])
+        got[token:, 0, 1] = clean[token:, 0, 1]
+        assert torch.equal(got, clean)
+    elif name in "qk" and value != value:
+        assert not torch.isfinite(got[token]).all()

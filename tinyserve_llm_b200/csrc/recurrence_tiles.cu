@@ -24,6 +24,10 @@
 //
 // No decay is ever divided by another: products of decays are taken as they are needed.
 //
+// A token's values, keys and decays reach its own and later tokens only, also where they are infinite or NaN: coefficients above the
+// diagonal are zeros, and a value that has no split is left out of the product with them (0 times it would be NaN) and added to the
+// rows from its own on.  A tile pays a vote for it.
+//
 // A first kernel works out, per tile and q/k head (time mixing: head), what all columns of the state share: the
 // "pack" (16 rows for the q side, 16 or 32 for the k side, one with the channels' decays over the tile) and the coefficients
 // (W = M diag(b); P W, so that O = diag(c) S_0^T Q + (P W) (V - diag(c) R) does not wait for U; c; G[B]).  The second
@@ -155,9 +159,9 @@ __global__ void __launch_bounds__(128) delta_tile_prepare_kernel(PrepareArgs p) 
             float pw = 0.f;
 #pragma unroll
             for (int s = 0; s <= t; ++s) pw = fmaf(__shfl_sync(0xffffffffu, P[t], s), M[s] * b, pw);
-            if (lane < B) {
-                out[t * CP + j] = M[t] * b;
-                out[B * CP + t * CP + j] = pw;
+            if (lane < B) {                              // 0 where t < j, whatever the later token's step size is
+                out[t * CP + j] = t >= j ? M[t] * b : 0.f;
+                out[B * CP + t * CP + j] = t >= j ? pw : 0.f;
             }
         }
         if (lane < B) {
@@ -459,9 +463,9 @@ __global__ void __launch_bounds__(128) channel_tile_prepare_kernel(ChannelArgs p
         float pw = 0.f;
 #pragma unroll
         for (int s = 0; s <= t; ++s) pw = fmaf(__shfl_sync(0xffffffffu, P, s), M[s] * b, pw);
-        if (lane < B) {
-            out[t * CP + j] = M[t] * b;
-            out[B * CP + t * CP + j] = pw;
+        if (lane < B) {                                  // 0 where t < j, whatever the later token's step size is
+            out[t * CP + j] = t >= j ? M[t] * b : 0.f;
+            out[B * CP + t * CP + j] = t >= j ? pw : 0.f;
         }
     }
 }
@@ -503,6 +507,27 @@ __device__ __forceinline__ void mma_split(float (&big)[4], float (&small)[4], co
     mma_tf32(big, a.hi, b0.hi, b1.hi);
     mma_tf32(small, a.hi, b0.lo, b1.lo);
     mma_tf32(small, a.lo, b0.hi, b1.hi);
+}
+
+// Numbers from here on have no split (their hi would be infinite).
+constexpr float SPLITS = 3.4e38f;
+
+// What the tokens without a split (as a B fragment: tokens c, c + 4, c + 8, c + 12 of column r) add to tokens at or after them, by the
+// coefficients m [16][CP]: a C fragment.  Out of line: it is hardly ever called.
+__device__ __noinline__ float4 add_odd_tokens(const float* m, float x0, float x4, float x8, float x12, int r, int c) {
+    const float x[4] = {x0, x4, x8, x12};
+    float y[4] = {};
+#pragma unroll
+    for (int j = 0; j < B; ++j)
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            const float v = __shfl_sync(0xffffffffu, x[j >> 2], 4 * (2 * c + side) + (j & 3));
+            if (fabsf(v) < SPLITS) continue;
+#pragma unroll
+            for (int half = 0; half < 2; ++half)
+                if (j <= r + 8 * half) y[2 * half + side] = fmaf(m[(r + 8 * half) * CP + j], v, y[2 * half + side]);
+        }
+    return make_float4(y[0], y[1], y[2], y[3]);
 }
 
 // NT: eights of rows of the state a warp holds.  Fragments of mma.m16n8k8, lane = 4 r + c (r 0..7, c 0..3):
@@ -626,15 +651,26 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
             if (MODE != MIX || makes_o) {
                 const float* m = coef + (makes_o ? B * CP : 0);
                 float big[4] = {}, small[4] = {};
+                float kept[4];                               // what is not finite stays out of the product, where 0 times it is NaN
+                bool odd = false;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const bool ok = fabsf(x[k]) < SPLITS;
+                    kept[k] = ok ? x[k] : 0.f;
+                    odd |= !ok;
+                }
 #pragma unroll
                 for (int ks = 0; ks < 2; ++ks) {
                     const float* a = m + r * CP + 8 * ks + c;
-                    mma_split(big, small, split_a(a[0], a[8 * CP], a[4], a[8 * CP + 4]), split_tf32(x[2 * ks]), split_tf32(x[2 * ks + 1]));
+                    mma_split(big, small, split_a(a[0], a[8 * CP], a[4], a[8 * CP + 4]), split_tf32(kept[2 * ks]), split_tf32(kept[2 * ks + 1]));
                 }
+                float4 late = make_float4(0.f, 0.f, 0.f, 0.f);   // and reaches its own and later tokens by itself
+                if (__any_sync(0xffffffffu, odd)) late = add_odd_tokens(m, x[0], x[1], x[2], x[3], r, c);
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
                     const int t = r + 8 * half;
-                    float y0 = big[2 * half] + small[2 * half], y1 = big[2 * half + 1] + small[2 * half + 1];
+                    float y0 = big[2 * half] + small[2 * half] + (half ? late.z : late.x);
+                    float y1 = big[2 * half + 1] + small[2 * half + 1] + (half ? late.w : late.y);
                     if (!makes_o) {
                         const float g = MODE == DELTA ? coef[2 * B * CP + B + t] : 1.f;
                         *reinterpret_cast<float2*>(G_s + t * RP + 8 * nt_uo + 2 * c) = make_float2(g * y0, g * y1);
