@@ -208,3 +208,52 @@ def test_what_is_not_finite_reaches_no_earlier_token(mode, name, value):
         assert torch.equal(got, clean)
     elif name in "qk" and value != value:
         assert not torch.isfinite(got[token]).all()
+
+
+@pytest.mark.parametrize("form,tokens,heads", [("channel", 70, 3), ("head", 70, 4), ("head", 400, 2), ("delta", 300, 3)])
+def test_tiles_are_no_further_from_64_bits_than_the_walk(form, tokens, heads):
+    """bfloat16 values, decays as trained models spread them: outputs and states of both ways against the same recurrence in 64 bits."""
+    ops, H, D, V, T = get_ops(), heads, 128, 48, tokens
+    g = torch.Generator().manual_seed(tokens)
+    y = (torch.randn(T, H * (2 * D + V), generator=g) * 0.9).to(torch.bfloat16)
+    z, state = torch.randn(T, H * D, generator=g) * 0.7, torch.randn(1, H * D * V, generator=g) * 0.05
+    cuts = (0, H * D, 2 * H * D, H * (2 * D + V))
+    q, k, v = (y[:, a:b] for a, b in zip(cuts, cuts[1:]))
+    per_head = torch.tensor([1 - 2.0 ** (-5 - h) for h in range(H)])
+    wide = lambda t: t.double().view(T, H, -1)
+    if form == "delta":
+        q, k, v = (torch.nn.functional.silu(t.float()) for t in (q, k, v))
+        logits, rate, bias = torch.randn(T, H, generator=g), torch.linspace(0, 2.5, H), torch.linspace(-6, -2, H * D)
+        qd, kd = (wide(t) / (wide(t).pow(2).sum(-1, keepdim=True) + 1e-6).sqrt() for t in (q, k))
+        qd, beta = qd * 0.25, torch.sigmoid(logits.double())
+        a = torch.exp(-rate.double().exp()[:, None] * torch.nn.functional.softplus(wide(z) + bias.double().view(H, D)))
+    else:
+        qd, kd = wide(q) * 0.25, wide(k)
+        a = per_head.double()[None, :, None].expand(T, H, D) if form == "head" else torch.sigmoid(wide(z)).pow(1 / 16)
+    S, want = state.double().view(H, D, V).clone(), torch.empty(T, H, V, dtype=torch.float64)
+    for t in range(T):
+        S *= a[t][:, :, None]
+        u = wide(v)[t] if form != "delta" else beta[t][:, None] * (wide(v)[t] - torch.einsum("hdv,hd->hv", S, kd[t]))
+        S += kd[t][:, :, None] * u[:, None, :]
+        want[t] = torch.einsum("hdv,hd->hv", S, qd[t])
+    off = []
+    for tiles in (True, False):
+        held = state.cuda()
+        ctx, binding = _step(held, [T])
+        if form == "delta":
+            parts, rest = [t.cuda() for t in (q, k, v)], [t.cuda() for t in (z, logits, bias, rate)]
+            sizes = dict(heads=H, kv_heads=H, dim=D, unit_eps=1e-6, q_scale=0.25)
+            if tiles:
+                got = ops.channel_tiles(*parts, *rest, ctx, binding, vdim=V, **sizes)
+            else:
+                prepared, b = ops.delta_prepare(parts[0], parts[1], rest[0], rest[2], rest[3], rest[1], **sizes)
+                got = ops.recurrence_scan(prepared, parts[2], ctx, binding, heads=H, dim=D, vdim=V, beta=b)
+        else:
+            if not tiles:
+                ctx.prefill_seqs = None
+            yd = y.cuda()
+            got = ops.linear_recurrence(*(yd[:, i:j] for i, j in zip(cuts, cuts[1:])), ctx, binding, heads=H, dim=D, vdim=V, bias=None,
+                                        z=z.cuda() if form == "channel" else None, head_decays=per_head.cuda() if form == "head" else None,
+                                        inv_tau=1 / 16, q_scale=0.25, k_scale=1.0)
+        off += [float((x.double().cpu().view(-1) - y64.reshape(-1)).norm() / y64.norm()) for x, y64 in ((got, want), (held, S))]
+    assert off[0] <= off[2] and off[1] <= off[3], off

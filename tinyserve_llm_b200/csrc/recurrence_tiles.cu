@@ -24,6 +24,14 @@
 //
 // No decay is ever divided by another: products of decays are taken as they are needed.
 //
+// What the plain recurrence and the delta rule with decays per channel hold to (relative error of outputs / states against 64 bits, the
+// walk token by token and here): gated linear attention over 2,048 tokens 1.72e-7 / 1.46e-7 and 1.35e-7 / 6.2e-8, constant decays
+// 2.5e-7 / 2.4e-7 and 1.6e-7 / 1.1e-7, the delta rule over portions of 1,001, 667 and 333 tokens 3.0e-7 / 4.2e-7 and 1.9e-7 / 1.8e-7.
+// Three things bring that: the products of decays from a tile's ends are taken in 64 bits and rounded once (sixteen roundings of one
+// constant decay all err to one side, tile after tile: 6.2e-7 / 5.9e-7); a decay near one enters them with the bits past float32's that
+// 1 + expm1 knows; no accumulator of the tensor cores, which cut what it cannot hold, takes more than one large part.  Sums inside a
+// tile stay in float32 (in 64 bits they cost 20 us and gained nothing by then).
+//
 // A token's values, keys and decays reach its own and later tokens only, also where they are infinite or NaN: coefficients above the
 // diagonal are zeros, and a value that has no split is left out of the product with them (0 times it would be NaN) and added to the
 // rows from its own on.  A tile pays a vote for it.
@@ -243,6 +251,19 @@ __global__ void __launch_bounds__(128) mix_tile_prepare_kernel(PrepareArgs p) {
     }
 }
 
+// exp(x), x <= 0, as a float32 number and what that lacks: near one, where a portion multiplies many of them, 1 + expm1(x) is known to
+// more bits than float32 holds.
+__device__ __forceinline__ float decay_of(float x, float& rest) {
+    const float a = expf(x);
+    rest = 0.f;
+    if (!(x > -0.6f)) return a;
+    const float m = expm1f(x), near = 1.f + m;
+    rest = m - (near - 1.f);
+    return near;
+}
+
+__device__ __forceinline__ double whole(float a, __nv_bfloat16 rest) { return (double)a + (double)__bfloat162float(rest); }
+
 struct PlainArgs {
     const void* q; const void* k; long long q_stride, k_stride;
     const float* z; long long z_stride; const float* bias;   // decay logits a channel (a = sigmoid(z + bias)^inv_tau), or
@@ -256,8 +277,8 @@ struct PlainArgs {
 
 // The plain recurrence's pack and P.  grid (tiles, heads, portions), 128 threads.  Bound by its own arithmetic (a decay and,
 // with rotation, a sine and a cosine an element, then the running products); it takes the place of a kernel that wrote q, k and the
-// decays of every token to memory.  2,048 tokens, 8 heads of 128: 27 us (34 before ROWS was a constant and the warps skipped the t
-// ahead of their j); the scan behind it 133 us where the walk token by token took 262.
+// decays of every token to memory.  2,048 tokens, 8 heads of 128: 31 us (34 before ROWS was a constant and the warps skipped the t
+// ahead of their j); the scan behind it 141 us where the walk token by token took 262.
 template <typename T, int ROWS>
 __global__ void __launch_bounds__(128) plain_tile_prepare_kernel(PlainArgs p) {
     extern __shared__ float smem[];
@@ -270,11 +291,12 @@ __global__ void __launch_bounds__(128) plain_tile_prepare_kernel(PlainArgs p) {
     float* qs = smem;                                    // [16][pitch]
     float* ks = qs + B * pitch;
     float* as = ks + B * pitch;
+    __nv_bfloat16* rest = reinterpret_cast<__nv_bfloat16*>(as + B * pitch);        // what the decays lack
     const int half = p.rot_dims / 2;
 #pragma unroll 4
     for (int e = threadIdx.x; e < B * ROWS; e += 128) {
         const int t = e / ROWS, i = e % ROWS;
-        float qv = 0.f, kv = 0.f, av = 1.f;              // a token past the portion's end changes nothing
+        float qv = 0.f, kv = 0.f, av = 1.f, more = 0.f;  // a token past the portion's end changes nothing
         if (t < m && i < p.dim) {
             const T* qr = (const T*)p.q + (long long)(t0 + t) * p.q_stride + (long long)h * p.dim;
             const T* kr = (const T*)p.k + (long long)(t0 + t) * p.k_stride + (long long)h * p.dim;
@@ -292,7 +314,7 @@ __global__ void __launch_bounds__(128) plain_tile_prepare_kernel(PlainArgs p) {
             kv *= p.k_scale;
             if (p.z) {
                 const float x = p.z[(long long)(t0 + t) * p.z_stride + (long long)h * p.dim + i] + (p.bias ? p.bias[h * p.dim + i] : 0.f);
-                av = expf((fminf(x, 0.f) - log1pf(expf(-fabsf(x)))) * p.inv_tau);
+                av = decay_of((fminf(x, 0.f) - log1pf(expf(-fabsf(x)))) * p.inv_tau, more);
             } else {
                 av = p.head_decay[h];
             }
@@ -300,6 +322,7 @@ __global__ void __launch_bounds__(128) plain_tile_prepare_kernel(PlainArgs p) {
         qs[t * pitch + i] = qv;
         ks[t * pitch + i] = kv;
         as[t * pitch + i] = av;
+        rest[t * pitch + i] = __float2bfloat16_rn(more);
     }
     __syncthreads();
     const long long slot = tile_slot(seq, begin, tile);
@@ -329,18 +352,18 @@ __global__ void __launch_bounds__(128) plain_tile_prepare_kernel(PlainArgs p) {
     float* pack = p.pack + (slot * p.heads + h) * pack_floats(ROWS, 1);
     for (int i = threadIdx.x; i < ROWS; i += 128) {    // a thread a channel: products from the left and from the right
         const int pp = pack_pitch(ROWS);
-        float left = 1.f, right = 1.f;
+        double left = 1.0, right = 1.0;
 #pragma unroll
         for (int t = 0; t < B; ++t) {
-            left *= as[t * pitch + i];
-            pack[t * pp + i] = qs[t * pitch + i] * left;
+            left *= whole(as[t * pitch + i], rest[t * pitch + i]);
+            pack[t * pp + i] = (float)((double)qs[t * pitch + i] * left);
         }
 #pragma unroll
         for (int t = B - 1; t >= 0; --t) {
-            pack[(B + t) * pp + i] = ks[t * pitch + i] * right;
-            right *= as[t * pitch + i];
+            pack[(B + t) * pp + i] = (float)((double)ks[t * pitch + i] * right);
+            right *= whole(as[t * pitch + i], rest[t * pitch + i]);
         }
-        pack[2 * B * pp + i] = left;
+        pack[2 * B * pp + i] = (float)left;
     }
 }
 
@@ -356,7 +379,7 @@ struct ChannelArgs {
 };
 
 // The pack and the coefficients of the delta rule with decays per channel.  grid (tiles, value heads, portions), 128 threads.
-// Three portions of 1,001, 667 and 333 tokens, 8 heads of 128: 32 us; the scan behind it 94 us, token by token 300.
+// Three portions of 1,001, 667 and 333 tokens, 8 heads of 128: 33 us; the scan behind it 100 us, token by token 300.
 template <typename T, int ROWS>
 __global__ void __launch_bounds__(128) channel_tile_prepare_kernel(ChannelArgs p) {
     extern __shared__ float smem[];
@@ -371,6 +394,7 @@ __global__ void __launch_bounds__(128) channel_tile_prepare_kernel(ChannelArgs p
     float* as = ks + B * pitch;
     float* kk = as + B * pitch;                          // [16][17]: sum_i k_t k_j G[t][j]
     float* qk = kk + B * (B + 1);                        // sum_i q_t k_j G[t][j]
+    __nv_bfloat16* rest = reinterpret_cast<__nv_bfloat16*>(qk + B * (B + 1));      // [16][pitch]: what the decays lack
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float rate = expf(p.rate[h]);
     for (int t = warp; t < B; t += 4) {
@@ -384,7 +408,9 @@ __global__ void __launch_bounds__(128) channel_tile_prepare_kernel(ChannelArgs p
             const float qv = ok ? qr[i] : 0.f, kv = ok ? kr[i] : 0.f;
             qs[t * pitch + i] = qv;
             ks[t * pitch + i] = kv;
-            as[t * pitch + i] = ok ? expf(-rate * softplus(zr[i] + p.bias[h * p.dim + i])) : 1.f;
+            float more = 0.f;
+            as[t * pitch + i] = ok ? decay_of(-rate * softplus(zr[i] + p.bias[h * p.dim + i]), more) : 1.f;
+            rest[t * pitch + i] = __float2bfloat16_rn(more);
             sq += qv * qv;
             sk += kv * kv;
         }
@@ -428,19 +454,19 @@ __global__ void __launch_bounds__(128) channel_tile_prepare_kernel(ChannelArgs p
     float* pack = p.pack + (slot * p.heads + h) * pack_floats(ROWS, 2);
     for (int i = threadIdx.x; i < ROWS; i += 128) {    // a thread a channel: products from the left and from the right
         const int pp = pack_pitch(ROWS);
-        float left = 1.f, right = 1.f;
+        double left = 1.0, right = 1.0;
 #pragma unroll
         for (int t = 0; t < B; ++t) {
-            left *= as[t * pitch + i];
-            pack[t * pp + i] = qs[t * pitch + i] * left;
-            pack[(B + t) * pp + i] = ks[t * pitch + i] * left;
+            left *= whole(as[t * pitch + i], rest[t * pitch + i]);
+            pack[t * pp + i] = (float)((double)qs[t * pitch + i] * left);
+            pack[(B + t) * pp + i] = (float)((double)ks[t * pitch + i] * left);
         }
 #pragma unroll
         for (int t = B - 1; t >= 0; --t) {
-            pack[(2 * B + t) * pp + i] = ks[t * pitch + i] * right;
-            right *= as[t * pitch + i];
+            pack[(2 * B + t) * pp + i] = (float)((double)ks[t * pitch + i] * right);
+            right *= whole(as[t * pitch + i], rest[t * pitch + i]);
         }
-        pack[3 * B * pp + i] = left;
+        pack[3 * B * pp + i] = (float)left;
     }
     if (warp) return;
     // lane j holds column j (lanes 16..31 mirror lanes 0..15 and store nothing)
@@ -492,6 +518,8 @@ __device__ __forceinline__ Split split_tf32(float x) {
     s.lo = __float_as_uint(x - __uint_as_float(s.hi));
     return s;
 }
+// What the tensor cores drop of lo.
+__device__ __forceinline__ uint32_t rest_of(uint32_t lo) { return __float_as_uint(__uint_as_float(lo) - __uint_as_float(lo & 0xffffe000u)); }
 __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -502,11 +530,39 @@ __device__ __forceinline__ SplitA split_a(float a0, float a1, float a2, float a3
     const Split s0 = split_tf32(a0), s1 = split_tf32(a1), s2 = split_tf32(a2), s3 = split_tf32(a3);
     return SplitA{{s0.hi, s1.hi, s2.hi, s3.hi}, {s0.lo, s1.lo, s2.lo, s3.lo}};
 }
-// The two large and the small parts of a product of split factors, each in an accumulator of its own (no long chain).
+// The two large and the small parts of a product of split factors, each in an accumulator of its own (no long chain).  FRESH: every
+// large part begins at zero and is added by an ordinary rounded addition, where the tensor cores cut what an accumulator cannot hold.
+template <bool FRESH>
 __device__ __forceinline__ void mma_split(float (&big)[4], float (&small)[4], const SplitA& a, Split b0, Split b1) {
-    mma_tf32(big, a.hi, b0.hi, b1.hi);
+    if (FRESH) {
+        float part[4] = {};
+        mma_tf32(part, a.hi, b0.hi, b1.hi);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) big[i] += part[i];
+    } else {
+        mma_tf32(big, a.hi, b0.hi, b1.hi);
+    }
     mma_tf32(small, a.hi, b0.lo, b1.lo);
     mma_tf32(small, a.lo, b0.hi, b1.hi);
+}
+
+// Products of which one factor is a TF32 number itself (bfloat16 values): the other in three pieces, all of it.
+__device__ __forceinline__ void mma_exact_b(float (&big)[4], float (&small)[4], const SplitA& a, float b0, float b1) {
+    const uint32_t rest[4] = {rest_of(a.lo[0]), rest_of(a.lo[1]), rest_of(a.lo[2]), rest_of(a.lo[3])};
+    float part[4] = {};
+    mma_tf32(part, a.hi, __float_as_uint(b0), __float_as_uint(b1));
+    mma_tf32(small, a.lo, __float_as_uint(b0), __float_as_uint(b1));
+    mma_tf32(small, rest, __float_as_uint(b0), __float_as_uint(b1));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) big[i] += part[i];
+}
+__device__ __forceinline__ void mma_exact_a(float (&big)[4], float (&small)[4], const uint32_t (&a)[4], Split b0, Split b1) {
+    float part[4] = {};
+    mma_tf32(part, a, b0.hi, b1.hi);
+    mma_tf32(small, a, b0.lo, b1.lo);
+    mma_tf32(small, a, rest_of(b0.lo), rest_of(b1.lo));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) big[i] += part[i];
 }
 
 // Numbers from here on have no split (their hi would be infinite).
@@ -541,6 +597,8 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
     constexpr int PP = pack_pitch(ROWS);
     constexpr int SETS = sets_of(MODE), PACK = pack_floats(ROWS, SETS), STAGE = PACK + COEF;
     constexpr int TQ = MODE == MIX ? B : 2 * B;          // rows of the pack that meet S_0
+    constexpr bool FRESH = MODE != DELTA;                // (a decay a head: the sums as they have always been)
+    constexpr bool EXACT = MODE == MIX && sizeof(T) == 2;   // the values are TF32 numbers
     extern __shared__ __align__(16) float smem[];
     float* red = smem + 2 * STAGE;                       // [WARPS][TQ][RP]
     float* G_s = red + WARPS * TQ * RP;                  // [B][RP]: what the state's update takes, G[B] U or V
@@ -621,8 +679,8 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
                     const float* row = pack + (mt * B + r) * PP + warp * WROWS + 8 * nt + 2 * c;
                     const float2 lo = *reinterpret_cast<const float2*>(row), hi = *reinterpret_cast<const float2*>(row + 8 * PP);
                     const SplitA a = split_a(lo.x, hi.x, lo.y, hi.y);
-                    mma_split(big[mt][0], small[mt][0], a, b[0], b[1]);
-                    mma_split(big[mt][1], small[mt][1], a, b[2], b[3]);
+                    mma_split<FRESH>(big[mt][0], small[mt][0], a, b[0], b[1]);
+                    mma_split<FRESH>(big[mt][1], small[mt][1], a, b[2], b[3]);
                 }
             }
 #pragma unroll
@@ -662,7 +720,9 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
 #pragma unroll
                 for (int ks = 0; ks < 2; ++ks) {
                     const float* a = m + r * CP + 8 * ks + c;
-                    mma_split(big, small, split_a(a[0], a[8 * CP], a[4], a[8 * CP + 4]), split_tf32(kept[2 * ks]), split_tf32(kept[2 * ks + 1]));
+                    const SplitA w = split_a(a[0], a[8 * CP], a[4], a[8 * CP + 4]);
+                    if (EXACT) mma_exact_b(big, small, w, kept[2 * ks], kept[2 * ks + 1]);
+                    else mma_split<FRESH>(big, small, w, split_tf32(kept[2 * ks]), split_tf32(kept[2 * ks + 1]));
                 }
                 float4 late = make_float4(0.f, 0.f, 0.f, 0.f);   // and reaches its own and later tokens by itself
                 if (__any_sync(0xffffffffu, odd)) late = add_odd_tokens(m, x[0], x[1], x[2], x[3], r, c);
@@ -710,8 +770,11 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
                 float big[4] = {}, small[4] = {};
                 const float* k = pack + (SETS * B + c) * PP + warp * WROWS + 8 * nt + r;
 #pragma unroll
-                for (int ks = 0; ks < 2; ++ks)
-                    mma_split(big, small, a[ks], split_tf32(k[8 * ks * PP]), split_tf32(k[(8 * ks + 4) * PP]));
+                for (int ks = 0; ks < 2; ++ks) {
+                    const Split k0 = split_tf32(k[8 * ks * PP]), k1 = split_tf32(k[(8 * ks + 4) * PP]);
+                    if (EXACT) mma_exact_a(big, small, a[ks].hi, k0, k1);
+                    else mma_split<FRESH>(big, small, a[ks], k0, k1);
+                }
                 float2 d = make_float2(cB, cB);
                 if (MODE != DELTA) d = *reinterpret_cast<const float2*>(pack + (1 + SETS) * B * PP + warp * WROWS + 8 * nt + 2 * c);
                 S[nt][0] = fmaf(d.x, S[nt][0], big[0] + small[0]);
@@ -832,7 +895,7 @@ TS_API int ts_plain_tiles(const void* q, const void* k, const void* v, long long
     const PlainArgs a{q, k, q_stride, k_stride, z, z_stride, bias, head_decay, inv_tau, q_scale, k_scale, freq, freq ? rot_dims : 0,
                       positions, cu_q, prefill_seqs, pack, coef, heads, dim};
     const int rows = padded_rows(dim);
-    const size_t smem = sizeof(float) * (3 * B * (rows + 1));
+    const size_t smem = sizeof(float) * (3 * B * (rows + 1)) + 2 * B * (rows + 1);      // 29 KB at 128 channels: seven CTAs an SM
     const dim3 grid((max_q_len + B - 1) / B, heads, portions);
     const ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, vdim};
 #define TS_PLAIN_PREPARE(T)                                                                                                    \
@@ -870,7 +933,7 @@ TS_API int ts_channel_tiles(const float* q, const float* k, long long qk_stride,
     const ChannelArgs a{q, k, qk_stride, z, b, b_stride, dt_bias, a_log, cu_q, prefill_seqs, pack, coef, heads, kv_heads, dim,
                         unit_eps, q_scale};
     const int rows = padded_rows(dim);
-    const size_t smem = sizeof(float) * (3 * B * (rows + 1) + 2 * B * (B + 1));
+    const size_t smem = sizeof(float) * (3 * B * (rows + 1) + 2 * B * (B + 1)) + 2 * B * (rows + 1);
     const dim3 grid((max_q_len + B - 1) / B, heads, portions);
     TS_REQUIRE(b_dtype == TS_F32 || b_dtype == TS_BF16, "channel_tiles: unknown dtype code %d", b_dtype);
 #define TS_CHANNEL_PREPARE(T)                                                                                                  \
