@@ -257,3 +257,63 @@ def test_tiles_are_no_further_from_64_bits_than_the_walk(form, tokens, heads):
                                         inv_tau=1 / 16, q_scale=0.25, k_scale=1.0)
         off += [float((x.double().cpu().view(-1) - y64.reshape(-1)).norm() / y64.norm()) for x, y64 in ((got, want), (held, S))]
     assert off[0] <= off[2] and off[1] <= off[3], off
+
+
+def _recurrence_part(kind, dtype):
+    from tinyserve_llm_b200.config.spec import GatedDeltaRuleSpec, LinearRecurrenceSpec
+    from tinyserve_llm_b200.parts.base import Runtime, part_class
+    g = torch.Generator().manual_seed(3)
+    w = lambda *shape: torch.randn(shape, generator=g) * 0.05
+    if kind == "plain":
+        spec = LinearRecurrenceSpec(q_scale=0.125, decay="channel_logits", decay_rank=16, tau=16.0, hidden_size=128, num_heads=2, key_dim=64, value_dim=128,
+                                    out_norm_eps=1e-6)
+        tensors = {"q": w(128, 128), "k": w(128, 128), "v": w(256, 128), "g": w(256, 128), "o": w(128, 256), "a1": w(16, 128), "a2": w(128, 16) * 4,
+                   "a2.b": w(128), "norm": 1 + w(128)}
+    else:
+        spec = GatedDeltaRuleSpec(hidden_size=128, num_heads=2, num_kv_heads=1, key_dim=64, value_dim=128, conv_taps=4, q_scale=0.125, unit_eps=1e-6,
+                                  out_norm_eps=1e-6, decay_rank=16, gate_rank=16, decay_scope="channel", gate="low_rank_sigmoid")
+        tensors = {"q": w(64, 128), "k": w(64, 128), "v": w(256, 128), "b": w(2, 128), "o": w(128, 256), "q.conv": w(64, 4) * 8, "k.conv": w(64, 4) * 8,
+                   "v.conv": w(256, 4) * 8, "norm": 1 + w(128), "a1": w(16, 128), "a2": w(128, 16) * 4, "g1": w(16, 128), "g2": w(256, 16) * 4,
+                   "dt_bias": w(128) * 20 - 4, "A_log": w(2) + 1}
+    rt = Runtime(dtype=dtype, device=torch.device("cuda", 0), ops=get_ops())
+    part = part_class("mixer", spec)(spec, {n: t.to(dtype) if n not in ("norm", "dt_bias", "A_log") else t for n, t in tensors.items()}, rt)
+    return part, torch.randn(400, 128, generator=g).to(dtype).cuda()
+
+
+def _fed(part, x, cuts, state):
+    """The part's outputs for one request whose tokens come in portions that end at `cuts`."""
+    out, at = [], 0
+    for end in cuts:
+        ctx = make_ctx([end - at], [end])
+        ctx.prefill_seqs = i32([0] if end - at > 1 else [])
+        out.append(part.forward(x[at:end], ctx, EntryBinding(None, None, 0, 0, 16, 0, state=state.view(torch.uint8).view(1, -1), state_slots=i32([0]))))
+        at = end
+    return torch.cat(out)
+
+
+@pytest.mark.parametrize("kind", ["plain", "delta"])
+def test_float32_recurrences_do_not_depend_on_the_cut(kind):
+    part, x = _recurrence_part(kind, torch.float32)
+    states = [torch.zeros(part.state_bytes() // 4, device="cuda") for _ in range(2)]
+    whole, cut = (_fed(part, x, cuts, s) for cuts, s in zip(([400], [150, 157, 158, 400]), states))
+    assert torch.equal(whole, cut) and torch.equal(*states)
+
+
+@pytest.mark.parametrize("form", ["channel", "head"])
+def test_tiles_do_not_depend_on_cuts_at_multiples_of_sixteen(form):
+    ops, H, D, V, T = get_ops(), 2, 64, 80, 400
+    g = torch.Generator().manual_seed(9)
+    y, z = (torch.randn(T, H * (2 * D + V), generator=g) * 0.5).to(torch.bfloat16).cuda(), torch.randn(T, H * D, generator=g).cuda()
+    logits = dict(z=None, head_decays=torch.tensor([0.99, 0.8]).cuda()) if form == "head" else dict(head_decays=None)
+    results = []
+    for cuts in ([T], [176, 208, T]):
+        state, out, at = torch.ones(1, H * D * V).cuda(), [], 0
+        for end in cuts:
+            ctx, binding = _step(state, [end - at])
+            ctx.positions += at - int(ctx.positions[0])
+            part = y[at:end]
+            out.append(ops.linear_recurrence(part[:, :H * D], part[:, H * D:2 * H * D], part[:, 2 * H * D:], ctx, binding, heads=H, dim=D, vdim=V, bias=None,
+                                             inv_tau=0.1, q_scale=1.0, k_scale=1.0, **{"z": z[at:end].contiguous(), **logits}))
+            at = end
+        results.append((torch.cat(out), state))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])

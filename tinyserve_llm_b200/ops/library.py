@@ -578,12 +578,13 @@ class Ops:
     # ------------------------------------------------------------------ linear recurrences
     def linear_recurrence(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, ctx, binding, *, heads: int, dim: int,
                           vdim: int, z: torch.Tensor | None, bias: torch.Tensor | None, head_decays: torch.Tensor | None,
-                          inv_tau: float, q_scale: float, k_scale: float, position=None) -> torch.Tensor:
+                          inv_tau: float, q_scale: float, k_scale: float, position=None, tiles: bool | None = None) -> torch.Tensor:
         """
         float32 [T, heads * vdim]: o_t = S_t^T q_t with S_t = diag(a_t) S_(t-1) + k_t v_t^T per request and
         head, the state read from and written back to the request's slot (`binding.state`).  q, k, v are
         column slices of one projection output (unit stride inside a row).  Decays: `z` (float32
-        [T, heads * dim] logits, a = sigmoid(z + bias)^inv_tau) or `head_decays` (float32 [heads]).
+        [T, heads * dim] logits, a = sigmoid(z + bias)^inv_tau) or `head_decays` (float32 [heads]).  `tiles`: whether the
+        step's prompt portions go sixteen tokens at a time (None: any that the context lists).
         """
         for t, name, cols in ((q, "q", heads * dim), (k, "k", heads * dim), (v, "v", heads * vdim)):
             if not t.is_cuda or t.dim() != 2 or t.stride(1) != 1 or t.shape[1] != cols or t.dtype not in _DTYPE_CODE:
@@ -602,7 +603,8 @@ class Ops:
         if position is not None:
             freq, rot = position.frequencies, position.dims
         out = torch.empty((T, heads * vdim), dtype=torch.float32, device=q.device)
-        tiles = self.portions_by_tiles(ctx)
+        if tiles is None:
+            tiles = self.portions_by_tiles(ctx)
         if tiles:                                            # prompt portions sixteen tokens at a time
             pack, coef = self._tile_buffers(ctx, T, heads, heads, dim, q.device)
             self._call("ts_plain_tiles", _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(z),

@@ -134,7 +134,8 @@ class GatedDeltaRule(Mixer):
                                         qk_group=H // G, singles=tiles, out=o)
         else:
             z = self.decay_up(y[:, C:C + self.decay_rank].contiguous(), out_dtype=torch.float32)  # decay logits, float32 from here on
-            o, tiles = None, ops.portions_by_tiles(ctx)
+            # float32 activations token by token (as in parts/recurrence.py)
+            o, tiles = None, x.dtype != torch.float32 and ops.portions_by_tiles(ctx)
             if tiles:
                 o = ops.channel_tiles(q, k, v, z, b, self.dt_bias, self.a_log, ctx, matrices, vdim=V, **sizes)
             if not tiles or ctx.min_q_len <= 1:

@@ -28,6 +28,8 @@ from tinyserve_llm_b200.parts.base import Mixer, Runtime, TensorDecl, part_class
 from tinyserve_llm_b200.parts.linear import Linear, fuse_rows
 
 MAX_KEY_DIM = 256       # csrc/linear_recurrence.cu: 16 row groups x 16 rows in registers
+# Prompt portions go sixteen tokens at a time (csrc/recurrence_tiles.cu), but not with float32 activations: those walk token by
+# token, so that a token's result depends on nothing but the tokens before it, wherever the step was cut.
 
 
 @register_part("mixer", "linear_recurrence")
@@ -103,6 +105,7 @@ class LinearRecurrence(Mixer):
         o = ops.linear_recurrence(q, k, v, ctx, binding, heads=H, dim=D, vdim=V, z=z,
                                   bias=self.decay_bias if self.decay_rank else None, head_decays=self.head_decays,
                                   inv_tau=1.0 / spec.tau, q_scale=spec.q_scale, k_scale=spec.k_scale,
-                                  position=self.position)                 # float32 [T, H V]
+                                  position=self.position,
+                                  tiles=x.dtype != torch.float32 and ops.portions_by_tiles(ctx))      # float32 [T, H V]
         gated = ops.head_norm_gate(o, g, self.norm_weight, H, V, spec.out_norm_eps, x.dtype)
         return self.out(gated)
