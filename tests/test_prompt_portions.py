@@ -8,6 +8,8 @@ import torch
 from gpu_util import i32, make_ctx
 from tinyserve_llm_b200.cache.storage import EntryBinding
 from tinyserve_llm_b200.ops import get_ops
+from tinyserve_llm_b200.parts.delta_rule import CHANNEL_TILE_TOKENS
+from tinyserve_llm_b200.parts.recurrence import TILE_TOKENS
 
 pytestmark = pytest.mark.gpu
 
@@ -317,3 +319,30 @@ def test_tiles_do_not_depend_on_cuts_at_multiples_of_sixteen(form):
             at = end
         results.append((torch.cat(out), state))
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+@pytest.mark.parametrize("kind,entry,tokens", [("plain", "ts_plain_tiles", TILE_TOKENS), ("delta", "ts_channel_tiles", CHANNEL_TILE_TOKENS)])
+def test_short_portions_walk_token_by_token(kind, entry, tokens):
+    """Two portions and single tokens: either side of the longest portion from which tiles pay."""
+    ops = get_ops()
+    part, x = _recurrence_part(kind, torch.bfloat16)
+    for lens, tiles in (([tokens, 1, 9, 1], True), ([tokens - 1, 1, 9, 1], False)):
+        ctx = make_ctx(lens, lens)
+        ctx.prefill_seqs = i32([0, 2])
+        state = torch.zeros(len(lens), part.state_bytes(), dtype=torch.uint8, device="cuda")
+        before = ops.calls.get(entry, 0)
+        part.forward(x[:sum(lens)], ctx, EntryBinding(None, None, 0, 0, 16, 0, state=state, state_slots=i32(list(range(len(lens))))))
+        assert ops.calls.get(entry, 0) == before + tiles
+
+
+def test_every_tile_of_a_step_has_room_in_the_buffer():
+    """The kernels number a request's tiles from cu_q / 16 + its index on; the buffer holds T / 16 + requests + 1."""
+    g = torch.Generator().manual_seed(0)
+    for _ in range(200):
+        lens = torch.randint(0, 50, (int(torch.randint(1, 40, (1,), generator=g)),), generator=g).tolist()
+        begin, end = 0, 0
+        for s, n in enumerate(lens):
+            assert begin // 16 + s >= end
+            end = begin // 16 + s + -(-n // 16)
+            begin += n
+        assert end <= begin // 16 + len(lens) + 1

@@ -201,6 +201,7 @@ class Ops:
         self.swiglu_skinny_rows = self.skinny_max_rows
         # TINYSERVE_B200_TILES=0 keeps the recurrences that have a form of sixteen tokens at a time on the scan token by token
         self.recurrence_tiles = os.environ.get("TINYSERVE_B200_TILES", "1") != "0"
+        self._tile_floats: dict[tuple[int, int, int, int], tuple[int, int]] = {}   # sizes of a tile's buffers
         # TINYSERVE_B200_OVERLAP=0 keeps a replayed step's kernels on one stream (see parts/overlap.py)
         self.overlap = os.environ.get("TINYSERVE_B200_OVERLAP", "1") != "0"
         # TINYSERVE_B200_LRU=split keeps a gated linear recurrent unit's decode steps on the kernels of prompt portions
@@ -606,11 +607,11 @@ class Ops:
         if tiles is None:
             tiles = self.portions_by_tiles(ctx)
         if tiles:                                            # prompt portions sixteen tokens at a time
-            pack, coef = self._tile_buffers(ctx, T, heads, heads, dim, q.device)
+            buffer, pack, coef = self._tile_buffers(ctx, T, heads, heads, dim, q.device)
             self._call("ts_plain_tiles", _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(z),
                        z.stride(0) if z is not None else 0, _ptr(bias), _ptr(head_decays), inv_tau, q_scale, k_scale, _ptr(freq),
                        rot, _ptr(ctx.positions), _ptr(ctx.cu_q), _ptr(binding.state_slots), _ptr(ctx.prefill_seqs),
-                       ctx.prefill_seqs.shape[0], ctx.max_q_len, state.data_ptr(), state.stride(0) // 4, _ptr(pack), _ptr(coef),
+                       ctx.prefill_seqs.shape[0], ctx.max_q_len, state.data_ptr(), state.stride(0) // 4, pack, coef,
                        _ptr(out), heads, dim, vdim, _DTYPE_CODE[q.dtype], _stream())
             self.launches += 1                               # what the columns of a tile share, then the scan
             if ctx.min_q_len > 1:
@@ -1103,16 +1104,24 @@ class Ops:
             raise KernelError(f"a scan's out is {tuple(out.shape)}, expected {(rows, cols)}")
         return out
 
-    def portions_by_tiles(self, ctx) -> bool:
-        """Whether the step holds prompt portions, which go sixteen tokens at a time (a bare context may not list them)."""
-        return bool(self.recurrence_tiles and getattr(ctx, "max_q_len", 0) > 1 and getattr(ctx, "prefill_seqs", None) is not None
-                    and ctx.prefill_seqs.shape[0] > 0)
+    def portions_by_tiles(self, ctx, longest: int = 2) -> bool:
+        """
+        Whether the step holds prompt portions (a bare context may not list them), the longest of at least `longest` tokens,
+        which then go sixteen tokens at a time.  A replayed step is judged by the bound its grids are sized by.
+        """
+        portions = getattr(ctx, "prefill_seqs", None)
+        return bool(self.recurrence_tiles and getattr(ctx, "max_q_len", 0) >= longest and portions is not None and portions.shape[0] > 0)
 
-    def _tile_buffers(self, ctx, T: int, qk_heads: int, heads: int, dim: int, device, sets: int = 1) -> tuple[torch.Tensor, torch.Tensor]:
-        seqs = ctx.cu_q.shape[0] - 1
-        floats = (int(self.lib.ts_recurrence_tiles_pack_floats(T, seqs, qk_heads, dim, sets)),
-                  int(self.lib.ts_recurrence_tiles_coef_floats(T, seqs, heads)))
-        return tuple(torch.empty((n,), dtype=torch.float32, device=device) for n in floats)
+    def _tile_buffers(self, ctx, T: int, qk_heads: int, heads: int, dim: int, device, sets: int = 1) -> tuple[torch.Tensor, int, int]:
+        """A buffer for packs and coefficients, and where in it both begin (addresses)."""
+        key = (qk_heads, heads, dim, sets)
+        floats = self._tile_floats.get(key)
+        if floats is None:                                   # of one tile, both multiples of four
+            floats = self._tile_floats[key] = (int(self.lib.ts_recurrence_tiles_pack_floats(0, 0, qk_heads, dim, sets)),
+                                               int(self.lib.ts_recurrence_tiles_coef_floats(0, 0, heads)))
+        slots = T // 16 + ctx.cu_q.shape[0]                  # as the kernels number them: a request's first tile at cu_q / 16 + its index
+        buffer = torch.empty((slots * (floats[0] + floats[1]),), dtype=torch.float32, device=device)
+        return buffer, buffer.data_ptr(), buffer.data_ptr() + 4 * slots * floats[0]
 
     def delta_tiles(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gates: torch.Tensor, dt_bias: torch.Tensor,
                     a_log: torch.Tensor, ctx, binding, *, heads: int, kv_heads: int, dim: int, vdim: int, unit_eps: float,
@@ -1130,11 +1139,11 @@ class Ops:
         if tuple(gates.shape) != (T, 2 * heads) or dt_bias.numel() != heads or a_log.numel() != heads:
             raise KernelError("delta_tiles: gates [T, 2 heads] and a bias and a rate a head are needed")
         state, stride = self._state_floats(binding, heads * dim * vdim, "delta_tiles")
-        pack, coef = self._tile_buffers(ctx, T, kv_heads, heads, dim, q.device)
+        buffer, pack, coef = self._tile_buffers(ctx, T, kv_heads, heads, dim, q.device)
         out = torch.empty((T, heads * vdim), dtype=torch.float32, device=q.device)
         self._call("ts_delta_tiles", _ptr(q), _ptr(k), q.stride(0), _ptr(gates), _ptr(dt_bias), _ptr(a_log), _ptr(v), v.stride(0),
                    _ptr(ctx.cu_q), _ptr(binding.state_slots), _ptr(ctx.prefill_seqs), ctx.prefill_seqs.shape[0], ctx.max_q_len,
-                   state.data_ptr(), stride, _ptr(pack), _ptr(coef), _ptr(out), heads, kv_heads, dim, vdim, unit_eps, q_scale, _stream())
+                   state.data_ptr(), stride, pack, coef, _ptr(out), heads, kv_heads, dim, vdim, unit_eps, q_scale, _stream())
         self.launches += 1                                   # what the columns of a tile share, then the scan
         return out
 
@@ -1156,11 +1165,11 @@ class Ops:
         if dt_bias.numel() != heads * dim or a_log.numel() != heads:
             raise KernelError("channel_tiles: a bias a channel and a rate a head are needed")
         state, stride = self._state_floats(binding, heads * dim * vdim, "channel_tiles")
-        pack, coef = self._tile_buffers(ctx, T, heads, heads, dim, q.device, sets=2)
+        buffer, pack, coef = self._tile_buffers(ctx, T, heads, heads, dim, q.device, sets=2)
         out = torch.empty((T, heads * vdim), dtype=torch.float32, device=q.device)
         self._call("ts_channel_tiles", _ptr(q), _ptr(k), q.stride(0), _ptr(z), _ptr(b), b.stride(0), _DTYPE_CODE[b.dtype], _ptr(dt_bias),
                    _ptr(a_log), _ptr(v), v.stride(0), _ptr(ctx.cu_q), _ptr(binding.state_slots), _ptr(ctx.prefill_seqs),
-                   ctx.prefill_seqs.shape[0], ctx.max_q_len, state.data_ptr(), stride, _ptr(pack), _ptr(coef), _ptr(out), heads,
+                   ctx.prefill_seqs.shape[0], ctx.max_q_len, state.data_ptr(), stride, pack, coef, _ptr(out), heads,
                    kv_heads, dim, vdim, unit_eps, q_scale, _stream())
         self.launches += 1                                   # what the columns of a tile share, then the scan
         return out
@@ -1180,11 +1189,11 @@ class Ops:
         if tuple(z.shape) != (T, heads * dim) or w0.numel() != heads * dim or u.numel() != heads * dim:
             raise KernelError("mix_tiles: decay logits [T, heads * dim], w0 and u [heads * dim] are needed")
         state, stride = self._state_floats(binding, heads * dim * dim, "mix_tiles")
-        pack, coef = self._tile_buffers(ctx, T, heads, heads, dim, r.device)
+        buffer, pack, coef = self._tile_buffers(ctx, T, heads, heads, dim, r.device)
         out = torch.empty((T, heads * dim), dtype=torch.float32, device=r.device)
         self._call("ts_mix_tiles", _ptr(r), _ptr(k), r.stride(0), _ptr(z), _ptr(w0), _ptr(u), _ptr(v), v.stride(0), _ptr(ctx.cu_q),
                    _ptr(binding.state_slots), _ptr(ctx.prefill_seqs), ctx.prefill_seqs.shape[0], ctx.max_q_len, state.data_ptr(),
-                   stride, _ptr(pack), _ptr(coef), _ptr(out), heads, dim, _DTYPE_CODE[r.dtype], _stream())
+                   stride, pack, coef, _ptr(out), heads, dim, _DTYPE_CODE[r.dtype], _stream())
         self.launches += 1
         return out
 

@@ -32,6 +32,10 @@ from tinyserve_llm_b200.parts.base import Mixer, Runtime, TensorDecl, register_p
 from tinyserve_llm_b200.parts.linear import Linear, fuse_rows
 
 MAX_KEY_DIM = 256       # csrc/linear_recurrence.cu
+# The same line for the delta rule with a decay a channel (parts/recurrence.py), whose walk waits for more.  A layer of 8 heads of 128
+# channels, captured, us, walk and tiles: one portion of 64 tokens 52 / 58, 100 63 / 65, 145 73 / 70, 256 98 / 80; two of 100 67 / 66, of
+# 145 80 / 72; four of 64 65 / 64; 4 heads: four of 64 56 / 61, of 145 80 / 73.
+CHANNEL_TILE_TOKENS = 144
 
 
 @register_part("mixer", "gated_delta_rule")
@@ -135,7 +139,7 @@ class GatedDeltaRule(Mixer):
         else:
             z = self.decay_up(y[:, C:C + self.decay_rank].contiguous(), out_dtype=torch.float32)  # decay logits, float32 from here on
             # float32 activations token by token (as in parts/recurrence.py)
-            o, tiles = None, x.dtype != torch.float32 and ops.portions_by_tiles(ctx)
+            o, tiles = None, x.dtype != torch.float32 and ops.portions_by_tiles(ctx, CHANNEL_TILE_TOKENS)
             if tiles:
                 o = ops.channel_tiles(q, k, v, z, b, self.dt_bias, self.a_log, ctx, matrices, vdim=V, **sizes)
             if not tiles or ctx.min_q_len <= 1:
