@@ -346,3 +346,17 @@ def test_every_tile_of_a_step_has_room_in_the_buffer():
             end = begin // 16 + s + -(-n // 16)
             begin += n
         assert end <= begin // 16 + len(lens) + 1
+
+
+@pytest.mark.parametrize("kind", ["plain", "delta"])
+def test_a_context_that_does_not_say_its_shortest_request(kind):
+    part, x = _recurrence_part(kind, torch.bfloat16)
+    lens, results = [300, 1], []
+    for bare in (False, True):
+        ctx = make_ctx(lens, lens)
+        ctx.prefill_seqs = i32([0])
+        if bare:
+            del ctx.min_q_len
+        state = torch.zeros(2, part.state_bytes(), dtype=torch.uint8, device="cuda")
+        results.append(part.forward(x[:301], ctx, EntryBinding(None, None, 0, 0, 16, 0, state=state, state_slots=i32([0, 1]))))
+    assert torch.equal(*results)

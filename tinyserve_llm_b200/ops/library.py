@@ -614,7 +614,7 @@ class Ops:
                        ctx.prefill_seqs.shape[0], ctx.max_q_len, state.data_ptr(), state.stride(0) // 4, pack, coef,
                        _ptr(out), heads, dim, vdim, _DTYPE_CODE[q.dtype], _stream())
             self.launches += 1                               # what the columns of a tile share, then the scan
-            if ctx.min_q_len > 1:
+            if getattr(ctx, "min_q_len", 1) > 1:             # a bare context may not say: single tokens are then looked for
                 return out
         prepared = torch.empty((3, T, heads * dim), dtype=torch.float32, device=q.device)   # q, k, decays as they enter the scan
         self._call("ts_linear_recurrence", _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(z),
