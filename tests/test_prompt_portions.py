@@ -360,3 +360,25 @@ def test_a_context_that_does_not_say_its_shortest_request(kind):
         state = torch.zeros(2, part.state_bytes(), dtype=torch.uint8, device="cuda")
         results.append(part.forward(x[:301], ctx, EntryBinding(None, None, 0, 0, 16, 0, state=state, state_slots=i32([0, 1]))))
     assert torch.equal(*results)
+
+
+@pytest.mark.parametrize("kind", ["plain", "delta"])
+def test_beside_tiles_only_single_tokens_are_prepared(kind, monkeypatch):
+    """What the walk reads is written for the single tokens of the step and for no others (every new tensor begins as sevens)."""
+    part, x = _recurrence_part(kind, torch.bfloat16)
+    lens, made, empty = [300, 1, 40, 1], [], torch.empty
+    ctx = make_ctx(lens, lens)
+    ctx.prefill_seqs = i32([0, 2])
+    state = torch.zeros(4, part.state_bytes(), dtype=torch.uint8, device="cuda")
+
+    def sevens(*args, **kwargs):
+        t = empty(*args, **kwargs)
+        made.append(t.fill_(7) if t.is_floating_point() else t)
+        return t
+
+    monkeypatch.setattr(torch, "empty", sevens)
+    part.forward(x[:342], ctx, EntryBinding(None, None, 0, 0, 16, 0, state=state, state_slots=i32([0, 1, 2, 3])))
+    monkeypatch.undo()
+    prepared, = [t for t in made if t.dim() == 3 and t.shape[:2] == (3, 342)]
+    written = (prepared != 7).any(dim=2).all(dim=0)
+    assert written.nonzero().flatten().tolist() == [300, 341]

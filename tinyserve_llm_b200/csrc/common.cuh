@@ -147,3 +147,10 @@ struct KVGeometry {
     int page_tokens;
     int num_pages;
 };
+
+// With `single_of` (the request of every token): whether the token's request feeds it alone (a padding row does not).
+__device__ __forceinline__ bool feeds_one(const int* single_of, const int* cu_q, long long t) {
+    if (!single_of) return true;
+    const int seq = single_of[t];
+    return seq >= 0 && cu_q[seq + 1] - cu_q[seq] == 1;
+}

@@ -45,16 +45,19 @@ __device__ __forceinline__ float log_sigmoid(float x) { return fminf(x, 0.f) - l
 
 // What enters the recurrence, computed once per token, head and key channel (the scan's CTAs of one head all read it):
 // prepared[0] = rotated, scaled q; prepared[1] = rotated, scaled k; prepared[2] = the decay a.  Each [tokens, heads * dim].
+// `single_of` (optional): only tokens of requests that feed one are prepared.
 template <typename T>
 __global__ void recurrence_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, long long q_stride,
                                           long long k_stride, const float* __restrict__ z, long long z_stride,
                                           const float* __restrict__ bias, const float* __restrict__ head_decay,
                                           float inv_tau, float q_scale, float k_scale, const float* __restrict__ freq,
                                           int rot_dims, const int* __restrict__ positions, float* __restrict__ prepared,
-                                          long long total, int heads, int dim) {
+                                          long long total, int heads, int dim, const int* __restrict__ single_of,
+                                          const int* __restrict__ cu_q) {
     const int width = heads * dim, half = rot_dims / 2;
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
         const long long t = e / width;
+        if (!feeds_one(single_of, cu_q, t)) continue;
         const int c = (int)(e % width), h = c / dim, i = c % dim;
         const T* qr = q + t * q_stride + (long long)h * dim;
         const T* kr = k + t * k_stride + (long long)h * dim;
@@ -355,13 +358,13 @@ TS_API int ts_recurrence_scan(const float* qk, int qk_group, const float* decay,
     return ts_fail("recurrence_scan: unknown dtype code %d", v_dtype);
 }
 
-// `singles` 1: only requests that feed one token are walked (prompt portions: recurrence_tiles.cu).
+// `singles` 1: only requests that feed one token are walked (prompt portions: recurrence_tiles.cu), and with `seq_of_token` prepared.
 TS_API int ts_linear_recurrence(const void* q, const void* k, const void* v, long long q_stride, long long k_stride,
                                 long long v_stride, const float* z, long long z_stride, const float* bias,
                                 const float* head_decay, float inv_tau, float q_scale, float k_scale, const float* freq,
                                 int rot_dims, const int* positions, const int* cu_q, const int* slots, int num_seqs,
                                 float* state, long long slot_stride, float* out, int heads, int dim, int vdim,
-                                int num_tokens, float* prepared, int singles, int dtype, cudaStream_t stream) {
+                                int num_tokens, float* prepared, int singles, const int* seq_of_token, int dtype, cudaStream_t stream) {
     TS_REQUIRE(heads > 0 && dim > 0 && vdim > 0 && num_seqs >= 0 && num_tokens >= 0, "linear_recurrence: bad sizes");
     TS_REQUIRE(dim <= 16 * LR_ROWGROUPS, "linear_recurrence: %d key channels a head are not supported (up to %d)", dim,
                16 * LR_ROWGROUPS);
@@ -375,13 +378,15 @@ TS_API int ts_linear_recurrence(const void* q, const void* k, const void* v, lon
     const long long total = (long long)num_tokens * heads * dim;
     const unsigned blocks = (unsigned)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
     const float* fr = rot_dims > 0 ? freq : nullptr;
+    const int* single_of = singles ? seq_of_token : nullptr;
     if (dtype == TS_F32)
         recurrence_prepare_kernel<float><<<blocks, 256, 0, stream>>>((const float*)q, (const float*)k, q_stride, k_stride, z,
-            z_stride, bias, head_decay, inv_tau, q_scale, k_scale, fr, rot_dims, positions, prepared, total, heads, dim);
+            z_stride, bias, head_decay, inv_tau, q_scale, k_scale, fr, rot_dims, positions, prepared, total, heads, dim,
+            single_of, cu_q);
     else if (dtype == TS_BF16)
         recurrence_prepare_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k,
             q_stride, k_stride, z, z_stride, bias, head_decay, inv_tau, q_scale, k_scale, fr, rot_dims, positions, prepared,
-            total, heads, dim);
+            total, heads, dim, single_of, cu_q);
     else
         return ts_fail("linear_recurrence: unknown dtype code %d", dtype);
     TS_LAUNCH_CHECK("linear_recurrence (prepare)");

@@ -30,11 +30,13 @@ __global__ void delta_prepare_kernel(const float* __restrict__ q, const float* _
                                      const float* __restrict__ z, const float* __restrict__ dt_bias,
                                      const float* __restrict__ a_log, const T* __restrict__ b, long long b_stride,
                                      float* __restrict__ prepared, float* __restrict__ beta, long long items, long long total,
-                                     int heads, int kv_heads, int dim, float unit_eps, float q_scale) {
+                                     int heads, int kv_heads, int dim, float unit_eps, float q_scale,
+                                     const int* __restrict__ single_of, const int* __restrict__ cu_q) {
     const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (item >= items) return;
     const int lane = threadIdx.x & 31;
     const long long t = item / heads;
+    if (!feeds_one(single_of, cu_q, t)) return;
     const int h = (int)(item % heads), g = h / (heads / kv_heads);
     const float* qr = q + t * qk_stride + (long long)g * dim;
     const float* kr = k + t * qk_stride + (long long)g * dim;
@@ -53,8 +55,8 @@ __global__ void delta_prepare_kernel(const float* __restrict__ q, const float* _
 
 TS_API int ts_delta_prepare(const float* q, const float* k, long long qk_stride, const float* z, const float* dt_bias,
                             const float* a_log, const void* b, long long b_stride, float* prepared, float* beta,
-                            int num_tokens, int heads, int kv_heads, int dim, float unit_eps, float q_scale, int dtype,
-                            cudaStream_t stream) {
+                            int num_tokens, int heads, int kv_heads, int dim, float unit_eps, float q_scale,
+                            const int* single_of, const int* cu_q, int dtype, cudaStream_t stream) {
     TS_REQUIRE(heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && dim > 0, "delta_prepare: %d heads over %d q/k heads",
                heads, kv_heads);
     if (num_tokens <= 0) return 0;
@@ -62,21 +64,14 @@ TS_API int ts_delta_prepare(const float* q, const float* k, long long qk_stride,
     const unsigned blocks = (unsigned)((items + 3) / 4);
     if (dtype == TS_F32)
         delta_prepare_kernel<float><<<blocks, 128, 0, stream>>>(q, k, qk_stride, z, dt_bias, a_log, (const float*)b, b_stride,
-            prepared, beta, items, total, heads, kv_heads, dim, unit_eps, q_scale);
+            prepared, beta, items, total, heads, kv_heads, dim, unit_eps, q_scale, single_of, cu_q);
     else if (dtype == TS_BF16)
         delta_prepare_kernel<__nv_bfloat16><<<blocks, 128, 0, stream>>>(q, k, qk_stride, z, dt_bias, a_log,
-            (const __nv_bfloat16*)b, b_stride, prepared, beta, items, total, heads, kv_heads, dim, unit_eps, q_scale);
+            (const __nv_bfloat16*)b, b_stride, prepared, beta, items, total, heads, kv_heads, dim, unit_eps, q_scale, single_of, cu_q);
     else
         return ts_fail("delta_prepare: unknown dtype code %d", dtype);
     TS_LAUNCH_CHECK("delta_prepare");
     return 0;
-}
-
-// With `single_of` (the request of every token): whether the token's request feeds it alone (a padding row does not).
-__device__ __forceinline__ bool feeds_one(const int* single_of, const int* cu_q, long long t) {
-    if (!single_of) return true;
-    const int seq = single_of[t];
-    return seq >= 0 && cu_q[seq + 1] - cu_q[seq] == 1;
 }
 
 // The same with one decay a head: one warp a (token, q/k head), which also takes its value heads' gates.  gates

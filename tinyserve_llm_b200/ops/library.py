@@ -61,7 +61,7 @@ _SIGNATURES = {
     "ts_skinny_linear_groups": ("int", "pppiiiillllip"),
     "ts_gemm_tcgen05_gated": ("int", "pppiiilliffpp"),
     "ts_stream_norm": ("int", "ppppppiifppifiippp" "pppff" "ppppill" "p"),
-    "ts_linear_recurrence": ("int", "ppplllplppfffpipppiplpiiiipiip"),
+    "ts_linear_recurrence": ("int", "ppplllplppfffpipppiplpiiiipi" "pip"),
     "ts_head_norm_gate": ("int", "piplpippliiififip"),
     "ts_latent_prepare": ("int", "pliiippfp" "f" "pppplliipiiiip"),
     "ts_latent_attention": ("int", "pllpliip" "fp" "plliipipp" "pii" "piiiifiiplip"),
@@ -98,7 +98,7 @@ _SIGNATURES = {
     "ts_mix_tiles": ("int", "pplppppl" "pppii" "plppp" "iiip"),
     "ts_plain_tiles": ("int", "ppplll" "plpp" "fffpip" "pppii" "plppp" "iiiip"),
     "ts_channel_tiles": ("int", "pplpplipp" "pl" "pppii" "plppp" "iiiiffp"),
-    "ts_delta_prepare": ("int", "pplppppl" "ppiiiiffip"),
+    "ts_delta_prepare": ("int", "pplppppl" "ppiiiiff" "ppip"),
     "ts_mlstm_prepare": ("int", "ppllpplppffppiplpppiiiip"),
     "ts_row_scaled_activation": ("int", "ppppiiiip"),
     "ts_difference_head_norm": ("int", "plipl" "piiii" "fffip"),
@@ -621,7 +621,7 @@ class Ops:
                    z.stride(0) if z is not None else 0, _ptr(bias), _ptr(head_decays), inv_tau, q_scale, k_scale,
                    _ptr(freq), rot, _ptr(ctx.positions), _ptr(ctx.cu_q), _ptr(binding.state_slots),
                    binding.state_slots.shape[0], state.data_ptr(), state.stride(0) // 4, _ptr(out), heads, dim, vdim,
-                   T, _ptr(prepared), 1 if tiles else 0, _DTYPE_CODE[q.dtype], _stream())
+                   T, _ptr(prepared), 1 if tiles else 0, _ptr(getattr(ctx, "seq_of_token", None)), _DTYPE_CODE[q.dtype], _stream())
         self.launches += 1                                   # the kernel that prepares the scan's inputs
         return out
 
@@ -1198,11 +1198,12 @@ class Ops:
         return out
 
     def delta_prepare(self, q: torch.Tensor, k: torch.Tensor, z: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor,
-                      b: torch.Tensor, *, heads: int, kv_heads: int, dim: int, unit_eps: float, q_scale: float):
+                      b: torch.Tensor, *, heads: int, kv_heads: int, dim: int, unit_eps: float, q_scale: float, singles=None):
         """
         (prepared [3, T, heads * dim], beta [T, heads]), float32, for the delta rule's scan: q, k (float32
         [T, kv_heads * dim] stretches with one row stride) as unit vectors per head, q scaled; decays
-        exp(-exp(a_log) softplus(z + dt_bias)); beta = sigmoid(b).
+        exp(-exp(a_log) softplus(z + dt_bias)); beta = sigmoid(b).  `singles` (a step context): only the rows of requests
+        that feed one token are prepared.
         """
         T = q.shape[0]
         for t, name, cols in ((q, "q", kv_heads * dim), (k, "k", kv_heads * dim)):
@@ -1217,6 +1218,7 @@ class Ops:
         beta = torch.empty((T, heads), dtype=torch.float32, device=q.device)
         self._call("ts_delta_prepare", _ptr(q), _ptr(k), q.stride(0), _ptr(z), _ptr(dt_bias), _ptr(a_log), _ptr(b),
                    b.stride(0), _ptr(prepared), _ptr(beta), T, heads, kv_heads, dim, unit_eps, q_scale,
+                   0 if singles is None else _ptr(singles.seq_of_token), 0 if singles is None else _ptr(singles.cu_q),
                    _DTYPE_CODE[b.dtype], _stream())
         return prepared, beta
 

@@ -143,7 +143,7 @@ class GatedDeltaRule(Mixer):
             if tiles:
                 o = ops.channel_tiles(q, k, v, z, b, self.dt_bias, self.a_log, ctx, matrices, vdim=V, **sizes)
             if not tiles or getattr(ctx, "min_q_len", 1) <= 1:
-                prepared, beta = ops.delta_prepare(q, k, z, self.dt_bias, self.a_log, b, **sizes)
+                prepared, beta = ops.delta_prepare(q, k, z, self.dt_bias, self.a_log, b, singles=ctx if tiles else None, **sizes)
                 o = ops.recurrence_scan(prepared, v, ctx, matrices, heads=H, dim=D, vdim=V, beta=beta, singles=tiles, out=o)
         return ops.head_norm_gate(o, gate, self.norm_weight, H, V, s.out_norm_eps, x.dtype,
                                   gate_kind="silu" if self.full_gate else "sigmoid", scale=scale, out=out)
