@@ -643,3 +643,63 @@ def test_latent_attention_of_portions_four_tokens_a_tile(heads, rank, rot, page,
     pool[table[s][j // page], 0, 0, j % page] = float("nan")
     again = run(portions)
     assert torch.equal(again[cu[s]:cu[s] + 41], got[cu[s]:cu[s] + 41]) and not bool(torch.isfinite(again[cu[s] + 41]).any())
+
+
+@pytest.mark.parametrize("heads, rank, rot, window, sink", [(16, 512, 64, 600, False), (5, 384, 32, 0, True), (17, 512, 64, 2, False), (16, 384, 0, 33, False)])
+def test_latent_attention_rows_do_not_depend_on_the_step(heads, rank, rot, window, sink):
+    """
+    A request that feeds one token takes the same kernel alone and beside a long portion; a long portion's rows are the same bits cut
+    anywhere, as long as the portions are those of the kernel of four tokens a CTA, and what 64 bits give.
+    """
+    from types import SimpleNamespace
+
+    from gpu_util import i32, make_ctx
+    from tinyserve_llm_b200.cache.storage import EntryBinding
+    from tinyserve_llm_b200.ops import get_ops
+    ops, g, width, dev, page = get_ops(), torch.Generator().manual_seed(3), rank + rot, "cuda", 64
+    least = 514 if window == 0 or window >= 512 else 1026               # tokens that the kernel takes, and one
+    n = 2 * least + 372
+    pages = -(-n // page)
+    pool = (torch.randn(2 * pages, 1, 1, page, width, generator=g) * 0.5).to(torch.bfloat16).to(dev)
+    table = [list(range(pages)), list(range(pages, 2 * pages))]
+    q_lat, q = torch.randn(n, heads, rank, generator=g).to(dev), torch.randn(n, heads * (4 + rot), generator=g).to(torch.bfloat16).to(dev)
+    freq = torch.tensor([100.0 ** (-2.0 * i / rot) for i in range(rot // 2)], dtype=torch.float32, device=dev) if rot else None
+    sinks = torch.linspace(-3, 3, heads, device=dev) if sink else None
+
+    def attend(rows, ctx, tables):
+        binding = EntryBinding(pool, None, page * width, 0, page, 2 * pages, i32(tables), pages, True)
+        return ops.latent_attention(q_lat[rows], q[rows], ctx, binding, heads, 4 + rot, 4, rank, rot, freq, 0.1, window, sink=sinks)
+
+    def run(rows, lens, ends):
+        return attend(rows, make_ctx(lens, ends), table[:len(lens)])
+
+    def by_fours(lens, ends):
+        return bool(ops.lib.ts_latent_attention_portions(sum(lens), len(lens), max(lens), heads, rank, rot, min(window, max(ends)) if window else max(ends)))
+
+    assert by_fours([n], [n]) and not by_fours([least - 2], [n]) and not by_fours([1] * n, [n] * n)
+    whole = run(torch.arange(n), [n], [n])
+    for cut in (least - 1, least + 186, least + 187, n - least):
+        assert by_fours([cut], [cut]) and by_fours([n - cut], [n])
+        assert torch.equal(run(torch.arange(cut), [cut], [cut]), whole[:cut])
+        assert torch.equal(run(torch.arange(cut, n), [n - cut], [n]), whole[cut:])
+    both = run(torch.arange(n), [n - 1, 1], [n - 1, n])                 # beside a single token: neither knows of the other
+    assert torch.equal(both[:n - 1], whole[:n - 1])
+    enough = torch.arange(n - 300, n)                                   # so many that none is split over CTAs
+    alone = attend(enough, SimpleNamespace(positions=i32([n - 1] * 300), seq_of_token=i32([0] * 300), max_ctx_len=n), [table[1]])
+    assert torch.equal(both[n - 1], alone[299])
+    keys = pool[:pages, 0, 0].reshape(-1, width)[:n].double()
+    for p in (0, 1, 2, 3, 4, 5, 32, 600, 601, 602, 603, n - 1):
+        seen = keys[max(0, p - window + 1) if window else 0:p + 1]
+        s = torch.einsum("hd,jd->hj", q_lat[p].double(), seen[:, :rank])
+        if rot:
+            part = q[p].double().view(heads, 4 + rot)[:, 4:].cpu()
+            s += torch.einsum("hr,jr->hj", plain.rotate_half(part[None], torch.tensor([p]), rot, 100.0)[0].to(dev), seen[:, rank:])
+        s = s * 0.1
+        if sink:
+            s = torch.cat([s, sinks.double()[:, None]], 1)
+        weights = torch.softmax(s, -1)[:, :seen.shape[0]]
+        want = weights @ seen[:, :rank]
+        assert float((whole[p].double() - want).norm() / want.norm()) < 4e-3, p      # the output's own rounding to bfloat16 is 1.6e-3
+    pool[601 // page, 0, 0, 601 % page] = float("nan")                  # a later token of the same four reaches no earlier one
+    again = run(torch.arange(n), [n], [n])
+    assert torch.equal(again[:601], whole[:601]) and not bool(torch.isfinite(again[601]).any())

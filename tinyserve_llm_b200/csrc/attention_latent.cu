@@ -12,14 +12,17 @@
 // ts_latent_prepare: per token, norms the query latent and the key/value latent (plain weights),
 // rotates the shared key part (rotate-half, angle = position * freq[i], float32) and stores [c | k_rot]
 // into the token's slot of the paged cache.
-// ts_latent_attention: bfloat16 with sizes it takes runs on the tensor-core kernel of attention_latent_mma.cu;
+// ts_latent_attention: bfloat16 with sizes it takes runs on the tensor-core kernels of attention_latent_mma.cu and, for the prompt
+// portions of steps that hold many such tokens, attention_latent_tokens.cu;
 // float32 and all other sizes here: one CTA per token and group of up to 8 heads (a warp a head).  Keys come in
 // tiles of 32 into shared memory as float32, shared by the heads; lane j scores key j of the tile, the
 // online softmax runs across the warp, and lane l accumulates channels l, l + 32, ... of the output.
 // A query at position p sees keys max(0, p - window + 1) .. p (window 0: all).  The order of every sum
 // depends on the query's position only.  In a step of few tokens (decoding) a token's keys are split over
 // several CTAs, 128 keys each counted from the window's first key, and a second kernel merges the
-// partial results in key order: again nothing depends on the rest of the batch.
+// partial results in key order: again nothing depends on the rest of the batch.  Only which of the two bfloat16 kernels takes a prompt
+// portion does (`ts_latent_attention_portions`): their sums have different orders, each of which follows from the token's position.  A
+// request that feeds one token takes the same kernel whatever stands beside it.
 // With `sink` (a number a head), exp(sink[h]) takes part in the sum of head h's softmax without a key or a value: it
 // is added once, where the output is divided by the sum (the merging kernel of a split step).
 #include "common.cuh"
@@ -28,8 +31,9 @@ bool ts_latent_mma_supported(int rank, int rot);
 int ts_latent_attention_mma_launch(const float* q_lat, long long ql_t, long long ql_h, const void* q, long long q_stride,
                                    int q_head_width, int q_rot_offset, const float* freq, float magnitude,
                                    const float* sink, const void* k_pool, KVGeometry geo, const int* block_table, int table_width, const int* positions,
-                                   const int* seq_of_token, void* out, int num_tokens, int heads, int rank, int rot,
-                                   float scale, int window, int split_keys, int splits, float* partial, cudaStream_t stream);
+                                   const int* seq_of_token, const int* singles_of, void* out, int num_tokens, int heads,
+                                   int rank, int rot, float scale, int window, int split_keys, int splits, float* partial,
+                                   cudaStream_t stream);
 
 constexpr int LA_WARPS = 8;
 constexpr int LA_KEYS = 32;
@@ -312,19 +316,12 @@ static int launch_latent(const float* q_lat, long long ql_t, long long ql_h, con
     return 0;
 }
 
-bool ts_latent_tokens_supported(int rank, int rot);
+bool ts_latent_tokens_supported(int rank, int rot);                  // attention_latent_tokens.cu
 int ts_latent_attention_tokens_launch(const float* q_lat, long long ql_t, long long ql_h, const void* q, long long q_stride,
                                       int q_head_width, int q_rot_offset, const float* freq, float magnitude, const float* sink,
                                       const void* k_pool, KVGeometry geo, const int* block_table, int table_width,
                                       const int* positions, const int* cu_q, int num_seqs, void* out, int num_tokens, int heads,
                                       int rank, int rot, float scale, int window, cudaStream_t stream);
-
-// Whether four tokens a CTA pay.  Such a CTA holds an SM by itself and takes as long as 1.5 rounds of two CTAs of a token each do
-// (183 against 122 us over windows of 1,024 keys), so the rounds decide.
-static bool tokens_pay(int num_tokens, int num_seqs, int heads) {
-    const long long groups = (heads + 15) / 16, tiles = ((long long)num_tokens / 4 + num_seqs) * groups, singles = num_tokens * groups;
-    return 3 * ((tiles + 147) / 148) < 2 * ((singles + 295) / 296);
-}
 
 // How many floats of scratch a call with these sizes needs (0: the step is large enough to run without splits).
 TS_API long long ts_latent_attention_scratch_floats(int num_tokens, int heads, int rank, int max_keys) {
@@ -334,11 +331,27 @@ TS_API long long ts_latent_attention_scratch_floats(int num_tokens, int heads, i
     return (long long)num_tokens * heads * splits * (rank + 2);
 }
 
+// Whether a step's prompt portions go four tokens a CTA: where a step has so many tokens of them and so many keys to see that one copy
+// of a key tile for four tokens is worth an SM held by one CTA.  Measured on a B200, us, one token a CTA and four, 16 heads, by window:
+//   latent 512   tokens          514         700         1,000       1,200       2,048       300, 300, 300
+//     128                                  69 / 73                 106 / 78    203 / 166     72 / 73
+//     1,024                   106 / 98    162 / 129   282 / 179   362 / 229   723 / 504    113 / 88
+//     none                                                        381 / 246   976 / 659
+//   384: 1,200 tokens, window 37 72 / 59, 1,024 303 / 195.   256: window 256 83 / 82, 1,024 189 / 161, but 2,048 tokens 137 / 160 and
+//   365 / 344, 37 59 / 75.   128: 1,024 109 / 126, 199 / 265; 37 32 / 61: two and more of those CTAs share an SM, and four of the others.
+// Fewer than 512 such tokens (300: 57 / 67) keep the other kernel, replayed steps among them.  384 channels and up; what is captured, small
+// or narrow stays as it was.
+TS_API int ts_latent_attention_portions(int num_tokens, int num_seqs, int max_q_len, int heads, int rank, int rot, int max_keys) {
+    return max_q_len > 1 && num_seqs > 0 && num_tokens - num_seqs >= (max_keys >= 512 ? 512 : 1024) && num_tokens <= 1 << 24 && heads <= 65535 && rank >= 384 &&
+           ts_latent_mma_supported(rank, rot) && ts_latent_tokens_supported(rank, rot) &&
+           ts_latent_attention_scratch_floats(num_tokens, heads, rank, max_keys) == 0;
+}
+
 TS_API int ts_latent_attention(const float* q_lat, long long ql_token_stride, long long ql_head_stride, const void* q,
                                long long q_stride, int q_head_width, int q_rot_offset, const float* freq,
                                float magnitude, const float* sink, const void* k_pool, long long page_stride, long long entry_offset, int page_tokens,
                                int num_pages, const int* block_table, int table_width, const int* positions,
-                               const int* seq_of_token, const int* cu_q, int num_seqs, int max_q_len, void* out, int num_tokens,
+                               const int* seq_of_token, const int* cu_q, int num_seqs, int min_q_len, int max_q_len, void* out, int num_tokens,
                                int heads, int rank, int rot, float scale, int window, int max_keys, float* scratch,
                                long long scratch_floats, int dtype, cudaStream_t stream) {
     TS_REQUIRE(num_tokens >= 0 && heads > 0 && rank > 0 && rot >= 0 && rot % 2 == 0, "latent_attention: bad sizes");
@@ -361,16 +374,20 @@ TS_API int ts_latent_attention(const float* q_lat, long long ql_token_stride, lo
     }
     if (dtype == TS_BF16 && ts_latent_mma_supported(rank, rot) && page_stride % 8 == 0 && entry_offset % 8 == 0 &&
         (uintptr_t)k_pool % 16 == 0) {
-        // prompt portions, where the context says which tokens are whose: four tokens a CTA
-        if (need == 0 && cu_q && num_seqs > 0 && max_q_len > 1 && num_tokens <= 1 << 24 && heads <= 65535 &&
-            tokens_pay(num_tokens, num_seqs, heads) && ts_latent_tokens_supported(rank, rot))
-            return ts_latent_attention_tokens_launch(q_lat, ql_token_stride, ql_head_stride, q, q_stride, q_head_width, q_rot_offset, freq,
-                                                     magnitude, sink, k_pool, geo, block_table, table_width, positions, cu_q, num_seqs,
-                                                     out, num_tokens, heads, rank, rot, scale, window, stream);
+        // prompt portions, where the context says which tokens are whose
+        const bool portions = cu_q && ts_latent_attention_portions(num_tokens, num_seqs, max_q_len, heads, rank, rot, max_keys);
+        if (portions) {
+            if (ts_latent_attention_tokens_launch(q_lat, ql_token_stride, ql_head_stride, q, q_stride, q_head_width, q_rot_offset, freq,
+                                                  magnitude, sink, k_pool, geo, block_table, table_width, positions, cu_q, num_seqs,
+                                                  out, num_tokens, heads, rank, rot, scale, window, stream))
+                return 1;
+            if (min_q_len > 1) return 0;
+        }
         // bfloat16 with sizes the tensor-core kernel takes: heads as the rows of mma.sync products
         if (ts_latent_attention_mma_launch(q_lat, ql_token_stride, ql_head_stride, q, q_stride, q_head_width, q_rot_offset,
-                                           freq, magnitude, sink, k_pool, geo, block_table, table_width, positions, seq_of_token, out,
-                                           num_tokens, heads, rank, rot, scale, window, split_keys, splits, scratch, stream))
+                                           freq, magnitude, sink, k_pool, geo, block_table, table_width, positions, seq_of_token,
+                                           portions ? cu_q : nullptr, out, num_tokens, heads, rank, rot, scale, window, split_keys, splits,
+                                           scratch, stream))
             return 1;
         if (split_keys > 0) {
             const long long items = (long long)num_tokens * heads;

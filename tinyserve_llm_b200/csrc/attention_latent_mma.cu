@@ -14,6 +14,7 @@
 // logits then differ from the float32 kernel's no more than that kernel's from the plain model (measured: the
 // largest error of a replay fell from 0.5 to 0.3 of its bound, for 15 % of the kernel's time).
 // A sink (a number a head) joins a head's sum where the output is divided by it.
+// With `singles_of` (the requests' first tokens) only requests that feed one token are taken.
 // A small step's keys may be split over CTAs exactly as in the FFMA kernel; the partial results have the
 // same form and the same kernel merges them.
 #include "common.cuh"
@@ -49,7 +50,8 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, long long ql_token_
                             const float* __restrict__ freq, float magnitude, const float* __restrict__ sink,
                             const __nv_bfloat16* __restrict__ k_pool, KVGeometry geo,
                             const int* __restrict__ block_table, int table_width, const int* __restrict__ positions,
-                            const int* __restrict__ seq_of_token, __nv_bfloat16* __restrict__ out, int heads, int rot,
+                            const int* __restrict__ seq_of_token, const int* __restrict__ singles_of,
+                            __nv_bfloat16* __restrict__ out, int heads, int rot,
                             float scale, int window, int split_keys, float* __restrict__ partial) {
     constexpr int RANK = 32 * NT;
     extern __shared__ __align__(16) unsigned char raw[];
@@ -64,7 +66,7 @@ latent_attention_mma_kernel(const float* __restrict__ q_lat, long long ql_token_
     long long* row_base = reinterpret_cast<long long*>(red + LM_WARPS * LM_HEADS);   // [64] element offset of a key's row, -1: none
     const int t = blockIdx.x;
     const int seq = seq_of_token[t];
-    if (seq < 0) return;
+    if (seq < 0 || (singles_of && singles_of[seq + 1] - singles_of[seq] > 1)) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int h0 = blockIdx.y * LM_HEADS;
     const int pos = positions[t];
@@ -279,8 +281,8 @@ bool ts_latent_mma_supported(int rank, int rot) {
 int ts_latent_attention_mma_launch(const float* q_lat, long long ql_t, long long ql_h, const void* q, long long q_stride,
                                    int q_head_width, int q_rot_offset, const float* freq, float magnitude,
                                    const float* sink, const void* k_pool, KVGeometry geo, const int* block_table, int table_width, const int* positions,
-                                   const int* seq_of_token, void* out, int num_tokens, int heads, int rank, int rot,
-                                   float scale, int window, int split_keys, int splits, float* partial,
+                                   const int* seq_of_token, const int* singles_of, void* out, int num_tokens, int heads,
+                                   int rank, int rot, float scale, int window, int split_keys, int splits, float* partial,
                                    cudaStream_t stream) {
     const int width = rank + rot, pitch = width + LM_PAD;
     const size_t smem = (size_t)(LM_HEADS + LM_KEYS) * pitch * 2 + (size_t)LM_HEADS * (rank + LM_PAD) * 2 +
@@ -293,7 +295,7 @@ int ts_latent_attention_mma_launch(const float* q_lat, long long ql_t, long long
             cudaFuncSetAttribute(latent_attention_mma_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
         latent_attention_mma_kernel<NT><<<grid, LM_WARPS * 32, smem, stream>>>(                                        \
             q_lat, ql_t, ql_h, (const __nv_bfloat16*)q, q_stride, q_head_width, q_rot_offset, freq, magnitude, sink,   \
-            (const __nv_bfloat16*)k_pool, geo, block_table, table_width, positions, seq_of_token, (__nv_bfloat16*)out, \
+            (const __nv_bfloat16*)k_pool, geo, block_table, table_width, positions, seq_of_token, singles_of, (__nv_bfloat16*)out, \
             heads, rot, scale, window, split_keys, partial);                                                           \
     } while (0)
     switch (rank / 32) {

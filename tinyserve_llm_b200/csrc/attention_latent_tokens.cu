@@ -1,6 +1,8 @@
 // Attention over a cached latent for prompt portions: the computation of attention_latent_mma.cu (mma.sync m16n8k16 on bfloat16
 // operands, the folded query's latent part and the probabilities each as the sum of two bfloat16 pieces, float32 softmax and
-// sums), four consecutive tokens of a request a CTA instead of one.
+// sums), four consecutive tokens of a request a CTA instead of one: those whose positions are the same but for their last two bits, so
+// that the order of a token's sums depends on its position only, wherever the portion was cut.  Requests that feed one token are left
+// to the other kernel.
 //
 // The tokens' windows overlap in all but three keys at either end, so a tile of keys is read from L2 once for 4 x 16 rows (token,
 // head) where it was read for 16.  Eight warps.  Scores: a warp takes one token's 16 heads and 16 of the tile's 32 keys.  Output: a
@@ -54,19 +56,23 @@ __global__ void __launch_bounds__(WARPS * 32, 1) latent_attention_tokens_kernel(
     float* corr_s = red + 2 * ROWS;                                       // [64]
     float2* turn = reinterpret_cast<float2*>(Ps);                         // [4][rot / 2] at first: cosines and sines (rot <= 256)
 
-    // request s's tiles begin at cu_q[s] / 4 + s, which leaves room for its last, partly filled one; the last ones, whose
-    // tokens see most, go first
+    // request s's tiles begin at cu_q[s] / 4 + 2 s, which leaves room for its first and last, partly filled ones; the last
+    // ones, whose tokens see most, go first
     const int tile_at = gridDim.x - 1 - blockIdx.x;
     int seq = 0;
     for (int step = p.steps; step > 0; step >>= 1)
-        if (seq + step < p.num_seqs && p.cu_q[seq + step] / TOKENS + seq + step <= tile_at) seq += step;
-    const int begin = p.cu_q[seq], t0 = begin + (tile_at - begin / TOKENS - seq) * TOKENS;
-    const int tokens = min(TOKENS, p.cu_q[seq + 1] - t0);
+        if (seq + step < p.num_seqs && p.cu_q[seq + step] / TOKENS + 2 * (seq + step) <= tile_at) seq += step;
+    const int begin = p.cu_q[seq], n = p.cu_q[seq + 1] - begin;
+    if (n <= 1) return;
+    const int start = p.positions[begin], last = start + n - 1;
+    // the run's positions, pos0 .. pos1, of which the portion may hold the middle or one end: first .. first + tokens - 1
+    const int pos0 = (start / TOKENS + tile_at - begin / TOKENS - 2 * seq) * TOKENS, pos1 = pos0 + TOKENS - 1;
+    const int first = max(pos0, start), t0 = begin + first - start, tokens = min(pos1, last) - first + 1;
     if (tokens <= 0) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int h0 = blockIdx.y * HEADS, pos0 = p.positions[t0], pos1 = pos0 + tokens - 1;
+    const int h0 = blockIdx.y * HEADS;
     const int lo0 = p.window > 0 ? max(0, pos0 - p.window + 1) : 0, lo1 = p.window > 0 ? max(0, pos1 - p.window + 1) : 0;
-    // keys all tokens see, and the others: below lo1 and above pos0 (a window shorter than the run: there is no key in between)
+    // keys all of the run see, and the others: below lo1 and above pos0 (a window shorter than the run: there is no key in between)
     const int body0 = min(lo1, pos0 + 1), body = pos0 + 1 - body0, edges = (body0 - lo0) + (pos1 - pos0);
     const int tiles = (body + KEYS - 1) / KEYS, first_tile = edges > 0 ? -1 : 0;
     auto edge_key = [&](int e) { return e < body0 - lo0 ? lo0 + e : pos0 + 1 + e - (body0 - lo0); };
@@ -77,7 +83,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) latent_attention_tokens_kernel(
             const bool any = tile < 0 ? tid < edges : tile * KEYS + tid < body;
             const int j = tile < 0 ? edge_key(tid) : body0 + tile * KEYS + tid;
             long long base = -1;
-            if (any) {
+            if (any && j <= last) {                  // a key behind the portion's end may lie past the table
                 const int page = table[j / p.geo.page_tokens];
                 if (page >= 0 && page < p.geo.num_pages)
                     base = (long long)page * p.geo.page_stride + p.geo.entry_offset + (long long)(j % p.geo.page_tokens) * width;
@@ -100,7 +106,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) latent_attention_tokens_kernel(
     const int half = p.rot / 2;
     for (int e = tid; e < TOKENS * half; e += THREADS) {
         float sn, cs;
-        sincosf((float)(pos0 + e / half) * p.freq[e % half], &sn, &cs);
+        sincosf((float)(first + e / half) * p.freq[e % half], &sn, &cs);
         turn[e] = make_float2(cs * p.magnitude, sn * p.magnitude);
     }
     __syncthreads();
@@ -188,7 +194,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) latent_attention_tokens_kernel(
                 mma_bf16(s[1], a, b[2], b[3]);
             }
             // thread: rows `row` (c 0, 1) and `row + 8` (c 2, 3); keys 16 side + 8 i + 2 quad + {0, 1}
-            const int pos = pos0 + mine, lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
+            const int pos = first + mine, lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
             float top[2] = {-INFINITY, -INFINITY};
 #pragma unroll
             for (int i = 0; i < 2; ++i)
@@ -349,7 +355,7 @@ int ts_latent_attention_tokens_launch(const float* q_lat, long long ql_t, long l
     const LatentArgs p{q_lat, ql_t, ql_h, (const __nv_bfloat16*)q, q_stride, q_head_width, q_rot_offset, freq, magnitude, sink,
                        (const __nv_bfloat16*)k_pool, geo, block_table, table_width, positions, cu_q, num_seqs, steps, (__nv_bfloat16*)out,
                        heads, rot, scale, window, wide};
-    const dim3 grid(num_tokens / TOKENS + num_seqs, (heads + HEADS - 1) / HEADS);
+    const dim3 grid(num_tokens / TOKENS + 2 * num_seqs, (heads + HEADS - 1) / HEADS);
     const size_t smem = latent_tokens_smem(rank, rot);
 #define TS_LATENT_TOKENS(NT)                                                                                                       \
     do {                                                                                                                           \

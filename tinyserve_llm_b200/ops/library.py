@@ -64,8 +64,9 @@ _SIGNATURES = {
     "ts_linear_recurrence": ("int", "ppplllplppfffpipppiplpiiiipi" "pip"),
     "ts_head_norm_gate": ("int", "piplpippliiififip"),
     "ts_latent_prepare": ("int", "pliiippfp" "f" "pppplliipiiiip"),
-    "ts_latent_attention": ("int", "pllpliip" "fp" "plliipipp" "pii" "piiiifiiplip"),
+    "ts_latent_attention": ("int", "pllpliip" "fp" "plliipipp" "piii" "piiiifiiplip"),
     "ts_latent_attention_scratch_floats": ("long long", "iiii"),
+    "ts_latent_attention_portions": ("int", "iiiiiii"),
     "ts_set_latent_mma": ("void", "i"),
     "ts_moe_route": ("int", "ppppppiiiip"),
     "ts_moe_route_few": ("int", "ppppppppiiiip"),
@@ -1404,7 +1405,7 @@ class Ops:
                    q_rot_offset, _ptr(freq), float(magnitude), _ptr(sink), _ptr(binding.k_pool), binding.page_stride, binding.entry_offset,
                    binding.page_tokens, binding.num_pages, _ptr(binding.block_table), binding.table_width,
                    _ptr(ctx.positions), _ptr(ctx.seq_of_token), _ptr(cu_q), cu_q.shape[0] - 1 if cu_q is not None else 0,
-                   int(getattr(ctx, "max_q_len", 0) or 0), _ptr(out), q.shape[0], heads, rank, rot, scale, window,
+                   int(getattr(ctx, "min_q_len", 0) or 0), int(getattr(ctx, "max_q_len", 0) or 0), _ptr(out), q.shape[0], heads, rank, rot, scale, window,
                    max_keys, _ptr(scratch), floats, _DTYPE_CODE[q.dtype], _stream())
         if floats:
             self.launches += 1                               # the kernel that merges the splits
