@@ -13,6 +13,11 @@
 // hide both; a step of a few rows the serial walk over its key tiles.  Measured on a B200, 32:8 heads of 64, us, before (one warp a
 // token and head, every key row read from L2 by each) and now: 512 tokens 598 / 61; 600 tokens 819 / 76; 4 portions of up to 150
 // behind up to 400 467 / 54; 64 tokens behind 4,000 1,114 / 290; 8 single tokens behind 2,000 163 / 157; one behind 400 42 / 38.
+// Taken are heads of 64 and 128 channels in groups of two and more.  Both sides over other sizes: heads of 16 and 32 have forms of
+// their own in the generic kernel (8 single tokens behind 2,000, 32:8 heads of 32: 108 / 157), heads between would be padded (32:8 of 80:
+// 171 / 260; of 112, 32:4: 209 / 255), and a group of one leaves fifteen of a single token's sixteen rows empty (64 single
+// tokens behind 500, 16:16 heads of 128: 163 / 261; 32 behind 150, 32:32 of 64: 32 / 43).  With groups of two nothing was slower
+// (16:8 heads of 64, 8 single tokens behind 2,000: 157 / 149, 512 tokens 323 / 47; of 128 426 / 252 and 654 / 81).
 #include <type_traits>
 
 #include "common.cuh"
@@ -36,7 +41,7 @@ struct Args {
     KVGeometry geo;
     const int* block_table; int table_width;
     const int* positions; const int* cu_q;
-    int num_seqs, steps, nh, nkv, hd, window;          // steps: the largest power of two up to num_seqs
+    int num_seqs, steps, nh, nkv, window;              // steps: the largest power of two up to num_seqs
     float scale;
 };
 
@@ -65,8 +70,8 @@ __global__ void __launch_bounds__(BQ * 4) paged_attention_f32_kernel(Args p) {
     for (int e = tid; e < BQ * (HD / 4); e += THREADS) {
         const int r = e / (HD / 4), d = e % (HD / 4) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < rows && d < p.hd)
-            v = *reinterpret_cast<const float4*>(p.q + (t0 + r / group) * p.q_stride + (long long)(kvh * group + r % group) * p.hd + d);
+        if (r < rows)
+            v = *reinterpret_cast<const float4*>(p.q + (t0 + r / group) * p.q_stride + (long long)(kvh * group + r % group) * HD + d);
         *reinterpret_cast<float4*>(qs + r * PITCH + d) = make_float4(v.x * p.scale, v.y * p.scale, v.z * p.scale, v.w * p.scale);
     }
     for (int r = tid; r < BQ; r += THREADS) {
@@ -78,21 +83,20 @@ __global__ void __launch_bounds__(BQ * 4) paged_attention_f32_kernel(Args p) {
     const int from = first_key[0] / BK, to = last_key[rows - 1] / BK;                 // positions rise along a run
     const int* table = p.block_table + (long long)seq * p.table_width;
     const int keys_end = last_key[rows - 1] + 1;
-    const long long head_off = p.geo.entry_offset + (long long)kvh * p.geo.page_tokens * p.hd;
+    const long long head_off = p.geo.entry_offset + (long long)kvh * p.geo.page_tokens * HD;
     // Where a tile's keys lie, looked up a tile ahead; -1: a page given back or a bad table, and the key is not seen.
     auto locate = [&](int tile) {
         for (int r = tid; r < BK; r += THREADS) {
             const int j = tile * BK + r, page = j < keys_end ? table[j / p.geo.page_tokens] : -1;
             key_at[tile & 1][r] = page >= 0 && page < p.geo.num_pages
-                                      ? (long long)page * p.geo.page_stride + head_off + (long long)(j % p.geo.page_tokens) * p.hd : -1;
+                                      ? (long long)page * p.geo.page_stride + head_off + (long long)(j % p.geo.page_tokens) * HD : -1;
         }
     };
     auto load = [&](float* dst, const float* pool, int tile) {
         for (int e = tid; e < BK * (HD / 4); e += THREADS) {
             const int r = e / (HD / 4), d = e % (HD / 4) * 4;
             const long long at = key_at[tile & 1][r];
-            const bool ok = at >= 0 && d < p.hd;
-            cp16(dst + r * PITCH + d, ok ? pool + at + d : pool, ok);
+            cp16(dst + r * PITCH + d, at >= 0 ? pool + at + d : pool, at >= 0);
         }
         commit();
     };
@@ -212,13 +216,10 @@ __global__ void __launch_bounds__(BQ * 4) paged_attention_f32_kernel(Args p) {
         const int r = ty * 4 + i;
         if (r >= rows) continue;
         const float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
-        float* out = p.out + ((long long)(t0 + r / group) * p.nh + kvh * group + r % group) * p.hd;
+        float* out = p.out + ((long long)(t0 + r / group) * p.nh + kvh * group + r % group) * HD;
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            const int d = 64 * c + tx * 4;
-            if (d < p.hd)
-                *reinterpret_cast<float4*>(out + d) = make_float4(o[i][4 * c] * inv, o[i][4 * c + 1] * inv, o[i][4 * c + 2] * inv, o[i][4 * c + 3] * inv);
-        }
+        for (int c = 0; c < NC; ++c)
+            *reinterpret_cast<float4*>(out + 64 * c + tx * 4) = make_float4(o[i][4 * c] * inv, o[i][4 * c + 1] * inv, o[i][4 * c + 2] * inv, o[i][4 * c + 3] * inv);
     }
 }
 
@@ -236,11 +237,11 @@ int launch(const Args& p, int num_tokens, cudaStream_t stream) {
 
 }  // namespace
 
-// Whether these sizes and addresses are taken: 16-byte rows, heads of up to 128 channels, a group's heads inside a tile.  Which
+// Whether these sizes and addresses are taken: 16-byte rows, the sizes named above, a group's heads inside a tile.  Which
 // of the two kernels takes a model's attention follows from its sizes alone, so a row's result stays independent of its step.
 bool paged_attention_f32_supported(const void* q, long long q_stride, const void* out, const void* k_pool, const void* v_pool,
                                    const KVGeometry& geo, int nh, int nkv, int hd) {
-    return hd % 4 == 0 && hd <= 128 && nh / nkv <= 16 && nkv <= 65535 && q_stride % 4 == 0 && geo.page_stride % 4 == 0 && geo.entry_offset % 4 == 0 &&
+    return (hd == 64 || hd == 128) && nh / nkv >= 2 && nh / nkv <= 16 && nkv <= 65535 && q_stride % 4 == 0 && geo.page_stride % 4 == 0 && geo.entry_offset % 4 == 0 &&
            ((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_pool | (uintptr_t)v_pool) % 16 == 0;
 }
 
@@ -249,9 +250,9 @@ int paged_attention_f32(const float* q, long long q_stride, float* out, const fl
                         int num_tokens, int max_q_len, int nh, int nkv, int hd, float scale, int window, cudaStream_t stream) {
     int steps = 1;
     while (2 * steps <= num_seqs) steps *= 2;
-    const Args p{q, q_stride, out, k_pool, v_pool, geo, block_table, table_width, positions, cu_q, num_seqs, steps, nh, nkv, hd, window, scale};
+    const Args p{q, q_stride, out, k_pool, v_pool, geo, block_table, table_width, positions, cu_q, num_seqs, steps, nh, nkv, window, scale};
     // 16 rows a CTA where every request feeds one token: its group's heads are all the rows there are.  Else 32, not 64: twice
     // the CTAs to share out (512 tokens, 32:8 heads of 64: 84 against 102 us before the tiles went longest first)
-    if (max_q_len <= 1) return hd <= 64 ? launch<64, 16>(p, num_tokens, stream) : launch<128, 16>(p, num_tokens, stream);
-    return hd <= 64 ? launch<64, 32>(p, num_tokens, stream) : launch<128, 32>(p, num_tokens, stream);
+    if (max_q_len <= 1) return hd == 64 ? launch<64, 16>(p, num_tokens, stream) : launch<128, 16>(p, num_tokens, stream);
+    return hd == 64 ? launch<64, 32>(p, num_tokens, stream) : launch<128, 32>(p, num_tokens, stream);
 }

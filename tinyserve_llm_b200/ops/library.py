@@ -419,8 +419,8 @@ class Ops:
                         window: int, generic: bool = False) -> torch.Tensor:
         """
         [T, nh * hd].  bfloat16 with head size 64 or 128 and pages of a multiple of 64 tokens runs on
-        the tensor-core kernels (prefill tiles and split-key decode), float32 on tiles of multiply-adds where the
-        step's context says which tokens are whose; everything else, and `generic=True`, on the generic kernel.
+        the tensor-core kernels (prefill tiles and split-key decode), float32 with head size 64 or 128 and groups of two
+        and more on tiles of multiply-adds where the step's context says which tokens are whose; everything else, and `generic=True`, on the generic kernel.
         """
         self._check(qkv, "qkv", tuple(_DTYPE_CODE), 2)
         out = torch.empty((qkv.shape[0], nh * hd), dtype=qkv.dtype, device=qkv.device)
