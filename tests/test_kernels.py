@@ -324,6 +324,22 @@ def test_float32_attention_tiles_do_not_depend_on_the_cut(ops, nh, nkv, hd, page
     assert torch.equal(run([n], [n])[:150], whole[:150])
 
 
+def test_float32_attention_of_more_tokens_than_a_grid_has_rows(ops):
+    """65,700 requests of one token, 16 heads over one key head: a tile a token, which goes to the generic kernel."""
+    import dataclasses
+    from types import SimpleNamespace
+    n, nh, hd, page = 65700, 16, 64, 16
+    binding = make_binding(4, 1, 1, page, hd, torch.float32, [[0, 1, 2, 3]])
+    fill_cache(binding, 0, rand((64, 1, hd), torch.float32, 3), rand((64, 1, hd), torch.float32, 4))
+    table = torch.stack([torch.arange(n) % 4], dim=1).to(torch.int32).to(DEV)
+    binding = dataclasses.replace(binding, block_table=table, table_width=1)
+    qkv = rand((n, 18 * hd), torch.float32, 5).to(DEV)
+    ctx = SimpleNamespace(positions=(torch.arange(n) % page).to(torch.int32).to(DEV), seq_of_token=torch.arange(n, dtype=torch.int32, device=DEV),
+                          cu_q=torch.arange(n + 1, dtype=torch.int32, device=DEV), max_q_len=1, min_q_len=1, max_ctx_len=page)
+    got = ops.paged_attention(qkv, ctx, binding, nh, 1, hd, 0.125, 0)
+    assert torch.equal(got, ops.paged_attention(qkv, ctx, binding, nh, 1, hd, 0.125, 0, generic=True))
+
+
 @pytest.mark.parametrize("hd, g", [(64, 4), (128, 3)])
 def test_tensor_core_attention_on_long_batches(ops, hd, g):
     """Decode over many splits (contexts up to 2,300 keys), prompts of several tiles, and a decode-only batch."""

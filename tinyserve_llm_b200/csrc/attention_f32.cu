@@ -223,26 +223,31 @@ __global__ void __launch_bounds__(BQ * 4) paged_attention_f32_kernel(Args p) {
     }
 }
 
+// Query rows a CTA: 16 where every request feeds one token, whose group's heads are all the rows there are.  Else 32, not 64: twice
+// the CTAs to share out (512 tokens, 32:8 heads of 64: 84 against 102 us before the tiles went longest first).
+int rows_of(int max_q_len) { return max_q_len <= 1 ? 16 : 32; }
+long long tiles_of(int num_tokens, int num_seqs, int group, int rows) { return (long long)num_tokens / (rows / group) + num_seqs; }
+
 template <int HD, int BQ>
 int launch(const Args& p, int num_tokens, cudaStream_t stream) {
     constexpr size_t smem = sizeof(float) * ((BQ + 2 * BK) * (HD + 4) + BQ * PP);
     auto kernel = paged_attention_f32_kernel<HD, BQ>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const dim3 grid(p.nkv, num_tokens / (BQ / (p.nh / p.nkv)) + p.num_seqs);
-    TS_REQUIRE(grid.y <= 65535, "paged_attention_f32: %d tokens are more than a grid holds", num_tokens);
-    kernel<<<grid, BQ * 4, smem, stream>>>(p);
+    kernel<<<dim3(p.nkv, (unsigned)tiles_of(num_tokens, p.num_seqs, p.nh / p.nkv, BQ)), BQ * 4, smem, stream>>>(p);
     TS_LAUNCH_CHECK("paged_attention_f32");
     return 0;
 }
 
 }  // namespace
 
-// Whether these sizes and addresses are taken: 16-byte rows, the sizes named above, a group's heads inside a tile.  Which
+// Whether these sizes and addresses are taken: 16-byte rows, the sizes named above, a group's heads inside a tile, no more tiles
+// than a grid holds (131,000 prompt tokens and more: so many have no steps of other sizes beside them).  Which
 // of the two kernels takes a model's attention follows from its sizes alone, so a row's result stays independent of its step.
 bool paged_attention_f32_supported(const void* q, long long q_stride, const void* out, const void* k_pool, const void* v_pool,
-                                   const KVGeometry& geo, int nh, int nkv, int hd) {
+                                   const KVGeometry& geo, int num_seqs, int num_tokens, int max_q_len, int nh, int nkv, int hd) {
     return (hd == 64 || hd == 128) && nh / nkv >= 2 && nh / nkv <= 16 && nkv <= 65535 && q_stride % 4 == 0 && geo.page_stride % 4 == 0 && geo.entry_offset % 4 == 0 &&
-           ((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_pool | (uintptr_t)v_pool) % 16 == 0;
+           ((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_pool | (uintptr_t)v_pool) % 16 == 0 &&
+           tiles_of(num_tokens, num_seqs, nh / nkv, rows_of(max_q_len)) <= 65535;
 }
 
 int paged_attention_f32(const float* q, long long q_stride, float* out, const float* k_pool, const float* v_pool, KVGeometry geo,
@@ -251,8 +256,6 @@ int paged_attention_f32(const float* q, long long q_stride, float* out, const fl
     int steps = 1;
     while (2 * steps <= num_seqs) steps *= 2;
     const Args p{q, q_stride, out, k_pool, v_pool, geo, block_table, table_width, positions, cu_q, num_seqs, steps, nh, nkv, window, scale};
-    // 16 rows a CTA where every request feeds one token: its group's heads are all the rows there are.  Else 32, not 64: twice
-    // the CTAs to share out (512 tokens, 32:8 heads of 64: 84 against 102 us before the tiles went longest first)
-    if (max_q_len <= 1) return hd == 64 ? launch<64, 16>(p, num_tokens, stream) : launch<128, 16>(p, num_tokens, stream);
+    if (rows_of(max_q_len) == 16) return hd == 64 ? launch<64, 16>(p, num_tokens, stream) : launch<128, 16>(p, num_tokens, stream);
     return hd == 64 ? launch<64, 32>(p, num_tokens, stream) : launch<128, 32>(p, num_tokens, stream);
 }

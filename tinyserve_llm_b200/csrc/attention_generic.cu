@@ -251,7 +251,7 @@ TS_API int ts_paged_attention_split(const void* q, long long q_stride, void* out
 }
 
 bool paged_attention_f32_supported(const void* q, long long q_stride, const void* out, const void* k_pool, const void* v_pool,
-                                   const KVGeometry& geo, int nh, int nkv, int hd);
+                                   const KVGeometry& geo, int num_seqs, int num_tokens, int max_q_len, int nh, int nkv, int hd);
 int paged_attention_f32(const float* q, long long q_stride, float* out, const float* k_pool, const float* v_pool, KVGeometry geo,
                         const int* block_table, int table_width, const int* positions, const int* cu_q, int num_seqs,
                         int num_tokens, int max_q_len, int nh, int nkv, int hd, float scale, int window, cudaStream_t stream);
@@ -268,7 +268,7 @@ TS_API int ts_paged_attention_generic(const void* qkv, void* out, const void* k_
     const long long q_stride = (long long)(nh + 2 * nkv) * hd;
     const KVGeometry geo{page_stride, entry_offset, page_tokens, num_pages};
     if (cu_q && num_seqs > 0 && dtype == TS_F32 && num_tokens > 0 && nkv > 0 && nh > 0 && nh % nkv == 0 && page_tokens > 0 && table_width > 0 && window >= 0 &&
-        paged_attention_f32_supported(qkv, q_stride, out, k_pool, v_pool, geo, nh, nkv, hd))
+        paged_attention_f32_supported(qkv, q_stride, out, k_pool, v_pool, geo, num_seqs, num_tokens, max_q_len, nh, nkv, hd))
         return paged_attention_f32((const float*)qkv, q_stride, (float*)out, (const float*)k_pool, (const float*)v_pool, geo, block_table,
                                    table_width, positions, cu_q, num_seqs, num_tokens, max_q_len, nh, nkv, hd, scale, window, stream);
     return ts_paged_attention_split(qkv, q_stride, out, k_pool, v_pool, page_stride, entry_offset,
