@@ -340,6 +340,27 @@ def test_float32_attention_of_more_tokens_than_a_grid_has_rows(ops):
     assert torch.equal(got, ops.paged_attention(qkv, ctx, binding, nh, 1, hd, 0.125, 0, generic=True))
 
 
+@pytest.mark.parametrize("nh, nkv, hd, lens", [(8, 2, 64, [70, 1]), (8, 2, 64, [1, 1, 1]), (6, 2, 32, [5, 1])])
+def test_float32_attention_leaves_no_padding_row_unwritten(ops, monkeypatch, nh, nkv, hd, lens):
+    """A step padded to 96 rows and 4 requests, as a replayed one is; every new tensor begins as NaNs."""
+    page, rows, ends = 16, 96, [90, 40, 7][:len(lens)]
+    tables, at = [], 0
+    for c in ends:
+        tables.append(list(range(at, at + -(-c // page))))
+        at += len(tables[-1])
+    binding = make_binding(at, 1, nkv, page, hd, torch.float32, tables + [[]] * (4 - len(lens)), poison=False)
+    ctx = make_ctx(lens, ends)
+    real = sum(lens)
+    pad = lambda t, size, value: torch.cat([t, torch.full((size - t.shape[0],), value, dtype=torch.int32, device=DEV)])
+    ctx.positions, ctx.seq_of_token, ctx.cu_q = pad(ctx.positions, rows, 0), pad(ctx.seq_of_token, rows, -1), pad(ctx.cu_q, 5, real)
+    qkv, empty = rand((rows, (nh + 2 * nkv) * hd), torch.float32, 5).to(DEV), torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: empty(*a, **k).fill_(math.nan) if k.get("dtype") == torch.float32 else empty(*a, **k))
+    got = [ops.paged_attention(qkv, ctx, binding, nh, nkv, hd, 0.125, 0, generic=generic) for generic in (False, True)]
+    monkeypatch.undo()
+    for out in got:
+        assert not out[real:].any() and torch.isfinite(out).all()
+
+
 @pytest.mark.parametrize("hd, g", [(64, 4), (128, 3)])
 def test_tensor_core_attention_on_long_batches(ops, hd, g):
     """Decode over many splits (contexts up to 2,300 keys), prompts of several tiles, and a decode-only batch."""

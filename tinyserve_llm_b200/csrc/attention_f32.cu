@@ -41,7 +41,7 @@ struct Args {
     KVGeometry geo;
     const int* block_table; int table_width;
     const int* positions; const int* cu_q;
-    int num_seqs, steps, nh, nkv, window;              // steps: the largest power of two up to num_seqs
+    int num_tokens, num_seqs, steps, nh, nkv, window;  // steps: the largest power of two up to num_seqs
     float scale;
 };
 
@@ -59,6 +59,9 @@ __global__ void __launch_bounds__(BQ * 4) paged_attention_f32_kernel(Args p) {
     // request s's tiles begin at cu_q[s] / per_tile + s, which leaves room for its last, partly filled one; the tiles with the
     // most keys before them go first
     const int tile_at = gridDim.y - 1 - blockIdx.y;
+    // padding rows behind the last request: zeros, so that nothing that reads them meets NaNs of someone else's memory
+    for (int t = p.cu_q[p.num_seqs] + tile_at; t < p.num_tokens; t += gridDim.y)
+        for (int d = threadIdx.x; d < group * HD; d += THREADS) p.out[((long long)t * p.nh + kvh * group) * HD + d] = 0.f;
     int seq = 0;
     for (int step = p.steps; step > 0; step >>= 1)
         if (seq + step < p.num_seqs && p.cu_q[seq + step] / per_tile + seq + step <= tile_at) seq += step;
@@ -255,7 +258,7 @@ int paged_attention_f32(const float* q, long long q_stride, float* out, const fl
                         int num_tokens, int max_q_len, int nh, int nkv, int hd, float scale, int window, cudaStream_t stream) {
     int steps = 1;
     while (2 * steps <= num_seqs) steps *= 2;
-    const Args p{q, q_stride, out, k_pool, v_pool, geo, block_table, table_width, positions, cu_q, num_seqs, steps, nh, nkv, window, scale};
+    const Args p{q, q_stride, out, k_pool, v_pool, geo, block_table, table_width, positions, cu_q, num_tokens, num_seqs, steps, nh, nkv, window, scale};
     if (rows_of(max_q_len) == 16) return hd == 64 ? launch<64, 16>(p, num_tokens, stream) : launch<128, 16>(p, num_tokens, stream);
     return hd == 64 ? launch<64, 32>(p, num_tokens, stream) : launch<128, 32>(p, num_tokens, stream);
 }

@@ -78,7 +78,13 @@ paged_attention_generic_kernel(const T* __restrict__ q, long long q_stride, T* _
     const int t = (int)(item / nh), h = (int)(item % nh);
     const int seq = seq_of_token[t];
     T* o_ptr = out + ((long long)t * nh + h) * vd;
-    if (seq < 0) return;                                      // padding row
+    if (seq < 0) {                                            // padding row: zeros, so that nothing that reads it meets NaNs of someone else's memory
+        for (int d = lane; d < vd; d += 32) {
+            if (extras.out_f32) reinterpret_cast<float*>(out)[((long long)t * nh + h) * vd + d] = 0.f;
+            else o_ptr[d] = from_float<T>(0.f);
+        }
+        return;
+    }
     const int pos = positions[t];
     const int kvh = h / (nh / nkv);
     const T* q_ptr = q + (long long)t * q_stride + (long long)h * hd;

@@ -256,17 +256,27 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                 if (failed) break;
                 float* y = p.y + it.segment * p.segment_stride + (long long)m_first * p.ldy + n;
                 const int k0 = (it.first + from) * BK, k1 = min(p.K, k0 + blocks * BK);
+                uint32_t odd = 0;
 #pragma unroll
                 for (int j = 0; j < OWN; ++j) {
                     if (n < p.N && m_first + j < p.M) {
-                        float v = sum[j];
-                        if (!isfinite(v)) {          // hi + lo does not stand for infinite or the largest numbers
-                            v = 0.f;
-                            for (int k = k0; k < k1; ++k) v = fmaf(p.x[(m_first + j) * p.ldx + k], p.w[n * p.ldw + k], v);
-                        }
-                        y[j * p.ldy] = from ? y[j * p.ldy] + v : v;
+                        if (isfinite(sum[j])) y[j * p.ldy] = from ? y[j * p.ldy] + sum[j] : sum[j];
+                        else odd |= 1u << j;         // hi + lo does not stand for infinite or the largest numbers
                     }
                     sum[j] = 0.f;
+                }
+                // Those again by multiply-adds.  A row of x with a NaN, which padding may be, gives NaN everywhere: one look tells.
+                for (int j = 0; j < OWN && __any_sync(0xffffffffu, odd >> j); ++j) {
+                    const bool mine = odd >> j & 1;
+                    if (!__any_sync(0xffffffffu, mine)) continue;
+                    const float* x = p.x + (m_first + j) * p.ldx;
+                    float v = 0.f;
+                    bool nan = false;
+                    for (int k = k0 + lane; k < k1; k += 32) nan |= x[k] != x[k];
+                    if (__any_sync(0xffffffffu, nan)) v = __uint_as_float(0x7fffffffu);
+                    else if (mine)
+                        for (int k = k0; k < k1; ++k) v = fmaf(x[k], p.w[n * p.ldw + k], v);
+                    if (mine) y[j * p.ldy] = from ? y[j * p.ldy] + v : v;
                 }
             }
         }
