@@ -188,8 +188,9 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         for (int at = blockIdx.x; at < p.items; at += gridDim.x) total += item_of(p, at, BX).count;
         for (int g = team; g < total; g += 2) {
             const int s = g % RING, a = g % PAIRS;
-            if (!mbar_wait(&raw_full_bar[s], (g / RING) & 1, p.error, 22) || failed) { failed = 1; break; }
-            if (!mbar_wait(&free_bar[a], ((g / PAIRS) & 1) ^ 1, p.error, 26)) { failed = 1; break; }
+            bool ok = mbar_wait(&raw_full_bar[s], (g / RING) & 1, p.error, 22) && !failed;
+            ok = ok && mbar_wait(&free_bar[a], ((g / PAIRS) & 1) ^ 1, p.error, 26);
+            if (!__all_sync(0xffffffffu, ok)) { failed = 1; break; }                  // what follows wants the whole warp
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const unsigned char* w_row = ring + s * RAW_BYTES + row * 128;            // 16-byte piece c lies at c ^ (row % 8)
 #pragma unroll
@@ -234,14 +235,16 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
 #pragma unroll
         for (int j = 0; j < OWN; ++j) sum[j] = 0.f;
         int sums = 0;
-        for (int at = blockIdx.x; at < p.items && !failed; at += gridDim.x) {
+        bool ok = true;                              // the same in all lanes
+        for (int at = blockIdx.x; at < p.items && ok; at += gridDim.x) {
             const Item it = item_of(p, at, BX);
             const int n = it.n0 + quarter * 32 + lane, m_first = it.m0 + side * OWN;
-            for (int from = 0; from < it.count && !failed; from += p.per_segment) {   // a segment
+            for (int from = 0; from < it.count && ok; from += p.per_segment) {        // a segment
                 const int blocks = min(p.per_segment, it.count - from);
                 for (int i = 0; i < blocks; i += SUM_BLOCKS, ++sums) {
                     const int b = sums % SUMS;
-                    if (!mbar_wait(&sum_full_bar[b], (sums / SUMS) & 1, p.error, 25) || failed) { failed = 1; break; }
+                    ok = __all_sync(0xffffffffu, mbar_wait(&sum_full_bar[b], (sums / SUMS) & 1, p.error, 25) && !failed);
+                    if (!ok) { failed = 1; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     uint32_t v[OWN];
 #pragma unroll
@@ -253,7 +256,7 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
 #pragma unroll
                     for (int j = 0; j < OWN; ++j) sum[j] += __uint_as_float(v[j]);
                 }
-                if (failed) break;
+                if (!ok) break;
                 float* y = p.y + it.segment * p.segment_stride + (long long)m_first * p.ldy + n;
                 const int k0 = (it.first + from) * BK, k1 = min(p.K, k0 + blocks * BK);
                 uint32_t odd = 0;
