@@ -141,6 +141,20 @@ def test_float32_matrix_product_on_split_operands(ops, m, n, k):
     ops.check_device_errors()
 
 
+@pytest.mark.parametrize("k", [4, 16, 32, 60, 64, 128, 2048])
+def test_float32_matrix_product_is_no_further_off_than_the_multiply_add_chain(ops, k):
+    """The chain takes weights that begin off a 16-byte boundary.  A row of one 1 gives short sums' weights as they are."""
+    x, w = rand((96, k), torch.float32, 5).to(DEV), rand((512, k), torch.float32, 6).to(DEV)
+    shifted = torch.empty(512 * k + 1, device=DEV)[1:].view(512, k).copy_(w)
+    want = x.double() @ w.double().T
+    split, chain = ((ops.linear(x, t).double() - want).norm() for t in (w, shifted))
+    assert bool(split <= chain)
+    if k < 64:
+        x = torch.zeros(3, k, device=DEV)
+        x[:, 1] = 1.0
+        assert torch.equal(ops.linear(x, w), w[:, 1].expand(3, -1))
+
+
 def test_float32_matrix_product_keeps_infinities_and_nans(ops):
     x, w = rand((40, 512), torch.float32, 5), rand((300, 512), torch.float32, 6)
     x[3, 5], x[9, 7], w[11, 100], w[12, 100] = math.inf, math.nan, -math.inf, 3e38

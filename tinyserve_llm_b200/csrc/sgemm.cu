@@ -1,6 +1,6 @@
 // float32 matrix product C[M, N] = A[M, K] . B[N, K]^T: the engine's true 32-bit projection (no tensor-core mode that
-// rounds its inputs).  A single product whose rows TMA takes runs in sgemm_tcgen05.cu, to the same accuracy; this file's
-// kernel, FFMA with float32 accumulation, takes the others and batches of products.  Each output element
+// rounds its inputs).  A single product of 64 terms and more whose rows TMA takes runs in sgemm_tcgen05.cu, no further from 64
+// bits; this file's kernel, FFMA with float32 accumulation, takes the others and batches of products.  Each output element
 // sums over k in ascending order, so a row's result does not depend on what else is in the batch.
 // Any M, N, K; rows of A and B are K-contiguous (the checkpoint's [out_features, in_features]).
 // A batched form runs one such product per blockIdx.z.
@@ -67,9 +67,9 @@ long long sgemm_tcgen05_scratch_floats(int M, int N, int K);
 int sgemm_tcgen05(const float* x, const float* w, float* y, int M, int N, int K, long long ldx, long long ldw, long long ldy,
                   float* scratch, int* error, cudaStream_t stream);
 
-// Floats of scratch `ts_sgemm_nt` may use (sgemm_tcgen05.cu).
+// Floats of scratch `ts_sgemm_nt` may use for rows without gaps (sgemm_tcgen05.cu).
 TS_API long long ts_sgemm_nt_scratch_floats(int M, int N, int K) {
-    return M > 0 && N > 0 && K > 0 ? sgemm_tcgen05_scratch_floats(M, N, K) : 0;
+    return M > 0 && N > 0 && sgemm_tcgen05_supported(nullptr, nullptr, K, K, K) ? sgemm_tcgen05_scratch_floats(M, N, K) : 0;
 }
 
 // On the tensor cores where TMA takes rows and addresses, whatever M is (a row's result must not depend on what else is in

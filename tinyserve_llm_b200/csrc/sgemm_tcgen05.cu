@@ -363,9 +363,14 @@ Shape choose(int M, int N, int blocks, int per_segment, int segments) {
 
 }  // namespace
 
-// 1 if TMA takes the sizes and addresses: 16-byte aligned bases and rows.
+// Terms from which on a sum of split products is no further from 64 bits than the multiply-add chain.  Below, what the split drops counts
+// for more than the chain's roundings (relative error, chain and here: 4 terms 4.0e-8 / 9.3e-8, 16 7.4e-8 / 1.0e-7, 32 1.03e-7 / 1.30e-7,
+// 48 1.25e-7 both, 64 1.43e-7 / 1.34e-7, 2,048 8.1e-7 / 1.5e-7).
+constexpr int MIN_TERMS = 64;
+
+// 1 if the sum is long enough and TMA takes the sizes and addresses: 16-byte aligned bases and rows.
 bool sgemm_tcgen05_supported(const float* x, const float* w, int K, long long ldx, long long ldw) {
-    return K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0;
+    return K >= MIN_TERMS && K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0;
 }
 
 // Floats of scratch a product of these sizes needs (0: none).
