@@ -4,7 +4,7 @@
 // of which the tensor cores drop the last bit: 2^-23 of v), and W x = W_hi x_hi + W_hi x_lo + W_lo x_hi in tcgen05.mma kind::tf32
 // with float32 accumulators; the small terms go first.  The tensor cores cut what an accumulator cannot hold, so they add up 32
 // terms of k only: a block's sum leaves tensor memory and is added to the running sum in registers by an ordinary rounded
-// addition.  Measured against 64-bit products: 1.9e-7 (2,048 terms) and 1.8e-7 (8,192), where the multiply-add chain of sgemm.cu is
+// addition (every second block's: 3 to 7 % faster, twice the error).  Measured against 64-bit products: 1.9e-7 (2,048 terms) and 1.8e-7 (8,192), where the multiply-add chain of sgemm.cu is
 // 8.0e-7 and 1.6e-6 off; 1.3e-7 against 1.5e-7 at 64 terms.  An element that comes out infinite or NaN (infinite inputs, for
 // which hi + lo does not stand, or an overflow) is worked out again by that chain, so such elements are what plain arithmetic gives.
 //
@@ -35,9 +35,6 @@ namespace {
 
 constexpr int BW = 128, BK = 32;                     // rows of W a tile; k a block: 128 bytes, one swizzled row
 constexpr int SPLIT_WARPS = 4, ADDERS_FROM = 2 + 2 * SPLIT_WARPS;    // two teams of split warps
-// Blocks of k the tensor cores add up before the sum goes to the registers.  2: 3 to 7 % faster, twice the error (3.8e-7 against
-// 1.9e-7 at 2,048 terms).
-constexpr int SUM_BLOCKS = 1;
 __host__ __device__ constexpr int share_of(int bx) { return bx >= 64 ? 4 : 2; }           // adder warps a quarter of the lanes
 __host__ __device__ constexpr int threads_of(int bx) { return 32 * (ADDERS_FROM + 4 * share_of(bx)); }
 constexpr int W_BYTES = BW * BK * 4;
@@ -155,29 +152,24 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     } else if (warp == 1 && lane == 0) {
         // float32 accumulator, TF32 operands, B K-major, 128 x BX
         const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(BX >> 3) << 17) | ((uint32_t)(BW >> 4) << 24);
-        int g = 0, sums = 0;
+        int g = 0;
         for (int at = blockIdx.x; at < p.items && !failed; at += gridDim.x) {
             const Item it = item_of(p, at, BX);
-            for (int i = 0, j = 0; i < it.count; ++i, ++g) {                          // j: the block's place in its segment
-                const int a = g % PAIRS, b = sums % SUMS;
-                const bool more = j % SUM_BLOCKS != 0;                                // the sum is begun already
-                if (!more && !mbar_wait(&sum_empty_bar[b], ((sums / SUMS) & 1) ^ 1, p.error, 24)) { failed = 1; break; }
+            for (int i = 0; i < it.count; ++i, ++g) {
+                const int a = g % PAIRS, b = g % SUMS;
+                if (!mbar_wait(&sum_empty_bar[b], ((g / SUMS) & 1) ^ 1, p.error, 24)) { failed = 1; break; }
                 if (!mbar_wait(&ready_bar[a], (g / PAIRS) & 1, p.error, 23)) { failed = 1; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t w_hi = tmem_base + A_COLS + a * 2 * BK, w_lo = w_hi + BK, d = tmem_base + b * BX;
                 const uint64_t x_hi = smem_desc(split + a * 2 * X_BYTES), x_lo = smem_desc(split + a * 2 * X_BYTES + X_BYTES);
 #pragma unroll
-                for (int k = 0; k < BK / 8; ++k) umma_tf32(d, w_hi + 8 * k, x_lo + 2 * k, idesc, k != 0 || more);   // 8 numbers of K: 8 columns, 32 bytes
+                for (int k = 0; k < BK / 8; ++k) umma_tf32(d, w_hi + 8 * k, x_lo + 2 * k, idesc, k != 0);   // 8 numbers of K: 8 columns, 32 bytes
 #pragma unroll
                 for (int k = 0; k < BK / 8; ++k) umma_tf32(d, w_lo + 8 * k, x_hi + 2 * k, idesc, 1);
 #pragma unroll
                 for (int k = 0; k < BK / 8; ++k) umma_tf32(d, w_hi + 8 * k, x_hi + 2 * k, idesc, 1);
                 umma_commit(&free_bar[a]);
-                j = j + 1 == p.per_segment ? 0 : j + 1;
-                if (j % SUM_BLOCKS == 0 || i + 1 == it.count) {
-                    umma_commit(&sum_full_bar[b]);
-                    ++sums;
-                }
+                umma_commit(&sum_full_bar[b]);
             }
         }
     } else if (warp >= 2 && warp < ADDERS_FROM) {
@@ -241,7 +233,7 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             const int n = it.n0 + quarter * 32 + lane, m_first = it.m0 + side * OWN;
             for (int from = 0; from < it.count && ok; from += p.per_segment) {        // a segment
                 const int blocks = min(p.per_segment, it.count - from);
-                for (int i = 0; i < blocks; i += SUM_BLOCKS, ++sums) {
+                for (int i = 0; i < blocks; ++i, ++sums) {
                     const int b = sums % SUMS;
                     ok = __all_sync(0xffffffffu, mbar_wait(&sum_full_bar[b], (sums / SUMS) & 1, p.error, 25) && !failed);
                     if (!ok) { failed = 1; break; }
