@@ -589,8 +589,8 @@ def test_greedy_generation_through_the_entry_point(folders, name):
 
 
 @pytest.mark.parametrize("heads, rank, rot, page, window, lens, before, sink", [
-    (16, 512, 64, 64, 1024, [301], [0], False), (16, 512, 64, 256, 0, [240, 75], [40, 0], False), (3, 128, 16, 16, 37, [303, 2, 66], [0, 9, 100], True),
-    (19, 256, 32, 64, 2, [181], [5], False), (16, 384, 0, 32, 64, [330], [64], True), (33, 128, 64, 64, 0, [100, 1, 33, 1], [3, 200, 0, 7], False)])
+    (16, 512, 64, 64, 1024, [601], [0], False), (16, 512, 64, 256, 0, [480, 75], [40, 0], False), (3, 384, 16, 16, 37, [1003, 2, 66], [0, 9, 100], True),
+    (19, 384, 32, 64, 2, [1101], [5], False), (16, 384, 0, 32, 64, [1090], [64], True), (33, 512, 64, 64, 0, [500, 1, 33, 1], [3, 200, 0, 7], False)])
 def test_latent_attention_of_portions_four_tokens_a_tile(heads, rank, rot, page, window, lens, before, sink):
     """The kernel of prompt portions against the one of single tokens (a context without `cu_q`) and the sums in 64 bits."""
     from types import SimpleNamespace
@@ -615,6 +615,7 @@ def test_latent_attention_of_portions_four_tokens_a_tile(heads, rank, rot, page,
     positions = [p for n, b in zip(lens, before) for p in range(b, b + n)]
     base = dict(positions=i32(positions), seq_of_token=i32([s for s, n in enumerate(lens) for _ in range(n)]), max_ctx_len=max(ends))
     portions = SimpleNamespace(cu_q=i32(cu), max_q_len=max(lens), **base)
+    assert ops.lib.ts_latent_attention_portions(T, len(lens), max(lens), heads, rank, rot, min(window, max(ends)) if window else max(ends))
     q_lat, q = torch.randn(T, heads, rank, generator=g), torch.randn(T, heads * (4 + rot), generator=g).to(torch.bfloat16)
     freq = torch.tensor([100.0 ** (-2.0 * i / rot) for i in range(rot // 2)], dtype=torch.float32, device=dev) if rot else None
     sinks = torch.linspace(-3, 3, heads, device=dev) if sink else None

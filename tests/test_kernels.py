@@ -313,6 +313,7 @@ def test_paged_attention(ops, dtype, generic, nh, nkv, hd, page, window):
 def test_float32_attention_tiles_do_not_depend_on_the_cut(ops, nh, nkv, hd, page, window):
     """A request of 203 tokens whole, in portions and with its last tokens alone: the same bits; a later key's NaN reaches no earlier row."""
     n, width = 203, (nh + 2 * nkv) * hd
+    assert bool(ops.lib.ts_paged_attention_f32_takes(nh, nkv, hd)) == (hd in (64, 128))       # the others: the generic kernel
     pages = -(-n // page)
     binding = make_binding(2 * pages, 1, nkv, page, hd, torch.float32, [list(range(pages))[::-1], list(range(pages, 2 * pages))])
     keys, values = rand((n, nkv, hd), torch.float32, 20), rand((n, nkv, hd), torch.float32, 30)

@@ -246,9 +246,11 @@ int launch(const Args& p, int num_tokens, cudaStream_t stream) {
 // Whether these sizes and addresses are taken: 16-byte rows, the sizes named above, a group's heads inside a tile, no more tiles
 // than a grid holds (131,000 prompt tokens and more: so many have no steps of other sizes beside them).  Which
 // of the two kernels takes a model's attention follows from its sizes alone, so a row's result stays independent of its step.
+TS_API int ts_paged_attention_f32_takes(int nh, int nkv, int hd) { return (hd == 64 || hd == 128) && nh / nkv >= 2 && nh / nkv <= 16; }
+
 bool paged_attention_f32_supported(const void* q, long long q_stride, const void* out, const void* k_pool, const void* v_pool,
                                    const KVGeometry& geo, int num_seqs, int num_tokens, int max_q_len, int nh, int nkv, int hd) {
-    return (hd == 64 || hd == 128) && nh / nkv >= 2 && nh / nkv <= 16 && nkv <= 65535 && q_stride % 4 == 0 && geo.page_stride % 4 == 0 && geo.entry_offset % 4 == 0 &&
+    return ts_paged_attention_f32_takes(nh, nkv, hd) && nkv <= 65535 && q_stride % 4 == 0 && geo.page_stride % 4 == 0 && geo.entry_offset % 4 == 0 &&
            ((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_pool | (uintptr_t)v_pool) % 16 == 0 &&
            tiles_of(num_tokens, num_seqs, nh / nkv, rows_of(max_q_len)) <= 65535;
 }

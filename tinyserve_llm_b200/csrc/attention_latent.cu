@@ -332,17 +332,16 @@ TS_API long long ts_latent_attention_scratch_floats(int num_tokens, int heads, i
 }
 
 // Whether a step's prompt portions go four tokens a CTA: where a step has so many tokens of them and so many keys to see that one copy
-// of a key tile for four tokens is worth an SM held by one CTA.  Measured on a B200, us, one token a CTA and four, 16 heads, by window:
-//   latent 512   tokens          514         700         1,000       1,200       2,048       300, 300, 300
-//     128                                  69 / 73                 106 / 78    203 / 166     72 / 73
-//     1,024                   106 / 98    162 / 129   282 / 179   362 / 229   723 / 504    113 / 88
-//     none                                                        381 / 246   976 / 659
-//   384: 1,200 tokens, window 37 72 / 59, 1,024 303 / 195.   256: window 256 83 / 82, 1,024 189 / 161, but 2,048 tokens 137 / 160 and
-//   365 / 344, 37 59 / 75.   128: 1,024 109 / 126, 199 / 265; 37 32 / 61: two and more of those CTAs share an SM, and four of the others.
-// Fewer than 512 such tokens (300: 57 / 67) keep the other kernel, replayed steps among them.  384 channels and up; what is captured, small
-// or narrow stays as it was.
+// of a key tile for four tokens is worth an SM held by one CTA.  Measured on a B200, 16 heads, us, one token a CTA / four:
+//   latent of 512, window 1,024   514 tokens 106 / 98, 700 162 / 129, 1,000 282 / 179, 2,048 723 / 504, 300 57 / 67
+//                  none           1,200 tokens 381 / 246, 2,048 976 / 659
+//                  128            700 tokens 69 / 73, three portions of 300 72 / 73, 1,200 106 / 78, 2,048 203 / 166
+//   latent of 384                 1,200 tokens, window 37 72 / 59, window 1,024 303 / 195
+//   latent of 256                 2,048 tokens, window 37 59 / 75, 256 137 / 160, 1,024 365 / 344
+//   latent of 128                 2,048 tokens, window 37 32 / 61, 1,024 199 / 265 (two of those CTAs share an SM, but four of the others)
+// So: latents of 384 and 512 channels, 512 such tokens (no replayed step has them) and 1,024 where fewer than 512 keys are seen.
 TS_API int ts_latent_attention_portions(int num_tokens, int num_seqs, int max_q_len, int heads, int rank, int rot, int max_keys) {
-    return max_q_len > 1 && num_seqs > 0 && num_tokens - num_seqs >= (max_keys >= 512 ? 512 : 1024) && num_tokens <= 1 << 24 && heads <= 65535 && rank >= 384 &&
+    return max_q_len > 1 && num_seqs > 0 && num_tokens - num_seqs >= (max_keys >= 512 ? 512 : 1024) && num_tokens <= 1 << 24 && heads <= 65535 &&
            ts_latent_mma_supported(rank, rot) && ts_latent_tokens_supported(rank, rot) &&
            ts_latent_attention_scratch_floats(num_tokens, heads, rank, max_keys) == 0;
 }

@@ -10,8 +10,8 @@
 // one on its way by cp.async.  Keys that only some of the four tokens see (at most six) come as a tile of their own, whose weights
 // meet the values by plain multiply-adds under a row's own mask; all other tiles hold keys that every token sees.
 //
-// Measured on a B200, 16 heads, latent of 512 + 64 channels, window 1,024, us, one token a CTA and now: 2,048 tokens 727 / 506, 1,000
-// behind 1,500 cached ones 501 / 361, 450 260 / 183, 300 229 / 183.  A tile takes 4.8 us, of which its MMAs are 2.2: two warps a
+// Measured on a B200, 16 heads, latent of 512 + 64 channels, window 1,024, us, one token a CTA and now: 2,048 tokens 723 / 504, 1,000
+// behind 2,000 cached ones 461 / 360, 514 242 / 181 (other sizes: ts_latent_attention_portions).  A tile takes 4.8 us, of which its MMAs are 2.2: two warps a
 // scheduler wait on one another's products and reads.  Tried and no faster: scores and values in warps of their own a tile apart (539
 // at 2,048 tokens), scores by quarters of the channels with half the ldmatrix (537).
 #include "mma_tile.cuh"
@@ -339,9 +339,9 @@ __global__ void __launch_bounds__(WARPS * 32, 1) latent_attention_tokens_kernel(
 
 }  // namespace
 
-// Latents of 128, 256, 384 or 512 channels whose tiles fit shared memory (the rotated part in steps of 16: ts_latent_mma_supported).
+// Latents of 384 or 512 channels whose tiles fit shared memory (the rotated part in steps of 16: ts_latent_mma_supported).
 bool ts_latent_tokens_supported(int rank, int rot) {
-    return rank % 128 == 0 && rank <= 512 && rot <= 256 && latent_tokens_smem(rank, rot) <= 227 * 1024;
+    return (rank == 384 || rank == 512) && rot <= 256 && latent_tokens_smem(rank, rot) <= 227 * 1024;
 }
 
 int ts_latent_attention_tokens_launch(const float* q_lat, long long ql_t, long long ql_h, const void* q, long long q_stride,
@@ -362,9 +362,7 @@ int ts_latent_attention_tokens_launch(const float* q_lat, long long ql_t, long l
         cudaFuncSetAttribute(latent_attention_tokens_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
         latent_attention_tokens_kernel<NT><<<grid, WARPS * 32, smem, stream>>>(p);                                                 \
     } while (0)
-    if (rank == 128) TS_LATENT_TOKENS(2);
-    else if (rank == 256) TS_LATENT_TOKENS(4);
-    else if (rank == 384) TS_LATENT_TOKENS(6);
+    if (rank == 384) TS_LATENT_TOKENS(6);
     else TS_LATENT_TOKENS(8);
 #undef TS_LATENT_TOKENS
     TS_LAUNCH_CHECK("latent_attention (tokens)");

@@ -29,6 +29,7 @@ _SIGNATURES = {
     "ts_attention_bf16_scratch_floats": ("long long", "iiii"),
     "ts_attention_bf16_supported": ("int", "iiii"),
     "ts_paged_attention_bf16": ("int", "pppplliipippiiiiiiifiplpip"),
+    "ts_paged_attention_f32_takes": ("int", "iii"),
     "ts_paged_attention_generic": ("int", "pppplliipipp" "pii" "iiiifiip"),
     "ts_paged_attention_bf16_sigmoid": ("int", "pl" "ppp" "lliipippiiiiiiifiplpi" "pppl" "p"),
     "ts_paged_attention_bf16_masked": ("int", "pl" "ppp" "lllliipippiiiiiiifiifi" "plpi" "fp"),
