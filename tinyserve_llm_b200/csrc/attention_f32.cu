@@ -18,6 +18,8 @@
 // 171 / 260; of 112, 32:4: 209 / 255), and a group of one leaves fifteen of a single token's sixteen rows empty (64 single
 // tokens behind 500, 16:16 heads of 128: 163 / 261; 32 behind 150, 32:32 of 64: 32 / 43).  With groups of two nothing was slower
 // (16:8 heads of 64, 8 single tokens behind 2,000: 157 / 149, 512 tokens 323 / 47; of 128 426 / 252 and 654 / 81).
+// The bounds by `hd` cut nothing off, but with HD in their place the compiler unrolls the loads of a tile ahead of everything else: 8
+// single tokens behind 2,000 take 171 us (16:8 of 64) and 288 (24:8 of 128) instead of 149 and 248.
 #include <type_traits>
 
 #include "common.cuh"
@@ -42,6 +44,7 @@ struct Args {
     const int* block_table; int table_width;
     const int* positions; const int* cu_q;
     int num_tokens, num_seqs, steps, nh, nkv, window;  // steps: the largest power of two up to num_seqs
+    int hd;                                          // HD, which the kernel takes as a number it does not know (see below)
     float scale;
 };
 
@@ -73,8 +76,8 @@ __global__ void __launch_bounds__(BQ * 4) paged_attention_f32_kernel(Args p) {
     for (int e = tid; e < BQ * (HD / 4); e += THREADS) {
         const int r = e / (HD / 4), d = e % (HD / 4) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < rows)
-            v = *reinterpret_cast<const float4*>(p.q + (t0 + r / group) * p.q_stride + (long long)(kvh * group + r % group) * HD + d);
+        if (r < rows && d < p.hd)
+            v = *reinterpret_cast<const float4*>(p.q + (t0 + r / group) * p.q_stride + (long long)(kvh * group + r % group) * p.hd + d);
         *reinterpret_cast<float4*>(qs + r * PITCH + d) = make_float4(v.x * p.scale, v.y * p.scale, v.z * p.scale, v.w * p.scale);
     }
     for (int r = tid; r < BQ; r += THREADS) {
@@ -86,20 +89,21 @@ __global__ void __launch_bounds__(BQ * 4) paged_attention_f32_kernel(Args p) {
     const int from = first_key[0] / BK, to = last_key[rows - 1] / BK;                 // positions rise along a run
     const int* table = p.block_table + (long long)seq * p.table_width;
     const int keys_end = last_key[rows - 1] + 1;
-    const long long head_off = p.geo.entry_offset + (long long)kvh * p.geo.page_tokens * HD;
+    const long long head_off = p.geo.entry_offset + (long long)kvh * p.geo.page_tokens * p.hd;
     // Where a tile's keys lie, looked up a tile ahead; -1: a page given back or a bad table, and the key is not seen.
     auto locate = [&](int tile) {
         for (int r = tid; r < BK; r += THREADS) {
             const int j = tile * BK + r, page = j < keys_end ? table[j / p.geo.page_tokens] : -1;
             key_at[tile & 1][r] = page >= 0 && page < p.geo.num_pages
-                                      ? (long long)page * p.geo.page_stride + head_off + (long long)(j % p.geo.page_tokens) * HD : -1;
+                                      ? (long long)page * p.geo.page_stride + head_off + (long long)(j % p.geo.page_tokens) * p.hd : -1;
         }
     };
     auto load = [&](float* dst, const float* pool, int tile) {
         for (int e = tid; e < BK * (HD / 4); e += THREADS) {
             const int r = e / (HD / 4), d = e % (HD / 4) * 4;
             const long long at = key_at[tile & 1][r];
-            cp16(dst + r * PITCH + d, at >= 0 ? pool + at + d : pool, at >= 0);
+            const bool ok = at >= 0 && d < p.hd;
+            cp16(dst + r * PITCH + d, ok ? pool + at + d : pool, ok);
         }
         commit();
     };
@@ -219,10 +223,13 @@ __global__ void __launch_bounds__(BQ * 4) paged_attention_f32_kernel(Args p) {
         const int r = ty * 4 + i;
         if (r >= rows) continue;
         const float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
-        float* out = p.out + ((long long)(t0 + r / group) * p.nh + kvh * group + r % group) * HD;
+        float* out = p.out + ((long long)(t0 + r / group) * p.nh + kvh * group + r % group) * p.hd;
 #pragma unroll
-        for (int c = 0; c < NC; ++c)
-            *reinterpret_cast<float4*>(out + 64 * c + tx * 4) = make_float4(o[i][4 * c] * inv, o[i][4 * c + 1] * inv, o[i][4 * c + 2] * inv, o[i][4 * c + 3] * inv);
+        for (int c = 0; c < NC; ++c) {
+            const int d = 64 * c + tx * 4;
+            if (d < p.hd)
+                *reinterpret_cast<float4*>(out + d) = make_float4(o[i][4 * c] * inv, o[i][4 * c + 1] * inv, o[i][4 * c + 2] * inv, o[i][4 * c + 3] * inv);
+        }
     }
 }
 
@@ -260,7 +267,7 @@ int paged_attention_f32(const float* q, long long q_stride, float* out, const fl
                         int num_tokens, int max_q_len, int nh, int nkv, int hd, float scale, int window, cudaStream_t stream) {
     int steps = 1;
     while (2 * steps <= num_seqs) steps *= 2;
-    const Args p{q, q_stride, out, k_pool, v_pool, geo, block_table, table_width, positions, cu_q, num_tokens, num_seqs, steps, nh, nkv, window, scale};
+    const Args p{q, q_stride, out, k_pool, v_pool, geo, block_table, table_width, positions, cu_q, num_tokens, num_seqs, steps, nh, nkv, window, hd, scale};
     if (rows_of(max_q_len) == 16) return hd == 64 ? launch<64, 16>(p, num_tokens, stream) : launch<128, 16>(p, num_tokens, stream);
     return hd == 64 ? launch<64, 32>(p, num_tokens, stream) : launch<128, 32>(p, num_tokens, stream);
 }
