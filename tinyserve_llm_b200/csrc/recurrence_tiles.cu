@@ -67,7 +67,7 @@ constexpr int RP = 24;             // pitch of the partial sums and of U: likewi
 // that does the same for it.
 __host__ __device__ constexpr int pack_pitch(int rows) { return rows + 8; }
 __host__ __device__ constexpr int pack_floats(int rows, int sets) { return ((1 + sets) * B + 1) * pack_pitch(rows); }
-enum { DELTA = 0, MIX = 1, CHANNEL = 2 };           // delta rule, a decay a head; time mixing and plain; delta rule, a decay a channel
+enum { DELTA = 0, MIX = 1, CHANNEL = 2, PLAIN = 3 };   // delta rule, a decay a head; time mixing; delta rule, a decay a channel; plain
 __host__ __device__ constexpr int sets_of(int mode) { return mode == CHANNEL ? 2 : 1; }
 
 __device__ __forceinline__ float softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
@@ -596,9 +596,10 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
     constexpr int WROWS = 8 * NT, ROWS = WARPS * WROWS;  // rows of a warp; rows of the state
     constexpr int PP = pack_pitch(ROWS);
     constexpr int SETS = sets_of(MODE), PACK = pack_floats(ROWS, SETS), STAGE = PACK + COEF;
-    constexpr int TQ = MODE == MIX ? B : 2 * B;          // rows of the pack that meet S_0
-    constexpr bool FRESH = MODE != DELTA;                // (a decay a head: the sums as they have always been)
-    constexpr bool EXACT = MODE == MIX && sizeof(T) == 2;   // the values are TF32 numbers
+    constexpr bool VALUES = MODE == MIX || MODE == PLAIN;   // the values themselves move the state on
+    constexpr int TQ = VALUES ? B : 2 * B;               // rows of the pack that meet S_0
+    constexpr bool FRESH = MODE == PLAIN || MODE == CHANNEL;   // (the others sum as they did before)
+    constexpr bool EXACT = MODE == PLAIN && sizeof(T) == 2;    // the values are TF32 numbers
     extern __shared__ __align__(16) float smem[];
     float* red = smem + 2 * STAGE;                       // [WARPS][TQ][RP]
     float* G_s = red + WARPS * TQ * RP;                  // [B][RP]: what the state's update takes, G[B] U or V
@@ -662,7 +663,7 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
         }
         const float* pack = smem + (tile & 1) * STAGE;
         const float* coef = pack + PACK;
-        if (MODE == MIX && !makes_o) {                   // what the update takes is there from the start
+        if (VALUES && !makes_o) {                   // what the update takes is there from the start
 #pragma unroll
             for (int k = 0; k < 4; ++k) G_s[(c + 4 * k) * RP + col] = to_float<T>(vnow[k]);
         }
@@ -699,14 +700,14 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 x[k] = to_float<T>(vnow[k]);
-                if (MODE != MIX) {
+                if (!VALUES) {
                     float sum = 0.f;
 #pragma unroll
                     for (int w = 0; w < WARPS; ++w) sum += red[(w * TQ + B + c + 4 * k) * RP + col];
                     x[k] = MODE == DELTA ? fmaf(-coef[2 * B * CP + c + 4 * k], sum, x[k]) : x[k] - sum;
                 }
             }
-            if (MODE != MIX || makes_o) {
+            if (!VALUES || makes_o) {
                 const float* m = coef + (makes_o ? B * CP : 0);
                 float big[4] = {}, small[4] = {};
                 float kept[4];                               // what is not finite stays out of the product, where 0 times it is NaN
@@ -755,7 +756,7 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
                 }
             }
         }
-        if (MODE != MIX) __syncthreads();                // what the update takes is in
+        if (!VALUES) __syncthreads();                // what the update takes is in
         // product 3, S^T <- decay S^T + G^T K, and the state after the tile
         {
             SplitA a[2];
@@ -802,7 +803,7 @@ int launch_scan(const ScanArgs& p, int portions, cudaStream_t stream) {
     const dim3 grid((p.vdim + COLS - 1) / COLS, p.heads, portions);
 #define TS_TILES(NT)                                                                                                 \
     do {                                                                                                             \
-        constexpr int TQ = MODE == MIX ? B : 2 * B;                                                                  \
+        constexpr int TQ = MODE == MIX || MODE == PLAIN ? B : 2 * B;                                                 \
         const size_t smem = sizeof(float) * (2 * (pack_floats(WARPS * 8 * NT, sets_of(MODE)) + COEF) + (WARPS * TQ + B) * RP); \
         auto kernel = recurrence_tiles_kernel<T, NT, MODE>;                                                          \
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                        \
@@ -908,11 +909,11 @@ TS_API int ts_plain_tiles(const void* q, const void* k, const void* v, long long
     } while (0)
     if (dtype == TS_F32) {
         TS_PLAIN_PREPARE(float);
-        return launch_scan<float, MIX>(s, portions, stream);
+        return launch_scan<float, PLAIN>(s, portions, stream);
     }
     if (dtype == TS_BF16) {
         TS_PLAIN_PREPARE(__nv_bfloat16);
-        return launch_scan<__nv_bfloat16, MIX>(s, portions, stream);
+        return launch_scan<__nv_bfloat16, PLAIN>(s, portions, stream);
     }
 #undef TS_PLAIN_PREPARE
     return ts_fail("plain_tiles: unknown dtype code %d", dtype);
