@@ -590,7 +590,7 @@ def test_greedy_generation_through_the_entry_point(folders, name):
 
 @pytest.mark.parametrize("heads, rank, rot, page, window, lens, before, sink", [
     (16, 512, 64, 64, 1024, [601], [0], False), (16, 512, 64, 256, 0, [480, 75], [40, 0], False), (3, 384, 16, 16, 37, [1003, 2, 66], [0, 9, 100], True),
-    (19, 384, 32, 64, 2, [1101], [5], False), (16, 384, 0, 32, 64, [1090], [64], True), (33, 512, 64, 64, 0, [500, 1, 33, 1], [3, 200, 0, 7], False)])
+    (19, 384, 32, 64, 2, [1101], [5], False), (16, 384, 0, 32, 64, [1090], [64], True), (33, 512, 64, 64, 0, [500, 1, 33, 1], [30, 200, 0, 7], False)])
 def test_latent_attention_of_portions_four_tokens_a_tile(heads, rank, rot, page, window, lens, before, sink):
     """The kernel of prompt portions against the one of single tokens (a context without `cu_q`) and the sums in 64 bits."""
     from types import SimpleNamespace
