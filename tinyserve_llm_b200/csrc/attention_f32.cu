@@ -48,6 +48,13 @@ struct Args {
     float scale;
 };
 
+// Padding rows behind the last request: zeros, so that nothing that reads them meets NaNs of someone else's memory.  Out of line: in line
+// it takes registers from the loop over the keys (24:8 heads of 128, 8 single tokens behind 2,000: 247 -> 257 us).
+__device__ __noinline__ void clear_padding(float* out, const int* end, int num_tokens, int first, int stride, long long row, int width) {
+    for (int t = *end + first; t < num_tokens; t += stride)
+        for (int d = threadIdx.x; d < width; d += blockDim.x) out[t * row + d] = 0.f;
+}
+
 template <int HD, int BQ>
 __global__ void __launch_bounds__(BQ * 4) paged_attention_f32_kernel(Args p) {
     constexpr int THREADS = BQ * 4, PITCH = HD + 4, NC = HD / 64;                     // NC: runs of four channels a thread
@@ -62,9 +69,7 @@ __global__ void __launch_bounds__(BQ * 4) paged_attention_f32_kernel(Args p) {
     // request s's tiles begin at cu_q[s] / per_tile + s, which leaves room for its last, partly filled one; the tiles with the
     // most keys before them go first
     const int tile_at = gridDim.y - 1 - blockIdx.y;
-    // padding rows behind the last request: zeros, so that nothing that reads them meets NaNs of someone else's memory
-    for (int t = p.cu_q[p.num_seqs] + tile_at; t < p.num_tokens; t += gridDim.y)
-        for (int d = threadIdx.x; d < group * HD; d += THREADS) p.out[((long long)t * p.nh + kvh * group) * HD + d] = 0.f;
+    clear_padding(p.out + (long long)kvh * group * HD, p.cu_q + p.num_seqs, p.num_tokens, tile_at, gridDim.y, p.nh * HD, group * HD);
     int seq = 0;
     for (int step = p.steps; step > 0; step >>= 1)
         if (seq + step < p.num_seqs && p.cu_q[seq + step] / per_tile + seq + step <= tile_at) seq += step;
