@@ -9,10 +9,11 @@
 // of a head, angle = position * freq[i]) and scaled on their way in.  Everything from the loaded
 // projections on is float32: rotation, decays, the state, the sums.
 //
-// The scan walks single decoded tokens (and prompt portions where the kernels of recurrence_tiles.cu, which take them sixteen tokens
-// at a time, are switched off): a CTA owns one request, one head and 16 value channels (8 for the delta rule), reads the state from
-// the request's slot, walks over the request's tokens of this step in order and writes the state back.  With `singles` it
-// leaves requests of more than one token alone.  A first kernel computes what enters the recurrence (rotated and scaled q
+// The scan walks single decoded tokens, and the prompt portions that the kernels of recurrence_tiles.cu do not take sixteen tokens at a
+// time (short ones; float32 activations): a CTA owns one request, one head and 16 value channels (8 for the delta rule), reads the
+// state from the request's slot, walks over the request's tokens of this step in order and writes the state back.  A token's
+// arithmetic does not depend on where the step was cut or on what else is in the batch.  With `singles` it leaves requests of more
+// than one token alone.  A first kernel computes what enters the recurrence (rotated and scaled q
 // and k, the decays) once per token, head and channel; the scan stages 16 tokens of it at a time, fetched one tile ahead.  Inside a
 // tile no thread waits for another: thread (r, j) holds a run of rows of column j of S (read from the staged tile four
 // channels a load) and leaves its share of o_t[j] in shared memory, and the sixteen shares are added

@@ -24,7 +24,7 @@
 //   16,384 x 2,048      192 / 53   192 / 53   306 / 68
 //   2,048 x 8,192                  677 / 29   636 / 40      - / 100
 //   3,072 x 2,048                                                 241 / 70
-// What bounds it: a block of k costs 0.75 to 0.93 us whatever BX is.  An MMA of 8 numbers of k takes some 107 cycles with up to 64
+// (a feed-forward of 100 rows, 2,048 x 8,192, since then 113 / 107).  What bounds it: a block of k costs 0.75 to 0.93 us whatever BX is.  An MMA of 8 numbers of k takes some 107 cycles with up to 64
 // rows of x and 137 with 128 (67 by the tensor cores' rate); with one of the twelve MMAs issued (timing only) the first column
 // is 34 us, and loads alone stream W at 4.4 TB/s.
 //

@@ -1109,7 +1109,7 @@ class Ops:
     def portions_by_tiles(self, ctx, longest: int = 2) -> bool:
         """
         Whether the step holds prompt portions (a bare context may not list them), the longest of at least `longest` tokens,
-        which then go sixteen tokens at a time.  A replayed step is judged by the bound its grids are sized by.
+        which then go sixteen tokens at a time.  For a replayed step the bound its grids are sized by decides.
         """
         portions = getattr(ctx, "prefill_seqs", None)
         return bool(self.recurrence_tiles and getattr(ctx, "max_q_len", 0) >= longest and portions is not None and portions.shape[0] > 0)
