@@ -382,3 +382,92 @@ def test_beside_tiles_only_single_tokens_are_prepared(kind, monkeypatch):
     prepared, = [t for t in made if t.dim() == 3 and t.shape[:2] == (3, 342)]
     written = (prepared != 7).any(dim=2).all(dim=0)
     assert written.nonzero().flatten().tolist() == [300, 341]
+
+
+def _windowed_latent(heads, dim, rot, rank, window, lens, cached, page, plant=None):
+    """A windowed latent layer over prompt portions: (output, cache rows written, what 64 bits give).  Pages before a window are given back."""
+    from tinyserve_llm_b200.config.spec import InlineRotarySpec, LatentAttentionSpec
+    from tinyserve_llm_b200.parts.base import Runtime, part_class
+    g = torch.Generator().manual_seed(dim + rank + window)
+    W, scale, eps = 96, 2.0 / (dim + rot) ** 0.5, 1e-5
+    spec = LatentAttentionSpec(hidden_size=W, num_heads=heads, head_dim=dim, rot_dim=rot, value_dim=dim, q_rank=0, kv_rank=rank, scale=scale, window=window,
+                               norm_eps=eps, position=InlineRotarySpec(dims=rot))
+    w = {"q": torch.randn(heads * (dim + rot), W, generator=g) * W ** -0.5, "dkv": torch.randn(rank + rot, W, generator=g) * W ** -0.5,
+         "uk": torch.randn(heads * dim, rank, generator=g) * rank ** -0.5, "uv": torch.randn(heads * dim, rank, generator=g) * rank ** -0.5,
+         "o": torch.randn(W, heads * dim, generator=g) * (heads * dim) ** -0.5}
+    w = {n: t.to(torch.bfloat16) for n, t in w.items()}
+    w["dkv.norm"] = 1 + torch.randn(rank, generator=g) * 0.1
+    rt = Runtime(dtype=torch.bfloat16, device=torch.device("cuda", 0), ops=get_ops())
+    part = part_class("mixer", spec)(spec, w, rt)
+    x = torch.randn(sum(lens), W, generator=g).to(torch.bfloat16)
+    if plant is not None:
+        x[plant, 3] = float("nan")
+    ends = [n + c for n, c in zip(lens, cached)]
+    counts = [-(-e // page) for e in ends]
+    order = torch.randperm(sum(counts) + 1, generator=g).tolist()
+    pool = torch.full((sum(counts) + 1, 2, 1, page, rank + rot), float("nan"), dtype=torch.bfloat16)
+    history, tables, at = [], [], 0
+    for c, n, end in zip(counts, cached, ends):
+        ids, at = order[at:at + c], at + c
+        rows = torch.randn(n, rank + rot, generator=g).to(torch.bfloat16)
+        for j in range(n):
+            pool[ids[j // page], 1, 0, j % page] = rows[j]
+        history.append(rows)
+        gone = max(0, n - window + 1) // page
+        for i in ids[:gone]:
+            pool[i] = float("nan")
+        tables.append([-1] * gone + ids[gone:] + [-1] * (max(counts) - c))
+    ctx = make_ctx(lens, ends)
+    ctx.replayed, ctx.prefill_seqs = False, i32([s for s, n in enumerate(lens) if n > 1])
+    per = page * (rank + rot)
+    dev = pool.cuda()
+    binding = EntryBinding(dev, None, 2 * per, per, page, pool.shape[0], i32(tables), max(counts))
+    before = rt.ops.calls.get("ts_prefill_attention_tcgen05_dense", 0)
+    got = part.forward(x.cuda(), ctx, binding)
+    assert rt.ops.calls.get("ts_prefill_attention_tcgen05_dense", 0) == before + 1
+    if plant is not None:
+        return got.cpu(), None
+    d = {n: t.double() for n, t in w.items()}
+    freq = 10000.0 ** (-2.0 * torch.arange(rot // 2, dtype=torch.float64) / rot)
+
+    def turned(t, positions):                            # [n, k, rot]
+        a = positions.double()[:, None, None] * freq
+        u, v = t.chunk(2, dim=-1)
+        return torch.cat([u * a.cos() - v * a.sin(), v * a.cos() + u * a.sin()], dim=-1)
+
+    want, at = [], 0
+    for n, c, rows in zip(lens, cached, history):
+        xs, positions = x[at:at + n].double(), torch.arange(c, c + n)
+        q, y = (xs @ d["q"].t()).view(n, heads, dim + rot), xs @ d["dkv"].t()
+        lat = y[:, :rank] / (y[:, :rank].pow(2).mean(-1, keepdim=True) + eps).sqrt() * d["dkv.norm"]
+        new = torch.cat([lat, turned(y[:, None, rank:], positions)[:, 0]], dim=-1)
+        full = torch.cat([rows.double(), new])
+        k = torch.cat([(full[:, :rank] @ d["uk"].t()).view(-1, heads, dim), full[:, None, rank:].expand(-1, heads, -1)], dim=-1)
+        q = torch.cat([q[..., :dim], turned(q[..., dim:], positions)], dim=-1)
+        s = torch.einsum("ihd,jhd->hij", q, k) * scale
+        j = torch.arange(c + n)[None]
+        s = s.masked_fill((j > positions[:, None]) | (j <= positions[:, None] - window), -float("inf"))
+        o = torch.einsum("hij,jhd->ihd", torch.softmax(s, -1), (full[:, :rank] @ d["uv"].t()).view(-1, heads, dim))
+        want.append(o.reshape(n, -1) @ d["o"].t())
+        at += n
+    return got.double().cpu(), torch.cat(want)
+
+
+@pytest.mark.parametrize("heads,dim,rot,rank,window,lens,cached,page", [
+    (2, 128, 64, 512, 100, [300, 1, 129, 2], [0, 500, 777, 130], 64), (3, 64, 24, 40, 1, [140], [260], 16), (1, 128, 40, 72, 1000, [150, 150], [0, 1300], 256),
+    (2, 64, 16, 64, 129, [128, 257], [127, 1], 64), (4, 128, 8, 128, 4096, [513], [64], 128)])
+def test_windowed_latent_portions_on_keys_and_values_of_their_own(heads, dim, rot, rank, window, lens, cached, page):
+    """Windows inside a key tile, over several, wider than the context; portions behind cached keys whose early pages are given back."""
+    got, want = _windowed_latent(heads, dim, rot, rank, window, lens, cached, page)
+    # bfloat16 queries, latents, keys, values, weights, heads and outputs: seven roundings of at most 2^-9, half of that on average; in a
+    # single row scores of up to 8 (two is their deviation), off by up to 2^-9 of themselves, move its weights by as much as 8 2^-9 more
+    err, off = (got - want).norm(dim=-1) / want.norm(dim=-1), float((got - want).norm() / want.norm())
+    assert float(err.max()) < 15 * 2.0 ** -9 and off < 3.5 * 2.0 ** -9, (float(err.max()), off)
+
+
+def test_a_latent_that_is_not_finite_reaches_the_queries_that_see_it_only():
+    sizes = (2, 128, 64, 256, 70, [400, 130], [30, 0], 64)
+    (clean, _), (got, _) = _windowed_latent(*sizes), _windowed_latent(*sizes, plant=201)
+    sees = torch.zeros(530, dtype=torch.bool)
+    sees[201:271] = True
+    assert torch.isnan(got[sees]).all() and torch.equal(got[~sees], clean[~sees].to(got.dtype))

@@ -407,42 +407,91 @@ TS_API int ts_latent_attention(const float* q_lat, long long ql_token_stride, lo
     return ts_fail("latent_attention: unknown dtype code %d", dtype);
 }
 
-// The queries' rotated parts for the unfolded form: out[t, h, 0 .. 63] = rotated q[t, h * head_width + rot_offset ..],
-// zeros past `rot` channels; rotation by halves, angle position * freq[i] in float32, cos and sin times `magnitude`.
-// A thread a pair of channels (i, i + rot / 2), the threads past the last pair write the zeros.
-__global__ void __launch_bounds__(256)
-latent_rotate_queries_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride, int head_width, int rot_offset,
-                             const float* __restrict__ freq, float magnitude, const int* __restrict__ positions,
-                             __nv_bfloat16* __restrict__ out, int heads, int rot) {
-    const int t = blockIdx.x, half = rot / 2, i = threadIdx.x & 31;
-    float sn = 0.f, cs = 0.f;
-    if (i < half) {                                       // a thread keeps its pair of channels over all heads
-        sincosf((float)positions[t] * freq[i], &sn, &cs);
-        sn *= magnitude;
-        cs *= magnitude;
+// The cached rows [c | k_rot] that a step's prompt portions see, page by page into matrices of their own for the unfolded form: c
+// [rows, rank] and k_rot [rows, rot], the portions one after another in the order of their list, each from the first key its first
+// query sees, rounded down to a key tile of the attention (WINDOW_TILE), to its last; kv_start[s] is key 0's row (negative where it lies
+// before).  With a rotated part, the cosines and sines of the portions' tokens go to turn [T, 32], from which the attention rotates
+// its queries.  With `odd` a row whose latent is not finite is written as zeros and marked (its values, zeros in the products, would
+// otherwise reach queries that do not see it as 0 times NaN).  A warp a row, 16 bytes a lane; bound by its launch and one round trip
+// (2,048 rows of 576: 5 us, where torch's indexing, two copies and the upload of kv_start took five launches).
+constexpr int WINDOW_TILE = 128, GATHER_WARPS = 8;
+
+__device__ __forceinline__ int first_gathered(int ctx, int q_len, int window) {
+    return window > 0 ? max(0, ctx - q_len - window + 1) / WINDOW_TILE * WINDOW_TILE : 0;
+}
+
+template <typename V>                                    // what a lane copies at a time: 16 bytes or an element
+__global__ void __launch_bounds__(GATHER_WARPS * 32)
+latent_gather_kernel(const __nv_bfloat16* __restrict__ pool, KVGeometry geo, const int* __restrict__ block_table, int table_width,
+                     const int* __restrict__ cu_q, const int* __restrict__ ctx_lens, const int* __restrict__ portions, int window, int rank,
+                     int rot, const float* __restrict__ freq, float magnitude, float2* __restrict__ turn, long long num_rows, __nv_bfloat16* __restrict__ c, __nv_bfloat16* __restrict__ k_rot, unsigned char* __restrict__ odd,
+                     int* __restrict__ kv_start) {
+    constexpr int N = sizeof(V) / sizeof(__nv_bfloat16);
+    const int seq = portions ? portions[blockIdx.y] : (int)blockIdx.y;
+    if (seq < 0) return;
+    const int q_len = cu_q[seq + 1] - cu_q[seq], ctx = ctx_lens[seq];
+    if (q_len <= 1) return;
+    const int lo = first_gathered(ctx, q_len, window);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    long long start = 0;                                 // rows of the portions before this one
+    for (int i = lane; i < (int)blockIdx.y; i += 32) {
+        const int s = portions ? portions[i] : i;
+        if (s < 0) continue;
+        const int n = cu_q[s + 1] - cu_q[s];
+        if (n > 1) start += ctx_lens[s] - first_gathered(ctx_lens[s], n, window);
     }
-    const __nv_bfloat16* src = q + (long long)t * q_stride + rot_offset + i;
-    __nv_bfloat16* dst = out + (long long)t * heads * 64;
-    for (int h = threadIdx.x >> 5; h < heads; h += 8) {
-        if (i < half) {
-            const float u = __bfloat162float(src[(long long)h * head_width]), v = __bfloat162float(src[(long long)h * head_width + half]);
-            dst[h * 64 + i] = __float2bfloat16_rn(u * cs - v * sn);
-            dst[h * 64 + i + half] = __float2bfloat16_rn(v * cs + u * sn);
-        } else {
-            const int c = rot + 2 * (i - half);
-            dst[h * 64 + c] = dst[h * 64 + c + 1] = __float2bfloat16_rn(0.f);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) start += __shfl_xor_sync(0xffffffffu, start, o);
+    if (blockIdx.x == 0 && threadIdx.x == 0) kv_start[seq] = (int)(start - lo);
+    const int* table = block_table + (long long)seq * table_width;
+    for (int key = lo + blockIdx.x * GATHER_WARPS + warp; key < ctx; key += gridDim.x * GATHER_WARPS) {
+        const long long row = start + key - lo;
+        if (row >= num_rows) return;
+        const int at = key / geo.page_tokens, page = at < table_width ? table[at] : -1;
+        const bool held = page >= 0 && page < geo.num_pages;         // pages before a window are given back: zeros, which nobody sees
+        const __nv_bfloat16* src = pool + (long long)(held ? page : 0) * geo.page_stride + geo.entry_offset + (long long)(key % geo.page_tokens) * (rank + rot);
+        bool bad = false;
+        if (odd) {
+            for (int i = lane; i < rank / N; i += 32) {
+                const V v = reinterpret_cast<const V*>(src)[i];
+                const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v);
+#pragma unroll
+                for (int j = 0; j < N; ++j) bad |= !isfinite(__bfloat162float(e[j]));
+            }
+            bad = held && __any_sync(0xffffffffu, bad);
+            if (lane == 0) odd[row] = bad;
         }
+        const int t = key - (ctx - q_len);               // the portion's token at this position
+        if (t >= 0 && lane < rot / 2) {
+            float sn, cs;
+            sincosf((float)key * freq[lane], &sn, &cs);
+            turn[(long long)(cu_q[seq] + t) * 32 + lane] = make_float2(cs * magnitude, sn * magnitude);
+        }
+        V zero;
+        memset(&zero, 0, sizeof(V));
+        for (int i = lane; i < rank / N; i += 32)
+            reinterpret_cast<V*>(c + row * rank)[i] = held && !bad ? reinterpret_cast<const V*>(src)[i] : zero;
+        for (int i = lane; i < rot / N; i += 32)
+            reinterpret_cast<V*>(k_rot + row * rot)[i] = held ? reinterpret_cast<const V*>(src + rank)[i] : zero;
     }
 }
 
-TS_API int ts_latent_rotate_queries(const void* q, long long q_stride, int head_width, int rot_offset, const float* freq,
-                                    float magnitude, const int* positions, void* out, int num_tokens, int heads, int rot,
-                                    cudaStream_t stream) {
-    TS_REQUIRE(num_tokens >= 0 && heads > 0 && rot > 0 && rot % 2 == 0 && rot <= 64 && rot_offset + rot <= head_width,
-               "latent_rotate_queries: bad sizes");
-    if (num_tokens == 0) return 0;
-    latent_rotate_queries_kernel<<<num_tokens, 256, 0, stream>>>((const __nv_bfloat16*)q, q_stride, head_width, rot_offset, freq,
-                                                                 magnitude, positions, (__nv_bfloat16*)out, heads, rot);
-    TS_LAUNCH_CHECK("latent_rotate_queries");
+// `rows`: of the matrices (the keys of all portions, at most `max_keys` of one); portions [num_portions] or null (then every request,
+// of which those that feed one token are passed over); freq [rot / 2], turn [T, 32, 2] (rot 0: null); odd [rows] or null.
+TS_API int ts_latent_gather(const void* pool, long long page_stride, long long entry_offset, int page_tokens, int num_pages,
+                            const int* block_table, int table_width, const int* cu_q, const int* ctx_lens, const int* portions,
+                            int num_portions, int window, int max_keys, int rank, int rot, const float* freq, float magnitude,
+                            float* turn, long long rows, void* c, void* k_rot, unsigned char* odd, int* kv_start, cudaStream_t stream) {
+    TS_REQUIRE(rank > 0 && rot >= 0 && rot <= 64 && rot % 2 == 0 && (rot == 0 || (freq && turn)) && page_tokens > 0 && table_width > 0 && window >= 0, "latent_gather: bad sizes");
+    TS_REQUIRE(num_portions >= 0 && num_portions <= 65535 && rows < 0x7fffffffll, "latent_gather: %d portions, %lld rows", num_portions, rows);
+    if (num_portions == 0 || max_keys <= 0) return 0;
+    const KVGeometry geo{page_stride, entry_offset, page_tokens, num_pages};
+    const dim3 grid((max_keys + GATHER_WARPS - 1) / GATHER_WARPS, num_portions);
+    const bool wide = rank % 8 == 0 && rot % 8 == 0 && page_stride % 8 == 0 && entry_offset % 8 == 0 && (uintptr_t)pool % 16 == 0 &&
+                      (uintptr_t)c % 16 == 0 && (uintptr_t)k_rot % 16 == 0;
+    auto kernel = wide ? latent_gather_kernel<uint4> : latent_gather_kernel<__nv_bfloat16>;
+    kernel<<<grid, GATHER_WARPS * 32, 0, stream>>>((const __nv_bfloat16*)pool, geo, block_table, table_width, cu_q, ctx_lens, portions, window,
+                                                   rank, rot, freq, magnitude, (float2*)turn, rows, (__nv_bfloat16*)c, (__nv_bfloat16*)k_rot, odd, kv_start);
+    TS_LAUNCH_CHECK("latent_gather");
     return 0;
 }

@@ -23,8 +23,12 @@
 // (attention/torch_paged.py:36-45 of the reference, by positions); value rows beyond the request's
 // length are zeroed in shared memory before they are multiplied.
 //
-// A form for keys of which every head has its own part and all heads share a second, rotated one (ROT): queries and keys
-// have a further sub-tile of 64 channels, the keys' read from a matrix of its own, once for all heads.
+// A form for keys of which every head has its own part and all heads share a second, rotated one (ROT): the keys have a further
+// sub-tile of 64 channels, read from a matrix of its own once for all heads; the queries' part is rotated by the softmax threads, a
+// row each, into tensor memory as two bfloat16 pieces, x = hi + lo, both A operands against the shared sub-tile.  Behind a window it
+// also takes the probabilities as two pieces (PAIR): it stands in for a kernel on the latents themselves (attention_latent_tokens.cu)
+// that has both from float32, and is with them no further from 64 bits than that one (relative error of a layer of 2,048 tokens, 16
+// heads: 4.10e-3 against 4.16e-3; without the second pieces 4.41e-3).  With heads of 128 channels one CTA holds an SM.
 //
 // Every mbarrier wait gives up after about two seconds and records where in an error word.
 #include <cuda.h>
@@ -36,20 +40,20 @@ namespace {
 constexpr int QROWS = 128;                   // queries per CTA
 // Sizes that follow from the head size.  A tile row of more than 64 dims lies in shared memory as
 // sub-tiles of 64 dims (128 bytes, the widest row the 128-byte swizzle takes), one after the other.
-// ROT (0 or 64): channels of the shared part of queries and keys, a sub-tile behind the others.
-template <int HD, int ROT = 0>
+// ROT (0 or 64): channels of the shared part of queries and keys, a sub-tile of the keys behind the others.  PAIR: P in two pieces.
+template <int HD, int ROT = 0, bool PAIR = false>
 struct Shape {
     static constexpr int KEYS = (HD == 64) == (ROT == 0) ? 128 : 64;     // keys per tile: two CTAs must fit an SM (HD 128 with ROT: one)
-    static constexpr int SUBS = HD / 64, QK_SUBS = (HD + ROT) / 64;      // sub-tiles of 64 dims: of values, of queries and keys
+    static constexpr int SUBS = HD / 64, K_SUBS = (HD + ROT) / 64;       // sub-tiles of 64 dims: of queries and values, of keys
     static constexpr int SUB_Q = QROWS * 128, SUB_KV = KEYS * 128; // bytes of a sub-tile
-    static constexpr int Q_BYTES = QK_SUBS * SUB_Q, K_BYTES = QK_SUBS * SUB_KV, STAGE_BYTES = K_BYTES + SUBS * SUB_KV;
+    static constexpr int Q_BYTES = SUBS * SUB_Q, K_BYTES = K_SUBS * SUB_KV, STAGE_BYTES = K_BYTES + SUBS * SUB_KV;
     static constexpr int O_COL = KEYS;       // S at columns 0..KEYS-1, O after it, P (bfloat16 pairs) after O
-    static constexpr int P_COL = KEYS + HD;
-    static constexpr int TMEM_COLS = P_COL + KEYS / 2 <= 256 ? 256 : 512;
+    static constexpr int P_COL = KEYS + HD, ROT_COL = P_COL + (PAIR ? KEYS : KEYS / 2);    // P's second piece after the first; rotated queries
+    static constexpr int TMEM_USED = ROT_COL + ROT, TMEM_COLS = TMEM_USED <= 256 ? 256 : 512;
     static constexpr int CTAS = TMEM_COLS == 256 ? 2 : 1;                // on an SM
     static_assert(HD == 64 || HD == 128, "head sizes 64 and 128");
     static_assert(ROT == 0 || ROT == 64, "one shared sub-tile or none");
-    static_assert(P_COL + KEYS / 2 <= TMEM_COLS, "S, O and P must fit the allocation");
+    static_assert(TMEM_USED <= TMEM_COLS, "S, O, P and the rotated queries must fit the allocation");
 };
 constexpr int SOFTMAX_WARPS = 8;             // two threads a query row: each takes half of the tile's keys and half of O's dims
 constexpr int PRODUCER_WARP = SOFTMAX_WARPS, MMA_WARP = SOFTMAX_WARPS + 1, THREADS = (SOFTMAX_WARPS + 2) * 32;
@@ -190,6 +194,12 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// Two numbers as pairs of bfloat16 pieces, x = hi + lo to 2^-17 of x.
+__device__ __forceinline__ void pack_pair(float x0, float x1, uint32_t& hi, uint32_t& lo) {
+    hi = pack_bf16(x0, x1);
+    lo = pack_bf16(x0 - __uint_as_float(hi << 16), x1 - __uint_as_float(hi & 0xffff0000u));
+}
+
 // The two softmax warps of a quadrant meet at a named barrier of their own (ids 1..4; 0 is __syncthreads).
 __device__ __forceinline__ void pair_barrier(int quadrant) {
     switch (quadrant) {
@@ -225,8 +235,15 @@ struct FlashParams {
     float sink2;                      // a score (times log2(e)) that joins the softmax's sum without a key or a value; -inf: none
     // keys and values in matrices of their own instead of pages: [rows, nkv * HD], request s's key j in row kv_start[s] + j
     const int* kv_start;              // null: keys and values come from the paged pools
+    const unsigned char* odd_rows;    // BOUNDED, [odd_count], not null: 1 where a key stands for NaN (a query that sees it comes out NaN)
+    int odd_count;
     int q_head_cols;                  // columns of a head in q's rows (HD, and more where q holds other parts between the heads)
     const float* sinks;               // [nh], not null: a sink a head, in place of sink2
+    // ROT: the queries' channels HD .. HD + rot - 1 of a head are rotated here, by halves
+    const __nv_bfloat16* q;
+    long long q_stride;
+    const float2* turn;               // [T, 32] cosine and sine of a token's angles
+    int rot;
 };
 
 // SIG: a visible key's weight is sigmoid(score * scale - slope (position - key) + bias): no maximum, no sum, no
@@ -234,18 +251,19 @@ struct FlashParams {
 // This form and BOUNDED take a window: the first key tile is the one that holds the first key the tile's first query sees.
 // BOUNDED: softmax as in the plain form; a row's keys begin at first_visible(position); capped scores go through
 // tanh in registers before the maximum is taken.
-// ROT: map_q_rot [T, nh * 64] and map_k_rot [keys, <= 64] are the shared part of queries and keys (dense keys only).
+// ROT: map_k_rot [keys, <= 64] is the shared part of the keys (dense keys only).
 template <int HD, int FORM, int ROT>
-__global__ void __launch_bounds__(THREADS, (Shape<HD, ROT>::CTAS)) prefill_attention_tcgen05_kernel(
+__global__ void __launch_bounds__(THREADS, (Shape<HD, ROT, FORM == BOUNDED && ROT != 0>::CTAS)) prefill_attention_tcgen05_kernel(
         const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-        const __grid_constant__ CUtensorMap map_q_rot, const __grid_constant__ CUtensorMap map_k_rot, FlashParams p) {
-    using S_ = Shape<HD, ROT>;
+        const __grid_constant__ CUtensorMap map_k_rot, FlashParams p) {
+    constexpr bool PAIR = FORM == BOUNDED && ROT != 0;
+    using S_ = Shape<HD, ROT, PAIR>;
     constexpr int TMEM_COLS = S_::TMEM_COLS;
     constexpr bool SIG = FORM == SIGMOID, LOW = FORM == BOUNDED;
     constexpr int KEYS = S_::KEYS, SUBS = S_::SUBS, SUB_Q = S_::SUB_Q, SUB_KV = S_::SUB_KV, Q_BYTES = S_::Q_BYTES,
                   K_BYTES = S_::K_BYTES, STAGE_BYTES = S_::STAGE_BYTES, O_COL = S_::O_COL, P_COL = S_::P_COL;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t q_full, kv_full[2], stage_free[2], s_done, p_ready, all_done;
+    __shared__ __align__(8) uint64_t q_full, kv_full[2], stage_free[2], s_done, p_ready, all_done, rot_ready;
     __shared__ uint32_t tmem_base_slot;
     __shared__ int failed;
     __shared__ float half_max[2][2][QROWS];          // [tile parity][half][row]: the two threads of a row exchange their maxima
@@ -276,7 +294,8 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT>::CTAS)) prefill_atten
     const int nv = LOW ? p.value_heads : p.nkv, vh = LOW ? kvh / (p.nkv / p.value_heads) : kvh;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int* table = p.block_table + (long long)seq * p.table_width;
-    const int dense_row0 = p.kv_start ? p.kv_start[seq] : -1;
+    const bool dense = p.kv_start != nullptr;
+    const int dense_row0 = dense ? p.kv_start[seq] : 0;
 
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* q_tile = base;
@@ -291,6 +310,7 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT>::CTAS)) prefill_atten
         mbar_init(&s_done, 1);
         mbar_init(&p_ready, SOFTMAX_WARPS * 32);
         mbar_init(&all_done, 1);
+        if (ROT) mbar_init(&rot_ready, SOFTMAX_WARPS * 32);
         failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -312,7 +332,6 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT>::CTAS)) prefill_atten
         mbar_expect_tx(&q_full, Q_BYTES);
 #pragma unroll
         for (int h = 0; h < SUBS; ++h) tma_load_2d(q_tile + h * SUB_Q, &map_q, &q_full, head * p.q_head_cols + h * 64, q_begin + row0);
-        if (ROT) tma_load_2d(q_tile + SUBS * SUB_Q, &map_q_rot, &q_full, head * 64, q_begin + row0);
         for (int j = kv_begin; j < num_kv; ++j) {
             const int it = j - kv_begin, s = it & 1;
             if (!mbar_wait(&stage_free[s], ((it >> 1) & 1) ^ 1, p.error, 11)) { failed = 1; break; }
@@ -323,7 +342,7 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT>::CTAS)) prefill_atten
             for (int b = 0; b < KEYS / 64; ++b) {    // boxes of 64 keys x 64 dims: a box never crosses a page
                 const int key = j * KEYS + b * 64;
                 int row, v_row, col = 0, v_col = 0;
-                if (dense_row0 >= 0) {               // rows past the request's last key belong to the next request, or to nobody
+                if (dense) {                         // rows past the request's last key belong to the next request, or to nobody
                     row = v_row = dense_row0 + key;  // (the copy fills those with zeros): masked anyway
                     col = kvh * HD;
                     v_col = vh * HD;
@@ -346,17 +365,23 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT>::CTAS)) prefill_atten
         const uint32_t idesc_s = instr_desc(QROWS, KEYS, false);
         const uint32_t idesc_o = instr_desc(QROWS, 64, true);        // O in column blocks of 64 dims, one per sub-tile of V
         bool ok = mbar_wait(&q_full, 0, p.error, 12);
+        if (ROT) ok = ok && mbar_wait(&rot_ready, 0, p.error, 18);
         // S = Q K^T of tile j, once its keys have landed
         auto issue_scores = [&](int it) -> bool {
             const int s = it & 1;
             if (!mbar_wait(&kv_full[s], (it >> 1) & 1, p.error, 13)) return false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-            for (int h = 0; h < S_::QK_SUBS; ++h) {
+            for (int h = 0; h < SUBS; ++h) {
                 const uint64_t q_desc = smem_desc(q_tile + h * SUB_Q);
                 const uint64_t k_desc = smem_desc(kv_tiles + s * STAGE_BYTES + h * SUB_KV);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) umma_ss(tmem, q_desc + 2 * k, k_desc + 2 * k, idesc_s, (h | k) != 0);
+            }
+            if (ROT) {                               // 16 channels are 8 columns of packed queries: four of the first piece, four of the second
+                const uint64_t k_desc = smem_desc(kv_tiles + s * STAGE_BYTES + SUBS * SUB_KV);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) umma_ts(tmem, tmem + S_::ROT_COL + 8 * k, k_desc + 2 * (k & 3), idesc_s, 1);
             }
             umma_commit(&s_done);
             return true;
@@ -377,6 +402,11 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT>::CTAS)) prefill_atten
 #pragma unroll
                 for (int k = 0; k < KEYS / 16; ++k)
                     umma_ts(tmem + O_COL + 64 * h, tmem + P_COL + 8 * k, v_desc + 128 * k, idesc_o, (j | k) != 0);
+                if (PAIR) {
+#pragma unroll
+                    for (int k = 0; k < KEYS / 16; ++k)
+                        umma_ts(tmem + O_COL + 64 * h, tmem + P_COL + KEYS / 2 + 8 * k, v_desc + 128 * k, idesc_o, 1);
+                }
             }
             umma_commit(&stage_free[s]);
         }
@@ -399,9 +429,56 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT>::CTAS)) prefill_atten
         const float slope2 = SIG && p.slopes ? p.slopes[head] * LOG2E : 0.f;
         const float bias2 = (SIG && p.head_bias ? p.head_bias[head] * LOG2E : 0.f) - slope2 * (float)pos;
         bool ok = true;
+        if constexpr (ROT != 0) {                    // this thread's half of the row's rotated channels, 32 of them
+            float x[32];
+            const long long t = q_begin + row0 + r;
+            const __nv_bfloat16* qr = p.q + t * p.q_stride + (long long)head * p.q_head_cols + HD;
+            const float2* turn = p.turn + t * 32;
+            if (p.rot == 64 && r < rows) {
+#pragma unroll
+                for (int c = 0; c < 32; c += 8) {
+                    const uint4 u4 = *reinterpret_cast<const uint4*>(qr + c), v4 = *reinterpret_cast<const uint4*>(qr + 32 + c);
+                    const __nv_bfloat16 *u = reinterpret_cast<const __nv_bfloat16*>(&u4), *v = reinterpret_cast<const __nv_bfloat16*>(&v4);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const float2 cs = turn[c + e];
+                        const float a = __bfloat162float(u[e]), b = __bfloat162float(v[e]);
+                        x[c + e] = half == 0 ? a * cs.x - b * cs.y : b * cs.x + a * cs.y;
+                    }
+                }
+            } else {
+                const int pairs = p.rot / 2;
+#pragma unroll
+                for (int c = 0; c < 32; ++c) {
+                    const int d = half * 32 + c, i = d < pairs ? d : d - pairs;
+                    x[c] = 0.f;
+                    if (r < rows && d < p.rot) {
+                        const float2 cs = turn[i];
+                        const float a = __bfloat162float(qr[i]), b = __bfloat162float(qr[i + pairs]);
+                        x[c] = d < pairs ? a * cs.x - b * cs.y : b * cs.x + a * cs.y;
+                    }
+                }
+            }
+            uint32_t hi[16], lo[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) pack_pair(x[2 * i], x[2 * i + 1], hi[i], lo[i]);
+            tmem_st16(lane_addr + S_::ROT_COL + half * 16, hi);
+            tmem_st16(lane_addr + S_::ROT_COL + 32 + half * 16, lo);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            mbar_arrive(&rot_ready);
+        }
         for (int j = kv_begin; j < num_kv; ++j) {
             const int it = j - kv_begin, s = it & 1;
             const int key0 = j * KEYS;
+            uint32_t odd[HK / 32] = {};              // which of this thread's keys stand for NaN
+            if (LOW && p.odd_rows) {
+#pragma unroll
+                for (int ch = 0; ch < HK / 32; ++ch) {
+                    const int row = dense_row0 + key0 + col0 + ch * 32 + lane;
+                    odd[ch] = row >= 0 && row < p.odd_count ? p.odd_rows[row] : 0;
+                }
+            }
             // a wait that ran out: the warp (as one) skips the work of this and the later tiles but still meets its
             // partner at the barrier below and still arrives at p_ready, so that nobody is left waiting for it
             if (ok && !mbar_wait(&s_done, it & 1, p.error, 15)) ok = false;
@@ -474,6 +551,17 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT>::CTAS)) prefill_atten
                         for (int i = 0; i < 32; ++i)
                             sv[ch][i] = __float_as_uint(exp_tanh(__uint_as_float(sv[ch][i]) * p.cap_pre));
                 }
+                if (p.odd_rows) {
+#pragma unroll
+                    for (int ch = 0; ch < HK / 32; ++ch) {
+                        const uint32_t bits = __ballot_sync(0xffffffffu, odd[ch] != 0);
+                        if (bits) {                  // hardly ever: such a score is NaN, and with it the row that sees it
+#pragma unroll
+                            for (int i = 0; i < 32; ++i)
+                                if (bits >> i & 1) sv[ch][i] = 0x7fffffffu;
+                        }
+                    }
+                }
             }
             // pass 1: the maximum over them (four running maxima: no long dependent chain)
 #pragma unroll
@@ -518,7 +606,7 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT>::CTAS)) prefill_atten
 #pragma unroll
                 for (int ch = 0; ch < HK / 32; ++ch) {
                     const int c = col0 + ch * 32;
-                    uint32_t packed[16];
+                    uint32_t packed[16], rest[16];
                     const uint32_t (&v)[32] = sv[ch];
 #pragma unroll
                     for (int i = 0; i < 32; i += 2) {
@@ -527,24 +615,28 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT>::CTAS)) prefill_atten
                         if (key0 + c + i > pos || (LOW && key0 + c + i < lo)) p0 = 0.f;
                         if (key0 + c + i + 1 > pos || (LOW && key0 + c + i + 1 < lo)) p1 = 0.f;
                         l4[(i >> 1) & 3] += p0 + p1;
-                        packed[i >> 1] = pack_bf16(p0, p1);
+                        if (PAIR) pack_pair(p0, p1, packed[i >> 1], rest[i >> 1]);
+                        else packed[i >> 1] = pack_bf16(p0, p1);
                     }
                     tmem_st16(lane_addr + P_COL + (c >> 1), packed);
+                    if (PAIR) tmem_st16(lane_addr + P_COL + KEYS / 2 + (c >> 1), rest);
                 }
             } else {
 #pragma unroll
                 for (int ch = 0; ch < HK / 32; ++ch) {
                     const int c = col0 + ch * 32;
-                    uint32_t packed[16];
+                    uint32_t packed[16], rest[16];
                     const uint32_t (&v)[32] = sv[ch];
 #pragma unroll
                     for (int i = 0; i < 32; i += 2) {
                         const float p0 = fast_exp2(fmaf(__uint_as_float(v[i]), p.scale_log2, -m_use));
                         const float p1 = fast_exp2(fmaf(__uint_as_float(v[i + 1]), p.scale_log2, -m_use));
                         l4[(i >> 1) & 3] += p0 + p1;
-                        packed[i >> 1] = pack_bf16(p0, p1);
+                        if (PAIR) pack_pair(p0, p1, packed[i >> 1], rest[i >> 1]);
+                        else packed[i >> 1] = pack_bf16(p0, p1);
                     }
                     tmem_st16(lane_addr + P_COL + (c >> 1), packed);
+                    if (PAIR) tmem_st16(lane_addr + P_COL + KEYS / 2 + (c >> 1), rest);
                 }
             }
             l_run = l_run * corr + ((l4[0] + l4[1]) + (l4[2] + l4[3]));
@@ -657,10 +749,10 @@ TS_API int ts_attention_tcgen05_supported(int hd, int page_tokens, int nh, int n
 
 namespace {
 
-// The part of queries and keys beside the heads' own: q_rot [T, nh * 64] (zeros past `rot` channels of a head), k_rot rows of
-// `rot` channels, k_rot_stride elements apart; sinks [nh] or null.
+// The part of queries and keys beside the heads' own: the `rot` channels of a query head behind its first hd, rotated by `turn` [T, 32]
+// (cosine, sine), and k_rot rows of `rot` channels, k_rot_stride elements apart; sinks [nh] or null.
 struct SharedPart {
-    const void* q_rot;
+    const float2* turn;
     const void* k_rot;
     long long k_rot_stride;
     int rot;                          // 0: no such part
@@ -674,7 +766,8 @@ int run_prefill(const void* q, long long q_cols, long long q_stride, void* out, 
                 float scale, const int* prefill_seqs, int num_prefill_seqs, int* error, bool sigmoid, int window,
                 const float* slopes, const float* head_bias, const void* gate, long long gate_stride, cudaStream_t stream,
                 bool bounded = false, int chunk = 0, float softcap = 0.f, int value_heads = 0, const int* kv_start = nullptr,
-                long long dense_rows = 0, float sink = -INFINITY, const SharedPart* shared = nullptr) {
+                long long dense_rows = 0, float sink = -INFINITY, const SharedPart* shared = nullptr, long long dense_stride = 0,
+                const unsigned char* odd_rows = nullptr) {
     TS_REQUIRE(ts_attention_tcgen05_supported(hd, page_tokens, nh, nkv, 0), "attention_tcgen05: sizes not taken (head_dim %d, page %d)", hd, page_tokens);
     TS_REQUIRE(sigmoid || bounded || window == 0, "attention_tcgen05: the plain form takes no window");
     TS_REQUIRE(window >= 0 && chunk >= 0 && softcap >= 0.f, "attention_tcgen05: a negative window, chunk or cap");
@@ -691,31 +784,34 @@ int run_prefill(const void* q, long long q_cols, long long q_stride, void* out, 
     if (prefill_seqs != nullptr && num_prefill_seqs == 0) return 0;
     const long long pool_rows = (long long)num_pages * entries * nkv * page_tokens;
     TS_REQUIRE(pool_rows < 0x7fffffffll, "attention_tcgen05: the pool has too many rows for 32-bit TMA coordinates");
-    CUtensorMap map_q, map_k, map_v, map_q_rot, map_k_rot;
+    CUtensorMap map_q, map_k, map_v, map_k_rot;
     if (make_map(&map_q, q, num_tokens, q_cols, q_stride, QROWS)) return 1;
     if (kv_start != nullptr) {                           // matrices [dense_rows, heads * hd]
         TS_REQUIRE(dense_rows > 0 && dense_rows < 0x7fffffffll, "attention_tcgen05: %lld rows of keys", dense_rows);
-        if (make_map(&map_k, k_pool, dense_rows, (long long)nkv * hd, (long long)nkv * hd, 64)) return 1;
-        if (make_map(&map_v, v_pool, dense_rows, (long long)value_heads * hd, (long long)value_heads * hd, 64)) return 1;
+        TS_REQUIRE(dense_stride >= (long long)nkv * hd && dense_stride % 8 == 0, "attention_tcgen05: key and value rows %lld elements apart", dense_stride);
+        if (make_map(&map_k, k_pool, dense_rows, (long long)nkv * hd, dense_stride, 64)) return 1;
+        if (make_map(&map_v, v_pool, dense_rows, (long long)value_heads * hd, dense_stride, 64)) return 1;
     } else {
         if (make_map(&map_k, k_pool, pool_rows, hd, hd, 64)) return 1;
         if (make_map(&map_v, v_pool, pool_rows / nkv * value_heads, hd, hd, 64)) return 1;
     }
     const int rot = shared ? shared->rot : 0;
     if (rot > 0) {
-        TS_REQUIRE(kv_start != nullptr && !sigmoid && !bounded, "attention_tcgen05: a shared key part comes with dense keys in the plain form");
-        TS_REQUIRE(rot <= 64 && rot % 8 == 0 && shared->q_head_cols % 8 == 0 && shared->k_rot_stride % 8 == 0 &&
-                   (uintptr_t)shared->q_rot % 16 == 0 && (uintptr_t)shared->k_rot % 16 == 0,
+        TS_REQUIRE(kv_start != nullptr && !sigmoid, "attention_tcgen05: a shared key part comes with dense keys and softmax");
+        TS_REQUIRE(rot <= 64 && rot % 8 == 0 && shared->q_head_cols % 8 == 0 && shared->q_head_cols >= hd + rot && shared->k_rot_stride % 8 == 0 &&
+                   (uintptr_t)shared->turn % 8 == 0 && (uintptr_t)shared->k_rot % 16 == 0,
                    "attention_tcgen05: a shared key part of %d channels, or its alignment", rot);
-        if (make_map(&map_q_rot, shared->q_rot, num_tokens, (long long)nh * 64, (long long)nh * 64, QROWS)) return 1;
         if (make_map(&map_k_rot, shared->k_rot, dense_rows, rot, shared->k_rot_stride, 64)) return 1;
     } else {
-        map_q_rot = map_q;                               // not read
-        map_k_rot = map_k;
+        map_k_rot = map_k;                               // not read
     }
     FlashParams p;
     p.q_head_cols = shared ? shared->q_head_cols : hd;
     p.sinks = shared ? shared->sinks : nullptr;
+    p.q = (const __nv_bfloat16*)q;
+    p.q_stride = q_stride;
+    p.turn = shared ? shared->turn : nullptr;
+    p.rot = rot;
     p.out = (__nv_bfloat16*)out;
     p.block_table = block_table;
     p.table_width = table_width;
@@ -734,6 +830,8 @@ int run_prefill(const void* q, long long q_cols, long long q_stride, void* out, 
     p.value_heads = value_heads;
     p.sink2 = sink > -INFINITY ? sink * LOG2E : -INFINITY;
     p.kv_start = kv_start;
+    p.odd_rows = odd_rows;
+    p.odd_count = (int)dense_rows;
     p.error = error;
     p.window = window;
     p.slopes = slopes;
@@ -743,13 +841,16 @@ int run_prefill(const void* q, long long q_cols, long long q_stride, void* out, 
     dim3 grid(nh, (max_q_len + QROWS - 1) / QROWS, prefill_seqs ? num_prefill_seqs : num_seqs);
 #define TS_FLASH_LAUNCH(HD, FORM, ROT)                                                                                    \
     do {                                                                                                                  \
-        const size_t smem = (size_t)Shape<HD, ROT>::Q_BYTES + 2 * Shape<HD, ROT>::STAGE_BYTES + 1024;                     \
+        using Sizes = Shape<HD, ROT, (FORM) == BOUNDED && (ROT) != 0>;                                                    \
+        const size_t smem = (size_t)Sizes::Q_BYTES + 2 * Sizes::STAGE_BYTES + 1024;                                       \
         auto kernel = prefill_attention_tcgen05_kernel<HD, FORM, ROT>;                                                    \
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                             \
         TS_CHAINED_CHECK("attention_tcgen05", launch_chained(kernel, grid, dim3(THREADS), smem, stream, map_q, map_k, map_v, \
-                                                             map_q_rot, map_k_rot, p));                                   \
+                                                             map_k_rot, p));                                              \
     } while (0)
-    if (hd == 64 && rot > 0) TS_FLASH_LAUNCH(64, PLAIN, 64);
+    if (hd == 64 && rot > 0 && bounded) TS_FLASH_LAUNCH(64, BOUNDED, 64);
+    else if (rot > 0 && bounded) TS_FLASH_LAUNCH(128, BOUNDED, 64);
+    else if (hd == 64 && rot > 0) TS_FLASH_LAUNCH(64, PLAIN, 64);
     else if (rot > 0) TS_FLASH_LAUNCH(128, PLAIN, 64);
     else if (hd == 64 && sigmoid) TS_FLASH_LAUNCH(64, SIGMOID, 0);
     else if (hd == 64 && bounded) TS_FLASH_LAUNCH(64, BOUNDED, 0);
@@ -814,22 +915,26 @@ TS_API int ts_prefill_attention_tcgen05_masked(const void* q, long long q_stride
 }
 
 // Causal softmax attention of prompt portions over keys and values that lie in matrices of their own,
-// k [kv_rows, nkv * hd] and v [kv_rows, nkv * hd] (bfloat16, rows back to back), request s's key j in row kv_start[s] + j
+// k and v [kv_rows, nkv * hd] (bfloat16, rows kv_stride elements apart), request s's key j in row kv_start[s] + j
 // (kv_start: int32 [num_seqs] on the device; ctx_lens[s] keys a request).  For keys and values that are worked out
 // for the step instead of read from pages.  Queries [T, q_stride] in a matrix of their own, head h's hd columns from
-// h * q_head_cols on.  With `rot` > 0 a score also has q_rot . k_rot, q_rot [T, nh * 64] (a head's channels past `rot` zero)
-// and k_rot one row of `rot` channels a key for all heads, k_rot_stride elements apart, in the same row order as k.
+// h * q_head_cols on.  With `rot` > 0 a score also has q_rot . k_rot, q_rot the `rot` channels behind those hd, rotated by halves by `turn`
+// [T, 32] (cosine and sine of a token's angles, times whatever magnitude), and k_rot one row of `rot` channels a key for all heads,
+// k_rot_stride elements apart, in the same row order as k.
 // `sinks` [nh] (null: none): a score a head that joins every softmax's sum without a key or a value.
+// `window` n > 0: query i sees keys i - n + 1 .. i; rows of keys no query of the step sees need not be there (kv_start may then be
+// negative), and `odd_rows` [kv_rows] (null: none) marks keys that stand for NaN, whose rows of k and v hold zeros.
 TS_API int ts_prefill_attention_tcgen05_dense(const void* q, long long q_stride, void* out, const void* k, const void* v,
-                                              long long kv_rows, const int* kv_start, const int* cu_q, const int* ctx_lens,
-                                              int num_seqs, int num_tokens, int max_q_len, int nh, int nkv, int hd,
-                                              float scale, const int* prefill_seqs, int num_prefill_seqs, int* error,
-                                              int q_head_cols, const void* q_rot, const void* k_rot, long long k_rot_stride, int rot,
-                                              const float* sinks, cudaStream_t stream) {
+                                              long long kv_rows, long long kv_stride, const int* kv_start, const int* cu_q,
+                                              const int* ctx_lens, int num_seqs, int num_tokens, int max_q_len, int nh, int nkv, int hd,
+                                              float scale, int window, const unsigned char* odd_rows, const int* prefill_seqs,
+                                              int num_prefill_seqs, int* error, int q_head_cols, const float* turn, const void* k_rot,
+                                              long long k_rot_stride, int rot, const float* sinks, cudaStream_t stream) {
     TS_REQUIRE(kv_start != nullptr, "attention_tcgen05: the first rows of the requests' keys are needed");
-    TS_REQUIRE(q_head_cols >= hd && (rot == 0 || (q_rot && k_rot)), "attention_tcgen05: the queries' columns, or the shared key part");
-    const SharedPart shared{q_rot, k_rot, k_rot_stride, rot, q_head_cols, sinks};
+    TS_REQUIRE(q_head_cols >= hd && (rot == 0 || (turn && k_rot)), "attention_tcgen05: the queries' columns, or the shared key part");
+    TS_REQUIRE((odd_rows == nullptr || window > 0) && (window == 0 || rot > 0), "attention_tcgen05: a window comes with a shared key part, marked keys with a window");
+    const SharedPart shared{(const float2*)turn, k_rot, k_rot_stride, rot, q_head_cols, sinks};
     return run_prefill(q, (long long)nh * q_head_cols, q_stride, out, k, v, 1, 1, 0, 64, nullptr, 1, cu_q, ctx_lens, num_seqs, num_tokens,
-                       max_q_len, nh, nkv, hd, scale, prefill_seqs, num_prefill_seqs, error, false, 0, nullptr, nullptr,
-                       nullptr, 0, stream, false, 0, 0.f, 0, kv_start, kv_rows, -INFINITY, &shared);
+                       max_q_len, nh, nkv, hd, scale, prefill_seqs, num_prefill_seqs, error, false, window, nullptr, nullptr, nullptr, 0,
+                       stream, window > 0, 0, 0.f, 0, kv_start, kv_rows, -INFINITY, &shared, kv_stride, odd_rows);
 }

@@ -34,8 +34,8 @@ _SIGNATURES = {
     "ts_paged_attention_bf16_sigmoid": ("int", "pl" "ppp" "lliipippiiiiiiifiplpi" "pppl" "p"),
     "ts_paged_attention_bf16_masked": ("int", "pl" "ppp" "lllliipippiiiiiiifiifi" "plpi" "fp"),
     "ts_attention_tcgen05_supported": ("int", "iiiii"),
-    "ts_prefill_attention_tcgen05_dense": ("int", "pl" "ppp" "lpppiiiiiifpip" "ipplip" "p"),
-    "ts_latent_rotate_queries": ("int", "pliipfppiiip"),
+    "ts_prefill_attention_tcgen05_dense": ("int", "pl" "ppp" "llpppiiiiiif" "ippip" "ipplip" "p"),
+    "ts_latent_gather": ("int", "plliipipppiiiiipfplppppp"),
     "ts_prefill_attention_tcgen05_masked": ("int", "pl" "ppp" "iiiipippiiiiiifiifi" "pipfp"),
     "ts_prefill_attention_tcgen05": ("int", "ppppiiiipippiiiiiifpipp"),
     "ts_prefill_attention_tcgen05_sigmoid": ("int", "pl" "ppp" "iiiipippiiiiiifi" "pppl" "pipp"),
@@ -858,34 +858,44 @@ class Ops:
 
     def dense_prompt_attention(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, kv_start: torch.Tensor, ctx, nh: int,
                                nkv: int, hd: int, scale: float, out: torch.Tensor | None = None, *, q_head_cols: int = 0,
-                               shared: tuple[torch.Tensor, torch.Tensor] | None = None, sink: torch.Tensor | None = None) -> torch.Tensor:
+                               shared: tuple[torch.Tensor, torch.Tensor] | None = None, sink: torch.Tensor | None = None,
+                               window: int = 0, odd_rows: torch.Tensor | None = None) -> torch.Tensor:
         """
         Causal softmax attention of the step's prompt portions (requests that feed more than one token) over keys
-        and values worked out for the step: k, v [rows, nkv * hd] bfloat16, request s's key j in row kv_start[s] + j
-        (int32 [requests] on the device), ctx.ctx_lens[s] keys a request.  Rows of requests that feed one token are
+        and values worked out for the step: k, v [rows, nkv * hd] bfloat16 (stretches of one row stride), request s's key j in row
+        kv_start[s] + j (int32 [requests] on the device), ctx.ctx_lens[s] keys a request.  Rows of requests that feed one token are
         left as they are in `out` ([T, nh * hd]; made here if not given).  The tcgen05 prompt kernel.
 
-        `q_head_cols` (0: hd): columns of a head in q's rows, its first hd being the ones that meet k.  `shared` (q_rot
-        [T, nh * 64], k_rot [rows, rot <= 64]): a score also has q_rot . k_rot, k_rot being the same for all heads and
-        q_rot's channels past rot zero.  `sink` (float32 [nh]): exp(sink[h]) joins every softmax's sum of head h.
+        `q_head_cols` (0: hd): columns of a head in q's rows, its first hd being the ones that meet k.  `shared` (turn
+        float32 [T, 32, 2], k_rot [rows, rot <= 64]): a score also has q_rot . k_rot, k_rot being the same for all heads and q_rot the
+        head's next rot columns, rotated by halves by the cosines and sines in turn.  `sink` (float32 [nh]): exp(sink[h]) joins every softmax's sum of head h.
+        `window` n > 0 (with `shared`): a query sees its own key and the n - 1 before it; with `odd_rows` (uint8 [rows]) keys marked there stand for
+        NaN and their rows of k and v hold zeros.
         """
         q_head_cols = q_head_cols or hd
         self._check_rows(q, "q")
-        self._check(k, "k", torch.bfloat16, 2)
-        self._check(v, "v", torch.bfloat16, 2)
+        self._check_rows(k, "k")
+        self._check_rows(v, "v")
+        if k.dtype != torch.bfloat16 or v.dtype != torch.bfloat16 or k.stride(0) != v.stride(0):
+            raise KernelError(f"dense_prompt_attention: k and v are bfloat16 with one row stride, not {k.dtype}, {v.dtype}, {k.stride(0)}, {v.stride(0)}")
+        if odd_rows is not None:
+            self._check(odd_rows, "odd_rows", torch.uint8, 1)
+            if odd_rows.shape[0] != k.shape[0]:
+                raise KernelError(f"dense_prompt_attention: {odd_rows.shape[0]} marks for {k.shape[0]} keys")
         self._check(kv_start, "kv_start", torch.int32, 1)
         if k.shape != v.shape or k.shape[1] != nkv * hd or q.shape[1] != nh * q_head_cols or kv_start.shape[0] != ctx.ctx_lens.shape[0]:
             raise KernelError(f"dense_prompt_attention: q {tuple(q.shape)}, k {tuple(k.shape)}, v {tuple(v.shape)} for "
                               f"{nh}:{nkv} heads of {hd}")
         if not self.dense_prompt_attention_supported(q, nh, nkv, hd):
             raise KernelError(f"dense_prompt_attention: sizes not taken ({nh}:{nkv} heads of {hd}, {q.dtype})")
-        q_rot = k_rot = None
+        turn = k_rot = None
         if shared is not None:
-            q_rot, k_rot = shared
-            self._check(q_rot, "q_rot", torch.bfloat16, 2)
+            turn, k_rot = shared
+            self._check(turn, "turn", torch.float32, 3)
             self._check_rows(k_rot, "k_rot")
-            if tuple(q_rot.shape) != (q.shape[0], nh * 64) or k_rot.shape[0] != k.shape[0] or k_rot.shape[1] > 64 or k_rot.dtype != torch.bfloat16:
-                raise KernelError(f"dense_prompt_attention: a shared part of {tuple(q_rot.shape)} and {tuple(k_rot.shape)}")
+            if (tuple(turn.shape) != (q.shape[0], 32, 2) or k_rot.shape[0] != k.shape[0] or k_rot.shape[1] > q_head_cols - hd
+                    or k_rot.shape[1] > 64 or k_rot.dtype != torch.bfloat16):
+                raise KernelError(f"dense_prompt_attention: a shared part of {tuple(turn.shape)} and {tuple(k_rot.shape)}")
         if sink is not None:
             self._check(sink, "sink", torch.float32, 1)
             if sink.shape[0] != nh:
@@ -895,21 +905,41 @@ class Ops:
         prefill_seqs = getattr(ctx, "prefill_seqs", None)
         num_prefill = prefill_seqs.shape[0] if prefill_seqs is not None else 0
         self._call("ts_prefill_attention_tcgen05_dense", _ptr(q), q.stride(0), _ptr(out), _ptr(k), _ptr(v), k.shape[0],
-                   _ptr(kv_start), _ptr(ctx.cu_q), _ptr(ctx.ctx_lens), ctx.ctx_lens.shape[0], q.shape[0], ctx.max_q_len, nh, nkv,
-                   hd, scale, _ptr(prefill_seqs), num_prefill, self.error_word().data_ptr(), q_head_cols, _ptr(q_rot), _ptr(k_rot),
+                   k.stride(0), _ptr(kv_start), _ptr(ctx.cu_q), _ptr(ctx.ctx_lens), ctx.ctx_lens.shape[0], q.shape[0], ctx.max_q_len,
+                   nh, nkv, hd, scale, window, _ptr(odd_rows), _ptr(prefill_seqs), num_prefill, self.error_word().data_ptr(), q_head_cols, _ptr(turn), _ptr(k_rot),
                    k_rot.stride(0) if k_rot is not None else 0, k_rot.shape[1] if k_rot is not None else 0, _ptr(sink), _stream())
         return out
 
-    def latent_rotate_queries(self, q: torch.Tensor, ctx, heads: int, head_width: int, rot_offset: int, rot: int,
-                              freq: torch.Tensor, magnitude: float) -> torch.Tensor:
-        """bfloat16 [T, heads * 64]: every head's `rot` channels of q from `rot_offset` on, rotated by halves, zeros behind them."""
-        self._check_rows(q, "q")
-        if q.dtype != torch.bfloat16 or q.shape[1] != heads * head_width or not 0 < rot <= 64:
-            raise KernelError(f"latent_rotate_queries: q {tuple(q.shape)} {q.dtype}, {heads} heads of {head_width}, rotation over {rot}")
-        out = torch.empty((q.shape[0], heads * 64), dtype=q.dtype, device=q.device)
-        self._call("ts_latent_rotate_queries", _ptr(q), q.stride(0), head_width, rot_offset, _ptr(freq), float(magnitude),
-                   _ptr(ctx.positions), _ptr(out), q.shape[0], heads, rot, _stream())
-        return out
+    def latent_gather(self, ctx, binding, rows: int, max_keys: int, rank: int, rot: int, window: int, freq: torch.Tensor | None,
+                      magnitude: float = 1.0) -> tuple[torch.Tensor, tuple | None, torch.Tensor | None, torch.Tensor]:
+        """
+        The cached rows [c | k_rot] that the step's prompt portions see, gathered from the pages: (c [rows, rank], (turn, k_rot [rows,
+        rot]) or None for rot 0, odd uint8 [rows], kv_start int32 [requests]) for `dense_prompt_attention`, turn by `freq` [rot / 2] and
+        `magnitude`.  `rows`: of all portions together, at most `max_keys`
+        of one: ctx_len - latent_first_key(...) each.  With a window, rows whose latent is not finite are zeros and marked in odd;
+        without one they are copied as they are and odd is None.
+        """
+        pool = binding.k_pool
+        if pool.dtype != torch.bfloat16:
+            raise KernelError(f"latent_gather: a pool of {pool.dtype}")
+        c = torch.empty((rows, rank), dtype=pool.dtype, device=pool.device)
+        turn = k_rot = None
+        if rot:
+            k_rot = torch.empty((rows, rot), dtype=pool.dtype, device=pool.device)
+            turn = torch.empty((ctx.num_tokens, 32, 2), dtype=torch.float32, device=pool.device)
+        odd = torch.empty((rows,), dtype=torch.uint8, device=pool.device) if window > 0 else None
+        kv_start = torch.empty((ctx.ctx_lens.shape[0],), dtype=torch.int32, device=pool.device)
+        portions = getattr(ctx, "prefill_seqs", None)
+        self._call("ts_latent_gather", _ptr(pool), binding.page_stride, binding.entry_offset, binding.page_tokens, binding.num_pages,
+                   _ptr(binding.block_table), binding.table_width, _ptr(ctx.cu_q), _ptr(ctx.ctx_lens), _ptr(portions),
+                   (portions if portions is not None else ctx.ctx_lens).shape[0], window, max_keys, rank, rot,
+                   _ptr(freq) if rot else None, float(magnitude), _ptr(turn), rows, _ptr(c), _ptr(k_rot), _ptr(odd), _ptr(kv_start), _stream())
+        return c, (turn, k_rot) if rot else None, odd, kv_start
+
+    @staticmethod
+    def latent_first_key(ctx_len: int, q_len: int, window: int) -> int:
+        """The first key `latent_gather` takes of a request: the first its first query sees, rounded down to a tile of 128."""
+        return max(0, ctx_len - q_len - window + 1) // 128 * 128 if window > 0 else 0
 
     def tensor_core_attention(self, q: torch.Tensor, binding, nh: int, nkv: int, hd: int, vd: int, ctx=None) -> bool:
         """Whether the bfloat16 tensor-core attention kernels take these sizes (else the generic kernel runs)."""

@@ -22,10 +22,10 @@ over the channels, so the order does not show), and the kernels rotate by halves
 
 Prompt portions of a step that is launched once (not replayed from a CUDA graph) take another way where the
 sizes allow (bfloat16, key and value heads of one size the tcgen05 prompt kernel takes, up to 64 rotated channels): the
-latents of the requests' whole contexts are gathered from the pages (their rotated parts, one for all heads, go to the
-kernel as they lie), a head's keys and values are worked out for the step (K = C W_uk^T, V = C W_uv^T, two library products: a quarter of the folded form's arithmetic at
-a latent of 512 channels and heads of 128) and the tcgen05 prompt kernel attends over them; requests that feed
-one token in the same step stay on the folded form.  The two ways differ by rounding only.
+latents the portions see, their whole contexts or what a window leaves, are gathered from the pages (their rotated parts, one for
+all heads, go to the kernel as they lie), a head's keys and values are worked out for the step ([K | V] = C [W_uk; W_uv]^T, one library
+product: a quarter of the folded form's arithmetic at a latent of 512 channels and heads of 128) and the tcgen05 prompt kernel
+attends over them; requests that feed one token in the same step stay on the folded form.  The two ways differ by rounding only.
 
 Tensors (local names): dq, dq.norm, uq (or q), dkv, dkv.norm, uk, uv, o, g with an output gate, sink.
 """
@@ -40,6 +40,8 @@ from tinyserve_llm_b200.parts.linear import Linear, fuse_rows
 
 MAX_KV_RANK = 512       # csrc/attention_latent.cu: 16 output channels a lane
 MATERIALIZE_MIN_TOKENS = 128    # prompt portions of a step, together, from which keys and values are worked out for the step
+MATERIALIZE_MAX_KEYS = 32       # with a window: keys a token fed, over all portions, up to which they are (16 heads, 160 .. 290 tokens behind
+                                # windows of 1,024, us folded / unfolded: 172 / 149 at 23 keys, 179 / 172 at 48, 163 / 336 at 95)
 
 
 def evens_then_odds(rows: torch.Tensor) -> torch.Tensor:
@@ -109,10 +111,14 @@ class LatentAttention(Mixer):
         self.kv_norm = tensors["dkv.norm"].to(device=rt.device, dtype=torch.float32).contiguous()
         # W_uk per head, transposed to [H, rank, D]: the product that folds it into the query reads rows of D
         self.uk_t = tensors["uk"].to(device=rt.device, dtype=rt.dtype).view(H, D, rank).transpose(1, 2).contiguous()
-        self.uv = tensors["uv"].to(device=rt.device, dtype=rt.dtype).view(H, V, rank).contiguous()
-        # the unfolded form of prompt portions: W_uk as stored, [H D, rank] (W_uv's stored form is self.uv's memory)
-        # (rotated parts go to the kernel as TMA sub-tiles of 64 channels out of rows [c | k_rot]: 16-byte boundaries)
-        self.uk = self.uk_t.transpose(1, 2).reshape(H * D, rank).contiguous() if D == V and R <= 64 and R % 8 == 0 and (R == 0 or rank % 8 == 0) else None
+        # the unfolded form of prompt portions: [W_uk; W_uv] as stored, one product for keys and values (its second half is self.uv's
+        # memory); rotated parts go to the kernel as TMA sub-tiles of 64 channels: rows on 16-byte boundaries
+        self.uk_uv = None
+        if D == V and R <= 64 and R % 8 == 0 and (R == 0 or rank % 8 == 0):
+            self.uk_uv = torch.cat([tensors[n].to(device=rt.device, dtype=rt.dtype).reshape(H * D, rank) for n in ("uk", "uv")])
+            self.uv = self.uk_uv[H * D:].view(H, V, rank)
+        else:
+            self.uv = tensors["uv"].to(device=rt.device, dtype=rt.dtype).view(H, V, rank).contiguous()
         self.out = Linear(tensors["o"], rt)
         self.sink = tensors["sink"].to(device=rt.device, dtype=torch.float32).contiguous() if spec.sink else None
 
@@ -121,16 +127,20 @@ class LatentAttention(Mixer):
 
     # ------------------------------------------------------------------ prompt portions on keys and values of their own
     def _portions(self, q: torch.Tensor, ctx) -> list[int] | None:
-        """The step's requests that feed more than one token, if their attention is to run on keys and values worked out for the step."""
-        spec, host = self.spec, getattr(ctx, "host", None)
-        if (self.uk is None or spec.window or getattr(ctx, "replayed", True) or host is None or ctx.max_q_len <= 1
-                or not self.rt.ops.dense_prompt_attention_supported(q, spec.num_heads, spec.num_heads, spec.head_dim)):
+        """How many keys each of the step's prompt portions sees, if they are to attend over keys and values worked out for the step."""
+        spec, host, ops = self.spec, getattr(ctx, "host", None), self.rt.ops
+        if (self.uk_uv is None or (spec.window and not spec.rot_dim) or getattr(ctx, "replayed", True) or host is None or ctx.max_q_len <= 1
+                or not ops.dense_prompt_attention_supported(q, spec.num_heads, spec.num_heads, spec.head_dim)):
             return None
+        # (windows come in the kernel's form with a rotated part, whose queries and probabilities have the folded form's precision)
         lens = [b - a for a, b in zip(host.cu_q, host.cu_q[1:])]
-        portions = [s for s, n in enumerate(lens) if n > 1]
-        if sum(lens[s] for s in portions) < MATERIALIZE_MIN_TOKENS:
+        fed = sum(n for n in lens if n > 1)
+        if fed < MATERIALIZE_MIN_TOKENS:
             return None
-        return portions
+        keys = [ctx_len - ops.latent_first_key(ctx_len, n, spec.window) for n, ctx_len in zip(lens, host.ctx_lens) if n > 1]
+        if spec.window and sum(keys) > MATERIALIZE_MAX_KEYS * fed:
+            return None
+        return keys
 
     @staticmethod
     def _single_tokens_only(ctx):
@@ -143,28 +153,13 @@ class LatentAttention(Mixer):
         out.seq_of_token = torch.where((ctx.seq_of_token >= 0) & (lens[seqs] == 1), ctx.seq_of_token, -1).to(torch.int32)
         return out
 
-    def _attend_unfolded(self, q: torch.Tensor, ctx, binding, portions: list[int], out: torch.Tensor | None) -> torch.Tensor:
-        spec, ops, host = self.spec, self.rt.ops, ctx.host
-        H, D, R, rank, B = spec.num_heads, spec.head_dim, spec.rot_dim, spec.kv_rank, binding.page_tokens
-        width = rank + R
-        entries = binding.page_stride // (B * width)
-        pool = binding.k_pool.view(binding.num_pages, entries, B, width)[:, binding.entry_offset // (B * width)]
-        starts, latents, at = [0] * len(host.ctx_lens), [], 0
-        for s in portions:                                  # the latents of the whole context, page by page
-            n = host.ctx_lens[s]
-            pages = binding.block_table[s, :-(-n // B)].long()
-            latents.append(pool[pages].reshape(-1, width)[:n])
-            starts[s], at = at, at + n
-        rows = torch.cat(latents) if len(latents) > 1 else latents[0].contiguous()
-        c, shared = rows, None
-        if R:
-            c = rows[:, :rank].contiguous()
-            shared = ops.latent_rotate_queries(q, ctx, H, D + R, D, R, self.frequencies, self.magnitude), rows[:, rank:]
-        kv_start = torch.tensor(starts, dtype=torch.int32).to(q.device, non_blocking=True)
-        k = ops.linear(c, self.uk)                          # [keys, H D]
-        v = ops.linear(c, self.uv.view(H * spec.value_dim, rank))
-        return ops.dense_prompt_attention(q, k, v, kv_start, ctx, H, H, D, spec.scale, out, q_head_cols=D + R, shared=shared,
-                                          sink=self.sink)
+    def _attend_unfolded(self, q: torch.Tensor, ctx, binding, keys: list[int], out: torch.Tensor | None) -> torch.Tensor:
+        spec, ops = self.spec, self.rt.ops
+        H, D, R, rank = spec.num_heads, spec.head_dim, spec.rot_dim, spec.kv_rank
+        c, shared, odd, kv_start = ops.latent_gather(ctx, binding, sum(keys), max(keys), rank, R, spec.window, self.frequencies, self.magnitude)
+        kv = ops.linear(c, self.uk_uv)                      # [keys, H D | H D]
+        return ops.dense_prompt_attention(q, kv[:, :H * D], kv[:, H * D:], kv_start, ctx, H, H, D, spec.scale, out, q_head_cols=D + R,
+                                          shared=shared, sink=self.sink, window=spec.window, odd_rows=odd)
 
     def forward(self, x: torch.Tensor, ctx, binding) -> torch.Tensor:
         spec, ops = self.spec, self.rt.ops
