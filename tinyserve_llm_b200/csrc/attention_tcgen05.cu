@@ -114,17 +114,17 @@ __device__ __forceinline__ uint32_t instr_desc(int m, int n, bool b_mn) {
     d |= (uint32_t)(m >> 4) << 24;
     return d;
 }
-__device__ __forceinline__ void umma_ss(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
+__device__ __forceinline__ void umma_ss(uint32_t leader, uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc), "r"(leader) : "memory");
 }
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
+__device__ __forceinline__ void umma_ts(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(acc), "r"(leader) : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -360,37 +360,40 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT, FORM == BOUNDED && RO
                 if (ROT) tma_load_2d(k_tile + SUBS * SUB_KV + b * (64 * 128), &map_k_rot, &kv_full[s], 0, row);
             }
         }
-    } else if (warp == MMA_WARP && lane == 0) {
-        // ---------------------------------------------------------------- MMA issuer
+    } else if (warp == MMA_WARP) {
+        // ---------------------------------------------------------------- MMA issuer: the warp as one, so that operands stay in uniform registers
+        const uint32_t leader = elect_one();
         const uint32_t idesc_s = instr_desc(QROWS, KEYS, false);
         const uint32_t idesc_o = instr_desc(QROWS, 64, true);        // O in column blocks of 64 dims, one per sub-tile of V
         bool ok = mbar_wait(&q_full, 0, p.error, 12);
         if (ROT) ok = ok && mbar_wait(&rot_ready, 0, p.error, 18);
+        ok = __all_sync(0xffffffffu, ok);
         // S = Q K^T of tile j, once its keys have landed
         auto issue_scores = [&](int it) -> bool {
             const int s = it & 1;
-            if (!mbar_wait(&kv_full[s], (it >> 1) & 1, p.error, 13)) return false;
+            if (!__all_sync(0xffffffffu, mbar_wait(&kv_full[s], (it >> 1) & 1, p.error, 13))) return false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
             for (int h = 0; h < SUBS; ++h) {
                 const uint64_t q_desc = smem_desc(q_tile + h * SUB_Q);
                 const uint64_t k_desc = smem_desc(kv_tiles + s * STAGE_BYTES + h * SUB_KV);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) umma_ss(tmem, q_desc + 2 * k, k_desc + 2 * k, idesc_s, (h | k) != 0);
+                for (int k = 0; k < 4; ++k) umma_ss(leader, tmem, q_desc + 2 * k, k_desc + 2 * k, idesc_s, (h | k) != 0);
             }
             if (ROT) {                               // 16 channels are 8 columns of packed queries: four of the first piece, four of the second
                 const uint64_t k_desc = smem_desc(kv_tiles + s * STAGE_BYTES + SUBS * SUB_KV);
 #pragma unroll
-                for (int k = 0; k < 8; ++k) umma_ts(tmem, tmem + S_::ROT_COL + 8 * k, k_desc + 2 * (k & 3), idesc_s, 1);
+                for (int k = 0; k < 8; ++k) umma_ts(leader, tmem, tmem + S_::ROT_COL + 8 * k, k_desc + 2 * (k & 3), idesc_s, 1);
             }
-            umma_commit(&s_done);
+            if (leader) umma_commit(&s_done);
+            __syncwarp();
             return true;
         };
         ok = ok && issue_scores(0);
         const int num_it = num_kv - kv_begin;
         for (int j = 0; j < num_it && ok; ++j) {       // j counts the tiles from the first one here
             const int s = j & 1;
-            if (!mbar_wait(&p_ready, j & 1, p.error, 14)) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, mbar_wait(&p_ready, j & 1, p.error, 14))) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             // The softmax has read S of tile j (P lies in columns of its own), so the next tile's scores go first:
             // its softmax can begin while O += P V of this tile is still running.  The softmax waits for that
@@ -401,17 +404,19 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT, FORM == BOUNDED && RO
                 const uint64_t v_desc = smem_desc(kv_tiles + s * STAGE_BYTES + K_BYTES + h * SUB_KV);
 #pragma unroll
                 for (int k = 0; k < KEYS / 16; ++k)
-                    umma_ts(tmem + O_COL + 64 * h, tmem + P_COL + 8 * k, v_desc + 128 * k, idesc_o, (j | k) != 0);
+                    umma_ts(leader, tmem + O_COL + 64 * h, tmem + P_COL + 8 * k, v_desc + 128 * k, idesc_o, (j | k) != 0);
                 if (PAIR) {
 #pragma unroll
                     for (int k = 0; k < KEYS / 16; ++k)
-                        umma_ts(tmem + O_COL + 64 * h, tmem + P_COL + KEYS / 2 + 8 * k, v_desc + 128 * k, idesc_o, 1);
+                        umma_ts(leader, tmem + O_COL + 64 * h, tmem + P_COL + KEYS / 2 + 8 * k, v_desc + 128 * k, idesc_o, 1);
                 }
             }
-            umma_commit(&stage_free[s]);
+            if (leader) umma_commit(&stage_free[s]);
+            __syncwarp();
         }
         if (!ok) failed = 1;
-        umma_commit(&all_done);
+        if (leader) umma_commit(&all_done);
+        __syncwarp();
     } else if (warp < SOFTMAX_WARPS) {
         // ---------------------------------------------------------------- softmax: two threads own query row r
         // Warp w reads the tensor-memory lanes of quadrant w % 4 (a warp can reach no others); the two

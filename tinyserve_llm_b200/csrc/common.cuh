@@ -106,6 +106,16 @@ __device__ __forceinline__ float block_sum(float v, float* scratch /* >= 32 floa
     return t;
 }
 
+// Nonzero in one lane of a warp that has come together, always the same one.  tcgen05.mma takes its operands from uniform registers:
+// in code that one lane alone runs, behind `lane == 0`, each of them is moved there anew (58 cycles from one MMA to the next whatever
+// its size), where a whole warp that runs the loop and issues under this predicate keeps them (15 cycles at 16 columns, 34 at 64,
+// which is the tensor cores' own rate).
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t leader;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(leader));
+    return leader;
+}
+
 // Programmatic dependent launch.  A kernel launched through launch_chained() may start while the
 // kernel before it on the stream is still running: it may read what no kernel on the stream writes
 // (weights, tables) at once, and must call chain_wait() before it reads anything an earlier kernel
