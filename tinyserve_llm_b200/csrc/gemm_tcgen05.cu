@@ -272,19 +272,6 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
 // the epilogue warps of both.  A cluster barrier after the barriers' initialisation keeps either CTA
 // from signalling a barrier that does not exist yet, another before the tensor memory is given back
 // keeps either from leaving while the other still reads its shared memory.
-__device__ __forceinline__ uint32_t pair_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t in_first_cta(const void* local) {      // the same object in the pair's first CTA
-    uint32_t remote;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(local)), "r"(0));
-    return remote;
-}
-__device__ __forceinline__ void pair_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void tma_load_2d_pair(void* smem, const CUtensorMap* map, uint32_t bar_in_first, int x, int y) {
     asm volatile(
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -296,14 +283,6 @@ __device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t a_desc, uint
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
         ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(zero) : "memory");
-}
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {          // arrives on `bar` in both CTAs
-    const uint16_t both = 3;
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(smem_u32(bar)), "h"(both) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar_in_cluster) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_in_cluster) : "memory");
 }
 
 template <int EPI>

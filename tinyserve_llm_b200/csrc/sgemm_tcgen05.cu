@@ -11,34 +11,38 @@
 // A row's result does not depend on what else is in the batch: the blocks of k, the segments k is cut into and the order
 // they are added up in follow from N and K alone, and the rows' tile (the MMA's N side) does not enter an element's sum.
 //
-// One CTA: 128 rows of W (the MMA's 128 lanes) against BX rows of x.  Warp 0 issues TMA loads into a ring of raw tiles, warp 1 the
-// MMAs, warps 2..9 split (two teams, a block each): a thread puts its row of W into tensor memory as hi and lo (the MMA's A
-// operand, so that neither passes through shared memory again) and its share of x into two swizzled tiles; the warps from 10
+// Two CTAs a tile (`cta_group::2`): 256 rows of W, 128 in each CTA (the MMA's lanes), against BX rows of x, of which each CTA loads and
+// splits half; the first CTA's thread issues the MMAs for both.  Per CTA: warp 0 issues TMA loads into a ring of raw tiles, warp 1 the
+// MMAs, warps 4..11 split (two teams, a block each): a thread puts its row of W into tensor memory as hi and lo (the MMA's A
+// operand, so that neither passes through shared memory again) and its share of x into two swizzled tiles; the warps from 12
 // on add the blocks' sums up.
-// mbarriers: `raw_full` / `raw_empty` TMA <-> split, `ready` / `free` split <-> MMA, `sum_full` / `sum_empty` MMA <-> adders.
+// mbarriers: `raw_full` / `raw_empty` TMA <-> split, `ready` / `free` split <-> MMA, `sum_full` / `sum_empty` MMA <-> adders; `ready` and
+// `sum_empty` are the first CTA's, on which both CTAs' warps arrive, `free` and `sum_full` are signalled in both.
 // K is cut into segments, enough of them that the tiles of W times the segments fill the SMs.  Where there are rows of x enough
-// to fill them anyway a CTA takes the segments one after another and adds each one's sum to y; else each segment is a CTA's
+// to fill them anyway a pair takes the segments one after another and adds each one's sum to y; else each segment is a pair's
 // work, its sums go to scratch, and a second kernel adds them up in the same order.
-// Measured on a B200, products with cold weights one after another, us, before (sgemm.cu) and now:
-//   rows of x             1          8         100        300      512
-//   16,384 x 2,048      192 / 53   192 / 53   306 / 68
-//   2,048 x 8,192                  677 / 29   636 / 40      - / 100
-//   3,072 x 2,048                                                 241 / 70
-// (a feed-forward of 100 rows, 2,048 x 8,192, since then 113 / 107).  What bounds it: a block of k costs 0.75 to 0.93 us whatever BX is.  An MMA of 8 numbers of k takes some 107 cycles with up to 64
-// rows of x and 137 with 128 (67 by the tensor cores' rate); with one of the twelve MMAs issued (timing only) the first column
-// is 34 us, and loads alone stream W at 4.4 TB/s.
+// Measured on a B200, products with cold weights one after another, us: sgemm.cu, this product with one CTA a tile and the MMAs issued by
+// one lane, and now:
+//   rows of x             1                8               100              300             512             1,024
+//   16,384 x 2,048   192 / 53 / 32   192 / 53 / 32    306 / 63 / 45     - / 170 / 128   - / 222 / 177    - / 405 / 333
+//   2,048 x 8,192                    677 / 29 / 19    636 / 36 / 28     -  / 89 / 65    - / 118 / 90     - / 275 / 177
+//   3,072 x 2,048                                                                     241 /  86 / 46     - / 115 / 91
+// A block of k took 0.75 to 0.93 us whatever BX was: 12 MMAs issued by one lane are 58 cycles each at the least (elect_one), and x's
+// tile, loaded and split whole by every CTA, moved more bytes through shared memory than W's.  Now 0.48 (BX 32), 0.57 (64) and 0.68 us
+// (128), of which the MMAs at the tensor cores' rate are 0.1, 0.22 and 0.41; W's stream alone takes 30 us in the first row.  What is left
+// is the adders' reading of tensor memory (7 us in the first row at 128 rows), the split (3) and a pair in seven without a tile there.
 //
 // Every wait on an mbarrier gives up after about two seconds and records where in an error word the host reads.
 #include "tcgen05.cuh"
 
 namespace {
 
-constexpr int BW = 128, BK = 32;                     // rows of W a tile; k a block: 128 bytes, one swizzled row
-constexpr int SPLIT_WARPS = 4, ADDERS_FROM = 2 + 2 * SPLIT_WARPS;    // two teams of split warps
+constexpr int BW = 128, BK = 32;                     // rows of W a CTA, half of a tile; k a block: 128 bytes, one swizzled row
+constexpr int SPLIT_WARPS = 4, SPLITS_FROM = 4, ADDERS_FROM = SPLITS_FROM + 2 * SPLIT_WARPS;    // two teams of split warps
 __host__ __device__ constexpr int share_of(int bx) { return bx >= 64 ? 4 : 2; }           // adder warps a quarter of the lanes
 __host__ __device__ constexpr int threads_of(int bx) { return 32 * (ADDERS_FROM + 4 * share_of(bx)); }
 constexpr int W_BYTES = BW * BK * 4;
-constexpr int SMS = 148;
+constexpr int PAIRS_OF_SMS = 74;
 constexpr long long MAX_SCRATCH = 64ll << 20;        // floats: more than that and the segments are taken in turn
 constexpr int MIN_SEGMENT = 8;                       // blocks of k a segment has at least (256 terms)
 
@@ -49,16 +53,16 @@ struct SgemmParams {
     int M, N, K;
     long long ldx, ldw, ldy, segment_stride;
     int blocks, per_segment, in_turn;                // blocks of k in all, and a segment; 1: a CTA takes all segments in turn
-    int items;                                       // tiles, times segments unless in turn
+    int items;                                       // tiles, times segments unless in turn: a pair's
     int* error;
 };
 
-// A from tensor memory (its 128 lanes the rows, a column a number of K), B from shared memory
-__device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// A from tensor memory (the 128 lanes of either CTA the rows, a column a number of K), B from both CTAs' shared memory
+__device__ __forceinline__ void umma_tf32(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
 }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* r) {
     asm volatile(
@@ -76,11 +80,11 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
 // the largest number hi is infinite and the rest NaN, and for a NaN the rest is one, so the sum never hides either.
 __device__ __forceinline__ float to_tf32(float v) { return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u); }
 
-struct Item { int n0, m0, segment, first, count; };    // a CTA's piece of work: a tile and the blocks of k it takes
+struct Item { int n0, m0, segment, first, count; };    // a pair's piece of work: a tile and the blocks of k it takes
 __device__ __forceinline__ Item item_of(const SgemmParams& p, int item, int bx) {
-    const int n_tiles = (p.N + BW - 1) / BW, m_tiles = (p.M + bx - 1) / bx;
+    const int n_tiles = (p.N + 2 * BW - 1) / (2 * BW), m_tiles = (p.M + bx - 1) / bx;
     Item it;
-    it.n0 = item % n_tiles * BW;
+    it.n0 = item % n_tiles * 2 * BW;
     it.m0 = item / n_tiles % m_tiles * bx;
     it.segment = item / n_tiles / m_tiles;
     it.first = it.segment * p.per_segment;
@@ -93,13 +97,14 @@ __device__ __forceinline__ Item item_of(const SgemmParams& p, int item, int bx) 
 template <int BX, int RING, int PAIRS, int SUMS>
 __global__ void __launch_bounds__(threads_of(BX), 1)
 sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, SgemmParams p) {
-    constexpr int X_BYTES = BX * BK * 4, RAW_BYTES = W_BYTES + X_BYTES;               // ring of [W | x]; PAIRS of [x hi | x lo]
+    constexpr int X_BYTES = BX / 2 * BK * 4, RAW_BYTES = W_BYTES + X_BYTES;           // ring of [W | x]; PAIRS of [x hi | x lo]: this CTA's half
     constexpr int A_COLS = SUMS * BX, TMEM_USED = A_COLS + PAIRS * 2 * BK;            // PAIRS of [W hi | W lo]
     constexpr int TMEM_COLS = TMEM_USED <= 256 ? 256 : 512;
     static_assert(TMEM_USED <= 512, "tensor memory has 512 columns");
     // a slot's barrier is waited on by one team only: the other could come to it a round early, where the parity it waits
     // for stands for the round before the first
     static_assert(RING % 2 == 0 && PAIRS % 2 == 0, "a ring slot and a pair of operand tiles belong to one team");
+    static_assert(RAW_BYTES % 1024 == 0 && X_BYTES % 1024 == 0, "tiles lie on the swizzle's boundaries");
     constexpr int OWN = BX / share_of(BX);           // columns of an adder
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t raw_full_bar[RING], raw_empty_bar[RING], ready_bar[PAIRS], free_bar[PAIRS], sum_full_bar[SUMS], sum_empty_bar[SUMS];
@@ -108,6 +113,7 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* split = ring + RING * RAW_BYTES;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = (int)pair_rank(), pair = blockIdx.x / 2, pairs = gridDim.x / 2;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < RING; ++s) {
@@ -115,69 +121,83 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             mbar_init(&raw_empty_bar[s], SPLIT_WARPS);
         }
         for (int b = 0; b < PAIRS; ++b) {
-            mbar_init(&ready_bar[b], SPLIT_WARPS);
+            mbar_init(&ready_bar[b], 2 * SPLIT_WARPS);
             mbar_init(&free_bar[b], 1);
         }
         for (int b = 0; b < SUMS; ++b) {
             mbar_init(&sum_full_bar[b], 1);
-            mbar_init(&sum_empty_bar[b], 4 * share_of(BX));
+            mbar_init(&sum_empty_bar[b], 2 * 4 * share_of(BX));
         }
         failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)),
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)),
                      "r"(TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_slot;
+    pair_sync();                                     // both CTAs' barriers exist
     chain_wait();
     chain_release();
 
-    if (warp == 0 && lane == 0) {
-        int g = 0;
-        for (int at = blockIdx.x; at < p.items && !failed; at += gridDim.x) {
-            const Item it = item_of(p, at, BX);
-            for (int i = 0; i < it.count; ++i, ++g) {
-                const int s = g % RING;
-                if (!mbar_wait(&raw_empty_bar[s], ((g / RING) & 1) ^ 1, p.error, 21)) { failed = 1; break; }
-                mbar_expect_tx(&raw_full_bar[s], RAW_BYTES);
-                tma_load_2d(ring + s * RAW_BYTES, &map_w, &raw_full_bar[s], (it.first + i) * BK, it.n0);
-                tma_load_2d(ring + s * RAW_BYTES + W_BYTES, &map_x, &raw_full_bar[s], (it.first + i) * BK, it.m0);
+    // The adders' sums want more registers than an even share: the launch's 896 x 72 as 128 x 40 + 256 x 56 + 512 x 88.
+    constexpr bool SHARES = threads_of(BX) == 896;
+    if (warp < SPLITS_FROM) {
+        if (SHARES) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        if (warp == 0 && lane == 0) {
+            int g = 0;
+            for (int at = pair; at < p.items && !failed; at += pairs) {
+                const Item it = item_of(p, at, BX);
+                for (int i = 0; i < it.count; ++i, ++g) {
+                    const int s = g % RING;
+                    if (!mbar_wait(&raw_empty_bar[s], ((g / RING) & 1) ^ 1, p.error, 21)) { failed = 1; break; }
+                    mbar_expect_tx(&raw_full_bar[s], RAW_BYTES);
+                    tma_load_2d(ring + s * RAW_BYTES, &map_w, &raw_full_bar[s], (it.first + i) * BK, it.n0 + rank * BW);
+                    tma_load_2d(ring + s * RAW_BYTES + W_BYTES, &map_x, &raw_full_bar[s], (it.first + i) * BK, it.m0 + rank * (BX / 2));
+                }
+            }
+        } else if (warp == 1 && rank == 0) {
+            // float32 accumulator, TF32 operands, B K-major, 256 x BX over both CTAs; the warp as one, so that operands stay in uniform registers
+            const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(BX >> 3) << 17) | ((uint32_t)(2 * BW >> 4) << 24);
+            const uint32_t leader = elect_one();
+            int g = 0;
+            bool ok = true;                          // the same in all lanes
+            for (int at = pair; at < p.items && ok; at += pairs) {
+                const Item it = item_of(p, at, BX);
+                for (int i = 0; i < it.count; ++i, ++g) {
+                    const int a = g % PAIRS, b = g % SUMS;
+                    ok = mbar_wait(&sum_empty_bar[b], ((g / SUMS) & 1) ^ 1, p.error, 24) &&
+                         mbar_wait(&ready_bar[a], (g / PAIRS) & 1, p.error, 23) && !failed;
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) { failed = 1; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t w_hi = tmem_base + A_COLS + a * 2 * BK, w_lo = w_hi + BK, d = tmem_base + b * BX;
+                    const uint64_t x_hi = smem_desc(split + a * 2 * X_BYTES), x_lo = smem_desc(split + a * 2 * X_BYTES + X_BYTES);
+#pragma unroll
+                    for (int k = 0; k < BK / 8; ++k) umma_tf32(leader, d, w_hi + 8 * k, x_lo + 2 * k, idesc, k != 0);   // 8 numbers of K: 8 columns, 32 bytes
+#pragma unroll
+                    for (int k = 0; k < BK / 8; ++k) umma_tf32(leader, d, w_lo + 8 * k, x_hi + 2 * k, idesc, 1);
+#pragma unroll
+                    for (int k = 0; k < BK / 8; ++k) umma_tf32(leader, d, w_hi + 8 * k, x_hi + 2 * k, idesc, 1);
+                    if (leader) {
+                        umma_commit_pair(&free_bar[a]);
+                        umma_commit_pair(&sum_full_bar[b]);
+                    }
+                    __syncwarp();
+                }
             }
         }
-    } else if (warp == 1 && lane == 0) {
-        // float32 accumulator, TF32 operands, B K-major, 128 x BX
-        const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(BX >> 3) << 17) | ((uint32_t)(BW >> 4) << 24);
-        int g = 0;
-        for (int at = blockIdx.x; at < p.items && !failed; at += gridDim.x) {
-            const Item it = item_of(p, at, BX);
-            for (int i = 0; i < it.count; ++i, ++g) {
-                const int a = g % PAIRS, b = g % SUMS;
-                if (!mbar_wait(&sum_empty_bar[b], ((g / SUMS) & 1) ^ 1, p.error, 24)) { failed = 1; break; }
-                if (!mbar_wait(&ready_bar[a], (g / PAIRS) & 1, p.error, 23)) { failed = 1; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t w_hi = tmem_base + A_COLS + a * 2 * BK, w_lo = w_hi + BK, d = tmem_base + b * BX;
-                const uint64_t x_hi = smem_desc(split + a * 2 * X_BYTES), x_lo = smem_desc(split + a * 2 * X_BYTES + X_BYTES);
-#pragma unroll
-                for (int k = 0; k < BK / 8; ++k) umma_tf32(d, w_hi + 8 * k, x_lo + 2 * k, idesc, k != 0);   // 8 numbers of K: 8 columns, 32 bytes
-#pragma unroll
-                for (int k = 0; k < BK / 8; ++k) umma_tf32(d, w_lo + 8 * k, x_hi + 2 * k, idesc, 1);
-#pragma unroll
-                for (int k = 0; k < BK / 8; ++k) umma_tf32(d, w_hi + 8 * k, x_hi + 2 * k, idesc, 1);
-                umma_commit(&free_bar[a]);
-                umma_commit(&sum_full_bar[b]);
-            }
-        }
-    } else if (warp >= 2 && warp < ADDERS_FROM) {
+    } else if (warp < ADDERS_FROM) {
+        if (SHARES) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
         // blocks in turn between the teams: a block's split is a chain of waits, loads and stores, and two run side by side
-        const int team = (warp - 2) / SPLIT_WARPS, quarter = warp & 3, row = quarter * 32 + lane;   // a warp reaches the quarter of the lanes its number gives
+        const int team = (warp - SPLITS_FROM) / SPLIT_WARPS, quarter = warp & 3, row = quarter * 32 + lane;   // a warp reaches the quarter of the lanes its number gives
         const uint32_t lane_addr = tmem_base + A_COLS + ((uint32_t)(quarter * 32) << 16);
         int total = 0;
-        for (int at = blockIdx.x; at < p.items; at += gridDim.x) total += item_of(p, at, BX).count;
+        for (int at = pair; at < p.items; at += pairs) total += item_of(p, at, BX).count;
         for (int g = team; g < total; g += 2) {
             const int s = g % RING, a = g % PAIRS;
             bool ok = mbar_wait(&raw_full_bar[s], (g / RING) & 1, p.error, 22) && !failed;
@@ -216,11 +236,12 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive(&ready_bar[a]);
+                mbar_arrive_remote_tcgen05(in_first_cta(&ready_bar[a]));
                 mbar_arrive(&raw_empty_bar[s]);
             }
         }
-    } else if (warp >= ADDERS_FROM) {
+    } else {
+        if (SHARES) asm volatile("setmaxnreg.inc.sync.aligned.u32 88;");
         const int quarter = warp & 3, side = (warp - ADDERS_FROM) >> 2;
         const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + side * OWN;
         float sum[OWN];
@@ -228,9 +249,9 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         for (int j = 0; j < OWN; ++j) sum[j] = 0.f;
         int sums = 0;
         bool ok = true;                              // the same in all lanes
-        for (int at = blockIdx.x; at < p.items && ok; at += gridDim.x) {
+        for (int at = pair; at < p.items && ok; at += pairs) {
             const Item it = item_of(p, at, BX);
-            const int n = it.n0 + quarter * 32 + lane, m_first = it.m0 + side * OWN;
+            const int n = it.n0 + rank * BW + quarter * 32 + lane, m_first = it.m0 + side * OWN;
             for (int from = 0; from < it.count && ok; from += p.per_segment) {        // a segment
                 const int blocks = min(p.per_segment, it.count - from);
                 for (int i = 0; i < blocks; ++i, ++sums) {
@@ -244,20 +265,38 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");  // read: the accumulator goes back before the additions
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&sum_empty_bar[b]);
+                    if (lane == 0) mbar_arrive_remote_tcgen05(in_first_cta(&sum_empty_bar[b]));
 #pragma unroll
                     for (int j = 0; j < OWN; ++j) sum[j] += __uint_as_float(v[j]);
                 }
                 if (!ok) break;
                 float* y = p.y + it.segment * p.segment_stride + (long long)m_first * p.ldy + n;
                 const int k0 = (it.first + from) * BK, k1 = min(p.K, k0 + blocks * BK);
+                const int rows = n < p.N ? p.M - m_first : 0;
                 uint32_t odd = 0;
+                if (from) {                          // the segments before this one: a few loads under way together
+                    const float* at_y = y;
 #pragma unroll
-                for (int j = 0; j < OWN; ++j) {
-                    if (n < p.N && m_first + j < p.M) {
-                        if (isfinite(sum[j])) y[j * p.ldy] = from ? y[j * p.ldy] + sum[j] : sum[j];
-                        else odd |= 1u << j;         // hi + lo does not stand for infinite or the largest numbers
+                    for (int j0 = 0; j0 < OWN; j0 += 8) {
+                        float before[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j, at_y += p.ldy) before[j] = j0 + j < rows ? *at_y : 0.f;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            if (!isfinite(sum[j0 + j])) odd |= 1u << (j0 + j);
+                            sum[j0 + j] += before[j];
+                        }
                     }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < OWN; ++j)
+                        if (!isfinite(sum[j])) odd |= 1u << j;
+                }
+                if (rows < OWN) odd &= rows > 0 ? (1u << rows) - 1 : 0;      // hi + lo does not stand for infinite or the largest numbers
+                float* to_y = y;
+#pragma unroll
+                for (int j = 0; j < OWN; ++j, to_y += p.ldy) {
+                    if (j < rows && !(odd >> j & 1)) *to_y = sum[j];
                     sum[j] = 0.f;
                 }
                 // Those again by multiply-adds.  A row of x with a NaN, which padding may be, gives NaN everywhere: one look tells.
@@ -278,9 +317,10 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    pair_sync();                                     // neither CTA leaves while the other's MMAs or arrivals may reach it
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
     }
 }
 
@@ -311,8 +351,8 @@ __global__ void __launch_bounds__(256) add_segments_kernel(const float* __restri
 // How K is cut, from N and K alone: enough segments that the tiles of W fill the SMs once, none shorter than MIN_SEGMENT blocks.
 void cut(int N, int K, int* blocks, int* per_segment, int* segments) {
     *blocks = (K + BK - 1) / BK;
-    const int tiles = (N + BW - 1) / BW;
-    int s = SMS / tiles;
+    const int tiles = (N + 2 * BW - 1) / (2 * BW);
+    int s = PAIRS_OF_SMS / tiles;
     if (s > *blocks / MIN_SEGMENT) s = *blocks / MIN_SEGMENT;
     if (s < 1) s = 1;
     *per_segment = (*blocks + s - 1) / s;
@@ -323,27 +363,42 @@ template <int BX, int RING, int PAIRS, int SUMS>
 int launch(SgemmParams p, int segments, cudaStream_t stream) {
     CUtensorMap map_w, map_x;
     if (make_tile_map(&map_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.w, p.N, p.K, p.ldw, BW, "sgemm_tcgen05")) return 1;
-    if (make_tile_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.x, p.M, p.K, p.ldx, BX, "sgemm_tcgen05")) return 1;
-    constexpr size_t smem = (size_t)RING * (W_BYTES + BX * BK * 4) + PAIRS * 2 * BX * BK * 4 + 1024;
+    if (make_tile_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.x, p.M, p.K, p.ldx, BX / 2, "sgemm_tcgen05")) return 1;
+    constexpr size_t smem = (size_t)RING * (W_BYTES + BX / 2 * BK * 4) + PAIRS * BX * BK * 4 + 1024;
     auto kernel = sgemm_tcgen05_kernel<BX, RING, PAIRS, SUMS>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    p.items = ((p.N + BW - 1) / BW) * ((p.M + BX - 1) / BX) * (p.in_turn ? 1 : segments);
-    TS_CHAINED_CHECK("sgemm_tcgen05", launch_chained(kernel, dim3(p.items < SMS ? p.items : SMS), dim3(threads_of(BX)), smem, stream,
-                                                     map_w, map_x, p));
+    p.items = ((p.N + 2 * BW - 1) / (2 * BW)) * ((p.M + BX - 1) / BX) * (p.in_turn ? 1 : segments);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * (p.items < PAIRS_OF_SMS ? p.items : PAIRS_OF_SMS));
+    cfg.blockDim = dim3(threads_of(BX));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = ts_chaining_enabled() ? 2 : 1;
+    TS_CHAINED_CHECK("sgemm_tcgen05", cudaLaunchKernelEx(&cfg, kernel, map_w, map_x, p));
     return 0;
 }
 
 // Rows of x a CTA, and whether it takes the segments in turn.  Neither enters an element's sum.
 struct Shape { int bx, in_turn; };
 Shape choose(int M, int N, int blocks, int per_segment, int segments) {
-    static const struct { int bx; double ns; } kinds[4] = {{16, 750}, {32, 770}, {64, 820}, {128, 930}};   // of a block of k, as measured
+    static const struct { int bx; double ns; } kinds[3] = {{32, 480}, {64, 570}, {128, 680}};   // of a block of k, as measured
     Shape best{128, segments > 1};
     double least = 1e30;
     for (const auto& kind : kinds)
         for (int in_turn = 0; in_turn < (segments > 1 ? 2 : 1); ++in_turn) {
             if (segments > 1 && !in_turn && (long long)segments * M * N > MAX_SCRATCH) continue;
-            const long long items = (long long)((N + BW - 1) / BW) * ((M + kind.bx - 1) / kind.bx) * (in_turn ? 1 : segments);
-            double ns = (double)((items + SMS - 1) / SMS) * (500.0 + (in_turn ? blocks : per_segment) * kind.ns);
+            const long long items = (long long)((N + 2 * BW - 1) / (2 * BW)) * ((M + kind.bx - 1) / kind.bx) * (in_turn ? 1 : segments);
+            // in turn, each segment but the first waits for the sums before it to come back from memory
+            double ns = (double)((items + PAIRS_OF_SMS - 1) / PAIRS_OF_SMS) *
+                        (500.0 + (in_turn ? blocks : per_segment) * kind.ns + (in_turn ? (segments - 1) * 3000.0 : 0.0));
             if (segments > 1 && !in_turn) ns += 2500.0 + (double)segments * M * N * 8.0 / 5000.0;     // the second kernel
             if (ns < least) {
                 least = ns;
@@ -380,8 +435,8 @@ int sgemm_tcgen05(const float* x, const float* w, float* y, int M, int N, int K,
     const bool parts = segments > 1 && !shape.in_turn;
     SgemmParams p{parts ? scratch : y, x, w, M, N, K, ldx, ldw, parts ? N : ldy, parts ? (long long)M * N : 0, blocks, per,
                   shape.in_turn, 0, error};
-    const int failed = shape.bx == 16 ? launch<16, 8, 4, 4>(p, segments, stream) : shape.bx == 32 ? launch<32, 8, 4, 4>(p, segments, stream)
-                     : shape.bx == 64 ? launch<64, 6, 4, 4>(p, segments, stream) : launch<128, 4, 2, 3>(p, segments, stream);
+    const int failed = shape.bx == 32 ? launch<32, 10, 4, 4>(p, segments, stream)
+                     : shape.bx == 64 ? launch<64, 8, 4, 4>(p, segments, stream) : launch<128, 6, 4, 2>(p, segments, stream);
     if (failed || !parts) return failed;
     const bool vec = N % 4 == 0 && ldy % 4 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)scratch % 16 == 0;
     const long long items = (long long)M * N / (vec ? 4 : 1);
