@@ -236,7 +236,7 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive_remote_tcgen05(in_first_cta(&ready_bar[a]));
+                mbar_arrive_remote(in_first_cta(&ready_bar[a]));
                 mbar_arrive(&raw_empty_bar[s]);
             }
         }
@@ -265,7 +265,7 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");  // read: the accumulator goes back before the additions
                     __syncwarp();
-                    if (lane == 0) mbar_arrive_remote_tcgen05(in_first_cta(&sum_empty_bar[b]));
+                    if (lane == 0) mbar_arrive_remote(in_first_cta(&sum_empty_bar[b]));
 #pragma unroll
                     for (int j = 0; j < OWN; ++j) sum[j] += __uint_as_float(v[j]);
                 }

@@ -78,12 +78,10 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {          // ar
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                  ::"r"(smem_u32(bar)), "h"(both) : "memory");
 }
+// An arrival on the other CTA's barrier for hand-offs to the tensor cores, whose reads and writes are ordered by tcgen05's fences and, in
+// shared memory, by the proxy fence: without an order at cluster scope between this thread's own writes to memory and what the other
+// CTA reads, which costs a microsecond.
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t bar_in_cluster) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_in_cluster) : "memory");
-}
-// The same without an order between this thread's own writes to memory and what the other CTA reads (which costs a microsecond): for
-// hand-offs to the tensor cores, whose reads and writes are ordered by tcgen05's fences and, in shared memory, by the proxy fence.
-__device__ __forceinline__ void mbar_arrive_remote_tcgen05(uint32_t bar_in_cluster) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_in_cluster) : "memory");
 }
 
