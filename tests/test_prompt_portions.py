@@ -261,6 +261,53 @@ def test_tiles_are_no_further_from_64_bits_than_the_walk(form, tokens, heads):
     assert off[0] <= off[2] and off[1] <= off[3], off
 
 
+def _stretched(dim, vdim, T, plant=None):
+    """bfloat16 portions of T, 1 and 130 tokens by stretches: (output, states, what 64 bits give for both)."""
+    ops, H, lens = get_ops(), 3, [T, 1, 130]
+    g = torch.Generator().manual_seed(dim + vdim)
+    n = sum(lens)
+    y = (torch.randn(n, H * (2 * dim + vdim) + 4, generator=g) * 0.5).to(torch.bfloat16)
+    z, state = torch.randn(n, H * dim, generator=g) + 3, torch.randn(len(lens) + 3, H * dim * vdim, generator=g)
+    cuts = (0, H * dim, 2 * H * dim, H * (2 * dim + vdim))
+    if plant is not None:
+        row, column, value = plant
+        y[row, cuts[2] + column] = value
+    dev, yd = state.cuda(), y.cuda()
+    ctx, binding = _step(dev, lens)
+    before = ops.calls.get("ts_plain_tiles", 0)
+    got = ops.linear_recurrence(*(yd[:, a:b] for a, b in zip(cuts, cuts[1:])), ctx, binding, heads=H, dim=dim, vdim=vdim, z=z.cuda(), bias=None, head_decays=None,
+                                inv_tau=1 / 16, q_scale=0.25, k_scale=1.0)
+    assert ops.calls.get("ts_plain_tiles", 0) == before + 1
+    q, k, v = (y[:, a:b].double().view(n, H, -1) for a, b in zip(cuts, cuts[1:]))
+    a = torch.sigmoid(z.double()).pow(1 / 16).view(n, H, dim)
+    want, left, at = torch.empty(n, H, vdim, dtype=torch.float64), state.double().view(-1, H, dim, vdim).clone(), 0
+    for s, m in enumerate(lens if plant is None else []):
+        S = left[len(left) - 1 - s]
+        for t in range(at, at + m):
+            S.mul_(a[t][:, :, None]).add_(k[t][:, :, None] * v[t][:, None, :])
+            want[t] = 0.25 * torch.einsum("hdv,hd->hv", S, q[t])
+        at += m
+    return got.cpu(), dev.cpu(), want, left
+
+
+@pytest.mark.parametrize("dim,vdim,T", [(64, 64, 129), (100, 129, 300), (128, 72, 257), (256, 33, 128), (36, 8, 513)])
+def test_plain_recurrence_by_stretches(dim, vdim, T):
+    """Portions around one stretch of 128 tokens and over several, rows and columns that fill their blocks and do not."""
+    got, states, want, left = _stretched(dim, vdim, T)
+    # as test_plain_recurrence_of_portions, over T tokens: a product within 2^-21, decays within sqrt(T) 2^-24 once roundings go both ways
+    for mine, true in ((got, want), (states, left)):
+        mine = mine.double().reshape(true.shape)
+        assert float((mine - true).norm() / true.norm()) < 2.0 ** -21 + T ** 0.5 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf")])
+def test_a_value_that_is_not_finite_stays_in_its_column_by_stretches(value):
+    (clean, *_), (got, *_) = _stretched(64, 40, 300), _stretched(64, 40, 300, (201, 2 * 40 + 17, value))
+    assert torch.equal(got[:201], clean[:201]) and not torch.isfinite(got[201:300, 2 * 40 + 17]).any()
+    got[201:300, 2 * 40 + 17] = clean[201:300, 2 * 40 + 17]
+    assert torch.equal(got, clean)
+
+
 def _recurrence_part(kind, dtype):
     from tinyserve_llm_b200.config.spec import GatedDeltaRuleSpec, LinearRecurrenceSpec
     from tinyserve_llm_b200.parts.base import Runtime, part_class

@@ -25,8 +25,8 @@
 // No decay is ever divided by another: products of decays are taken as they are needed.
 //
 // What the plain recurrence and the delta rule with decays per channel hold to (relative error of outputs / states against 64 bits, the
-// walk token by token and here): gated linear attention over 2,048 tokens 1.72e-7 / 1.46e-7 and 1.35e-7 / 6.2e-8, constant decays
-// 2.5e-7 / 2.4e-7 and 1.6e-7 / 1.1e-7, the delta rule over portions of 1,001, 667 and 333 tokens 3.0e-7 / 4.2e-7 and 1.9e-7 / 1.8e-7.
+// walk token by token and here; the plain recurrence over bfloat16 values: recurrence_stretches.cu): gated linear attention over 2,048 tokens
+// 1.73e-7 / 1.47e-7 and 1.20e-7 / 5.4e-8, constant decays 2.5e-7 / 2.4e-7 and 1.45e-7 / 1.04e-7, the delta rule over portions of 1,001, 667 and 333 tokens 3.0e-7 / 4.2e-7 and 1.9e-7 / 1.8e-7.
 // Three things bring that: the products of decays from a tile's ends are taken in 64 bits and rounded once (sixteen roundings of one
 // constant decay all err to one side, tile after tile: 6.2e-7 / 5.9e-7); a decay near one enters them with the bits past float32's that
 // 1 + expm1 knows; no accumulator of the tensor cores, which cut what it cannot hold, takes more than one large part.  Sums inside a
@@ -53,11 +53,10 @@
 // A tile cut short by the portion's end is filled up with tokens that change nothing (k = 0, decay 1).  Requests that
 // feed one token are left to the other scan.  Tiles count from the portion's first token, so where a prompt was cut
 // moves sums inside rounding only.
-#include "common.cuh"
+#include "recurrence_tiles.cuh"
 
 namespace {
 
-constexpr int B = 16;              // tokens a tile
 constexpr int COLS = 16;           // value channels a CTA
 constexpr int WARPS = 4, THREADS = WARPS * 32;   // of the scan
 constexpr int CP = 20;             // pitch of a coefficient matrix: a warp's fragment loads fall into different banks
@@ -71,10 +70,6 @@ enum { DELTA = 0, MIX = 1, CHANNEL = 2, PLAIN = 3 };   // delta rule, a decay a 
 __host__ __device__ constexpr int sets_of(int mode) { return mode == CHANNEL ? 2 : 1; }
 
 __device__ __forceinline__ float softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
-
-// Where a request's tiles lie among all tiles: request s's first at cu_q[s] / 16 + s.  Every request has room for its own
-// (a portion of n tokens takes ceil(n / 16), and the next request's first lies at least that much further on).
-__device__ __forceinline__ long long tile_slot(int seq, int begin, int tile) { return begin / B + seq + tile; }
 
 struct PrepareArgs {
     const void* q; const void* k; long long qk_stride;   // delta: float32 after the convolution; mixing: r, k as projected
@@ -251,119 +246,24 @@ __global__ void __launch_bounds__(128) mix_tile_prepare_kernel(PrepareArgs p) {
     }
 }
 
-// exp(x), x <= 0, as a float32 number and what that lacks: near one, where a portion multiplies many of them, 1 + expm1(x) is known to
-// more bits than float32 holds.
-__device__ __forceinline__ float decay_of(float x, float& rest) {
-    const float a = expf(x);
-    rest = 0.f;
-    if (!(x > -0.6f)) return a;
-    const float m = expm1f(x), near = 1.f + m;
-    rest = m - (near - 1.f);
-    return near;
-}
-
-__device__ __forceinline__ double whole(float a, __nv_bfloat16 rest) { return (double)a + (double)__bfloat162float(rest); }
-
-struct PlainArgs {
-    const void* q; const void* k; long long q_stride, k_stride;
-    const float* z; long long z_stride; const float* bias;   // decay logits a channel (a = sigmoid(z + bias)^inv_tau), or
-    const float* head_decay;                                 // one decay a head
-    float inv_tau, q_scale, k_scale;
-    const float* freq; int rot_dims; const int* positions;   // rotation by halves over the first rot_dims channels
-    const int* cu_q; const int* prefill_seqs;
-    float* pack; float* coef;
-    int heads, dim;
-};
-
-// The plain recurrence's pack and P.  grid (tiles, heads, portions), 128 threads.  Bound by its own arithmetic (a decay and,
-// with rotation, a sine and a cosine an element, then the running products); it takes the place of a kernel that wrote q, k and the
-// decays of every token to memory.  2,048 tokens, 8 heads of 128: 31 us (34 before ROWS was a constant and the warps skipped the t
-// ahead of their j); the scan behind it 141 us where the walk token by token took 262.
-template <typename T, int ROWS>
+// The plain recurrence's pack and P, float32.  grid (tiles, heads, portions), 128 threads.
+template <int ROWS>
 __global__ void __launch_bounds__(128) plain_tile_prepare_kernel(PlainArgs p) {
     extern __shared__ float smem[];
     const int seq = p.prefill_seqs[blockIdx.z], tile = blockIdx.x, h = blockIdx.y;
     if (seq < 0) return;
     const int begin = p.cu_q[seq], n = p.cu_q[seq + 1] - begin;
     if (n <= 1 || tile * B >= n) return;
-    const int t0 = begin + tile * B, m = min(B, n - tile * B);
-    const int pitch = ROWS + 1;
-    float* qs = smem;                                    // [16][pitch]
-    float* ks = qs + B * pitch;
-    float* as = ks + B * pitch;
-    __nv_bfloat16* rest = reinterpret_cast<__nv_bfloat16*>(as + B * pitch);        // what the decays lack
-    const int half = p.rot_dims / 2;
-#pragma unroll 4
-    for (int e = threadIdx.x; e < B * ROWS; e += 128) {
-        const int t = e / ROWS, i = e % ROWS;
-        float qv = 0.f, kv = 0.f, av = 1.f, more = 0.f;  // a token past the portion's end changes nothing
-        if (t < m && i < p.dim) {
-            const T* qr = (const T*)p.q + (long long)(t0 + t) * p.q_stride + (long long)h * p.dim;
-            const T* kr = (const T*)p.k + (long long)(t0 + t) * p.k_stride + (long long)h * p.dim;
-            qv = to_float<T>(qr[i]);
-            kv = to_float<T>(kr[i]);
-            if (i < p.rot_dims) {
-                const int f = i < half ? i : i - half, other = i < half ? i + half : i - half;
-                float sn, cs;
-                sincosf((float)p.positions[t0 + t] * p.freq[f], &sn, &cs);
-                const float qo = to_float<T>(qr[other]), ko = to_float<T>(kr[other]);
-                qv = i < half ? qv * cs - qo * sn : qv * cs + qo * sn;
-                kv = i < half ? kv * cs - ko * sn : kv * cs + ko * sn;
-            }
-            qv *= p.q_scale;
-            kv *= p.k_scale;
-            if (p.z) {
-                const float x = p.z[(long long)(t0 + t) * p.z_stride + (long long)h * p.dim + i] + (p.bias ? p.bias[h * p.dim + i] : 0.f);
-                av = decay_of((fminf(x, 0.f) - log1pf(expf(-fabsf(x)))) * p.inv_tau, more);
-            } else {
-                av = p.head_decay[h];
-            }
-        }
-        qs[t * pitch + i] = qv;
-        ks[t * pitch + i] = kv;
-        as[t * pitch + i] = av;
-        rest[t * pitch + i] = __float2bfloat16_rn(more);
-    }
+    const PlainTile<ROWS> x(smem);
+    load_plain<float, ROWS>(p, x, h, begin + tile * B, min(B, n - tile * B));
     __syncthreads();
     const long long slot = tile_slot(seq, begin, tile);
-    {   // P[t][j], t >= j: thread j = tid / 8 walks t with the running product of its channels
-        const int j = threadIdx.x >> 3, part = threadIdx.x & 7;
-        float sum[B];
-#pragma unroll
-        for (int t = 0; t < B; ++t) sum[t] = 0.f;
-        for (int i = part; i < p.dim; i += 8) {
-            float run = ks[j * pitch + i];
-#pragma unroll
-            for (int t = 0; t < B; ++t) {
-                if (t < (int)(threadIdx.x >> 5) * 4) continue;                          // the warp's four j begin here
-                if (t > j) run *= as[t * pitch + i];
-                if (t >= j) sum[t] = fmaf(qs[t * pitch + i], run, sum[t]);
-            }
-        }
-        float* out = p.coef + (slot * p.heads + h) * COEF + B * CP;
-#pragma unroll
-        for (int t = 0; t < B; ++t) {
-            float s = sum[t];
-#pragma unroll
-            for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (part == 0) out[t * CP + j] = s;                                         // 0 where t < j
-        }
-    }
+    float* out = p.coef + (slot * p.heads + h) * COEF + B * CP;
+    plain_scores<ROWS>(x, p.dim, [&](int t, int j, float s) { out[t * CP + j] = s; });
     float* pack = p.pack + (slot * p.heads + h) * pack_floats(ROWS, 1);
-    for (int i = threadIdx.x; i < ROWS; i += 128) {    // a thread a channel: products from the left and from the right
+    for (int i = threadIdx.x; i < ROWS; i += 128) {
         const int pp = pack_pitch(ROWS);
-        double left = 1.0, right = 1.0;
-#pragma unroll
-        for (int t = 0; t < B; ++t) {
-            left *= whole(as[t * pitch + i], rest[t * pitch + i]);
-            pack[t * pp + i] = (float)((double)qs[t * pitch + i] * left);
-        }
-#pragma unroll
-        for (int t = B - 1; t >= 0; --t) {
-            pack[(B + t) * pp + i] = (float)((double)ks[t * pitch + i] * right);
-            right *= whole(as[t * pitch + i], rest[t * pitch + i]);
-        }
-        pack[2 * B * pp + i] = (float)left;
+        pack[2 * B * pp + i] = plain_sides<ROWS>(x, i, [&](int t, float q) { pack[t * pp + i] = q; }, [&](int t, float k) { pack[(B + t) * pp + i] = k; });
     }
 }
 
@@ -505,66 +405,6 @@ struct ScanArgs {
     int heads, qk_group, dim, vdim;
 };
 
-__device__ __forceinline__ void cp16(void* smem, const void* gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
-}
-
-// A float32 number as the sum of two TF32 numbers (11 significant bits each): hi is x to the nearest (half of its last
-// place added before the low 13 bits go), lo what is left, of which the tensor cores read the leading bits: 2^-23 of x is lost.
-struct Split { uint32_t hi, lo; };
-__device__ __forceinline__ Split split_tf32(float x) {
-    Split s;
-    s.hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-    s.lo = __float_as_uint(x - __uint_as_float(s.hi));
-    return s;
-}
-// What the tensor cores drop of lo.
-__device__ __forceinline__ uint32_t rest_of(uint32_t lo) { return __float_as_uint(__uint_as_float(lo) - __uint_as_float(lo & 0xffffe000u)); }
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-struct SplitA { uint32_t hi[4], lo[4]; };
-__device__ __forceinline__ SplitA split_a(float a0, float a1, float a2, float a3) {
-    const Split s0 = split_tf32(a0), s1 = split_tf32(a1), s2 = split_tf32(a2), s3 = split_tf32(a3);
-    return SplitA{{s0.hi, s1.hi, s2.hi, s3.hi}, {s0.lo, s1.lo, s2.lo, s3.lo}};
-}
-// The two large and the small parts of a product of split factors, each in an accumulator of its own (no long chain).  FRESH: every
-// large part begins at zero and is added by an ordinary rounded addition, where the tensor cores cut what an accumulator cannot hold.
-template <bool FRESH>
-__device__ __forceinline__ void mma_split(float (&big)[4], float (&small)[4], const SplitA& a, Split b0, Split b1) {
-    if (FRESH) {
-        float part[4] = {};
-        mma_tf32(part, a.hi, b0.hi, b1.hi);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) big[i] += part[i];
-    } else {
-        mma_tf32(big, a.hi, b0.hi, b1.hi);
-    }
-    mma_tf32(small, a.hi, b0.lo, b1.lo);
-    mma_tf32(small, a.lo, b0.hi, b1.hi);
-}
-
-// Products of which one factor is a TF32 number itself (bfloat16 values): the other in three pieces, all of it.
-__device__ __forceinline__ void mma_exact_b(float (&big)[4], float (&small)[4], const SplitA& a, float b0, float b1) {
-    const uint32_t rest[4] = {rest_of(a.lo[0]), rest_of(a.lo[1]), rest_of(a.lo[2]), rest_of(a.lo[3])};
-    float part[4] = {};
-    mma_tf32(part, a.hi, __float_as_uint(b0), __float_as_uint(b1));
-    mma_tf32(small, a.lo, __float_as_uint(b0), __float_as_uint(b1));
-    mma_tf32(small, rest, __float_as_uint(b0), __float_as_uint(b1));
-#pragma unroll
-    for (int i = 0; i < 4; ++i) big[i] += part[i];
-}
-__device__ __forceinline__ void mma_exact_a(float (&big)[4], float (&small)[4], const uint32_t (&a)[4], Split b0, Split b1) {
-    float part[4] = {};
-    mma_tf32(part, a, b0.hi, b1.hi);
-    mma_tf32(small, a, b0.lo, b1.lo);
-    mma_tf32(small, a, rest_of(b0.lo), rest_of(b1.lo));
-#pragma unroll
-    for (int i = 0; i < 4; ++i) big[i] += part[i];
-}
-
 // Numbers from here on have no split (their hi would be infinite).
 constexpr float SPLITS = 3.4e38f;
 
@@ -599,7 +439,7 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
     constexpr bool VALUES = MODE == MIX || MODE == PLAIN;   // the values themselves move the state on
     constexpr int TQ = VALUES ? B : 2 * B;               // rows of the pack that meet S_0
     constexpr bool FRESH = MODE == PLAIN || MODE == CHANNEL;   // (the others sum as they did before)
-    constexpr bool EXACT = MODE == PLAIN && sizeof(T) == 2;    // the values are TF32 numbers
+    static_assert(MODE != PLAIN || sizeof(T) == 4, "bfloat16: recurrence_stretches.cu");
     extern __shared__ __align__(16) float smem[];
     float* red = smem + 2 * STAGE;                       // [WARPS][TQ][RP]
     float* G_s = red + WARPS * TQ * RP;                  // [B][RP]: what the state's update takes, G[B] U or V
@@ -722,8 +562,7 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
                 for (int ks = 0; ks < 2; ++ks) {
                     const float* a = m + r * CP + 8 * ks + c;
                     const SplitA w = split_a(a[0], a[8 * CP], a[4], a[8 * CP + 4]);
-                    if (EXACT) mma_exact_b(big, small, w, kept[2 * ks], kept[2 * ks + 1]);
-                    else mma_split<FRESH>(big, small, w, split_tf32(kept[2 * ks]), split_tf32(kept[2 * ks + 1]));
+                    mma_split<FRESH>(big, small, w, split_tf32(kept[2 * ks]), split_tf32(kept[2 * ks + 1]));
                 }
                 float4 late = make_float4(0.f, 0.f, 0.f, 0.f);   // and reaches its own and later tokens by itself
                 if (__any_sync(0xffffffffu, odd)) late = add_odd_tokens(m, x[0], x[1], x[2], x[3], r, c);
@@ -773,8 +612,7 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
 #pragma unroll
                 for (int ks = 0; ks < 2; ++ks) {
                     const Split k0 = split_tf32(k[8 * ks * PP]), k1 = split_tf32(k[(8 * ks + 4) * PP]);
-                    if (EXACT) mma_exact_a(big, small, a[ks].hi, k0, k1);
-                    else mma_split<FRESH>(big, small, a[ks], k0, k1);
+                    mma_split<FRESH>(big, small, a[ks], k0, k1);
                 }
                 float2 d = make_float2(cB, cB);
                 if (MODE != DELTA) d = *reinterpret_cast<const float2*>(pack + (1 + SETS) * B * PP + warp * WROWS + 8 * nt + 2 * c);
@@ -795,8 +633,6 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
             if (element(nt, e, i, j)) st[(long long)i * p.vdim + j] = S[nt][e];
         }
 }
-
-int padded_rows(int dim) { return dim <= 64 ? 64 : dim <= 128 ? 128 : 256; }
 
 template <typename T, int MODE>
 int launch_scan(const ScanArgs& p, int portions, cudaStream_t stream) {
@@ -880,43 +716,41 @@ TS_API int ts_mix_tiles(const void* r, const void* k, long long rk_stride, const
     return ts_fail("mix_tiles: unknown dtype code %d", dtype);
 }
 
-// The plain recurrence over a step's prompt portions: q, k, v as `ts_linear_recurrence` takes them.
+// Floats of the buffer of `ts_plain_tiles`.
+TS_API long long ts_plain_tiles_floats(int num_tokens, int num_seqs, int heads, int dim, int vdim, int dtype) {
+    if (dtype == TS_BF16) return plain_stretches_floats(num_tokens, num_seqs, heads, dim, vdim);
+    return ts_recurrence_tiles_pack_floats(num_tokens, num_seqs, heads, dim, 1) + ts_recurrence_tiles_coef_floats(num_tokens, num_seqs, heads);
+}
+
+// The plain recurrence over a step's prompt portions: q, k, v as `ts_linear_recurrence` takes them; `buffer` has the floats of
+// `ts_plain_tiles_floats`.  bfloat16 goes by stretches.
 TS_API int ts_plain_tiles(const void* q, const void* k, const void* v, long long q_stride, long long k_stride, long long v_stride,
                           const float* z, long long z_stride, const float* bias, const float* head_decay, float inv_tau,
                           float q_scale, float k_scale, const float* freq, int rot_dims, const int* positions, const int* cu_q,
-                          const int* slots, const int* prefill_seqs, int portions, int max_q_len, float* state,
-                          long long slot_stride, float* pack, float* coef, float* out, int heads, int dim, int vdim, int dtype,
+                          const int* slots, const int* prefill_seqs, int portions, int max_q_len, int num_tokens, int num_seqs,
+                          float* state, long long slot_stride, float* buffer, float* out, int heads, int dim, int vdim, int dtype,
                           cudaStream_t stream) {
     TS_REQUIRE(heads > 0 && dim > 0 && dim <= 256 && vdim > 0, "plain_tiles: %d heads of %d channels", heads, dim);
     TS_REQUIRE(rot_dims >= 0 && rot_dims <= dim && rot_dims % 2 == 0, "plain_tiles: rotation over %d of %d channels", rot_dims, dim);
     TS_REQUIRE((z != nullptr) != (head_decay != nullptr), "plain_tiles: either decay logits or one decay per head");
     TS_REQUIRE(slot_stride >= (long long)heads * dim * vdim, "plain_tiles: a state slot is too small");
     TS_REQUIRE(portions >= 0 && portions <= 65535 && heads <= 65535, "plain_tiles: grid too large");
+    TS_REQUIRE(dtype == TS_F32 || dtype == TS_BF16, "plain_tiles: unknown dtype code %d", dtype);
     if (portions == 0 || max_q_len <= 1) return 0;
-    const PlainArgs a{q, k, q_stride, k_stride, z, z_stride, bias, head_decay, inv_tau, q_scale, k_scale, freq, freq ? rot_dims : 0,
-                      positions, cu_q, prefill_seqs, pack, coef, heads, dim};
+    PlainArgs a{q, k, q_stride, k_stride, z, z_stride, bias, head_decay, inv_tau, q_scale, k_scale, freq, freq ? rot_dims : 0,
+                positions, cu_q, prefill_seqs, buffer, nullptr, heads, dim};
+    if (dtype == TS_BF16)
+        return plain_stretches(a, (const __nv_bfloat16*)v, v_stride, slots, portions, max_q_len, state, slot_stride, num_tokens, num_seqs, out, vdim, stream);
+    a.coef = buffer + ts_recurrence_tiles_pack_floats(num_tokens, num_seqs, heads, dim, 1);
     const int rows = padded_rows(dim);
-    const size_t smem = sizeof(float) * (3 * B * (rows + 1)) + 2 * B * (rows + 1);      // 29 KB at 128 channels: seven CTAs an SM
+    const size_t smem = rows == 64 ? PlainTile<64>::BYTES : rows == 128 ? PlainTile<128>::BYTES : PlainTile<256>::BYTES;   // 29 KB at 128 channels
     const dim3 grid((max_q_len + B - 1) / B, heads, portions);
-    const ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, vdim};
-#define TS_PLAIN_PREPARE(T)                                                                                                    \
-    do {                                                                                                                       \
-        auto kernel = rows == 64 ? plain_tile_prepare_kernel<T, 64> : rows == 128 ? plain_tile_prepare_kernel<T, 128>          \
-                                                                                  : plain_tile_prepare_kernel<T, 256>;         \
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                                  \
-        kernel<<<grid, 128, smem, stream>>>(a);                                                                                \
-        TS_LAUNCH_CHECK("plain_tiles (prepare)");                                                                              \
-    } while (0)
-    if (dtype == TS_F32) {
-        TS_PLAIN_PREPARE(float);
-        return launch_scan<float, PLAIN>(s, portions, stream);
-    }
-    if (dtype == TS_BF16) {
-        TS_PLAIN_PREPARE(__nv_bfloat16);
-        return launch_scan<__nv_bfloat16, PLAIN>(s, portions, stream);
-    }
-#undef TS_PLAIN_PREPARE
-    return ts_fail("plain_tiles: unknown dtype code %d", dtype);
+    const ScanArgs s{a.pack, a.coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, vdim};
+    auto kernel = rows == 64 ? plain_tile_prepare_kernel<64> : rows == 128 ? plain_tile_prepare_kernel<128> : plain_tile_prepare_kernel<256>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kernel<<<grid, 128, smem, stream>>>(a);
+    TS_LAUNCH_CHECK("plain_tiles (prepare)");
+    return launch_scan<float, PLAIN>(s, portions, stream);
 }
 
 // The delta rule with decays per channel over a step's prompt portions: q, k float32 [tokens, kv_heads * dim] stretches after the

@@ -98,7 +98,8 @@ _SIGNATURES = {
     "ts_recurrence_tiles_coef_floats": ("long long", "iii"),
     "ts_delta_tiles": ("int", "pplppppl" "pppii" "plppp" "iiiiffp"),
     "ts_mix_tiles": ("int", "pplppppl" "pppii" "plppp" "iiip"),
-    "ts_plain_tiles": ("int", "ppplll" "plpp" "fffpip" "pppii" "plppp" "iiiip"),
+    "ts_plain_tiles": ("int", "ppplll" "plpp" "fffpip" "pppiiii" "plpp" "iiiip"),
+    "ts_plain_tiles_floats": ("long long", "iiiiii"),
     "ts_channel_tiles": ("int", "pplpplipp" "pl" "pppii" "plppp" "iiiiffp"),
     "ts_delta_prepare": ("int", "pplppppl" "ppiiiiff" "ppip"),
     "ts_mlstm_prepare": ("int", "ppllpplppffppiplpppiiiip"),
@@ -610,13 +611,14 @@ class Ops:
         if tiles is None:
             tiles = self.portions_by_tiles(ctx)
         if tiles:                                            # prompt portions sixteen tokens at a time
-            buffer, pack, coef = self._tile_buffers(ctx, T, heads, heads, dim, q.device)
+            seqs, code = ctx.cu_q.shape[0] - 1, _DTYPE_CODE[q.dtype]
+            buffer = torch.empty((int(self.lib.ts_plain_tiles_floats(T, seqs, heads, dim, vdim, code)),), dtype=torch.float32, device=q.device)
             self._call("ts_plain_tiles", _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _ptr(z),
                        z.stride(0) if z is not None else 0, _ptr(bias), _ptr(head_decays), inv_tau, q_scale, k_scale, _ptr(freq),
                        rot, _ptr(ctx.positions), _ptr(ctx.cu_q), _ptr(binding.state_slots), _ptr(ctx.prefill_seqs),
-                       ctx.prefill_seqs.shape[0], ctx.max_q_len, state.data_ptr(), state.stride(0) // 4, pack, coef,
-                       _ptr(out), heads, dim, vdim, _DTYPE_CODE[q.dtype], _stream())
-            self.launches += 1                               # what the columns of a tile share, then the scan
+                       ctx.prefill_seqs.shape[0], ctx.max_q_len, T, seqs, state.data_ptr(), state.stride(0) // 4, _ptr(buffer),
+                       _ptr(out), heads, dim, vdim, code, _stream())
+            self.launches += 2 if code else 1                # what the columns of a tile share, (the states before stretches,) the scan
             if getattr(ctx, "min_q_len", 1) > 1:             # a bare context may not say: single tokens are then looked for
                 return out
         prepared = torch.empty((3, T, heads * dim), dtype=torch.float32, device=q.device)   # q, k, decays as they enter the scan

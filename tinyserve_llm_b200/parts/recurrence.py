@@ -28,13 +28,13 @@ from tinyserve_llm_b200.parts.base import Mixer, Runtime, TensorDecl, part_class
 from tinyserve_llm_b200.parts.linear import Linear, fuse_rows
 
 MAX_KEY_DIM = 256       # csrc/linear_recurrence.cu: 16 row groups x 16 rows in registers
-# Prompt portions go sixteen tokens at a time (csrc/recurrence_tiles.cu) in steps whose longest has this many tokens: a tile waits
-# longer for its first result than the walk takes for a few tokens.  A layer of 8 heads of 128 x 256 channels, captured, us, walk and
-# tiles: one portion of 145 tokens 48 / 56, 256 63 / 66, 300 71 / 72, 500 101 / 89; two of 200 66 / 69, of 300 86 / 80; four of 145
-# 74 / 72, of 256 109 / 90.  (A replayed step's bound is a power of two: from 257 tokens on.)
+# Prompt portions go sixteen tokens at a time (csrc/recurrence_stretches.cu) in steps whose longest has this many tokens: three kernels wait
+# longer for their first result than the walk takes for a few tokens.  A layer of 8 heads of 128 x 256 channels, captured, us, walk and
+# tiles: one portion of 145 tokens 44 / 50, 200 57 / 56, 256 61 / 54, 300 69 / 61; two of 200 64 / 59; four of 145 72 / 69; 4 heads 145
+# 40 / 46, 200 48 / 48, 256 55 / 49.  A replayed step's bound is a power of two, which 145 tokens share with 256: from 257 on there.
 # float32 activations walk token by token whatever their number, so that a token's result depends on nothing but the tokens before it,
 # wherever the step was cut.
-TILE_TOKENS = 288
+TILE_TOKENS, TILE_TOKENS_REPLAYED = 200, 257
 
 
 @register_part("mixer", "linear_recurrence")
@@ -111,6 +111,7 @@ class LinearRecurrence(Mixer):
                                   bias=self.decay_bias if self.decay_rank else None, head_decays=self.head_decays,
                                   inv_tau=1.0 / spec.tau, q_scale=spec.q_scale, k_scale=spec.k_scale,
                                   position=self.position,
-                                  tiles=x.dtype != torch.float32 and ops.portions_by_tiles(ctx, TILE_TOKENS))   # float32 [T, H V]
+                                  tiles=x.dtype != torch.float32 and ops.portions_by_tiles(
+                                      ctx, TILE_TOKENS_REPLAYED if getattr(ctx, "replayed", False) else TILE_TOKENS))   # float32 [T, H V]
         gated = ops.head_norm_gate(o, g, self.norm_weight, H, V, spec.out_norm_eps, x.dtype)
         return self.out(gated)
