@@ -1605,12 +1605,13 @@ class Ops:
         out_dtype = out_dtype or x.dtype
         if x.dtype == torch.float32 and out_dtype != torch.float32:
             raise KernelError("linear: the float32 product has float32 output")
-        if out is None:
-            out = torch.empty((x.shape[0], weight.shape[0]), dtype=out_dtype, device=x.device)
-        else:
+        skinny = self._skinny(x, weight)
+        if out is not None:
             self._check(out, "out", out_dtype, 2)
             if tuple(out.shape) != (x.shape[0], weight.shape[0]):
                 raise KernelError(f"linear: out is {tuple(out.shape)}, the product {(x.shape[0], weight.shape[0])}")
+        elif skinny or x.dtype == torch.float32:
+            out = torch.empty((x.shape[0], weight.shape[0]), dtype=out_dtype, device=x.device)
         if x.dtype == torch.float32:
             (M, K), N = x.shape, weight.shape[0]
             floats = int(self.lib.ts_sgemm_nt_scratch_floats(M, N, K))
@@ -1618,17 +1619,36 @@ class Ops:
             self._call("ts_sgemm_nt", _ptr(x), _ptr(weight), _ptr(out), M, N, K, K, K, N, _ptr(scratch), floats,
                        self.error_word().data_ptr(), _stream())
             return out
-        if self._skinny(x, weight):
+        if skinny:
             self._call("ts_skinny_linear", _ptr(weight), _ptr(x), _ptr(out), x.shape[0], weight.shape[0],
                        x.shape[1], x.shape[1], weight.shape[0], 0,
                        _DTYPE_CODE[out_dtype], _stream())
             if out_dtype == torch.float32:
                 self.calls["ts_skinny_linear:float32_out"] = self.calls.get("ts_skinny_linear:float32_out", 0) + 1
             return out
+        return self._library_mm(x, weight, out_dtype, out)
+
+    def _library_mm(self, x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype, out: torch.Tensor | None) -> torch.Tensor:
+        """The library's product; without `out` it makes its own result (2.4 us of host time less than a tensor made here and handed to it)."""
         self.calls["library_mm"] = self.calls.get("library_mm", 0) + 1
+        if out is None:
+            return torch.mm(x, weight.t()) if out_dtype == x.dtype else torch.mm(x, weight.t(), out_dtype=out_dtype)
         if out_dtype != x.dtype:
             return torch.mm(x, weight.t(), out_dtype=out_dtype, out=out)
         return torch.mm(x, weight.t(), out=out)
+
+    def linear_columns(self, x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None = None) -> torch.Tensor:
+        """
+        `linear` of a stretch of columns of wider rows: the library product takes it where it lies (a copy of its own took a launch,
+        3 us at 2,048 rows, and as long as a product on the host); the engine's kernels take a copy.
+        """
+        self._check_rows(x, "x")
+        if x.dtype == torch.bfloat16 and x.shape[0] > self.skinny_max_rows and x.shape[1] > 1:
+            self._check(weight, "weight", x.dtype, 2)
+            if x.shape[1] != weight.shape[1]:
+                raise KernelError(f"linear: x has {x.shape[1]} columns, the weight {weight.shape[1]}")
+            return self._library_mm(x, weight, out_dtype or x.dtype, None)
+        return self.linear(x.contiguous(), weight, out_dtype)
 
     def linear_groups(self, x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None = None) -> torch.Tensor:
         """

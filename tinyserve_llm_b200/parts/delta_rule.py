@@ -124,7 +124,7 @@ class GatedDeltaRule(Mixer):
         conv = ops.short_conv_silu(y[:, :C], self.taps, ctx, carried)                        # float32 [T, C]
         gate = y[:, C + self.decay_rank:C + self.decay_rank + self.gate_rank]
         if not self.full_gate:
-            gate = self.gate_up(gate.contiguous())
+            gate = self.gate_up.columns(gate)
         b = self.beta(x, out_dtype=torch.float32)
         q, k, v = conv[:, :G * D], conv[:, G * D:2 * G * D], conv[:, 2 * G * D:]
         sizes = dict(heads=H, kv_heads=G, dim=D, unit_eps=s.unit_eps, q_scale=s.q_scale)
@@ -137,7 +137,7 @@ class GatedDeltaRule(Mixer):
                 o = ops.recurrence_scan(prepared, v, ctx, matrices, heads=H, dim=D, vdim=V, beta=beta, head_decay=decay,
                                         qk_group=H // G, singles=tiles, out=o)
         else:
-            z = self.decay_up(y[:, C:C + self.decay_rank].contiguous(), out_dtype=torch.float32)  # decay logits, float32 from here on
+            z = self.decay_up.columns(y[:, C:C + self.decay_rank], out_dtype=torch.float32)   # decay logits, float32 from here on
             # float32 activations token by token (as in parts/recurrence.py)
             o, tiles = None, x.dtype != torch.float32 and ops.portions_by_tiles(ctx, CHANNEL_TILE_TOKENS)
             if tiles:

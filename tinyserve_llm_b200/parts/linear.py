@@ -29,3 +29,7 @@ class Linear:
     def __call__(self, x: torch.Tensor, out_dtype: torch.dtype | None = None,
                  out: torch.Tensor | None = None) -> torch.Tensor:
         return self.rt.ops.linear(x, self.weight, out_dtype=out_dtype, out=out)
+
+    def columns(self, x: torch.Tensor, out_dtype: torch.dtype | None = None) -> torch.Tensor:
+        """The product of a stretch of columns of wider rows."""
+        return self.rt.ops.linear_columns(x, self.weight, out_dtype=out_dtype)

@@ -105,8 +105,7 @@ class LinearRecurrence(Mixer):
         q, k, v, g = y[:, :H * D], y[:, H * D:2 * H * D], y[:, 2 * H * D:2 * H * D + H * V], y[:, 2 * H * D + H * V:2 * H * D + 2 * H * V]
         z = None
         if self.decay_rank:
-            low = y[:, 2 * H * D + 2 * H * V:].contiguous()
-            z = self.decay_up(low, out_dtype=torch.float32)               # decay logits, float32 from here on
+            z = self.decay_up.columns(y[:, 2 * H * D + 2 * H * V:], out_dtype=torch.float32)   # decay logits, float32 from here on
         o = ops.linear_recurrence(q, k, v, ctx, binding, heads=H, dim=D, vdim=V, z=z,
                                   bias=self.decay_bias if self.decay_rank else None, head_decays=self.head_decays,
                                   inv_tau=1.0 / spec.tau, q_scale=spec.q_scale, k_scale=spec.k_scale,
