@@ -279,16 +279,18 @@ struct ChannelArgs {
 };
 
 // The pack and the coefficients of the delta rule with decays per channel.  grid (tiles, value heads, portions), 128 threads.
-// Three portions of 1,001, 667 and 333 tokens, 8 heads of 128: 33 us; the scan behind it 100 us, token by token 300.
+// Bound by instructions (decays, running products) and by waits for its loads: all of a warp's four tokens' are under way together, seven
+// CTAs share an SM.  Three portions of 1,001, 667 and 333 tokens, 8 heads of 128: 29 us (33 with a token's loads at a time and one channel a
+// read of shared memory); the walk behind it 86, token by token 300.
 template <typename T, int ROWS>
-__global__ void __launch_bounds__(128) channel_tile_prepare_kernel(ChannelArgs p) {
+__global__ void __launch_bounds__(128, ROWS == 128 ? 7 : 1) channel_tile_prepare_kernel(ChannelArgs p) {
     extern __shared__ float smem[];
     const int seq = p.prefill_seqs[blockIdx.z], tile = blockIdx.x, h = blockIdx.y, g = h / (p.heads / p.kv_heads);
     if (seq < 0) return;
     const int begin = p.cu_q[seq], n = p.cu_q[seq + 1] - begin;
     if (n <= 1 || tile * B >= n) return;
     const int t0 = begin + tile * B, m = min(B, n - tile * B);
-    const int pitch = ROWS + 1;
+    constexpr int pitch = ROWS + 2;                      // even: two channels a read
     float* qs = smem;                                    // [16][pitch]
     float* ks = qs + B * pitch;
     float* as = ks + B * pitch;
@@ -297,25 +299,44 @@ __global__ void __launch_bounds__(128) channel_tile_prepare_kernel(ChannelArgs p
     __nv_bfloat16* rest = reinterpret_cast<__nv_bfloat16*>(qk + B * (B + 1));      // [16][pitch]: what the decays lack
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float rate = expf(p.rate[h]);
-    for (int t = warp; t < B; t += 4) {
-        const float* qr = p.q + (long long)(t0 + t) * p.qk_stride + (long long)g * p.dim;
-        const float* kr = p.k + (long long)(t0 + t) * p.qk_stride + (long long)g * p.dim;
-        const float* zr = p.z + ((long long)(t0 + t) * p.heads + h) * p.dim;
-        float sq = 0.f, sk = 0.f;
+    constexpr int EACH = ROWS / 32, DEEP = ROWS > 128 ? 1 : 4;          // channels a lane; tokens whose loads are under way together
+    for (int first = warp; first < B; first += 4 * DEEP) {
+        float q[DEEP][EACH], k[DEEP][EACH], z[DEEP][EACH];
 #pragma unroll
-        for (int i = lane; i < ROWS; i += 32) {
-            const bool ok = t < m && i < p.dim;          // a token past the portion's end changes nothing
-            const float qv = ok ? qr[i] : 0.f, kv = ok ? kr[i] : 0.f;
-            qs[t * pitch + i] = qv;
-            ks[t * pitch + i] = kv;
-            float more = 0.f;
-            as[t * pitch + i] = ok ? decay_of(-rate * softplus(zr[i] + p.bias[h * p.dim + i]), more) : 1.f;
-            rest[t * pitch + i] = __float2bfloat16_rn(more);
-            sq += qv * qv;
-            sk += kv * kv;
+        for (int e = 0; e < DEEP; ++e) {
+            const int t = first + 4 * e;
+            const float* qr = p.q + (long long)(t0 + t) * p.qk_stride + (long long)g * p.dim;
+            const float* kr = p.k + (long long)(t0 + t) * p.qk_stride + (long long)g * p.dim;
+            const float* zr = p.z + ((long long)(t0 + t) * p.heads + h) * p.dim;
+#pragma unroll
+            for (int u = 0; u < EACH; ++u) {
+                const int i = lane + 32 * u;
+                const bool ok = t < m && i < p.dim;      // a token past the portion's end changes nothing
+                q[e][u] = ok ? qr[i] : 0.f;
+                k[e][u] = ok ? kr[i] : 0.f;
+                z[e][u] = ok ? zr[i] : 0.f;
+            }
         }
-        const float iq = p.q_scale / sqrtf(warp_sum(sq) + p.unit_eps), ik = 1.f / sqrtf(warp_sum(sk) + p.unit_eps);
-        for (int i = lane; i < ROWS; i += 32) { qs[t * pitch + i] *= iq; ks[t * pitch + i] *= ik; }   // the lane's own elements
+#pragma unroll
+        for (int e = 0; e < DEEP; ++e) {
+            const int t = first + 4 * e;
+            float sq = 0.f, sk = 0.f;
+#pragma unroll
+            for (int u = 0; u < EACH; ++u) {
+                const int i = lane + 32 * u;
+                float more = 0.f;
+                as[t * pitch + i] = t < m && i < p.dim ? decay_of(-rate * softplus(z[e][u] + p.bias[h * p.dim + i]), more) : 1.f;
+                rest[t * pitch + i] = __float2bfloat16_rn(more);
+                sq += q[e][u] * q[e][u];
+                sk += k[e][u] * k[e][u];
+            }
+            const float iq = p.q_scale / sqrtf(warp_sum(sq) + p.unit_eps), ik = 1.f / sqrtf(warp_sum(sk) + p.unit_eps);
+#pragma unroll
+            for (int u = 0; u < EACH; ++u) {
+                qs[t * pitch + lane + 32 * u] = q[e][u] * iq;
+                ks[t * pitch + lane + 32 * u] = k[e][u] * ik;
+            }
+        }
     }
     __syncthreads();
     {   // t >= j: thread j = tid / 8 walks t with the running product of its channels
@@ -323,15 +344,20 @@ __global__ void __launch_bounds__(128) channel_tile_prepare_kernel(ChannelArgs p
         float sum_k[B], sum_q[B];
 #pragma unroll
         for (int t = 0; t < B; ++t) sum_k[t] = sum_q[t] = 0.f;
-        for (int i = part; i < p.dim; i += 8) {
-            float run = ks[j * pitch + i];
+        for (int i = 2 * part; i < p.dim; i += 16) {     // two channels (those past dim hold zeros)
+            float2 run = *reinterpret_cast<const float2*>(ks + j * pitch + i);
 #pragma unroll
             for (int t = 0; t < B; ++t) {
                 if (t < warp * 4) continue;                                             // the warp's four j begin here
-                if (t > j) run *= as[t * pitch + i];
+                if (t > j) {
+                    const float2 a = *reinterpret_cast<const float2*>(as + t * pitch + i);
+                    run.x *= a.x;
+                    run.y *= a.y;
+                }
                 if (t >= j) {
-                    sum_k[t] = fmaf(ks[t * pitch + i], run, sum_k[t]);
-                    sum_q[t] = fmaf(qs[t * pitch + i], run, sum_q[t]);
+                    const float2 kt = *reinterpret_cast<const float2*>(ks + t * pitch + i), qt = *reinterpret_cast<const float2*>(qs + t * pitch + i);
+                    sum_k[t] = fmaf(kt.y, run.y, fmaf(kt.x, run.x, sum_k[t]));
+                    sum_q[t] = fmaf(qt.y, run.y, fmaf(qt.x, run.x, sum_q[t]));
                 }
             }
         }
@@ -354,17 +380,18 @@ __global__ void __launch_bounds__(128) channel_tile_prepare_kernel(ChannelArgs p
     float* pack = p.pack + (slot * p.heads + h) * pack_floats(ROWS, 2);
     for (int i = threadIdx.x; i < ROWS; i += 128) {    // a thread a channel: products from the left and from the right
         const int pp = pack_pitch(ROWS);
-        double left = 1.0, right = 1.0;
+        double decay[B], left = 1.0, right = 1.0;
 #pragma unroll
         for (int t = 0; t < B; ++t) {
-            left *= whole(as[t * pitch + i], rest[t * pitch + i]);
+            decay[t] = whole(as[t * pitch + i], rest[t * pitch + i]);
+            left *= decay[t];
             pack[t * pp + i] = (float)((double)qs[t * pitch + i] * left);
             pack[(B + t) * pp + i] = (float)((double)ks[t * pitch + i] * left);
         }
 #pragma unroll
         for (int t = B - 1; t >= 0; --t) {
             pack[(2 * B + t) * pp + i] = (float)((double)ks[t * pitch + i] * right);
-            right *= whole(as[t * pitch + i], rest[t * pitch + i]);
+            right *= decay[t];
         }
         pack[3 * B * pp + i] = (float)left;
     }
@@ -403,6 +430,7 @@ struct ScanArgs {
     float* state; long long slot_stride;                 // floats between slots; a slot holds [heads, dim, vdim]
     float* out;                                          // [tokens, heads * vdim] float32
     int heads, qk_group, dim, vdim;
+    int* error;                                          // the delta rules' walk: where a wait that ran out says so
 };
 
 // Numbers from here on have no split (their hi would be infinite).
@@ -426,6 +454,34 @@ __device__ __noinline__ float4 add_odd_tokens(const float* m, float x0, float x4
     return make_float4(y[0], y[1], y[2], y[3]);
 }
 
+// Coefficients m [16][CP] times x (as a B fragment: tokens c, c + 4, c + 8, c + 12 of column r): a C fragment.
+template <bool FRESH>
+__device__ __forceinline__ void times_coefficients(float (&y)[4], const float* m, const float (&x)[4], int r, int c) {
+    float big[4], small[4];
+    float kept[4];                                       // what is not finite stays out of the product, where 0 times it is NaN
+    bool odd = false;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const bool ok = fabsf(x[k]) < SPLITS;
+        kept[k] = ok ? x[k] : 0.f;
+        odd |= !ok;
+    }
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks) {
+        const float* a = m + r * CP + 8 * ks + c;
+        const SplitA w = split_a(a[0], a[8 * CP], a[4], a[8 * CP + 4]);
+        const Split x0 = split_tf32(kept[2 * ks]), x1 = split_tf32(kept[2 * ks + 1]);
+        if (ks == 0) mma_split_first(big, small, w, x0, x1);
+        else mma_split<FRESH>(big, small, w, x0, x1);
+    }
+    float4 late = make_float4(0.f, 0.f, 0.f, 0.f);       // and reaches its own and later tokens by itself
+    if (__any_sync(0xffffffffu, odd)) late = add_odd_tokens(m, x[0], x[1], x[2], x[3], r, c);
+    y[0] = big[0] + small[0] + late.x;
+    y[1] = big[1] + small[1] + late.y;
+    y[2] = big[2] + small[2] + late.z;
+    y[3] = big[3] + small[3] + late.w;
+}
+
 // NT: eights of rows of the state a warp holds.  Fragments of mma.m16n8k8, lane = 4 r + c (r 0..7, c 0..3):
 //   A (16 x 8): (r, c), (r + 8, c), (r, c + 4), (r + 8, c + 4);   B (8 x 8): (c, r), (c + 4, r);
 //   C (16 x 8): (r, 2c), (r, 2c + 1), (r + 8, 2c), (r + 8, 2c + 1).
@@ -435,20 +491,17 @@ template <typename T, int NT, int MODE>
 __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
     constexpr int WROWS = 8 * NT, ROWS = WARPS * WROWS;  // rows of a warp; rows of the state
     constexpr int PP = pack_pitch(ROWS);
-    constexpr int SETS = sets_of(MODE), PACK = pack_floats(ROWS, SETS), STAGE = PACK + COEF;
-    constexpr bool VALUES = MODE == MIX || MODE == PLAIN;   // the values themselves move the state on
-    constexpr int TQ = VALUES ? B : 2 * B;               // rows of the pack that meet S_0
-    constexpr bool FRESH = MODE == PLAIN || MODE == CHANNEL;   // (the others sum as they did before)
-    static_assert(MODE != PLAIN || sizeof(T) == 4, "bfloat16: recurrence_stretches.cu");
+    constexpr int PACK = pack_floats(ROWS, 1), STAGE = PACK + COEF;
+    constexpr bool FRESH = MODE == PLAIN;                // (time mixing sums as it did before)
+    static_assert(MODE == MIX || MODE == PLAIN && sizeof(T) == 4, "delta rules: below; plain bfloat16: recurrence_stretches.cu");
     extern __shared__ __align__(16) float smem[];
-    float* red = smem + 2 * STAGE;                       // [WARPS][TQ][RP]
-    float* G_s = red + WARPS * TQ * RP;                  // [B][RP]: what the state's update takes, G[B] U or V
+    float* red = smem + 2 * STAGE;                       // [WARPS][B][RP]
+    float* G_s = red + WARPS * B * RP;                   // [B][RP]: the values
     const int seq = p.prefill_seqs[blockIdx.z], h = blockIdx.y, j0 = blockIdx.x * COLS;
     if (seq < 0) return;
     const int begin = p.cu_q[seq], n = p.cu_q[seq + 1] - begin, slot = p.slots[seq];
     if (n <= 1 || slot < 0) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, c = lane & 3;
-    const int qk_heads = p.heads / p.qk_group, qh = h / p.qk_group;
     float* st = p.state + (long long)slot * p.slot_stride + (long long)h * p.dim * p.vdim;
 
     auto element = [&](int nt, int e, int& i, int& j) {  // row and column of S of register e of tile nt
@@ -468,7 +521,7 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
     const long long first = tile_slot(seq, begin, 0);
     auto issue = [&](int tile) {
         float* stage = smem + (tile & 1) * STAGE;
-        const float* pack = p.pack + ((first + tile) * qk_heads + qh) * (long long)PACK;
+        const float* pack = p.pack + ((first + tile) * p.heads + h) * (long long)PACK;
         const float* coef = p.coef + ((first + tile) * p.heads + h) * (long long)COEF;
 #pragma unroll
         for (int e = 0; e < PACK / 4; e += THREADS)
@@ -478,11 +531,11 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
             if (e + tid < COEF / 4) cp16(stage + PACK + 4 * (e + tid), coef + 4 * (e + tid));
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
-    // Warps 0 and 1 make U (time mixing: hand the values on), warps 2 and 3 O, for columns 8 (warp & 1) .. + 7 each.
+    // Warps 0 and 1 hand the values on, warps 2 and 3 make O, for columns 8 (warp & 1) .. + 7 each.
     // Their values, as B fragments: tokens c, c + 4, c + 8, c + 12 of column r.
     const int nt_uo = warp & 1, col = 8 * nt_uo + r;
     const bool makes_o = warp >= 2;
-    static_assert(WARPS == 4, "two warps make U, two make O");
+    static_assert(WARPS == 4, "two warps hand the values on, two make O");
     const T* v = (const T*)p.v + (long long)(begin + c) * p.v_stride + (long long)h * p.vdim + j0 + col;
     T vnow[4], vnext[4];
     auto fetch_v = [&](int tile, T (&x)[4]) {            // as loaded: converting would wait for the load
@@ -503,99 +556,56 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
         }
         const float* pack = smem + (tile & 1) * STAGE;
         const float* coef = pack + PACK;
-        if (VALUES && !makes_o) {                   // what the update takes is there from the start
+        if (!makes_o) {                                  // what the update takes is there from the start
 #pragma unroll
             for (int k = 0; k < 4; ++k) G_s[(c + 4 * k) * RP + col] = to_float<T>(vnow[k]);
         }
         // product 1: the pack's rows against this warp's rows of S
         {
-            float big[TQ / B][2][4] = {}, small[TQ / B][2][4] = {};
+            float big[2][4] = {}, small[2][4] = {};
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
                 Split b[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) b[e] = split_tf32(S[nt][e]);
-#pragma unroll
-                for (int mt = 0; mt < TQ / B; ++mt) {
-                    const float* row = pack + (mt * B + r) * PP + warp * WROWS + 8 * nt + 2 * c;
-                    const float2 lo = *reinterpret_cast<const float2*>(row), hi = *reinterpret_cast<const float2*>(row + 8 * PP);
-                    const SplitA a = split_a(lo.x, hi.x, lo.y, hi.y);
-                    mma_split<FRESH>(big[mt][0], small[mt][0], a, b[0], b[1]);
-                    mma_split<FRESH>(big[mt][1], small[mt][1], a, b[2], b[3]);
-                }
+                const float* row = pack + r * PP + warp * WROWS + 8 * nt + 2 * c;
+                const float2 lo = *reinterpret_cast<const float2*>(row), hi = *reinterpret_cast<const float2*>(row + 8 * PP);
+                const SplitA a = split_a(lo.x, hi.x, lo.y, hi.y);
+                mma_split<FRESH>(big[0], small[0], a, b[0], b[1]);
+                mma_split<FRESH>(big[1], small[1], a, b[2], b[3]);
             }
 #pragma unroll
-            for (int mt = 0; mt < TQ / B; ++mt)
+            for (int nj = 0; nj < 2; ++nj)
 #pragma unroll
-                for (int nj = 0; nj < 2; ++nj)
-#pragma unroll
-                    for (int half = 0; half < 2; ++half)
-                        *reinterpret_cast<float2*>(red + (warp * TQ + mt * B + r + 8 * half) * RP + 8 * nj + 2 * c) =
-                            make_float2(big[mt][nj][2 * half] + small[mt][nj][2 * half],
-                                        big[mt][nj][2 * half + 1] + small[mt][nj][2 * half + 1]);
+                for (int half = 0; half < 2; ++half)
+                    *reinterpret_cast<float2*>(red + (warp * B + r + 8 * half) * RP + 8 * nj + 2 * c) =
+                        make_float2(big[nj][2 * half] + small[nj][2 * half], big[nj][2 * half + 1] + small[nj][2 * half + 1]);
         }
         __syncthreads();                                 // the partial sums are in
-        {
-            float x[4];                                  // V - c R (time mixing: V) at tokens c + 4 k of column `col`
+        if (makes_o) {
+            float x[4];                                  // V at tokens c + 4 k of column `col`
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                x[k] = to_float<T>(vnow[k]);
-                if (!VALUES) {
-                    float sum = 0.f;
+            for (int k = 0; k < 4; ++k) x[k] = to_float<T>(vnow[k]);
+            float y[4];
+            times_coefficients<FRESH>(y, coef + B * CP, x, r, c);
 #pragma unroll
-                    for (int w = 0; w < WARPS; ++w) sum += red[(w * TQ + B + c + 4 * k) * RP + col];
-                    x[k] = MODE == DELTA ? fmaf(-coef[2 * B * CP + c + 4 * k], sum, x[k]) : x[k] - sum;
+            for (int half = 0; half < 2; ++half) {
+                const int t = r + 8 * half;
+                float q0 = 0.f, q1 = 0.f;
+#pragma unroll
+                for (int w = 0; w < WARPS; ++w) {
+                    const float2 q = *reinterpret_cast<const float2*>(red + (w * B + t) * RP + 8 * nt_uo + 2 * c);
+                    q0 += q.x;
+                    q1 += q.y;
                 }
-            }
-            if (!VALUES || makes_o) {
-                const float* m = coef + (makes_o ? B * CP : 0);
-                float big[4] = {}, small[4] = {};
-                float kept[4];                               // what is not finite stays out of the product, where 0 times it is NaN
-                bool odd = false;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const bool ok = fabsf(x[k]) < SPLITS;
-                    kept[k] = ok ? x[k] : 0.f;
-                    odd |= !ok;
-                }
-#pragma unroll
-                for (int ks = 0; ks < 2; ++ks) {
-                    const float* a = m + r * CP + 8 * ks + c;
-                    const SplitA w = split_a(a[0], a[8 * CP], a[4], a[8 * CP + 4]);
-                    mma_split<FRESH>(big, small, w, split_tf32(kept[2 * ks]), split_tf32(kept[2 * ks + 1]));
-                }
-                float4 late = make_float4(0.f, 0.f, 0.f, 0.f);   // and reaches its own and later tokens by itself
-                if (__any_sync(0xffffffffu, odd)) late = add_odd_tokens(m, x[0], x[1], x[2], x[3], r, c);
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const int t = r + 8 * half;
-                    float y0 = big[2 * half] + small[2 * half] + (half ? late.z : late.x);
-                    float y1 = big[2 * half + 1] + small[2 * half + 1] + (half ? late.w : late.y);
-                    if (!makes_o) {
-                        const float g = MODE == DELTA ? coef[2 * B * CP + B + t] : 1.f;
-                        *reinterpret_cast<float2*>(G_s + t * RP + 8 * nt_uo + 2 * c) = make_float2(g * y0, g * y1);
-                    } else {
-                        float q0 = 0.f, q1 = 0.f;
-#pragma unroll
-                        for (int w = 0; w < WARPS; ++w) {
-                            const float2 q = *reinterpret_cast<const float2*>(red + (w * TQ + t) * RP + 8 * nt_uo + 2 * c);
-                            q0 += q.x;
-                            q1 += q.y;
-                        }
-                        const float ct = MODE == DELTA ? coef[2 * B * CP + t] : 1.f;
-                        y0 = fmaf(ct, q0, y0);
-                        y1 = fmaf(ct, q1, y1);
-                        const int j = j0 + 8 * nt_uo + 2 * c;
-                        if (tile * B + t < n) {
-                            float* dst = p.out + ((long long)(begin + tile * B + t) * p.heads + h) * p.vdim + j;
-                            if (j < p.vdim) dst[0] = y0;
-                            if (j + 1 < p.vdim) dst[1] = y1;
-                        }
-                    }
+                const int j = j0 + 8 * nt_uo + 2 * c;
+                if (tile * B + t < n) {
+                    float* dst = p.out + ((long long)(begin + tile * B + t) * p.heads + h) * p.vdim + j;
+                    if (j < p.vdim) dst[0] = q0 + y[2 * half];
+                    if (j + 1 < p.vdim) dst[1] = q1 + y[2 * half + 1];
                 }
             }
         }
-        if (!VALUES) __syncthreads();                // what the update takes is in
         // product 3, S^T <- decay S^T + G^T K, and the state after the tile
         {
             SplitA a[2];
@@ -604,18 +614,16 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
                 const float* g = G_s + (8 * ks + c) * RP + r;
                 a[ks] = split_a(g[0], g[8], g[4 * RP], g[4 * RP + 8]);
             }
-            const float cB = MODE == DELTA ? coef[2 * B * CP + B - 1] : 1.f;
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
                 float big[4] = {}, small[4] = {};
-                const float* k = pack + (SETS * B + c) * PP + warp * WROWS + 8 * nt + r;
+                const float* k = pack + (B + c) * PP + warp * WROWS + 8 * nt + r;
 #pragma unroll
                 for (int ks = 0; ks < 2; ++ks) {
                     const Split k0 = split_tf32(k[8 * ks * PP]), k1 = split_tf32(k[(8 * ks + 4) * PP]);
                     mma_split<FRESH>(big, small, a[ks], k0, k1);
                 }
-                float2 d = make_float2(cB, cB);
-                if (MODE != DELTA) d = *reinterpret_cast<const float2*>(pack + (1 + SETS) * B * PP + warp * WROWS + 8 * nt + 2 * c);
+                const float2 d = *reinterpret_cast<const float2*>(pack + 2 * B * PP + warp * WROWS + 8 * nt + 2 * c);
                 S[nt][0] = fmaf(d.x, S[nt][0], big[0] + small[0]);
                 S[nt][1] = fmaf(d.y, S[nt][1], big[1] + small[1]);
                 S[nt][2] = fmaf(d.x, S[nt][2], big[2] + small[2]);
@@ -634,16 +642,204 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
         }
 }
 
+// The delta rules' walk.  A CTA owns one request, one head and 16 columns.  Eight warps hold the state's rows.  A tile is a chain: k side
+// against S_0, its sum over the warps, U, the update.  What it does not wait for is beside it: the q side's product runs while two warps
+// without rows make U and two more (P W) (V - R), and those sum up and store the output under the update and the next tile's k side.
+// Packs and coefficients come by bulk copies, two tiles in shared memory.  Every wait for them gives up after about two seconds and says
+// so in an error word; the CTA then goes on with what is there.
+// Bound by the chain.  Three portions of 1,001, 667 and 333 tokens, 8 heads of 128 x 128: 86 us, where four warps that did both sides
+// before U, made U and O and copied the tiles themselves took 100.
+constexpr int DELTA_WARPS = 8, HELPERS = 4, HOLDERS = DELTA_WARPS * 32, DELTA_THREADS = HOLDERS + HELPERS * 32;
+
+template <int NT, int MODE>
+__global__ void __launch_bounds__(DELTA_THREADS) delta_tiles_kernel(ScanArgs p) {
+    constexpr int WROWS = 8 * NT, ROWS = DELTA_WARPS * WROWS;
+    constexpr int PP = pack_pitch(ROWS);
+    constexpr int SETS = sets_of(MODE), PACK = pack_floats(ROWS, SETS), STAGE = PACK + COEF, SUMS = DELTA_WARPS * B * RP;
+    constexpr bool FRESH = MODE == CHANNEL;
+    static_assert(MODE == DELTA || MODE == CHANNEL, "the delta rules");
+    extern __shared__ __align__(16) float smem[];
+    __shared__ __align__(8) uint64_t full[2];
+    float* red_k = smem + 2 * STAGE;                     // [DELTA_WARPS][B][RP], and of the q side
+    float* red_q = red_k + SUMS;
+    float* X_s = red_q + SUMS;                           // [B][RP]: V - R; (P W) of it
+    float* O_s = X_s + B * RP;
+    float* G_s = O_s + B * RP;                           // [2][B][RP]: G[B] U as two TF32 numbers
+    const int seq = p.prefill_seqs[blockIdx.z], h = blockIdx.y, j0 = blockIdx.x * COLS;
+    if (seq < 0) return;
+    const int begin = p.cu_q[seq], n = p.cu_q[seq + 1] - begin, slot = p.slots[seq];
+    if (n <= 1 || slot < 0) return;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, c = lane & 3;
+    const bool holds = warp < DELTA_WARPS;
+    const int qk_heads = p.heads / p.qk_group, qh = h / p.qk_group;
+    float* st = p.state + (long long)slot * p.slot_stride + (long long)h * p.dim * p.vdim;
+    auto element = [&](int nt, int e, int& i, int& j) {  // row and column of S of register e of tile nt
+        i = warp * WROWS + 8 * nt + 2 * c + (e & 1);
+        j = j0 + r + 8 * (e >> 1);
+        return i < p.dim && j < p.vdim;
+    };
+    float S[NT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            int i, j;
+            S[nt][e] = holds && element(nt, e, i, j) ? st[(long long)i * p.vdim + j] : 0.f;
+        }
+    const int tiles = (n + B - 1) / B;
+    const long long first = tile_slot(seq, begin, 0);
+    auto issue = [&](int tile) {                         // one thread
+        float* stage = smem + (tile & 1) * STAGE;
+        mbar_expect_tx(&full[tile & 1], STAGE * 4);
+        bulk_copy(stage, p.pack + ((first + tile) * qk_heads + qh) * (long long)PACK, PACK * 4, &full[tile & 1]);
+        bulk_copy(stage + PACK, p.coef + ((first + tile) * p.heads + h) * (long long)COEF, COEF * 4, &full[tile & 1]);
+    };
+    static_assert(PACK % 4 == 0 && COEF % 4 == 0, "bulk copies go by 16 bytes");
+    // the holders' threads a value of the tile: token tx, column cx; the helpers' two outputs: tokens tx and tx + 8
+    const int tx = (holds ? tid : tid - HOLDERS) / COLS, cx = tid % COLS;
+    static_assert(HOLDERS == B * COLS && HELPERS * 64 == B * COLS && HELPERS == 4, "a thread a value, or two; two helpers for U and two for O");
+    const bool in_columns = j0 + cx < p.vdim;
+    const float* v = (const float*)p.v + (long long)(begin + tx) * p.v_stride + (long long)h * p.vdim + j0 + cx;
+    float* out = p.out + ((long long)(begin + tx) * p.heads + h) * p.vdim + j0 + cx;
+    const long long v_step = B * p.v_stride, token_step = (long long)p.heads * p.vdim;
+    auto fetch_v = [&](int tile) { return holds && in_columns && tile * B + tx < n ? v[tile * v_step] : 0.f; };
+    if (tid == 0) {
+        mbar_init(&full[0], 1);
+        mbar_init(&full[1], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        issue(0);
+    }
+    float vnow = fetch_v(0);
+    bool ok = true;
+    for (int tile = 0; tile < tiles; ++tile) {
+        __syncthreads();                                 // the barriers exist; the other stage, U and the sums have been read
+        if (tid == 0 && tile + 1 < tiles) issue(tile + 1);
+        ok = ok && mbar_wait(&full[tile & 1], tile >> 1 & 1, p.error, holds ? 31 : 32);
+        float vnext = 0.f;
+        if (tile + 1 < tiles) vnext = fetch_v(tile + 1);
+        const float* pack = smem + (tile & 1) * STAGE;
+        const float* coef = pack + PACK;
+        Split s[NT][4];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[nt][e] = split_tf32(S[nt][e]);
+        auto against_state = [&](const float* rows, float* red) {    // 16 rows of the pack against this warp's rows of S
+            float big[2][4], small[2][4];
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                const float* row = rows + r * PP + warp * WROWS + 8 * nt + 2 * c;
+                const float2 lo = *reinterpret_cast<const float2*>(row), hi = *reinterpret_cast<const float2*>(row + 8 * PP);
+                const SplitA a = split_a(lo.x, hi.x, lo.y, hi.y);
+#pragma unroll
+                for (int nj = 0; nj < 2; ++nj) {
+                    if (nt == 0) mma_split_first(big[nj], small[nj], a, s[nt][2 * nj], s[nt][2 * nj + 1]);
+                    else mma_split<FRESH>(big[nj], small[nj], a, s[nt][2 * nj], s[nt][2 * nj + 1]);
+                }
+            }
+#pragma unroll
+            for (int nj = 0; nj < 2; ++nj)
+#pragma unroll
+                for (int half = 0; half < 2; ++half)
+                    *reinterpret_cast<float2*>(red + (warp * B + r + 8 * half) * RP + 8 * nj + 2 * c) =
+                        make_float2(big[nj][2 * half] + small[nj][2 * half], big[nj][2 * half + 1] + small[nj][2 * half + 1]);
+        };
+        if (holds) against_state(pack + B * PP, red_k);
+        __syncthreads();                                 // the k side's partial sums are in
+        if (holds) {
+            float sum = 0.f;
+#pragma unroll
+            for (int w = 0; w < DELTA_WARPS; ++w) sum += red_k[(w * B + tx) * RP + cx];
+            X_s[tx * RP + cx] = MODE == DELTA ? fmaf(-coef[2 * B * CP + tx], sum, vnow) : vnow - sum;
+        }
+        __syncthreads();                                 // V - R is in
+        if (holds) {
+            against_state(pack, red_q);
+        } else {
+            const bool makes_u = warp < DELTA_WARPS + 2;
+            const int col = 8 * (warp & 1);
+            float x[4], y[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) x[k] = X_s[(c + 4 * k) * RP + col + r];
+            times_coefficients<FRESH>(y, coef + (makes_u ? 0 : B * CP), x, r, c);
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int t = r + 8 * half;
+                if (makes_u) {
+                    const float g = MODE == DELTA ? coef[2 * B * CP + B + t] : 1.f;
+                    const Split a = split_tf32(g * y[2 * half]), b = split_tf32(g * y[2 * half + 1]);
+                    *reinterpret_cast<uint2*>(G_s + t * RP + col + 2 * c) = make_uint2(a.hi, b.hi);
+                    *reinterpret_cast<uint2*>(G_s + (B + t) * RP + col + 2 * c) = make_uint2(a.lo, b.lo);
+                } else {
+                    *reinterpret_cast<float2*>(O_s + t * RP + col + 2 * c) = make_float2(y[2 * half], y[2 * half + 1]);
+                }
+            }
+        }
+        __syncthreads();                                 // what the update takes is in, and all of the output
+        if (holds) {                                     // S^T <- decay S^T + G^T K: the state after the tile
+            SplitA a[2];
+#pragma unroll
+            for (int ks = 0; ks < 2; ++ks) {
+                const uint32_t* g = reinterpret_cast<const uint32_t*>(G_s) + (8 * ks + c) * RP + r;
+                a[ks] = SplitA{{g[0], g[8], g[4 * RP], g[4 * RP + 8]}, {g[B * RP], g[B * RP + 8], g[(B + 4) * RP], g[(B + 4) * RP + 8]}};
+            }
+            const float cB = MODE == DELTA ? coef[2 * B * CP + B - 1] : 1.f;
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                float big[4], small[4];
+                const float* k = pack + (SETS * B + c) * PP + warp * WROWS + 8 * nt + r;
+#pragma unroll
+                for (int ks = 0; ks < 2; ++ks) {
+                    const Split k0 = split_tf32(k[8 * ks * PP]), k1 = split_tf32(k[(8 * ks + 4) * PP]);
+                    if (ks == 0) mma_split_first(big, small, a[0], k0, k1);
+                    else mma_split<FRESH>(big, small, a[1], k0, k1);
+                }
+                float2 d = make_float2(cB, cB);
+                if (MODE != DELTA) d = *reinterpret_cast<const float2*>(pack + (1 + SETS) * B * PP + warp * WROWS + 8 * nt + 2 * c);
+                S[nt][0] = fmaf(d.x, S[nt][0], big[0] + small[0]);
+                S[nt][1] = fmaf(d.y, S[nt][1], big[1] + small[1]);
+                S[nt][2] = fmaf(d.x, S[nt][2], big[2] + small[2]);
+                S[nt][3] = fmaf(d.y, S[nt][3], big[3] + small[3]);
+            }
+        } else {
+#pragma unroll
+            for (int t = tx; t < B; t += B / 2) {
+                float sum = 0.f;
+#pragma unroll
+                for (int w = 0; w < DELTA_WARPS; ++w) sum += red_q[(w * B + t) * RP + cx];
+                const float y = O_s[t * RP + cx];
+                if (in_columns && tile * B + t < n) out[(tile * B + t - tx) * token_step] = MODE == DELTA ? fmaf(coef[2 * B * CP + t], sum, y) : y + sum;
+            }
+        }
+        vnow = vnext;
+    }
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            int i, j;
+            if (holds && element(nt, e, i, j)) st[(long long)i * p.vdim + j] = S[nt][e];
+        }
+}
+
 template <typename T, int MODE>
 int launch_scan(const ScanArgs& p, int portions, cudaStream_t stream) {
     const dim3 grid((p.vdim + COLS - 1) / COLS, p.heads, portions);
 #define TS_TILES(NT)                                                                                                 \
     do {                                                                                                             \
-        constexpr int TQ = MODE == MIX || MODE == PLAIN ? B : 2 * B;                                                 \
-        const size_t smem = sizeof(float) * (2 * (pack_floats(WARPS * 8 * NT, sets_of(MODE)) + COEF) + (WARPS * TQ + B) * RP); \
-        auto kernel = recurrence_tiles_kernel<T, NT, MODE>;                                                          \
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                        \
-        kernel<<<grid, THREADS, smem, stream>>>(p);                                                                  \
+        constexpr int ROWS = WARPS * 8 * NT;                                                                         \
+        if constexpr (MODE == DELTA || MODE == CHANNEL) {                                                            \
+            static_assert(sizeof(T) == 4, "the delta rules' values are float32");                                    \
+            const size_t smem = sizeof(float) * (2 * (pack_floats(ROWS, sets_of(MODE)) + COEF) + (2 * DELTA_WARPS + 4) * B * RP); \
+            auto kernel = delta_tiles_kernel<NT * WARPS / DELTA_WARPS, MODE>;                                        \
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                    \
+            kernel<<<grid, DELTA_THREADS, smem, stream>>>(p);                                                        \
+        } else {                                                                                                     \
+            const size_t smem = sizeof(float) * (2 * (pack_floats(ROWS, 1) + COEF) + (WARPS + 1) * B * RP);          \
+            auto kernel = recurrence_tiles_kernel<T, NT, MODE>;                                                      \
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                    \
+            kernel<<<grid, THREADS, smem, stream>>>(p);                                                              \
+        }                                                                                                            \
     } while (0)
     const int rows = padded_rows(p.dim);
     if (rows == 64) TS_TILES(2);
@@ -672,7 +868,8 @@ TS_API int ts_delta_tiles(const float* q, const float* k, long long qk_stride, c
                           const float* a_log, const float* v, long long v_stride, const int* cu_q, const int* slots,
                           const int* prefill_seqs, int portions, int max_q_len, float* state, long long slot_stride,
                           float* pack, float* coef, float* out, int heads, int kv_heads, int dim, int vdim,
-                          float unit_eps, float q_scale, cudaStream_t stream) {
+                          float unit_eps, float q_scale, int* error, cudaStream_t stream) {
+    TS_REQUIRE(error != nullptr, "delta_tiles: an error word is needed");
     TS_REQUIRE(heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && dim > 0 && dim <= 256 && vdim > 0,
                "delta_tiles: %d heads over %d q/k heads of %d channels", heads, kv_heads, dim);
     TS_REQUIRE(slot_stride >= (long long)heads * dim * vdim, "delta_tiles: a state slot is too small");
@@ -683,7 +880,7 @@ TS_API int ts_delta_tiles(const float* q, const float* k, long long qk_stride, c
     const size_t smem = sizeof(float) * (2 * B * (a.rows + 1) + 2 * B * (B + 1));
     delta_tile_prepare_kernel<<<dim3((max_q_len + B - 1) / B, kv_heads, portions), 128, smem, stream>>>(a);
     TS_LAUNCH_CHECK("delta_tiles (prepare)");
-    ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, heads / kv_heads, dim, vdim};
+    ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, heads / kv_heads, dim, vdim, error};
     return launch_scan<float, DELTA>(s, portions, stream);
 }
 
@@ -700,7 +897,7 @@ TS_API int ts_mix_tiles(const void* r, const void* k, long long rk_stride, const
     PrepareArgs a{r, k, rk_stride, z, w0, u, cu_q, prefill_seqs, pack, coef, heads, heads, dim, padded_rows(dim), 0.f, 1.f};
     const size_t smem = sizeof(float) * (3 * B * (a.rows + 1));
     const dim3 grid((max_q_len + B - 1) / B, heads, portions);
-    ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, dim};
+    ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, dim, nullptr};
     if (dtype == TS_F32) {
         cudaFuncSetAttribute(mix_tile_prepare_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         mix_tile_prepare_kernel<float><<<grid, 128, smem, stream>>>(a);
@@ -745,7 +942,7 @@ TS_API int ts_plain_tiles(const void* q, const void* k, const void* v, long long
     const int rows = padded_rows(dim);
     const size_t smem = rows == 64 ? PlainTile<64>::BYTES : rows == 128 ? PlainTile<128>::BYTES : PlainTile<256>::BYTES;   // 29 KB at 128 channels
     const dim3 grid((max_q_len + B - 1) / B, heads, portions);
-    const ScanArgs s{a.pack, a.coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, vdim};
+    const ScanArgs s{a.pack, a.coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, vdim, nullptr};
     auto kernel = rows == 64 ? plain_tile_prepare_kernel<64> : rows == 128 ? plain_tile_prepare_kernel<128> : plain_tile_prepare_kernel<256>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     kernel<<<grid, 128, smem, stream>>>(a);
@@ -759,7 +956,8 @@ TS_API int ts_channel_tiles(const float* q, const float* k, long long qk_stride,
                             int b_dtype, const float* dt_bias, const float* a_log, const float* v, long long v_stride,
                             const int* cu_q, const int* slots, const int* prefill_seqs, int portions, int max_q_len, float* state,
                             long long slot_stride, float* pack, float* coef, float* out, int heads, int kv_heads, int dim,
-                            int vdim, float unit_eps, float q_scale, cudaStream_t stream) {
+                            int vdim, float unit_eps, float q_scale, int* error, cudaStream_t stream) {
+    TS_REQUIRE(error != nullptr, "channel_tiles: an error word is needed");
     TS_REQUIRE(heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && dim > 0 && dim <= 256 && vdim > 0,
                "channel_tiles: %d heads over %d q/k heads of %d channels", heads, kv_heads, dim);
     TS_REQUIRE(slot_stride >= (long long)heads * dim * vdim, "channel_tiles: a state slot is too small");
@@ -768,7 +966,7 @@ TS_API int ts_channel_tiles(const float* q, const float* k, long long qk_stride,
     const ChannelArgs a{q, k, qk_stride, z, b, b_stride, dt_bias, a_log, cu_q, prefill_seqs, pack, coef, heads, kv_heads, dim,
                         unit_eps, q_scale};
     const int rows = padded_rows(dim);
-    const size_t smem = sizeof(float) * (3 * B * (rows + 1) + 2 * B * (B + 1)) + 2 * B * (rows + 1);
+    const size_t smem = sizeof(float) * (3 * B * (rows + 2) + 2 * B * (B + 1)) + 2 * B * (rows + 2);
     const dim3 grid((max_q_len + B - 1) / B, heads, portions);
     TS_REQUIRE(b_dtype == TS_F32 || b_dtype == TS_BF16, "channel_tiles: unknown dtype code %d", b_dtype);
 #define TS_CHANNEL_PREPARE(T)                                                                                                  \
@@ -782,6 +980,6 @@ TS_API int ts_channel_tiles(const float* q, const float* k, long long qk_stride,
     else TS_CHANNEL_PREPARE(__nv_bfloat16);
 #undef TS_CHANNEL_PREPARE
     TS_LAUNCH_CHECK("channel_tiles (prepare)");
-    const ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, vdim};
+    const ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, vdim, error};
     return launch_scan<float, CHANNEL>(s, portions, stream);
 }

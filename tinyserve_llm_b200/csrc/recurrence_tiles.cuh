@@ -1,7 +1,7 @@
 // What the recurrences over prompt portions sixteen tokens at a time share (recurrence_tiles.cu, recurrence_stretches.cu).
 #pragma once
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 // The plain recurrence's inputs.
 struct PlainArgs {
@@ -158,6 +158,13 @@ __device__ __forceinline__ float plain_sides(const PlainTile<ROWS>& x, int i, St
     return (float)left;
 }
 
+// `bytes` (a multiple of 16) from memory to shared memory by the copy engine, counted on `bar`: the threads' own 16-byte copies of a tile
+// of 29 KB held up the shared-memory pipe for 400 ns of 1,570.
+__device__ __forceinline__ void bulk_copy(void* smem, const void* gmem, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_u32(smem)), "l"(gmem), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+
 __device__ __forceinline__ void cp16(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
 }
@@ -185,6 +192,12 @@ __device__ __forceinline__ void mma_tf32_fresh(float (&d)[4], const uint32_t (&a
     asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
                  : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// The first of several products of split factors that are added up: both sums begin with it.
+__device__ __forceinline__ void mma_split_first(float (&big)[4], float (&small)[4], const SplitA& a, Split b0, Split b1) {
+    mma_tf32_fresh(big, a.hi, b0.hi, b1.hi);
+    mma_tf32_fresh(small, a.hi, b0.lo, b1.lo);
+    mma_tf32(small, a.lo, b0.hi, b1.hi);
 }
 // The two large and the small parts of a product of split factors, each in an accumulator of its own (no long chain).  FRESH: every
 // large part begins at zero and is added by an ordinary rounded addition, where the tensor cores cut what an accumulator cannot hold.

@@ -96,11 +96,11 @@ _SIGNATURES = {
     "ts_time_mix_prepare": ("int", "pplppppp" "iiipippiplipip"),
     "ts_recurrence_tiles_pack_floats": ("long long", "iiiii"),
     "ts_recurrence_tiles_coef_floats": ("long long", "iii"),
-    "ts_delta_tiles": ("int", "pplppppl" "pppii" "plppp" "iiiiffp"),
+    "ts_delta_tiles": ("int", "pplppppl" "pppii" "plppp" "iiiiffpp"),
     "ts_mix_tiles": ("int", "pplppppl" "pppii" "plppp" "iiip"),
     "ts_plain_tiles": ("int", "ppplll" "plpp" "fffpip" "pppiiii" "plpp" "iiiip"),
     "ts_plain_tiles_floats": ("long long", "iiiiii"),
-    "ts_channel_tiles": ("int", "pplpplipp" "pl" "pppii" "plppp" "iiiiffp"),
+    "ts_channel_tiles": ("int", "pplpplipp" "pl" "pppii" "plppp" "iiiiffpp"),
     "ts_delta_prepare": ("int", "pplppppl" "ppiiiiff" "ppip"),
     "ts_mlstm_prepare": ("int", "ppllpplppffppiplpppiiiip"),
     "ts_row_scaled_activation": ("int", "ppppiiiip"),
@@ -130,6 +130,8 @@ _WAIT_CODES: dict[int, tuple[str, str]] = {
     24: ("sgemm_tcgen05", "MMA issuer waiting for a drained accumulator"),
     25: ("sgemm_tcgen05", "adders waiting for a block's sums"),
     26: ("sgemm_tcgen05", "split warps waiting for free operand tiles"),
+    31: ("delta_tiles", "warps of the state waiting for a tile"),
+    32: ("delta_tiles", "warps of U and the output waiting for a tile"),
 }
 
 
@@ -1178,7 +1180,8 @@ class Ops:
         out = torch.empty((T, heads * vdim), dtype=torch.float32, device=q.device)
         self._call("ts_delta_tiles", _ptr(q), _ptr(k), q.stride(0), _ptr(gates), _ptr(dt_bias), _ptr(a_log), _ptr(v), v.stride(0),
                    _ptr(ctx.cu_q), _ptr(binding.state_slots), _ptr(ctx.prefill_seqs), ctx.prefill_seqs.shape[0], ctx.max_q_len,
-                   state.data_ptr(), stride, pack, coef, _ptr(out), heads, kv_heads, dim, vdim, unit_eps, q_scale, _stream())
+                   state.data_ptr(), stride, pack, coef, _ptr(out), heads, kv_heads, dim, vdim, unit_eps, q_scale,
+                   self.error_word().data_ptr(), _stream())
         self.launches += 1                                   # what the columns of a tile share, then the scan
         return out
 
@@ -1205,7 +1208,7 @@ class Ops:
         self._call("ts_channel_tiles", _ptr(q), _ptr(k), q.stride(0), _ptr(z), _ptr(b), b.stride(0), _DTYPE_CODE[b.dtype], _ptr(dt_bias),
                    _ptr(a_log), _ptr(v), v.stride(0), _ptr(ctx.cu_q), _ptr(binding.state_slots), _ptr(ctx.prefill_seqs),
                    ctx.prefill_seqs.shape[0], ctx.max_q_len, state.data_ptr(), stride, pack, coef, _ptr(out), heads,
-                   kv_heads, dim, vdim, unit_eps, q_scale, _stream())
+                   kv_heads, dim, vdim, unit_eps, q_scale, self.error_word().data_ptr(), _stream())
         self.launches += 1                                   # what the columns of a tile share, then the scan
         return out
 
