@@ -51,6 +51,11 @@ struct Shape {
     static constexpr int P_COL = KEYS + HD, ROT_COL = P_COL + (PAIR ? KEYS : KEYS / 2);    // P's second piece after the first; rotated queries
     static constexpr int TMEM_USED = ROT_COL + ROT, TMEM_COLS = TMEM_USED <= 256 ? 256 : 512;
     static constexpr int CTAS = TMEM_COLS == 256 ? 2 : 1;                // on an SM
+    // ROT: rotated queries on their way to tensor memory, in the second stage before its first load where they fit, else behind both
+    static constexpr int SCRATCH_PITCH = 65, SCRATCH_BYTES = QROWS * SCRATCH_PITCH * 4;
+    static constexpr bool IN_STAGE = SCRATCH_BYTES <= STAGE_BYTES;
+    static constexpr int SCRATCH_AT = IN_STAGE ? STAGE_BYTES : 2 * STAGE_BYTES;
+    static constexpr int SMEM = Q_BYTES + 2 * STAGE_BYTES + (ROT && !IN_STAGE ? SCRATCH_BYTES : 0) + 1024;
     static_assert(HD == 64 || HD == 128, "head sizes 64 and 128");
     static_assert(ROT == 0 || ROT == 64, "one shared sub-tile or none");
     static_assert(TMEM_USED <= TMEM_COLS, "S, O, P and the rotated queries must fit the allocation");
@@ -335,6 +340,7 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT, FORM == BOUNDED && RO
         for (int j = kv_begin; j < num_kv; ++j) {
             const int it = j - kv_begin, s = it & 1;
             if (!mbar_wait(&stage_free[s], ((it >> 1) & 1) ^ 1, p.error, 11)) { failed = 1; break; }
+            if (ROT && S_::IN_STAGE && it == 1 && !mbar_wait(&rot_ready, 0, p.error, 19)) { failed = 1; break; }
             unsigned char* k_tile = kv_tiles + s * STAGE_BYTES;
             unsigned char* v_tile = k_tile + K_BYTES;
             mbar_expect_tx(&kv_full[s], STAGE_BYTES);
@@ -434,36 +440,29 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT, FORM == BOUNDED && RO
         const float slope2 = SIG && p.slopes ? p.slopes[head] * LOG2E : 0.f;
         const float bias2 = (SIG && p.head_bias ? p.head_bias[head] * LOG2E : 0.f) - slope2 * (float)pos;
         bool ok = true;
-        if constexpr (ROT != 0) {                    // this thread's half of the row's rotated channels, 32 of them
-            float x[32];
-            const long long t = q_begin + row0 + r;
-            const __nv_bfloat16* qr = p.q + t * p.q_stride + (long long)head * p.q_head_cols + HD;
-            const float2* turn = p.turn + t * 32;
-            if (p.rot == 64 && r < rows) {
-#pragma unroll
-                for (int c = 0; c < 32; c += 8) {
-                    const uint4 u4 = *reinterpret_cast<const uint4*>(qr + c), v4 = *reinterpret_cast<const uint4*>(qr + 32 + c);
-                    const __nv_bfloat16 *u = reinterpret_cast<const __nv_bfloat16*>(&u4), *v = reinterpret_cast<const __nv_bfloat16*>(&v4);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const float2 cs = turn[c + e];
-                        const float a = __bfloat162float(u[e]), b = __bfloat162float(v[e]);
-                        x[c + e] = half == 0 ? a * cs.x - b * cs.y : b * cs.x + a * cs.y;
-                    }
+        if constexpr (ROT != 0) {
+            // The queries' shared part: a warp rotates 16 rows, a lane a pair of channels (so that loads are whole lines: a thread a row
+            // took half of the kernel's time), and a thread then takes its half of its own row from shared memory.
+            float* scratch = reinterpret_cast<float*>(kv_tiles + S_::SCRATCH_AT);
+            const int pairs = p.rot / 2, first = quadrant * 32 + half * 16;
+            const long long t0 = q_begin + row0;
+            const __nv_bfloat16* qr = p.q + t0 * p.q_stride + (long long)head * p.q_head_cols + HD;
+#pragma unroll 8
+            for (int k = 0; k < 16; ++k) {
+                const int row = first + k;
+                float2 cs = make_float2(0.f, 0.f);
+                float a = 0.f, b = 0.f;
+                if (lane < pairs && row < rows) {
+                    cs = p.turn[(t0 + row) * 32 + lane];
+                    a = __bfloat162float(qr[row * p.q_stride + lane]);
+                    b = __bfloat162float(qr[row * p.q_stride + lane + pairs]);
                 }
-            } else {
-                const int pairs = p.rot / 2;
-#pragma unroll
-                for (int c = 0; c < 32; ++c) {
-                    const int d = half * 32 + c, i = d < pairs ? d : d - pairs;
-                    x[c] = 0.f;
-                    if (r < rows && d < p.rot) {
-                        const float2 cs = turn[i];
-                        const float a = __bfloat162float(qr[i]), b = __bfloat162float(qr[i + pairs]);
-                        x[c] = d < pairs ? a * cs.x - b * cs.y : b * cs.x + a * cs.y;
-                    }
-                }
+                float* to = scratch + row * S_::SCRATCH_PITCH;
+                to[lane < pairs ? lane : 2 * lane] = a * cs.x - b * cs.y;                      // lanes past the pairs write zeros behind them
+                to[lane < pairs ? lane + pairs : 2 * lane + 1] = b * cs.x + a * cs.y;
             }
+            pair_barrier(quadrant);
+            const float* x = scratch + r * S_::SCRATCH_PITCH + half * 32;
             uint32_t hi[16], lo[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) pack_pair(x[2 * i], x[2 * i + 1], hi[i], lo[i]);
@@ -471,6 +470,7 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT, FORM == BOUNDED && RO
             tmem_st16(lane_addr + S_::ROT_COL + 32 + half * 16, lo);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");              // the scratch may be a stage of keys and values next
             mbar_arrive(&rot_ready);
         }
         for (int j = kv_begin; j < num_kv; ++j) {
@@ -847,7 +847,7 @@ int run_prefill(const void* q, long long q_cols, long long q_stride, void* out, 
 #define TS_FLASH_LAUNCH(HD, FORM, ROT)                                                                                    \
     do {                                                                                                                  \
         using Sizes = Shape<HD, ROT, (FORM) == BOUNDED && (ROT) != 0>;                                                    \
-        const size_t smem = (size_t)Sizes::Q_BYTES + 2 * Sizes::STAGE_BYTES + 1024;                                       \
+        const size_t smem = Sizes::SMEM;                                                                                  \
         auto kernel = prefill_attention_tcgen05_kernel<HD, FORM, ROT>;                                                    \
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                             \
         TS_CHAINED_CHECK("attention_tcgen05", launch_chained(kernel, grid, dim3(THREADS), smem, stream, map_q, map_k, map_v, \

@@ -124,6 +124,7 @@ _WAIT_CODES: dict[int, tuple[str, str]] = {
     16: ("attention_tcgen05", "epilogue waiting for the last product"),
     17: ("attention_tcgen05", "softmax waiting for the previous product before rescaling"),
     18: ("attention_tcgen05", "MMA issuer waiting for the rotated queries"),
+    19: ("attention_tcgen05", "loader waiting for the rotated queries' scratch"),
     21: ("sgemm_tcgen05", "TMA producer waiting for a free ring slot"),
     22: ("sgemm_tcgen05", "split warps waiting for operands"),
     23: ("sgemm_tcgen05", "MMA issuer waiting for split operands"),

@@ -129,7 +129,9 @@ class LatentAttention(Mixer):
     def _portions(self, q: torch.Tensor, ctx) -> list[int] | None:
         """How many keys each of the step's prompt portions sees, if they are to attend over keys and values worked out for the step."""
         spec, host, ops = self.spec, getattr(ctx, "host", None), self.rt.ops
-        if (self.uk_uv is None or (spec.window and not spec.rot_dim) or getattr(ctx, "replayed", True) or host is None or ctx.max_q_len <= 1
+        # (small steps leave first: they are bound by the host)
+        if (host is None or host.cu_q[-1] < MATERIALIZE_MIN_TOKENS or getattr(ctx, "replayed", True) or ctx.max_q_len <= 1
+                or self.uk_uv is None or (spec.window and not spec.rot_dim)
                 or not ops.dense_prompt_attention_supported(q, spec.num_heads, spec.num_heads, spec.head_dim)):
             return None
         # (windows come in the kernel's form with a rotated part, whose queries and probabilities have the folded form's precision)
