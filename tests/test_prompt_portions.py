@@ -518,3 +518,70 @@ def test_a_latent_that_is_not_finite_reaches_the_queries_that_see_it_only():
     sees = torch.zeros(530, dtype=torch.bool)
     sees[201:271] = True
     assert torch.isnan(got[sees]).all() and torch.equal(got[~sees], clean[~sees].to(got.dtype))
+
+
+def _both_forms(heads, dim, rot, rank, window, lens, cached, deviation):
+    """Relative errors against 64 bits of windowed latent attention alone, its scores of this deviation: (unfolded, folded), each (worst row, all)."""
+    from tinyserve_llm_b200.config.spec import InlineRotarySpec, LatentAttentionSpec
+    from tinyserve_llm_b200.parts.base import Runtime, part_class
+    g, page, T = torch.Generator().manual_seed(rank + dim), 64, sum(lens)
+    normal = lambda *shape, std=1.0: (torch.randn(shape, generator=g) * std).to(torch.bfloat16)
+    spec = LatentAttentionSpec(hidden_size=64, num_heads=heads, head_dim=dim, rot_dim=rot, value_dim=dim, q_rank=0, kv_rank=rank,
+                               scale=deviation / (dim + rot) ** 0.5, window=window, norm_eps=1e-5, position=InlineRotarySpec(dims=rot))
+    w = {"q": normal(heads * (dim + rot), 64), "dkv": normal(rank + rot, 64), "uk": normal(heads * dim, rank, std=rank ** -0.5),
+         "uv": normal(heads * dim, rank, std=rank ** -0.5), "o": normal(64, heads * dim), "dkv.norm": torch.ones(rank)}
+    part = part_class("mixer", spec)(spec, w, Runtime(dtype=torch.bfloat16, device=torch.device("cuda", 0), ops=get_ops()))
+    ends = [n + c for n, c in zip(lens, cached)]
+    counts = [-(-e // page) for e in ends]
+    pool, q = normal(sum(counts), 1, 1, page, rank + rot), normal(T, heads * (dim + rot))
+    tables = [list(range(sum(counts[:s]), sum(counts[:s + 1]))) + [-1] * (max(counts) - n) for s, n in enumerate(counts)]
+    binding = EntryBinding(pool.cuda(), None, page * (rank + rot), 0, page, pool.shape[0], i32(tables), max(counts))
+    freq = 10000.0 ** (-2.0 * torch.arange(rot // 2, dtype=torch.float64) / rot)
+    want, at = [], 0
+    for s, (n, c) in enumerate(zip(lens, cached)):
+        full = pool.view(-1, page, rank + rot)[tables[s][:counts[s]]].reshape(-1, rank + rot)[:c + n].double()
+        positions = torch.arange(c, c + n)
+        turned = q[at:at + n].double().view(n, heads, dim + rot)
+        a, (u, v) = positions.double()[:, None, None] * freq, turned[..., dim:].chunk(2, dim=-1)
+        turned = torch.cat([turned[..., :dim], u * a.cos() - v * a.sin(), v * a.cos() + u * a.sin()], dim=-1)
+        k = torch.cat([(full[:, :rank] @ w["uk"].double().t()).view(-1, heads, dim), full[:, None, rank:].expand(-1, heads, -1)], dim=-1)
+        j = torch.arange(c + n)[None]
+        scores = torch.einsum("ihd,jhd->hij", turned, k) * spec.scale
+        scores = scores.masked_fill((j > positions[:, None]) | (j <= positions[:, None] - window), -float("inf"))
+        want.append(torch.einsum("hij,jhd->ihd", torch.softmax(scores, -1), (full[:, :rank] @ w["uv"].double().t()).view(-1, heads, dim)))
+        at += n
+    want, results = torch.cat(want), []
+    for replayed in (False, True):                       # a step that is replayed stays on the folded form
+        ctx = make_ctx(lens, ends)
+        ctx.replayed, ctx.prefill_seqs = replayed, i32([s for s, n in enumerate(lens) if n > 1])
+        before = get_ops().calls.get("ts_prefill_attention_tcgen05_dense", 0)
+        got = part.attend(q.cuda(), ctx, binding).double().cpu().view(T, heads, dim)
+        assert get_ops().calls.get("ts_prefill_attention_tcgen05_dense", 0) == before + (not replayed)
+        off = (got - want).norm(dim=-1) / want.norm(dim=-1)
+        results.append((float(off.max()), float((got - want).norm() / want.norm())))
+    return results
+
+
+@pytest.mark.parametrize("deviation", [1.0, 3.0, 6.0])
+@pytest.mark.parametrize("heads,dim,rot,rank,window,lens,cached", [(4, 128, 64, 512, 256, [512], [0]), (3, 64, 32, 256, 100, [200, 150], [333, 0])])
+def test_keys_worked_out_for_a_step_are_no_further_from_64_bits_than_the_latents(heads, dim, rot, rank, window, lens, cached, deviation):
+    """
+    Flat and peaked scores.  Both forms round the outputs once to bfloat16 and, before that, the values or their weighted sum; with nothing
+    else rounded to less than two such pieces they differ by the luck of those roundings, hundredths over 10^5 of them.
+    """
+    (worst, off), (folded_worst, folded) = _both_forms(heads, dim, rot, rank, window, lens, cached, deviation)
+    assert off <= 1.02 * folded and worst <= 1.5 * folded_worst, (off, folded, worst, folded_worst)
+
+
+@pytest.mark.parametrize("rows,rank,cols,low", [(1, 40, 8, 8), (129, 72, 256, 128), (300, 512, 1032, 0), (2048, 512, 4096, 2048), (2900, 128, 10240, 5120)])
+def test_products_in_pieces(rows, rank, cols, low):
+    """Every tile shape of the product (one tile of rows, narrow, wide, pairs of CTAs), pieces of all, half and none of its columns."""
+    g = torch.Generator().manual_seed(rows)
+    x, w = torch.randn(rows, rank, generator=g).to(torch.bfloat16), (torch.randn(cols, rank, generator=g) * rank ** -0.5).to(torch.bfloat16)
+    y = get_ops().gemm_tcgen05_pieces(x.cuda(), w.cuda(), low)
+    want = (x.double().cuda() @ w.double().cuda().t())
+    # float32 sums of `rank` terms of about rank^-1/2: within sqrt(rank) 2^-24 of one; the sum of two pieces within 2^-17 of itself, a single one 2^-9
+    sums = rank ** 0.5 * 2.0 ** -22
+    assert bool(((y[:, :cols].double() - want).abs() <= want.abs() * 2.0 ** -8 + sums).all())
+    both = y[:, :low].double() + y[:, cols:].double()
+    assert bool(((both - want[:, :low]).abs() <= want[:, :low].abs() * 2.0 ** -16 + sums).all())

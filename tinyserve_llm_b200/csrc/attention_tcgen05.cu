@@ -26,9 +26,11 @@
 // A form for keys of which every head has its own part and all heads share a second, rotated one (ROT): the keys have a further
 // sub-tile of 64 channels, read from a matrix of its own once for all heads; the queries' part is rotated by the softmax threads, a
 // row each, into tensor memory as two bfloat16 pieces, x = hi + lo, both A operands against the shared sub-tile.  Behind a window it
-// also takes the probabilities as two pieces (PAIR): it stands in for a kernel on the latents themselves (attention_latent_tokens.cu)
-// that has both from float32, and is with them no further from 64 bits than that one (relative error of a layer of 2,048 tokens, 16
-// heads: 4.10e-3 against 4.16e-3; without the second pieces 4.41e-3).  With heads of 128 channels one CTA holds an SM.
+// also takes the heads' own keys and the probabilities as two pieces (PAIR): it stands in for kernels on the latents themselves
+// (attention_latent_mma.cu, attention_latent_tokens.cu), which round neither, and is with them no further from 64 bits than those
+// (relative error of the attention alone, 3 heads of 64 + 32 channels, latent of 256, window 100, scores of deviation 1 / 3 / 6: there 2.45 / 2.81 /
+// 3.23e-3, here 2.32 / 2.34 / 2.32e-3, with keys of one piece 2.62 / 3.35 / 4.02e-3; 2,048 tokens, 16 heads of 128, window 1,024: a layer takes 168 us, 141 with one).
+// With heads of 128 channels one CTA holds an SM.
 //
 // What a tile costs beside its arithmetic (4.5 instructions an element of the scores) is what bounds it: two CTAs an SM issue half of the
 // time, and taking out exponentials, sums or the second product changes little.  So: waits read the clock only where a first look was
@@ -49,19 +51,21 @@ constexpr int QROWS = 128;                   // queries per CTA
 // ROT (0 or 64): channels of the shared part of queries and keys, a sub-tile of the keys behind the others.  PAIR: P in two pieces.
 template <int HD, int ROT = 0, bool PAIR = false>
 struct Shape {
-    static constexpr int KEYS = (HD == 64) == (ROT == 0) ? 128 : 64;     // keys per tile: two CTAs must fit an SM (HD 128 with ROT: one)
-    static constexpr int SUBS = HD / 64, K_SUBS = (HD + ROT) / 64;       // sub-tiles of 64 dims: of queries and values, of keys
+    static constexpr int KEYS = !PAIR && (HD == 64) == (ROT == 0) ? 128 : 64;     // keys per tile: two CTAs must fit an SM (HD 128 with ROT: one)
+    // sub-tiles of 64 dims: of queries and values, of keys: the heads' own, the shared one, the own ones' second pieces
+    static constexpr int SUBS = HD / 64, K_SUBS = (HD + ROT + (PAIR ? HD : 0)) / 64;
     static constexpr int SUB_Q = QROWS * 128, SUB_KV = KEYS * 128; // bytes of a sub-tile
     static constexpr int Q_BYTES = SUBS * SUB_Q, K_BYTES = K_SUBS * SUB_KV, STAGE_BYTES = K_BYTES + SUBS * SUB_KV;
     static constexpr int O_COL = KEYS;       // S at columns 0..KEYS-1, O after it, P (bfloat16 pairs) after O
     static constexpr int P_COL = KEYS + HD, ROT_COL = P_COL + (PAIR ? KEYS : KEYS / 2);    // P's second piece after the first; rotated queries
     static constexpr int TMEM_USED = ROT_COL + ROT, TMEM_COLS = TMEM_USED <= 256 ? 256 : 512;
     static constexpr int CTAS = TMEM_COLS == 256 ? 2 : 1;                // on an SM
-    // ROT: rotated queries on their way to tensor memory, in the second stage before its first load where they fit, else behind both
+    // ROT: rotated queries on their way to tensor memory, from the second stage on before its first load where they (all but) fit, else behind both
     static constexpr int SCRATCH_PITCH = 65, SCRATCH_BYTES = QROWS * SCRATCH_PITCH * 4;
-    static constexpr bool IN_STAGE = SCRATCH_BYTES <= STAGE_BYTES;
+    static constexpr bool IN_STAGE = SCRATCH_BYTES <= STAGE_BYTES + 1024;
     static constexpr int SCRATCH_AT = IN_STAGE ? STAGE_BYTES : 2 * STAGE_BYTES;
-    static constexpr int SMEM = Q_BYTES + 2 * STAGE_BYTES + (ROT && !IN_STAGE ? SCRATCH_BYTES : 0) + 1024;
+    static constexpr int KV_BYTES = ROT && SCRATCH_AT + SCRATCH_BYTES > 2 * STAGE_BYTES ? SCRATCH_AT + SCRATCH_BYTES : 2 * STAGE_BYTES;
+    static constexpr int SMEM = Q_BYTES + KV_BYTES + 1024;
     static_assert(HD == 64 || HD == 128, "head sizes 64 and 128");
     static_assert(ROT == 0 || ROT == 64, "one shared sub-tile or none");
     static_assert(TMEM_USED <= TMEM_COLS, "S, O, P and the rotated queries must fit the allocation");
@@ -241,6 +245,7 @@ struct FlashParams {
     float sink2;                      // a score (times log2(e)) that joins the softmax's sum without a key or a value; -inf: none
     // keys and values in matrices of their own instead of pages: [rows, nkv * HD], request s's key j in row kv_start[s] + j
     const int* kv_start;              // null: keys and values come from the paged pools
+    int k_low_cols;                   // PAIR: columns from a key's first piece to its second
     const unsigned char* odd_rows;    // BOUNDED, [odd_count], not null: 1 where a key stands for NaN (a query that sees it comes out NaN)
     int odd_count;
     int q_head_cols;                  // columns of a head in q's rows (HD, and more where q holds other parts between the heads)
@@ -365,6 +370,11 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT, FORM == BOUNDED && RO
                     tma_load_2d(v_tile + h * SUB_KV + b * (64 * 128), &map_v, &kv_full[s], v_col + h * 64, v_row);
                 }
                 if (ROT) tma_load_2d(k_tile + SUBS * SUB_KV + b * (64 * 128), &map_k_rot, &kv_full[s], 0, row);
+                if (PAIR) {
+#pragma unroll
+                    for (int h = 0; h < SUBS; ++h)
+                        tma_load_2d(k_tile + (SUBS + 1 + h) * SUB_KV + b * (64 * 128), &map_k, &kv_full[s], col + p.k_low_cols + h * 64, row);
+                }
             }
         }
     } else if (warp == MMA_WARP) {
@@ -391,6 +401,14 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT, FORM == BOUNDED && RO
                 const uint64_t k_desc = smem_desc(kv_tiles + s * STAGE_BYTES + SUBS * SUB_KV);
 #pragma unroll
                 for (int k = 0; k < 8; ++k) umma_ts(leader, tmem, tmem + S_::ROT_COL + 8 * k, k_desc + 2 * (k & 3), idesc_s, 1);
+            }
+            if (PAIR) {
+#pragma unroll
+                for (int h = 0; h < SUBS; ++h) {
+                    const uint64_t q_desc = smem_desc(q_tile + h * SUB_Q), k_desc = smem_desc(kv_tiles + s * STAGE_BYTES + (SUBS + 1 + h) * SUB_KV);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) umma_ss(leader, tmem, q_desc + 2 * k, k_desc + 2 * k, idesc_s, 1);
+                }
             }
             if (leader) umma_commit(&s_done);
             __syncwarp();
@@ -768,7 +786,7 @@ int run_prefill(const void* q, long long q_cols, long long q_stride, void* out, 
                 const float* slopes, const float* head_bias, const void* gate, long long gate_stride, cudaStream_t stream,
                 bool bounded = false, int chunk = 0, float softcap = 0.f, int value_heads = 0, const int* kv_start = nullptr,
                 long long dense_rows = 0, float sink = -INFINITY, const SharedPart* shared = nullptr, long long dense_stride = 0,
-                const unsigned char* odd_rows = nullptr) {
+                const unsigned char* odd_rows = nullptr, long long k_low_cols = 0) {
     TS_REQUIRE(ts_attention_tcgen05_supported(hd, page_tokens, nh, nkv, 0), "attention_tcgen05: sizes not taken (head_dim %d, page %d)", hd, page_tokens);
     TS_REQUIRE(sigmoid || bounded || window == 0, "attention_tcgen05: the plain form takes no window");
     TS_REQUIRE(window >= 0 && chunk >= 0 && softcap >= 0.f, "attention_tcgen05: a negative window, chunk or cap");
@@ -790,7 +808,9 @@ int run_prefill(const void* q, long long q_cols, long long q_stride, void* out, 
     if (kv_start != nullptr) {                           // matrices [dense_rows, heads * hd]
         TS_REQUIRE(dense_rows > 0 && dense_rows < 0x7fffffffll, "attention_tcgen05: %lld rows of keys", dense_rows);
         TS_REQUIRE(dense_stride >= (long long)nkv * hd && dense_stride % 8 == 0, "attention_tcgen05: key and value rows %lld elements apart", dense_stride);
-        if (make_map(&map_k, k_pool, dense_rows, (long long)nkv * hd, dense_stride, 64)) return 1;
+        TS_REQUIRE(k_low_cols >= 0 && k_low_cols % 8 == 0 && k_low_cols + (long long)nkv * hd <= dense_stride,
+                   "attention_tcgen05: the keys' second pieces %lld columns behind the first, rows %lld apart", k_low_cols, dense_stride);
+        if (make_map(&map_k, k_pool, dense_rows, k_low_cols + (long long)nkv * hd, dense_stride, 64)) return 1;
         if (make_map(&map_v, v_pool, dense_rows, (long long)value_heads * hd, dense_stride, 64)) return 1;
     } else {
         if (make_map(&map_k, k_pool, pool_rows, hd, hd, 64)) return 1;
@@ -831,6 +851,7 @@ int run_prefill(const void* q, long long q_cols, long long q_stride, void* out, 
     p.value_heads = value_heads;
     p.sink2 = sink > -INFINITY ? sink * LOG2E : -INFINITY;
     p.kv_start = kv_start;
+    p.k_low_cols = (int)k_low_cols;
     p.odd_rows = odd_rows;
     p.odd_count = (int)dense_rows;
     p.error = error;
@@ -924,18 +945,20 @@ TS_API int ts_prefill_attention_tcgen05_masked(const void* q, long long q_stride
 // k_rot_stride elements apart, in the same row order as k.
 // `sinks` [nh] (null: none): a score a head that joins every softmax's sum without a key or a value.
 // `window` n > 0: query i sees keys i - n + 1 .. i; rows of keys no query of the step sees need not be there (kv_start may then be
-// negative), and `odd_rows` [kv_rows] (null: none) marks keys that stand for NaN, whose rows of k and v hold zeros.
+// negative), `odd_rows` [kv_rows] (null: none) marks keys that stand for NaN, whose rows of k and v hold zeros, and a key is the sum
+// of two pieces, the second one k_low_cols columns behind the first in the rows of k.
 TS_API int ts_prefill_attention_tcgen05_dense(const void* q, long long q_stride, void* out, const void* k, const void* v,
                                               long long kv_rows, long long kv_stride, const int* kv_start, const int* cu_q,
                                               const int* ctx_lens, int num_seqs, int num_tokens, int max_q_len, int nh, int nkv, int hd,
-                                              float scale, int window, const unsigned char* odd_rows, const int* prefill_seqs,
-                                              int num_prefill_seqs, int* error, int q_head_cols, const float* turn, const void* k_rot,
+                                              float scale, int window, long long k_low_cols, const unsigned char* odd_rows,
+                                              const int* prefill_seqs, int num_prefill_seqs, int* error, int q_head_cols, const float* turn, const void* k_rot,
                                               long long k_rot_stride, int rot, const float* sinks, cudaStream_t stream) {
     TS_REQUIRE(kv_start != nullptr, "attention_tcgen05: the first rows of the requests' keys are needed");
     TS_REQUIRE(q_head_cols >= hd && (rot == 0 || (turn && k_rot)), "attention_tcgen05: the queries' columns, or the shared key part");
-    TS_REQUIRE((odd_rows == nullptr || window > 0) && (window == 0 || rot > 0), "attention_tcgen05: a window comes with a shared key part, marked keys with a window");
+    TS_REQUIRE((odd_rows == nullptr || window > 0) && (window == 0 || rot > 0) && (window > 0) == (k_low_cols > 0),
+               "attention_tcgen05: a window comes with a shared key part and keys of two pieces, marked keys with a window");
     const SharedPart shared{(const float2*)turn, k_rot, k_rot_stride, rot, q_head_cols, sinks};
     return run_prefill(q, (long long)nh * q_head_cols, q_stride, out, k, v, 1, 1, 0, 64, nullptr, 1, cu_q, ctx_lens, num_seqs, num_tokens,
                        max_q_len, nh, nkv, hd, scale, prefill_seqs, num_prefill_seqs, error, false, window, nullptr, nullptr, nullptr, 0,
-                       stream, window > 0, 0, 0.f, 0, kv_start, kv_rows, -INFINITY, &shared, kv_stride, odd_rows);
+                       stream, window > 0, 0, 0.f, 0, kv_start, kv_rows, -INFINITY, &shared, kv_stride, odd_rows, k_low_cols);
 }

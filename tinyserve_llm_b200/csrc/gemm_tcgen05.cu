@@ -17,7 +17,8 @@
 //
 // Epilogues: plain store (bfloat16 or float32), or SwiGLU: the tile's BN columns are BN/2 gate rows
 // of W and the BN/2 up rows that belong to them, and it stores round(silu(gate)) * up
-// (model/llama.py:80-83 of the reference), which saves writing and re-reading the [T, 2I] product.
+// (model/llama.py:80-83 of the reference), which saves writing and re-reading the [T, 2I] product; or
+// pieces: the first columns as two bfloat16 numbers each, the others rounded.
 //
 // Every wait on an mbarrier gives up after about two seconds, records where in an error word the
 // host can read, and the CTA goes on to free its tensor memory and return.
@@ -29,7 +30,7 @@ constexpr int BM = 128, BK = 64, UMMA_K = 16;
 constexpr int EPI_WARPS = 8, THREADS = 64 + 32 * EPI_WARPS;     // two epilogue warps for each quarter of the accumulator's lanes
 constexpr int A_BYTES = BM * BK * 2;
 
-enum { EPI_STORE = 0, EPI_SWIGLU = 1 };
+enum { EPI_STORE = 0, EPI_SWIGLU = 1, EPI_PIECES = 2 };
 
 // Instruction descriptor: bfloat16 x bfloat16 -> float32, both operands K-major, tile M x N.
 __device__ __forceinline__ uint32_t instr_desc(int m, int n) {
@@ -69,7 +70,46 @@ struct GemmParams {
     int* error;
     int act;              // gated epilogue: the activation (TS_ACT_* of common.cuh; 0 = SiLU) and its constants
     float act_limit, act_alpha;
+    int low_cols;         // EPI_PIECES
 };
+
+// Eight columns of the product from `col` on.  EPI_PIECES: columns before low_cols are stored as two bfloat16 pieces, y = hi + lo to 2^-17
+// of y, lo behind the row's N columns (an infinite hi has none).
+template <int EPI>
+__device__ __forceinline__ void store_eight(const GemmParams& p, int row, int col, const uint32_t* acc) {
+    if (EPI == EPI_STORE && p.out_f32) {
+        float* out = (float*)p.y + (long long)row * p.ldy + col;
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (col + e < p.N) out[e] = __uint_as_float(acc[e]);
+        return;
+    }
+    __nv_bfloat16* out = (__nv_bfloat16*)p.y + (long long)row * p.ldy + col;
+    if (col + 8 <= p.N && (((uintptr_t)out) & 15) == 0) {
+        uint4 v;
+        __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) h[e] = __floats2bfloat162_rn(__uint_as_float(acc[2 * e]), __uint_as_float(acc[2 * e + 1]));
+        *reinterpret_cast<uint4*>(out) = v;
+    } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (col + e < p.N) out[e] = __float2bfloat16_rn(__uint_as_float(acc[e]));
+    }
+    if (EPI == EPI_PIECES && col < p.low_cols) {         // (low_cols and N are multiples of 8)
+        float rest[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float x = __uint_as_float(acc[e]), hi = round_to<__nv_bfloat16>(x);
+            rest[e] = isinf(hi) ? 0.f : x - hi;
+        }
+        uint4 v;
+        __nv_bfloat162* l = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) l[e] = __floats2bfloat162_rn(rest[2 * e], rest[2 * e + 1]);
+        *reinterpret_cast<uint4*>(out + p.N) = v;
+    }
+}
 
 template <int EPI, int BN, int STAGES>
 __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
@@ -230,26 +270,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
 #pragma unroll
                     for (int j = 0; j < SHARE; j += 8) {
                         const int c = c0 + j;
-                        if (p.out_f32) {
-                            float* out = (float*)p.y + (long long)row * p.ldy + n0 + c;
-#pragma unroll
-                            for (int e = 0; e < 8; ++e)
-                                if (n0 + c + e < p.N) out[e] = __uint_as_float(acc[j + e]);
-                        } else {
-                            __nv_bfloat16* out = (__nv_bfloat16*)p.y + (long long)row * p.ldy + n0 + c;
-                            if (n0 + c + 8 <= p.N && (((uintptr_t)out) & 15) == 0) {
-                                uint4 v;
-                                __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
-#pragma unroll
-                                for (int e = 0; e < 4; ++e)
-                                    h[e] = __floats2bfloat162_rn(__uint_as_float(acc[j + 2 * e]), __uint_as_float(acc[j + 2 * e + 1]));
-                                *reinterpret_cast<uint4*>(out) = v;
-                            } else {
-#pragma unroll
-                                for (int e = 0; e < 8; ++e)
-                                    if (n0 + c + e < p.N) out[e] = __float2bfloat16_rn(__uint_as_float(acc[j + e]));
-                            }
-                        }
+                        store_eight<EPI>(p, row, n0 + c, acc + j);
                     }
                 }
             }
@@ -447,26 +468,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_pair_kernel(const __grid
 #pragma unroll
                     for (int j = 0; j < SHARE; j += 8) {
                         const int c = c0 + j;
-                        if (p.out_f32) {
-                            float* out = (float*)p.y + (long long)row * p.ldy + n0 + c;
-#pragma unroll
-                            for (int e = 0; e < 8; ++e)
-                                if (n0 + c + e < p.N) out[e] = __uint_as_float(acc[j + e]);
-                        } else {
-                            __nv_bfloat16* out = (__nv_bfloat16*)p.y + (long long)row * p.ldy + n0 + c;
-                            if (n0 + c + 8 <= p.N && (((uintptr_t)out) & 15) == 0) {
-                                uint4 v;
-                                __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
-#pragma unroll
-                                for (int e = 0; e < 4; ++e)
-                                    h[e] = __floats2bfloat162_rn(__uint_as_float(acc[j + 2 * e]), __uint_as_float(acc[j + 2 * e + 1]));
-                                *reinterpret_cast<uint4*>(out) = v;
-                            } else {
-#pragma unroll
-                                for (int e = 0; e < 8; ++e)
-                                    if (n0 + c + e < p.N) out[e] = __float2bfloat16_rn(__uint_as_float(acc[j + e]));
-                            }
-                        }
+                        store_eight<EPI>(p, row, n0 + c, acc + j);
                     }
                 }
             }
@@ -504,10 +506,11 @@ TS_API int ts_gemm_tcgen05_supported(const void* W, const void* x, int M, int N,
 // read (0: fine; 1, 2, 3: a producer, MMA or epilogue wait ran out of time).
 static int gemm_tcgen05_launch(const void* W, const void* x, void* y, int M, int N, int K, long long ldx, long long ldy,
                                int epilogue, int out_dtype, int* error, int act, float act_limit, float act_alpha,
-                               cudaStream_t stream);
+                               cudaStream_t stream, int low_cols = 0);
 
 TS_API int ts_gemm_tcgen05(const void* W, const void* x, void* y, int M, int N, int K, long long ldx, long long ldy,
                            int epilogue, int out_dtype, int* error, cudaStream_t stream) {
+    TS_REQUIRE(epilogue == EPI_STORE || epilogue == EPI_SWIGLU, "gemm_tcgen05: unknown epilogue %d", epilogue);
     return gemm_tcgen05_launch(W, x, y, M, N, K, ldx, ldy, epilogue, out_dtype, error, TS_ACT_SILU, 0.f, 1.f, stream);
 }
 
@@ -518,12 +521,19 @@ TS_API int ts_gemm_tcgen05_gated(const void* W, const void* x, void* y, int M, i
     return gemm_tcgen05_launch(W, x, y, M, N, K, ldx, ldy, EPI_SWIGLU, TS_BF16, error, act, limit, alpha, stream);
 }
 
+// The product's rows of N columns, bfloat16, and behind them what that rounding left of the first low_cols: rows of N + low_cols.
+TS_API int ts_gemm_tcgen05_pieces(const void* W, const void* x, void* y, int M, int N, int K, long long ldx, int low_cols, int* error,
+                                  cudaStream_t stream) {
+    TS_REQUIRE(N % 8 == 0 && low_cols % 8 == 0 && low_cols >= 0 && low_cols <= N && (uintptr_t)y % 16 == 0,
+               "gemm_tcgen05: pieces of %d of %d columns, or their alignment", low_cols, N);
+    return gemm_tcgen05_launch(W, x, y, M, N, K, ldx, (long long)N + low_cols, EPI_PIECES, TS_BF16, error, TS_ACT_SILU, 0.f, 1.f, stream, low_cols);
+}
+
 static int gemm_tcgen05_launch(const void* W, const void* x, void* y, int M, int N, int K, long long ldx, long long ldy,
                                int epilogue, int out_dtype, int* error, int act, float act_limit, float act_alpha,
-                               cudaStream_t stream) {
+                               cudaStream_t stream, int low_cols) {
     TS_REQUIRE(ts_gemm_tcgen05_supported(W, x, M, N, K, ldx), "gemm_tcgen05: sizes or alignment TMA does not take (M=%d N=%d K=%d)", M, N, K);
     TS_REQUIRE(error != nullptr, "gemm_tcgen05: an error word is needed");
-    TS_REQUIRE(epilogue == EPI_STORE || epilogue == EPI_SWIGLU, "gemm_tcgen05: unknown epilogue %d", epilogue);
     TS_REQUIRE(out_dtype == TS_BF16 || (out_dtype == TS_F32 && epilogue == EPI_STORE), "gemm_tcgen05: unsupported output dtype");
     const int inter = N / 2;
     if (epilogue == EPI_SWIGLU) TS_REQUIRE(N % 2 == 0, "gemm_tcgen05: the SwiGLU epilogue needs gate and up halves (N=%d)", N);
@@ -539,7 +549,7 @@ static int gemm_tcgen05_launch(const void* W, const void* x, void* y, int M, int
     const int out_per_tile = epilogue == EPI_SWIGLU ? bn / 2 : bn;
     const int num_tiles = m_tiles * ((out_cols + out_per_tile - 1) / out_per_tile);
     CUtensorMap map_a, map_b;
-    GemmParams p{y, M, N, K, ldy, inter, out_dtype == TS_F32 ? 1 : 0, error, act, act_limit, act_alpha};
+    GemmParams p{y, M, N, K, ldy, inter, out_dtype == TS_F32 ? 1 : 0, error, act, act_limit, act_alpha, low_cols};
     // Two CTAs a tile of 256 x 256 where every pair of SMs gets at least six such tiles: measured on a B200, pairs were
     // 1 to 3 % faster than single CTAs from there on (Llama 3.2 1B's gate/up product at 2,048 and 8,192 rows, Llama
     // 3.1 8B's from 1,024 rows) and the same or slower with fewer tiles, whose last round leaves more pairs idle.
@@ -567,6 +577,9 @@ static int gemm_tcgen05_launch(const void* W, const void* x, void* y, int M, int
         if (epilogue == EPI_SWIGLU) {
             cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<EPI_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_smem);
             TS_CHAINED_CHECK("gemm_tcgen05", cudaLaunchKernelEx(&cfg, gemm_tcgen05_pair_kernel<EPI_SWIGLU>, map_a, map_b, p));
+        } else if (epilogue == EPI_PIECES) {
+            cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<EPI_PIECES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_smem);
+            TS_CHAINED_CHECK("gemm_tcgen05", cudaLaunchKernelEx(&cfg, gemm_tcgen05_pair_kernel<EPI_PIECES>, map_a, map_b, p));
         } else {
             cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<EPI_STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_smem);
             TS_CHAINED_CHECK("gemm_tcgen05", cudaLaunchKernelEx(&cfg, gemm_tcgen05_pair_kernel<EPI_STORE>, map_a, map_b, p));
@@ -590,6 +603,10 @@ static int gemm_tcgen05_launch(const void* W, const void* x, void* y, int M, int
         if (wide) TS_GEMM_LAUNCH(EPI_SWIGLU, 256, 4);
         else if (deep) TS_GEMM_LAUNCH(EPI_SWIGLU, 128, 6);
         else TS_GEMM_LAUNCH(EPI_SWIGLU, 128, 3);
+    } else if (epilogue == EPI_PIECES) {
+        if (wide) TS_GEMM_LAUNCH(EPI_PIECES, 256, 4);
+        else if (deep) TS_GEMM_LAUNCH(EPI_PIECES, 128, 6);
+        else TS_GEMM_LAUNCH(EPI_PIECES, 128, 3);
     } else {
         if (wide) TS_GEMM_LAUNCH(EPI_STORE, 256, 4);
         else if (deep) TS_GEMM_LAUNCH(EPI_STORE, 128, 6);

@@ -34,7 +34,7 @@ _SIGNATURES = {
     "ts_paged_attention_bf16_sigmoid": ("int", "pl" "ppp" "lliipippiiiiiiifiplpi" "pppl" "p"),
     "ts_paged_attention_bf16_masked": ("int", "pl" "ppp" "lllliipippiiiiiiifiifi" "plpi" "fp"),
     "ts_attention_tcgen05_supported": ("int", "iiiii"),
-    "ts_prefill_attention_tcgen05_dense": ("int", "pl" "ppp" "llpppiiiiiif" "ippip" "ipplip" "p"),
+    "ts_prefill_attention_tcgen05_dense": ("int", "pl" "ppp" "llpppiiiiiif" "ilppip" "ipplip" "p"),
     "ts_latent_gather": ("int", "plliipipppiiiiipfplppppp"),
     "ts_prefill_attention_tcgen05_masked": ("int", "pl" "ppp" "iiiipippiiiiiifiifi" "pipfp"),
     "ts_prefill_attention_tcgen05": ("int", "ppppiiiipippiiiiiifpipp"),
@@ -43,6 +43,7 @@ _SIGNATURES = {
     "ts_feed_tokens": ("int", "pipip"),
     "ts_gemm_tcgen05_supported": ("int", "ppiiil"),
     "ts_gemm_tcgen05": ("int", "pppiiilliipp"),
+    "ts_gemm_tcgen05_pieces": ("int", "pppiiilipp"),
     "ts_gemm_tcgen05_set_pairing": ("void", "i"),
     "ts_last_error": ("const char*", ""),
     "ts_abi_version": ("int", ""),
@@ -865,7 +866,7 @@ class Ops:
     def dense_prompt_attention(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, kv_start: torch.Tensor, ctx, nh: int,
                                nkv: int, hd: int, scale: float, out: torch.Tensor | None = None, *, q_head_cols: int = 0,
                                shared: tuple[torch.Tensor, torch.Tensor] | None = None, sink: torch.Tensor | None = None,
-                               window: int = 0, odd_rows: torch.Tensor | None = None) -> torch.Tensor:
+                               window: int = 0, odd_rows: torch.Tensor | None = None, k_low: torch.Tensor | None = None) -> torch.Tensor:
         """
         Causal softmax attention of the step's prompt portions (requests that feed more than one token) over keys
         and values worked out for the step: k, v [rows, nkv * hd] bfloat16 (stretches of one row stride), request s's key j in row
@@ -875,8 +876,8 @@ class Ops:
         `q_head_cols` (0: hd): columns of a head in q's rows, its first hd being the ones that meet k.  `shared` (turn
         float32 [T, 32, 2], k_rot [rows, rot <= 64]): a score also has q_rot . k_rot, k_rot being the same for all heads and q_rot the
         head's next rot columns, rotated by halves by the cosines and sines in turn.  `sink` (float32 [nh]): exp(sink[h]) joins every softmax's sum of head h.
-        `window` n > 0 (with `shared`): a query sees its own key and the n - 1 before it; with `odd_rows` (uint8 [rows]) keys marked there stand for
-        NaN and their rows of k and v hold zeros.
+        `window` n > 0 (with `shared`): a query sees its own key and the n - 1 before it, keys are k + k_low (columns behind k's in the same rows),
+        and with `odd_rows` (uint8 [rows]) keys marked there stand for NaN and their rows of k and v hold zeros.
         """
         q_head_cols = q_head_cols or hd
         self._check_rows(q, "q")
@@ -884,6 +885,14 @@ class Ops:
         self._check_rows(v, "v")
         if k.dtype != torch.bfloat16 or v.dtype != torch.bfloat16 or k.stride(0) != v.stride(0):
             raise KernelError(f"dense_prompt_attention: k and v are bfloat16 with one row stride, not {k.dtype}, {v.dtype}, {k.stride(0)}, {v.stride(0)}")
+        low_cols = 0
+        if (k_low is not None) != (window > 0):
+            raise KernelError("dense_prompt_attention: a window comes with keys of two pieces")
+        if k_low is not None:
+            self._check_rows(k_low, "k_low")
+            low_cols = (k_low.data_ptr() - k.data_ptr()) // 2
+            if k_low.dtype != k.dtype or k_low.shape != k.shape or k_low.stride(0) != k.stride(0) or not 0 < low_cols <= k.stride(0) - k.shape[1]:
+                raise KernelError(f"dense_prompt_attention: second pieces {tuple(k_low.shape)} {k_low.dtype} that are not columns behind k's {tuple(k.shape)}")
         if odd_rows is not None:
             self._check(odd_rows, "odd_rows", torch.uint8, 1)
             if odd_rows.shape[0] != k.shape[0]:
@@ -912,7 +921,7 @@ class Ops:
         num_prefill = prefill_seqs.shape[0] if prefill_seqs is not None else 0
         self._call("ts_prefill_attention_tcgen05_dense", _ptr(q), q.stride(0), _ptr(out), _ptr(k), _ptr(v), k.shape[0],
                    k.stride(0), _ptr(kv_start), _ptr(ctx.cu_q), _ptr(ctx.ctx_lens), ctx.ctx_lens.shape[0], q.shape[0], ctx.max_q_len,
-                   nh, nkv, hd, scale, window, _ptr(odd_rows), _ptr(prefill_seqs), num_prefill, self.error_word().data_ptr(), q_head_cols, _ptr(turn), _ptr(k_rot),
+                   nh, nkv, hd, scale, window, low_cols, _ptr(odd_rows), _ptr(prefill_seqs), num_prefill, self.error_word().data_ptr(), q_head_cols, _ptr(turn), _ptr(k_rot),
                    k_rot.stride(0) if k_rot is not None else 0, k_rot.shape[1] if k_rot is not None else 0, _ptr(sink), _stream())
         return out
 
@@ -1701,6 +1710,18 @@ class Ops:
         self._call("ts_gemm_tcgen05", _ptr(weight), _ptr(x), _ptr(out), M, N, K, K,
                    cols, 1 if swiglu else 0, _DTYPE_CODE[out_dtype],
                    self.error_word().data_ptr(), _stream())
+        return out
+
+    def gemm_tcgen05_pieces(self, x: torch.Tensor, weight: torch.Tensor, low_cols: int) -> torch.Tensor:
+        """bfloat16 [M, N + low_cols]: x [M, K] . weight[N, K]^T rounded, and behind it what that left of the first low_cols columns."""
+        self._check(x, "x", torch.bfloat16, 2)
+        self._check(weight, "weight", torch.bfloat16, 2)
+        (M, K), N = x.shape, weight.shape[0]
+        if weight.shape[1] != K:
+            raise KernelError(f"gemm_tcgen05: x has {K} columns, the weight {weight.shape[1]}")
+        out = torch.empty((M, N + low_cols), dtype=torch.bfloat16, device=x.device)
+        if M:
+            self._call("ts_gemm_tcgen05_pieces", _ptr(weight), _ptr(x), _ptr(out), M, N, K, K, low_cols, self.error_word().data_ptr(), _stream())
         return out
 
     def check_device_errors(self) -> None:

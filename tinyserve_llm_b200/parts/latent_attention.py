@@ -23,8 +23,8 @@ over the channels, so the order does not show), and the kernels rotate by halves
 Prompt portions of a step that is launched once (not replayed from a CUDA graph) take another way where the
 sizes allow (bfloat16, key and value heads of one size the tcgen05 prompt kernel takes, up to 64 rotated channels): the
 latents the portions see, their whole contexts or what a window leaves, are gathered from the pages (their rotated parts, one for
-all heads, go to the kernel as they lie), a head's keys and values are worked out for the step ([K | V] = C [W_uk; W_uv]^T, one library
-product: a quarter of the folded form's arithmetic at a latent of 512 channels and heads of 128) and the tcgen05 prompt kernel
+all heads, go to the kernel as they lie), a head's keys and values are worked out for the step ([K | V] = C [W_uk; W_uv]^T, one
+product, behind a window with keys of two pieces: a quarter of the folded form's arithmetic at a latent of 512 channels and heads of 128) and the tcgen05 prompt kernel
 attends over them; requests that feed one token in the same step stay on the folded form.  The two ways differ by rounding only.
 
 Tensors (local names): dq, dq.norm, uq (or q), dkv, dkv.norm, uk, uv, o, g with an output gate, sink.
@@ -134,7 +134,7 @@ class LatentAttention(Mixer):
                 or self.uk_uv is None or (spec.window and not spec.rot_dim)
                 or not ops.dense_prompt_attention_supported(q, spec.num_heads, spec.num_heads, spec.head_dim)):
             return None
-        # (windows come in the kernel's form with a rotated part, whose queries and probabilities have the folded form's precision)
+        # (windows come in the kernel's form with a rotated part, whose queries, keys and probabilities have the folded form's precision)
         lens = [b - a for a, b in zip(host.cu_q, host.cu_q[1:])]
         fed = sum(n for n in lens if n > 1)
         if fed < MATERIALIZE_MIN_TOKENS:
@@ -159,9 +159,30 @@ class LatentAttention(Mixer):
         spec, ops = self.spec, self.rt.ops
         H, D, R, rank = spec.num_heads, spec.head_dim, spec.rot_dim, spec.kv_rank
         c, shared, odd, kv_start = ops.latent_gather(ctx, binding, sum(keys), max(keys), rank, R, spec.window, self.frequencies, self.magnitude)
-        kv = ops.linear(c, self.uk_uv)                      # [keys, H D | H D]
-        return ops.dense_prompt_attention(q, kv[:, :H * D], kv[:, H * D:], kv_start, ctx, H, H, D, spec.scale, out, q_head_cols=D + R,
-                                          shared=shared, sink=self.sink, window=spec.window, odd_rows=odd)
+        if not spec.window:
+            kv, k_low = ops.linear(c, self.uk_uv), None     # [keys, H D | H D]
+        else:                                               # keys as two pieces: the folded form rounds none
+            kv = ops.gemm_tcgen05_pieces(c, self.uk_uv, H * D)
+            k_low = kv[:, 2 * H * D:]
+        return ops.dense_prompt_attention(q, kv[:, :H * D], kv[:, H * D:2 * H * D], kv_start, ctx, H, H, D, spec.scale, out, q_head_cols=D + R,
+                                          shared=shared, sink=self.sink, window=spec.window, odd_rows=odd, k_low=k_low)
+
+    def attend(self, q: torch.Tensor, ctx, binding) -> torch.Tensor:
+        """[T, H V] in q's dtype: the heads' outputs for queries q [T, H (D + R)], rotated here, over the cached rows [c | k_rot]."""
+        spec, ops = self.spec, self.rt.ops
+        H, D, R, V, rank = spec.num_heads, spec.head_dim, spec.rot_dim, spec.value_dim, spec.kv_rank
+        portions = self._portions(q, ctx)
+        if portions is not None and ctx.min_q_len > 1:
+            return self._attend_unfolded(q, ctx, binding, portions, None)
+        folded_ctx = ctx if portions is None else self._single_tokens_only(ctx)
+        q_lat = ops.per_head_linear(q, self.uk_t, H, D + R, D)            # float32 [T, H, rank]: W_uk^T q_flat
+        o_lat = ops.latent_attention(q_lat, q, folded_ctx, binding, H, D + R, D, rank, R, self.frequencies, spec.scale,
+                                     spec.window, magnitude=self.magnitude, sink=self.sink)   # [T, H, rank]: softmax-weighted sums of c
+        o = ops.per_head_linear(o_lat.view(-1, H * rank), self.uv, H, rank, rank, out_dtype=q.dtype)   # [T, H, V]
+        o = o.reshape(-1, H * V)
+        if portions is None:
+            return o
+        return self._attend_unfolded(q, ctx, binding, portions, o.contiguous())               # the portions' rows are written over
 
     def forward(self, x: torch.Tensor, ctx, binding) -> torch.Tensor:
         spec, ops = self.spec, self.rt.ops
@@ -177,18 +198,7 @@ class LatentAttention(Mixer):
             q = y[:, :H * (D + R)]
             ops.latent_prepare(y[:, H * (D + R):latents], ctx, binding, 0, rank, R, None, self.kv_norm, spec.norm_eps,
                                self.frequencies, self.magnitude)
-        portions = self._portions(q, ctx)
-        if portions is not None and ctx.min_q_len > 1:
-            o = self._attend_unfolded(q, ctx, binding, portions, None)
-        else:
-            folded_ctx = ctx if portions is None else self._single_tokens_only(ctx)
-            q_lat = ops.per_head_linear(q, self.uk_t, H, D + R, D)        # float32 [T, H, rank]: W_uk^T q_flat
-            o_lat = ops.latent_attention(q_lat, q, folded_ctx, binding, H, D + R, D, rank, R, self.frequencies, spec.scale,
-                                         spec.window, magnitude=self.magnitude, sink=self.sink)   # [T, H, rank]: softmax-weighted sums of c
-            o = ops.per_head_linear(o_lat.view(-1, H * rank), self.uv, H, rank, rank, out_dtype=x.dtype)   # [T, H, V]
-            o = o.reshape(-1, H * V)
-            if portions is not None:                                      # the portions' rows are written over
-                o = self._attend_unfolded(q, ctx, binding, portions, o.contiguous())
+        o = self.attend(q, ctx, binding)
         if spec.output_gate:
             o = ops.sigmoid_gate(o, y[:, latents:latents + H * V])
         return self.out(o)
