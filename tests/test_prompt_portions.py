@@ -585,3 +585,73 @@ def test_products_in_pieces(rows, rank, cols, low):
     assert bool(((y[:, :cols].double() - want).abs() <= want.abs() * 2.0 ** -8 + sums).all())
     both = y[:, :low].double() + y[:, cols:].double()
     assert bool(((both - want[:, :low]).abs() <= want[:, :low].abs() * 2.0 ** -16 + sums).all())
+
+
+def _latent_part(heads, dim, rot, rank, window, **extra):
+    from tinyserve_llm_b200.config.spec import InlineRotarySpec, LatentAttentionSpec
+    from tinyserve_llm_b200.parts.base import Runtime, part_class
+    g, gate = torch.Generator().manual_seed(heads + rank), extra.get("output_gate", False)
+    w = lambda *shape: (torch.randn(shape, generator=g) * shape[-1] ** -0.5).to(torch.bfloat16)
+    tensors = {"q": w(heads * (dim + rot), 96), "dkv": w(rank + rot, 96), "uk": w(heads * dim, rank), "uv": w(heads * dim, rank), "o": w(96, heads * dim),
+               "dkv.norm": torch.ones(rank)}
+    if gate:
+        tensors["g"] = w(heads * dim, 96)
+    spec = LatentAttentionSpec(hidden_size=96, num_heads=heads, head_dim=dim, rot_dim=rot, value_dim=dim, q_rank=0, kv_rank=rank,
+                               scale=(dim + rot) ** -0.5, window=window, norm_eps=1e-5, position=InlineRotarySpec(dims=rot), **extra)
+    return part_class("mixer", spec)(spec, tensors, Runtime(dtype=torch.bfloat16, device=torch.device("cuda", 0), ops=get_ops()))
+
+
+def test_a_windowed_portion_takes_its_form_whatever_else_is_in_the_step():
+    """A portion's own tokens and keys decide, and a portion that a replayed step may hold stays with the form of such steps."""
+    part = _latent_part(2, 128, 64, 128, 300)
+    for tokens, cached, limit, unfolded in ((128, 0, 0, True), (127, 0, 0, False), (128, 90000, 0, True), (512, 0, 512, False), (513, 0, 512, True),
+                                            (700, 5000, 512, True), (700, 5000, 1024, False)):
+        for lens, kept in (([], []), ([600], [0]), ([2, 1, 40], [0, 9, 3000]), ([1] * 9, [5] * 9), ([2000, 64], [0, 70000])):
+            lens, kept = [tokens] + lens, [cached] + kept
+            ctx = make_ctx(lens, [n + c for n, c in zip(lens, kept)])
+            ctx.replayed, ctx.replay_limit = False, limit
+            q = torch.empty(sum(lens), 2 * 192, dtype=torch.bfloat16, device="cuda")
+            assert (0 in part.unfolded_requests(q, ctx)) == unfolded, (tokens, cached, limit, lens)
+    far = _latent_part(2, 128, 64, 128, 20000)           # a window of 20,000 keys for 200 tokens: the latents are read as they are
+    ctx = make_ctx([200, 2000], [50000, 2000])
+    ctx.replayed = False
+    assert far.unfolded_requests(torch.empty(2200, 2 * 192, dtype=torch.bfloat16, device="cuda"), ctx) == [1]
+
+
+def test_the_engine_says_which_steps_it_may_replay():
+    from types import SimpleNamespace
+    from tinyserve_llm_b200.engine.step import HostView, StepContext
+    host = HostView([0], [0, 3], [0], [3], [0])
+    for runner, limit in ((None, 0), (SimpleNamespace(cuda_graphs=True, graph_max_tokens=512), 512), (SimpleNamespace(cuda_graphs=False, graph_max_tokens=512), 0)):
+        assert StepContext(runner, 3, 1, host).replay_limit == limit
+
+
+@pytest.mark.parametrize("rank", [512, 128])             # folded portions four tokens a CTA, and a token a CTA
+def test_portions_of_both_forms_in_one_step(rank):
+    """Long portions beside short ones and single tokens: every row as in a step in which its request is alone with its like."""
+    part, lens, cached, page = _latent_part(2, 128, 64, rank, 200), [700, 300, 1, 90, 600], [0, 40, 333, 10, 77], 64
+    g = torch.Generator().manual_seed(rank)
+    ends = [n + c for n, c in zip(lens, cached)]
+    counts = [-(-e // page) for e in ends]
+    pool = torch.randn(sum(counts), 1, 1, page, rank + 64, generator=g).to(torch.bfloat16).cuda()
+    q = torch.randn(sum(lens), 2 * 192, generator=g).to(torch.bfloat16).cuda()
+    tables = [list(range(sum(counts[:s]), sum(counts[:s + 1]))) + [-1] * (max(counts) - n) for s, n in enumerate(counts)]
+
+    def attend(which):
+        ctx = make_ctx([lens[s] for s in which], [ends[s] for s in which])
+        ctx.replayed, ctx.replay_limit, ctx.prefill_seqs = False, 512, i32([i for i, s in enumerate(which) if lens[s] > 1])
+        rows = torch.cat([torch.arange(sum(lens[:s]), sum(lens[:s + 1])) for s in which]).cuda()
+        out = part.attend(q[rows].contiguous(), ctx, EntryBinding(pool, None, page * (rank + 64), 0, page, pool.shape[0], i32([tables[s] for s in which]), max(counts)))
+        return out, torch.split(out, [lens[s] for s in which])
+
+    before = dict(get_ops().calls)
+    together, rows = attend([0, 1, 2, 3, 4])
+    assert torch.isfinite(together).all()
+    for name in ("ts_prefill_attention_tcgen05_dense", "ts_latent_attention"):
+        assert get_ops().calls[name] == before.get(name, 0) + 1
+    _, (first, last) = attend([0, 4])
+    assert torch.equal(rows[0], first) and torch.equal(rows[4], last)
+    # the folded form's products of other numbers of rows may sum in another order, in float32, before one rounding to bfloat16
+    _, others = attend([1, 2, 3])
+    for got, want in zip((rows[1], rows[2], rows[3]), others):
+        assert float((got.double() - want.double()).norm() / want.double().norm()) < 2.0 ** -9

@@ -320,8 +320,8 @@ bool ts_latent_tokens_supported(int rank, int rot);                  // attentio
 int ts_latent_attention_tokens_launch(const float* q_lat, long long ql_t, long long ql_h, const void* q, long long q_stride,
                                       int q_head_width, int q_rot_offset, const float* freq, float magnitude, const float* sink,
                                       const void* k_pool, KVGeometry geo, const int* block_table, int table_width,
-                                      const int* positions, const int* cu_q, int num_seqs, void* out, int num_tokens, int heads,
-                                      int rank, int rot, float scale, int window, cudaStream_t stream);
+                                      const int* positions, const int* seq_of_token, const int* cu_q, int num_seqs, void* out,
+                                      int num_tokens, int heads, int rank, int rot, float scale, int window, cudaStream_t stream);
 
 // How many floats of scratch a call with these sizes needs (0: the step is large enough to run without splits).
 TS_API long long ts_latent_attention_scratch_floats(int num_tokens, int heads, int rank, int max_keys) {
@@ -377,7 +377,7 @@ TS_API int ts_latent_attention(const float* q_lat, long long ql_token_stride, lo
         const bool portions = cu_q && ts_latent_attention_portions(num_tokens, num_seqs, max_q_len, heads, rank, rot, max_keys);
         if (portions) {
             if (ts_latent_attention_tokens_launch(q_lat, ql_token_stride, ql_head_stride, q, q_stride, q_head_width, q_rot_offset, freq,
-                                                  magnitude, sink, k_pool, geo, block_table, table_width, positions, cu_q, num_seqs,
+                                                  magnitude, sink, k_pool, geo, block_table, table_width, positions, seq_of_token, cu_q, num_seqs,
                                                   out, num_tokens, heads, rank, rot, scale, window, stream))
                 return 1;
             if (min_q_len > 1) return 0;

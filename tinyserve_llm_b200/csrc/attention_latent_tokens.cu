@@ -27,7 +27,7 @@ struct LatentArgs {
     const float* freq; float magnitude; const float* sink;
     const __nv_bfloat16* k_pool; KVGeometry geo;
     const int* block_table; int table_width;
-    const int* positions; const int* cu_q;
+    const int* positions; const int* seq_of_token; const int* cu_q;
     int num_seqs, steps;                             // steps: the largest power of two up to num_seqs
     __nv_bfloat16* out;
     int heads, rot; float scale; int window;
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) latent_attention_tokens_kernel(
     for (int step = p.steps; step > 0; step >>= 1)
         if (seq + step < p.num_seqs && p.cu_q[seq + step] / TOKENS + 2 * (seq + step) <= tile_at) seq += step;
     const int begin = p.cu_q[seq], n = p.cu_q[seq + 1] - begin;
-    if (n <= 1) return;
+    if (n <= 1 || p.seq_of_token[begin] < 0) return;     // a single token, or a request that is left out
     const int start = p.positions[begin], last = start + n - 1;
     // the run's positions, pos0 .. pos1, of which the portion may hold the middle or one end: first .. first + tokens - 1
     const int pos0 = (start / TOKENS + tile_at - begin / TOKENS - 2 * seq) * TOKENS, pos1 = pos0 + TOKENS - 1;
@@ -347,13 +347,13 @@ bool ts_latent_tokens_supported(int rank, int rot) {
 int ts_latent_attention_tokens_launch(const float* q_lat, long long ql_t, long long ql_h, const void* q, long long q_stride,
                                       int q_head_width, int q_rot_offset, const float* freq, float magnitude, const float* sink,
                                       const void* k_pool, KVGeometry geo, const int* block_table, int table_width,
-                                      const int* positions, const int* cu_q, int num_seqs, void* out, int num_tokens, int heads,
-                                      int rank, int rot, float scale, int window, cudaStream_t stream) {
+                                      const int* positions, const int* seq_of_token, const int* cu_q, int num_seqs, void* out,
+                                      int num_tokens, int heads, int rank, int rot, float scale, int window, cudaStream_t stream) {
     int steps = 1;
     while (2 * steps <= num_seqs) steps *= 2;
     const int wide = ql_t % 4 == 0 && ql_h % 4 == 0 && (uintptr_t)q_lat % 16 == 0;
     const LatentArgs p{q_lat, ql_t, ql_h, (const __nv_bfloat16*)q, q_stride, q_head_width, q_rot_offset, freq, magnitude, sink,
-                       (const __nv_bfloat16*)k_pool, geo, block_table, table_width, positions, cu_q, num_seqs, steps, (__nv_bfloat16*)out,
+                       (const __nv_bfloat16*)k_pool, geo, block_table, table_width, positions, seq_of_token, cu_q, num_seqs, steps, (__nv_bfloat16*)out,
                        heads, rot, scale, window, wide};
     const dim3 grid(num_tokens / TOKENS + 2 * num_seqs, (heads + HEADS - 1) / HEADS);
     const size_t smem = latent_tokens_smem(rank, rot);

@@ -75,6 +75,8 @@ class StepContext:
         # True: the step is captured into a CUDA graph or replayed from one, so a part must launch the same kernels on
         # buffers of the same sizes whatever the step holds; False: it runs once, and `host` says exactly what it holds
         self.replayed = False
+        # steps with prompt portions of up to so many tokens in all may be replayed; larger ones never are
+        self.replay_limit = runner.graph_max_tokens if runner is not None and runner.cuda_graphs else 0
 
     def binding(self, entry: RunEntry) -> EntryBinding | None:
         base = self._runner.bindings[entry.cache_entry]

@@ -25,12 +25,15 @@ sizes allow (bfloat16, key and value heads of one size the tcgen05 prompt kernel
 latents the portions see, their whole contexts or what a window leaves, are gathered from the pages (their rotated parts, one for
 all heads, go to the kernel as they lie), a head's keys and values are worked out for the step ([K | V] = C [W_uk; W_uv]^T, one
 product, behind a window with keys of two pieces: a quarter of the folded form's arithmetic at a latent of 512 channels and heads of 128) and the tcgen05 prompt kernel
-attends over them; requests that feed one token in the same step stay on the folded form.  The two ways differ by rounding only.
+attends over them; requests that feed one token in the same step stay on the folded form, and so do, behind a window, portions that a
+replayed step may hold or that see many keys for their tokens.  The two ways differ by rounding only.
 
 Tensors (local names): dq, dq.norm, uq (or q), dkv, dkv.norm, uk, uv, o, g with an output gate, sink.
 """
 
 from __future__ import annotations
+
+import copy
 
 import torch
 
@@ -39,8 +42,8 @@ from tinyserve_llm_b200.parts.base import KVNeed, Mixer, Runtime, TensorDecl, pa
 from tinyserve_llm_b200.parts.linear import Linear, fuse_rows
 
 MAX_KV_RANK = 512       # csrc/attention_latent.cu: 16 output channels a lane
-MATERIALIZE_MIN_TOKENS = 128    # prompt portions of a step, together, from which keys and values are worked out for the step
-MATERIALIZE_MAX_KEYS = 32       # with a window: keys a token fed, over all portions, up to which they are (16 heads, 160 .. 290 tokens behind
+MATERIALIZE_MIN_TOKENS = 128    # prompt portions of a step, together (with a window: each), from which keys and values are worked out for the step
+MATERIALIZE_MAX_KEYS = 32       # with a window: keys a token a portion feeds, up to which they are (16 heads, 160 .. 290 tokens behind
                                 # windows of 1,024, us folded / unfolded: 172 / 149 at 23 keys, 179 / 172 at 48, 163 / 336 at 95)
 
 
@@ -126,38 +129,53 @@ class LatentAttention(Mixer):
         return KVNeed(1, self.spec.kv_rank + self.spec.rot_dim, self.spec.window, values=False)
 
     # ------------------------------------------------------------------ prompt portions on keys and values of their own
-    def _portions(self, q: torch.Tensor, ctx) -> list[int] | None:
-        """How many keys each of the step's prompt portions sees, if they are to attend over keys and values worked out for the step."""
+    def unfolded_requests(self, q: torch.Tensor, ctx) -> list[int]:
+        """
+        The requests whose prompt portions attend over keys and values worked out for the step.  With a window that follows from the portion
+        alone, its tokens and the keys the window leaves it, so that a row's form does not depend on what else is in the step: a portion
+        that a step replayed from a graph may hold stays on the folded form, which such a step takes, in every step.
+        """
         spec, host, ops = self.spec, getattr(ctx, "host", None), self.rt.ops
         # (small steps leave first: they are bound by the host)
         if (host is None or host.cu_q[-1] < MATERIALIZE_MIN_TOKENS or getattr(ctx, "replayed", True) or ctx.max_q_len <= 1
                 or self.uk_uv is None or (spec.window and not spec.rot_dim)
                 or not ops.dense_prompt_attention_supported(q, spec.num_heads, spec.num_heads, spec.head_dim)):
-            return None
+            return []
         # (windows come in the kernel's form with a rotated part, whose queries, keys and probabilities have the folded form's precision)
         lens = [b - a for a, b in zip(host.cu_q, host.cu_q[1:])]
-        fed = sum(n for n in lens if n > 1)
-        if fed < MATERIALIZE_MIN_TOKENS:
-            return None
-        keys = [ctx_len - ops.latent_first_key(ctx_len, n, spec.window) for n, ctx_len in zip(lens, host.ctx_lens) if n > 1]
-        if spec.window and sum(keys) > MATERIALIZE_MAX_KEYS * fed:
-            return None
-        return keys
+        portions = [s for s, n in enumerate(lens) if n > 1]
+        if not spec.window:
+            return portions if sum(lens[s] for s in portions) >= MATERIALIZE_MIN_TOKENS else []
+        least = max(MATERIALIZE_MIN_TOKENS, getattr(ctx, "replay_limit", 0) + 1)
+        return [s for s in portions if lens[s] >= least and self._keys_of(host, s) <= MATERIALIZE_MAX_KEYS * lens[s]]
+
+    def _keys_of(self, host, s: int) -> int:
+        """How many keys of a request are gathered for its portion."""
+        return host.ctx_lens[s] - self.rt.ops.latent_first_key(host.ctx_lens[s], host.cu_q[s + 1] - host.cu_q[s], self.spec.window)
 
     @staticmethod
-    def _single_tokens_only(ctx):
-        """The step's context with the tokens of prompt portions marked as padding rows: the folded form skips them."""
-        import copy
-        lens = ctx.cu_q[1:] - ctx.cu_q[:-1]
-        seqs = ctx.seq_of_token.long().clamp_min(0)
-        out = copy.copy(ctx)
-        out.max_q_len = 1
-        out.seq_of_token = torch.where((ctx.seq_of_token >= 0) & (lens[seqs] == 1), ctx.seq_of_token, -1).to(torch.int32)
-        return out
+    def _divided(ctx, unfolded: list[int]):
+        """The step's context for the folded form, tokens of the unfolded requests marked as padding rows (that form skips them), and for the unfolded one."""
+        host = ctx.host
+        lens = [b - a for a, b in zip(host.cu_q, host.cu_q[1:])]
+        rest = [n for s, n in enumerate(lens) if s not in set(unfolded)]
+        flags = torch.zeros(len(lens), dtype=torch.bool)
+        flags[unfolded] = True
+        flags = flags.pin_memory().to(ctx.cu_q.device, non_blocking=True)
+        of_token = flags[ctx.seq_of_token.long().clamp_min(0)]
+        folded, others = copy.copy(ctx), copy.copy(ctx)
+        folded.seq_of_token = torch.where(of_token, -1, ctx.seq_of_token)
+        folded.min_q_len, folded.max_q_len = min(rest), max(rest)
+        listed = getattr(ctx, "prefill_seqs", None)
+        if any(n > 1 for n in rest):                     # portions on both forms
+            listed = torch.arange(len(lens), dtype=torch.int32, device=ctx.cu_q.device) if listed is None else listed
+            others.prefill_seqs = torch.where(flags[listed.long().clamp_min(0)], listed, -1)
+        return folded, others
 
-    def _attend_unfolded(self, q: torch.Tensor, ctx, binding, keys: list[int], out: torch.Tensor | None) -> torch.Tensor:
+    def _attend_unfolded(self, q: torch.Tensor, ctx, binding, unfolded: list[int], out: torch.Tensor | None) -> torch.Tensor:
         spec, ops = self.spec, self.rt.ops
         H, D, R, rank = spec.num_heads, spec.head_dim, spec.rot_dim, spec.kv_rank
+        keys = [self._keys_of(ctx.host, s) for s in unfolded]
         c, shared, odd, kv_start = ops.latent_gather(ctx, binding, sum(keys), max(keys), rank, R, spec.window, self.frequencies, self.magnitude)
         if not spec.window:
             kv, k_low = ops.linear(c, self.uk_uv), None     # [keys, H D | H D]
@@ -171,18 +189,18 @@ class LatentAttention(Mixer):
         """[T, H V] in q's dtype: the heads' outputs for queries q [T, H (D + R)], rotated here, over the cached rows [c | k_rot]."""
         spec, ops = self.spec, self.rt.ops
         H, D, R, V, rank = spec.num_heads, spec.head_dim, spec.rot_dim, spec.value_dim, spec.kv_rank
-        portions = self._portions(q, ctx)
-        if portions is not None and ctx.min_q_len > 1:
-            return self._attend_unfolded(q, ctx, binding, portions, None)
-        folded_ctx = ctx if portions is None else self._single_tokens_only(ctx)
+        unfolded = self.unfolded_requests(q, ctx)
+        if unfolded and len(unfolded) == len(ctx.host.ctx_lens):
+            return self._attend_unfolded(q, ctx, binding, unfolded, None)
+        folded_ctx, unfolded_ctx = self._divided(ctx, unfolded) if unfolded else (ctx, None)
         q_lat = ops.per_head_linear(q, self.uk_t, H, D + R, D)            # float32 [T, H, rank]: W_uk^T q_flat
         o_lat = ops.latent_attention(q_lat, q, folded_ctx, binding, H, D + R, D, rank, R, self.frequencies, spec.scale,
                                      spec.window, magnitude=self.magnitude, sink=self.sink)   # [T, H, rank]: softmax-weighted sums of c
         o = ops.per_head_linear(o_lat.view(-1, H * rank), self.uv, H, rank, rank, out_dtype=q.dtype)   # [T, H, V]
         o = o.reshape(-1, H * V)
-        if portions is None:
+        if not unfolded:
             return o
-        return self._attend_unfolded(q, ctx, binding, portions, o.contiguous())               # the portions' rows are written over
+        return self._attend_unfolded(q, unfolded_ctx, binding, unfolded, o.contiguous())      # those portions' rows are written over
 
     def forward(self, x: torch.Tensor, ctx, binding) -> torch.Tensor:
         spec, ops = self.spec, self.rt.ops
