@@ -655,3 +655,19 @@ def test_portions_of_both_forms_in_one_step(rank):
     _, others = attend([1, 2, 3])
     for got, want in zip((rows[1], rows[2], rows[3]), others):
         assert float((got.double() - want.double()).norm() / want.double().norm()) < 2.0 ** -9
+
+
+def test_queries_of_unfolded_portions_are_rotated_by_their_positions():
+    """A context's positions, which need not be the tokens' places among the keys."""
+    part, lens, page = _latent_part(2, 64, 24, 128, 100), [130, 1, 200], 64
+    ctx = make_ctx(lens, [150, 9, 200])
+    ctx.replayed, ctx.prefill_seqs = False, i32([0, 2])
+    ctx.positions += 1000
+    pool = torch.zeros(8, 1, 1, page, 152, dtype=torch.bfloat16, device="cuda")
+    binding = EntryBinding(pool, None, page * 152, 0, page, 8, i32([[0, 1, 2, -1], [3, -1, -1, -1], [4, 5, 6, 7]]), 4)
+    _, (turn, _), _, _ = get_ops().latent_gather(ctx, binding, 350, 200, 128, 24, 100, part.frequencies, 0.75)
+    angles = ctx.positions.double()[:, None] * part.frequencies.double()
+    for s, (a, b) in enumerate(((0, 130), (131, 331))):
+        want = 0.75 * torch.stack([angles[a:b].cos(), angles[a:b].sin()], dim=-1)
+        # an angle of up to 1,200 is a float32 product, within 2^-14 of itself; cosine and sine follow it
+        assert float((turn[a:b, :12].double() - want).abs().max()) < 2.0 ** -13

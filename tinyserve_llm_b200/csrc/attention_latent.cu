@@ -410,8 +410,8 @@ TS_API int ts_latent_attention(const float* q_lat, long long ql_token_stride, lo
 // The cached rows [c | k_rot] that a step's prompt portions see, page by page into matrices of their own for the unfolded form: c
 // [rows, rank] and k_rot [rows, rot], the portions one after another in the order of their list, each from the first key its first
 // query sees, rounded down to a key tile of the attention (WINDOW_TILE), to its last; kv_start[s] is key 0's row (negative where it lies
-// before).  With a rotated part, the cosines and sines of the portions' tokens go to turn [T, 32], from which the attention rotates
-// its queries.  With `odd` a row whose latent is not finite is written as zeros and marked (its values, zeros in the products, would
+// before).  With a rotated part, the cosines and sines of the portions' tokens, by their positions, go to turn [T, 32], from which the attention
+// rotates its queries.  With `odd` a row whose latent is not finite is written as zeros and marked (its values, zeros in the products, would
 // otherwise reach queries that do not see it as 0 times NaN).  A warp a row, 16 bytes a lane; bound by its launch and one round trip
 // (2,048 rows of 576: 5 us, where torch's indexing, two copies and the upload of kv_start took five launches).
 constexpr int WINDOW_TILE = 128, GATHER_WARPS = 8;
@@ -423,9 +423,10 @@ __device__ __forceinline__ int first_gathered(int ctx, int q_len, int window) {
 template <typename V>                                    // what a lane copies at a time: 16 bytes or an element
 __global__ void __launch_bounds__(GATHER_WARPS * 32)
 latent_gather_kernel(const __nv_bfloat16* __restrict__ pool, KVGeometry geo, const int* __restrict__ block_table, int table_width,
-                     const int* __restrict__ cu_q, const int* __restrict__ ctx_lens, const int* __restrict__ portions, int window, int rank,
-                     int rot, const float* __restrict__ freq, float magnitude, float2* __restrict__ turn, long long num_rows, __nv_bfloat16* __restrict__ c, __nv_bfloat16* __restrict__ k_rot, unsigned char* __restrict__ odd,
-                     int* __restrict__ kv_start) {
+                     const int* __restrict__ cu_q, const int* __restrict__ ctx_lens, const int* __restrict__ positions,
+                     const int* __restrict__ portions, int window, int rank, int rot, const float* __restrict__ freq, float magnitude,
+                     float2* __restrict__ turn, long long num_rows, __nv_bfloat16* __restrict__ c, __nv_bfloat16* __restrict__ k_rot,
+                     unsigned char* __restrict__ odd, int* __restrict__ kv_start) {
     constexpr int N = sizeof(V) / sizeof(__nv_bfloat16);
     const int seq = portions ? portions[blockIdx.y] : (int)blockIdx.y;
     if (seq < 0) return;
@@ -464,7 +465,7 @@ latent_gather_kernel(const __nv_bfloat16* __restrict__ pool, KVGeometry geo, con
         const int t = key - (ctx - q_len);               // the portion's token at this position
         if (t >= 0 && lane < rot / 2) {
             float sn, cs;
-            sincosf((float)key * freq[lane], &sn, &cs);
+            sincosf((float)positions[cu_q[seq] + t] * freq[lane], &sn, &cs);
             turn[(long long)(cu_q[seq] + t) * 32 + lane] = make_float2(cs * magnitude, sn * magnitude);
         }
         V zero;
@@ -477,12 +478,13 @@ latent_gather_kernel(const __nv_bfloat16* __restrict__ pool, KVGeometry geo, con
 }
 
 // `rows`: of the matrices (the keys of all portions, at most `max_keys` of one); portions [num_portions] or null (then every request,
-// of which those that feed one token are passed over); freq [rot / 2], turn [T, 32, 2] (rot 0: null); odd [rows] or null.
+// of which those that feed one token are passed over); positions [T], freq [rot / 2], turn [T, 32, 2] (rot 0: null); odd [rows] or null.
 TS_API int ts_latent_gather(const void* pool, long long page_stride, long long entry_offset, int page_tokens, int num_pages,
-                            const int* block_table, int table_width, const int* cu_q, const int* ctx_lens, const int* portions,
-                            int num_portions, int window, int max_keys, int rank, int rot, const float* freq, float magnitude,
+                            const int* block_table, int table_width, const int* cu_q, const int* ctx_lens, const int* positions,
+                            const int* portions, int num_portions, int window, int max_keys, int rank, int rot, const float* freq, float magnitude,
                             float* turn, long long rows, void* c, void* k_rot, unsigned char* odd, int* kv_start, cudaStream_t stream) {
-    TS_REQUIRE(rank > 0 && rot >= 0 && rot <= 64 && rot % 2 == 0 && (rot == 0 || (freq && turn)) && page_tokens > 0 && table_width > 0 && window >= 0, "latent_gather: bad sizes");
+    TS_REQUIRE(rank > 0 && rot >= 0 && rot <= 64 && rot % 2 == 0 && (rot == 0 || (freq && turn && positions)) && page_tokens > 0 &&
+               table_width > 0 && window >= 0, "latent_gather: bad sizes");
     TS_REQUIRE(num_portions >= 0 && num_portions <= 65535 && rows < 0x7fffffffll, "latent_gather: %d portions, %lld rows", num_portions, rows);
     if (num_portions == 0 || max_keys <= 0) return 0;
     const KVGeometry geo{page_stride, entry_offset, page_tokens, num_pages};
@@ -490,8 +492,9 @@ TS_API int ts_latent_gather(const void* pool, long long page_stride, long long e
     const bool wide = rank % 8 == 0 && rot % 8 == 0 && page_stride % 8 == 0 && entry_offset % 8 == 0 && (uintptr_t)pool % 16 == 0 &&
                       (uintptr_t)c % 16 == 0 && (uintptr_t)k_rot % 16 == 0;
     auto kernel = wide ? latent_gather_kernel<uint4> : latent_gather_kernel<__nv_bfloat16>;
-    kernel<<<grid, GATHER_WARPS * 32, 0, stream>>>((const __nv_bfloat16*)pool, geo, block_table, table_width, cu_q, ctx_lens, portions, window,
-                                                   rank, rot, freq, magnitude, (float2*)turn, rows, (__nv_bfloat16*)c, (__nv_bfloat16*)k_rot, odd, kv_start);
+    kernel<<<grid, GATHER_WARPS * 32, 0, stream>>>((const __nv_bfloat16*)pool, geo, block_table, table_width, cu_q, ctx_lens, positions,
+                                                   portions, window, rank, rot, freq, magnitude, (float2*)turn, rows, (__nv_bfloat16*)c,
+                                                   (__nv_bfloat16*)k_rot, odd, kv_start);
     TS_LAUNCH_CHECK("latent_gather");
     return 0;
 }

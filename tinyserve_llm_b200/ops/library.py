@@ -35,7 +35,7 @@ _SIGNATURES = {
     "ts_paged_attention_bf16_masked": ("int", "pl" "ppp" "lllliipippiiiiiiifiifi" "plpi" "fp"),
     "ts_attention_tcgen05_supported": ("int", "iiiii"),
     "ts_prefill_attention_tcgen05_dense": ("int", "pl" "ppp" "llpppiiiiiif" "ilppip" "ipplip" "p"),
-    "ts_latent_gather": ("int", "plliipipppiiiiipfplppppp"),
+    "ts_latent_gather": ("int", "plliipippppiiiiipfplppppp"),
     "ts_prefill_attention_tcgen05_masked": ("int", "pl" "ppp" "iiiipippiiiiiifiifi" "pipfp"),
     "ts_prefill_attention_tcgen05": ("int", "ppppiiiipippiiiiiifpipp"),
     "ts_prefill_attention_tcgen05_sigmoid": ("int", "pl" "ppp" "iiiipippiiiiiifi" "pppl" "pipp"),
@@ -929,8 +929,8 @@ class Ops:
                       magnitude: float = 1.0) -> tuple[torch.Tensor, tuple | None, torch.Tensor | None, torch.Tensor]:
         """
         The cached rows [c | k_rot] that the step's prompt portions see, gathered from the pages: (c [rows, rank], (turn, k_rot [rows,
-        rot]) or None for rot 0, odd uint8 [rows], kv_start int32 [requests]) for `dense_prompt_attention`, turn by `freq` [rot / 2] and
-        `magnitude`.  `rows`: of all portions together, at most `max_keys`
+        rot]) or None for rot 0, odd uint8 [rows], kv_start int32 [requests]) for `dense_prompt_attention`, turn by ctx.positions, `freq`
+        [rot / 2] and `magnitude`.  `rows`: of all portions together, at most `max_keys`
         of one: ctx_len - latent_first_key(...) each.  With a window, rows whose latent is not finite are zeros and marked in odd;
         without one they are copied as they are and odd is None.
         """
@@ -946,7 +946,7 @@ class Ops:
         kv_start = torch.empty((ctx.ctx_lens.shape[0],), dtype=torch.int32, device=pool.device)
         portions = getattr(ctx, "prefill_seqs", None)
         self._call("ts_latent_gather", _ptr(pool), binding.page_stride, binding.entry_offset, binding.page_tokens, binding.num_pages,
-                   _ptr(binding.block_table), binding.table_width, _ptr(ctx.cu_q), _ptr(ctx.ctx_lens), _ptr(portions),
+                   _ptr(binding.block_table), binding.table_width, _ptr(ctx.cu_q), _ptr(ctx.ctx_lens), _ptr(ctx.positions), _ptr(portions),
                    (portions if portions is not None else ctx.ctx_lens).shape[0], window, max_keys, rank, rot,
                    _ptr(freq) if rot else None, float(magnitude), _ptr(turn), rows, _ptr(c), _ptr(k_rot), _ptr(odd), _ptr(kv_start), _stream())
         return c, (turn, k_rot) if rot else None, odd, kv_start
