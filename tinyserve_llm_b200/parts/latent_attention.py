@@ -43,8 +43,11 @@ from tinyserve_llm_b200.parts.linear import Linear, fuse_rows
 
 MAX_KV_RANK = 512       # csrc/attention_latent.cu: 16 output channels a lane
 MATERIALIZE_MIN_TOKENS = 128    # prompt portions of a step, together (with a window: each), from which keys and values are worked out for the step
-MATERIALIZE_MAX_KEYS = 32       # with a window: keys a token a portion feeds, up to which they are (16 heads, 160 .. 290 tokens behind
-                                # windows of 1,024, us folded / unfolded: 172 / 149 at 23 keys, 179 / 172 at 48, 163 / 336 at 95)
+# With a window: keys a token a portion feeds, up to which they are.  The attention alone, heads of 128, latent of 512, us folded / unfolded, 8 heads
+# and 16: 128 tokens, 9 keys a token 115 / 71, 123 / 72; 33 keys 349 / 150, 410 / 170; 513 tokens, 9 keys 688 / 153, 693 / 172; 2,048 tokens, 3 keys
+# 2,693 / 164, 2,728 / 327.  Beyond that the latents gathered for few tokens cost more than they save (three portions of 160 .. 290 tokens, windows
+# of 1,024: 163 / 336 at 95 keys a token fed).
+MATERIALIZE_MAX_KEYS = 32
 
 
 def evens_then_odds(rows: torch.Tensor) -> torch.Tensor:
