@@ -7,7 +7,7 @@ import torch
 
 from gpu_util import i32, make_ctx
 from tinyserve_llm_b200.cache.storage import EntryBinding
-from tinyserve_llm_b200.ops import get_ops
+from tinyserve_llm_b200.ops import KernelError, get_ops
 from tinyserve_llm_b200.parts.delta_rule import CHANNEL_TILE_TOKENS
 from tinyserve_llm_b200.parts.recurrence import TILE_TOKENS
 
@@ -671,3 +671,33 @@ def test_queries_of_unfolded_portions_are_rotated_by_their_positions():
         want = 0.75 * torch.stack([angles[a:b].cos(), angles[a:b].sin()], dim=-1)
         # an angle of up to 1,200 is a float32 product, within 2^-14 of itself; cosine and sine follow it
         assert float((turn[a:b, :12].double() - want).abs().max()) < 2.0 ** -13
+
+
+@pytest.mark.parametrize("kind", ["delta", "channel"])
+def test_a_delta_walk_whose_wait_runs_out_stores_nothing(kind):
+    """A limit of no time at all: every CTA gives up at its first tile, waits for its copies, and leaves the state as it was."""
+    ops, H, D, lens = get_ops(), 2, 64, [40, 17, 1, 2]
+    g = torch.Generator().manual_seed(1)
+    T = sum(lens)
+    y, z, b, gates = (torch.randn(T, n, generator=g).cuda() for n in (3 * H * D, H * D, H, 2 * H))
+    per_head, per_channel = torch.zeros(H).cuda(), torch.zeros(H * D).cuda()
+    state = torch.randn(len(lens) + 3, H * D * D, generator=g).cuda()
+    sizes = dict(heads=H, kv_heads=H, dim=D, vdim=D, unit_eps=1e-6, q_scale=0.25)
+    parts, held, results = y.split(H * D, dim=1), state.clone(), []
+    for limit in ({"wait_cycles": 0}, {}, {}):
+        ctx, binding = _step(held, lens)
+        if kind == "delta":
+            results.append(ops.delta_tiles(*parts, gates, per_head, per_head, ctx, binding, **sizes, **limit))
+        else:
+            results.append(ops.channel_tiles(*parts, z, b, per_channel, per_head, ctx, binding, **sizes, **limit))
+        torch.cuda.synchronize()
+        if limit:
+            assert torch.equal(held, state)
+            with pytest.raises(KernelError, match="delta_tiles"):
+                ops.check_device_errors()
+        else:
+            assert not torch.equal(held, state)
+            ops.check_device_errors()
+            held = state.clone()
+    rows = [t for s, n in enumerate(lens) for t in range(sum(lens[:s]), sum(lens[:s + 1])) if n > 1]
+    assert torch.equal(results[1][rows], results[2][rows])

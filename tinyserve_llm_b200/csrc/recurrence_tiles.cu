@@ -430,7 +430,7 @@ struct ScanArgs {
     float* state; long long slot_stride;                 // floats between slots; a slot holds [heads, dim, vdim]
     float* out;                                          // [tokens, heads * vdim] float32
     int heads, qk_group, dim, vdim;
-    int* error;                                          // the delta rules' walk: where a wait that ran out says so
+    int* error; long long wait_cycles;                   // the delta rules' walk: where a wait that ran out says so, and when it does
 };
 
 // Numbers from here on have no split (their hi would be infinite).
@@ -646,7 +646,8 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
 // against S_0, its sum over the warps, U, the update.  What it does not wait for is beside it: the q side's product runs while two warps
 // without rows make U and two more (P W) (V - R), and those sum up and store the output under the update and the next tile's k side.
 // Packs and coefficients come by bulk copies, two tiles in shared memory.  Every wait for them gives up after about two seconds and says
-// so in an error word; the CTA then goes on with what is there.
+// so in an error word; the CTA then stores nothing of that tile and the later ones, leaves the state as it was, waits once more, as long, for
+// the copies on their way (the shared memory they write will be another CTA's) and returns.
 // Bound by the chain.  Three portions of 1,001, 667 and 333 tokens, 8 heads of 128 x 128: 86 us, where four warps that did both sides
 // before U, made U and O and copied the tiles themselves took 100.
 constexpr int DELTA_WARPS = 8, HELPERS = 4, HOLDERS = DELTA_WARPS * 32, DELTA_THREADS = HOLDERS + HELPERS * 32;
@@ -660,6 +661,7 @@ __global__ void __launch_bounds__(DELTA_THREADS) delta_tiles_kernel(ScanArgs p) 
     static_assert(MODE == DELTA || MODE == CHANNEL, "the delta rules");
     extern __shared__ __align__(16) float smem[];
     __shared__ __align__(8) uint64_t full[2];
+    __shared__ int failed;
     float* red_k = smem + 2 * STAGE;                     // [DELTA_WARPS][B][RP], and of the q side
     float* red_q = red_k + SUMS;
     float* X_s = red_q + SUMS;                           // [B][RP]: V - R; (P W) of it
@@ -704,17 +706,17 @@ __global__ void __launch_bounds__(DELTA_THREADS) delta_tiles_kernel(ScanArgs p) 
     const long long v_step = B * p.v_stride, token_step = (long long)p.heads * p.vdim;
     auto fetch_v = [&](int tile) { return holds && in_columns && tile * B + tx < n ? v[tile * v_step] : 0.f; };
     if (tid == 0) {
+        failed = 0;
         mbar_init(&full[0], 1);
         mbar_init(&full[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         issue(0);
     }
     float vnow = fetch_v(0);
-    bool ok = true;
     for (int tile = 0; tile < tiles; ++tile) {
         __syncthreads();                                 // the barriers exist; the other stage, U and the sums have been read
         if (tid == 0 && tile + 1 < tiles) issue(tile + 1);
-        ok = ok && mbar_wait(&full[tile & 1], tile >> 1 & 1, p.error, holds ? 31 : 32);
+        if (!mbar_wait(&full[tile & 1], tile >> 1 & 1, p.error, holds ? 31 : 32, p.wait_cycles)) failed = 1;
         float vnext = 0.f;
         if (tile + 1 < tiles) vnext = fetch_v(tile + 1);
         const float* pack = smem + (tile & 1) * STAGE;
@@ -746,6 +748,7 @@ __global__ void __launch_bounds__(DELTA_THREADS) delta_tiles_kernel(ScanArgs p) 
         };
         if (holds) against_state(pack + B * PP, red_k);
         __syncthreads();                                 // the k side's partial sums are in
+        const int gone = failed;                         // the same in all threads; looked at where its load has long come back
         if (holds) {
             float sum = 0.f;
 #pragma unroll
@@ -776,6 +779,10 @@ __global__ void __launch_bounds__(DELTA_THREADS) delta_tiles_kernel(ScanArgs p) 
             }
         }
         __syncthreads();                                 // what the update takes is in, and all of the output
+        if (gone) {
+            for (int t = tile; tid == 0 && t < tiles && t < tile + 2; ++t) mbar_wait(&full[t & 1], t >> 1 & 1, p.error, 31);
+            return;
+        }
         if (holds) {                                     // S^T <- decay S^T + G^T K: the state after the tile
             SplitA a[2];
 #pragma unroll
@@ -868,7 +875,7 @@ TS_API int ts_delta_tiles(const float* q, const float* k, long long qk_stride, c
                           const float* a_log, const float* v, long long v_stride, const int* cu_q, const int* slots,
                           const int* prefill_seqs, int portions, int max_q_len, float* state, long long slot_stride,
                           float* pack, float* coef, float* out, int heads, int kv_heads, int dim, int vdim,
-                          float unit_eps, float q_scale, int* error, cudaStream_t stream) {
+                          float unit_eps, float q_scale, int* error, long long wait_cycles, cudaStream_t stream) {
     TS_REQUIRE(error != nullptr, "delta_tiles: an error word is needed");
     TS_REQUIRE(heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && dim > 0 && dim <= 256 && vdim > 0,
                "delta_tiles: %d heads over %d q/k heads of %d channels", heads, kv_heads, dim);
@@ -880,7 +887,7 @@ TS_API int ts_delta_tiles(const float* q, const float* k, long long qk_stride, c
     const size_t smem = sizeof(float) * (2 * B * (a.rows + 1) + 2 * B * (B + 1));
     delta_tile_prepare_kernel<<<dim3((max_q_len + B - 1) / B, kv_heads, portions), 128, smem, stream>>>(a);
     TS_LAUNCH_CHECK("delta_tiles (prepare)");
-    ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, heads / kv_heads, dim, vdim, error};
+    ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, heads / kv_heads, dim, vdim, error, wait_cycles};
     return launch_scan<float, DELTA>(s, portions, stream);
 }
 
@@ -897,7 +904,7 @@ TS_API int ts_mix_tiles(const void* r, const void* k, long long rk_stride, const
     PrepareArgs a{r, k, rk_stride, z, w0, u, cu_q, prefill_seqs, pack, coef, heads, heads, dim, padded_rows(dim), 0.f, 1.f};
     const size_t smem = sizeof(float) * (3 * B * (a.rows + 1));
     const dim3 grid((max_q_len + B - 1) / B, heads, portions);
-    ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, dim, nullptr};
+    ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, dim, nullptr, 0};
     if (dtype == TS_F32) {
         cudaFuncSetAttribute(mix_tile_prepare_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         mix_tile_prepare_kernel<float><<<grid, 128, smem, stream>>>(a);
@@ -942,7 +949,7 @@ TS_API int ts_plain_tiles(const void* q, const void* k, const void* v, long long
     const int rows = padded_rows(dim);
     const size_t smem = rows == 64 ? PlainTile<64>::BYTES : rows == 128 ? PlainTile<128>::BYTES : PlainTile<256>::BYTES;   // 29 KB at 128 channels
     const dim3 grid((max_q_len + B - 1) / B, heads, portions);
-    const ScanArgs s{a.pack, a.coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, vdim, nullptr};
+    const ScanArgs s{a.pack, a.coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, vdim, nullptr, 0};
     auto kernel = rows == 64 ? plain_tile_prepare_kernel<64> : rows == 128 ? plain_tile_prepare_kernel<128> : plain_tile_prepare_kernel<256>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     kernel<<<grid, 128, smem, stream>>>(a);
@@ -956,7 +963,7 @@ TS_API int ts_channel_tiles(const float* q, const float* k, long long qk_stride,
                             int b_dtype, const float* dt_bias, const float* a_log, const float* v, long long v_stride,
                             const int* cu_q, const int* slots, const int* prefill_seqs, int portions, int max_q_len, float* state,
                             long long slot_stride, float* pack, float* coef, float* out, int heads, int kv_heads, int dim,
-                            int vdim, float unit_eps, float q_scale, int* error, cudaStream_t stream) {
+                            int vdim, float unit_eps, float q_scale, int* error, long long wait_cycles, cudaStream_t stream) {
     TS_REQUIRE(error != nullptr, "channel_tiles: an error word is needed");
     TS_REQUIRE(heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && dim > 0 && dim <= 256 && vdim > 0,
                "channel_tiles: %d heads over %d q/k heads of %d channels", heads, kv_heads, dim);
@@ -980,6 +987,6 @@ TS_API int ts_channel_tiles(const float* q, const float* k, long long qk_stride,
     else TS_CHANNEL_PREPARE(__nv_bfloat16);
 #undef TS_CHANNEL_PREPARE
     TS_LAUNCH_CHECK("channel_tiles (prepare)");
-    const ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, vdim, error};
+    const ScanArgs s{pack, coef, v, v_stride, cu_q, slots, prefill_seqs, state, slot_stride, out, heads, 1, dim, vdim, error, wait_cycles};
     return launch_scan<float, CHANNEL>(s, portions, stream);
 }

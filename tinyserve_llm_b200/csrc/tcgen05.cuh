@@ -19,22 +19,21 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// false: the wait ran out of time (the error word says which one)
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* error, int code) {
+// false: the wait ran out of time (the error word says which one); with a limit of 0 it does so without a look
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* error, int code, long long limit = WAIT_CYCLES) {
     const long long start = clock64();
     uint32_t done = 0;
-    while (true) {
+    while (limit > 0) {
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
             "selp.u32 %0, 1, 0, p;\n\t}"
             : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
         if (done) return true;
-        if (clock64() - start > WAIT_CYCLES) {
-            atomicExch(error, code);
-            return false;
-        }
+        if (clock64() - start > limit) break;
     }
+    atomicExch(error, code);
+    return false;
 }
 
 __device__ __forceinline__ void tma_load_2d(void* smem, const CUtensorMap* map, uint64_t* bar, int x, int y) {

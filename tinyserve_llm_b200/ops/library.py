@@ -97,11 +97,11 @@ _SIGNATURES = {
     "ts_time_mix_prepare": ("int", "pplppppp" "iiipippiplipip"),
     "ts_recurrence_tiles_pack_floats": ("long long", "iiiii"),
     "ts_recurrence_tiles_coef_floats": ("long long", "iii"),
-    "ts_delta_tiles": ("int", "pplppppl" "pppii" "plppp" "iiiiffpp"),
+    "ts_delta_tiles": ("int", "pplppppl" "pppii" "plppp" "iiiiffplp"),
     "ts_mix_tiles": ("int", "pplppppl" "pppii" "plppp" "iiip"),
     "ts_plain_tiles": ("int", "ppplll" "plpp" "fffpip" "pppiiii" "plpp" "iiiip"),
     "ts_plain_tiles_floats": ("long long", "iiiiii"),
-    "ts_channel_tiles": ("int", "pplpplipp" "pl" "pppii" "plppp" "iiiiffpp"),
+    "ts_channel_tiles": ("int", "pplpplipp" "pl" "pppii" "plppp" "iiiiffplp"),
     "ts_delta_prepare": ("int", "pplppppl" "ppiiiiff" "ppip"),
     "ts_mlstm_prepare": ("int", "ppllpplppffppiplpppiiiip"),
     "ts_row_scaled_activation": ("int", "ppppiiiip"),
@@ -110,6 +110,8 @@ _SIGNATURES = {
 }
 _CTYPES = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_longlong, "f": ctypes.c_float}
 _RETURNS = {"int": ctypes.c_int, "long long": ctypes.c_longlong, "void": None, "const char*": ctypes.c_char_p}
+
+TILE_WAIT_CYCLES = 4_000_000_000    # about two seconds at 2 GHz
 
 # Where a bounded wait inside a kernel gave up, by the code it left in the error word.
 _WAIT_CODES: dict[int, tuple[str, str]] = {
@@ -1172,11 +1174,12 @@ class Ops:
 
     def delta_tiles(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gates: torch.Tensor, dt_bias: torch.Tensor,
                     a_log: torch.Tensor, ctx, binding, *, heads: int, kv_heads: int, dim: int, vdim: int, unit_eps: float,
-                    q_scale: float) -> torch.Tensor:
+                    q_scale: float, wait_cycles: int = TILE_WAIT_CYCLES) -> torch.Tensor:
         """
         `delta_prepare_head` and its scan for the step's prompt portions, sixteen tokens at a time: float32
         [T, heads * vdim], of which the rows of requests that feed one token are left unwritten.  q, k, v float32
-        stretches after the convolution, gates [T, 2 heads].
+        stretches after the convolution, gates [T, 2 heads].  A wait for a tile gives up after `wait_cycles` clock cycles: the error
+        word says so, and the request's state is left as it was.
         """
         T = q.shape[0]
         for t, name, cols in ((q, "q", kv_heads * dim), (k, "k", kv_heads * dim), (v, "v", heads * vdim)):
@@ -1191,17 +1194,17 @@ class Ops:
         self._call("ts_delta_tiles", _ptr(q), _ptr(k), q.stride(0), _ptr(gates), _ptr(dt_bias), _ptr(a_log), _ptr(v), v.stride(0),
                    _ptr(ctx.cu_q), _ptr(binding.state_slots), _ptr(ctx.prefill_seqs), ctx.prefill_seqs.shape[0], ctx.max_q_len,
                    state.data_ptr(), stride, pack, coef, _ptr(out), heads, kv_heads, dim, vdim, unit_eps, q_scale,
-                   self.error_word().data_ptr(), _stream())
+                   self.error_word().data_ptr(), wait_cycles, _stream())
         self.launches += 1                                   # what the columns of a tile share, then the scan
         return out
 
     def channel_tiles(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tensor, b: torch.Tensor, dt_bias: torch.Tensor,
                       a_log: torch.Tensor, ctx, binding, *, heads: int, kv_heads: int, dim: int, vdim: int, unit_eps: float,
-                      q_scale: float) -> torch.Tensor:
+                      q_scale: float, wait_cycles: int = TILE_WAIT_CYCLES) -> torch.Tensor:
         """
         `delta_prepare` and its scan for the step's prompt portions, sixteen tokens at a time: float32 [T, heads * vdim], of
         which the rows of requests that feed one token are left unwritten.  q, k, v float32 stretches after the convolution,
-        z float32 [T, heads * dim] and b [T, heads] the logits of the decays and the step sizes.
+        z float32 [T, heads * dim] and b [T, heads] the logits of the decays and the step sizes.  `wait_cycles`: as in `delta_tiles`.
         """
         T = q.shape[0]
         for t, name, cols in ((q, "q", kv_heads * dim), (k, "k", kv_heads * dim), (v, "v", heads * vdim)):
@@ -1218,7 +1221,7 @@ class Ops:
         self._call("ts_channel_tiles", _ptr(q), _ptr(k), q.stride(0), _ptr(z), _ptr(b), b.stride(0), _DTYPE_CODE[b.dtype], _ptr(dt_bias),
                    _ptr(a_log), _ptr(v), v.stride(0), _ptr(ctx.cu_q), _ptr(binding.state_slots), _ptr(ctx.prefill_seqs),
                    ctx.prefill_seqs.shape[0], ctx.max_q_len, state.data_ptr(), stride, pack, coef, _ptr(out), heads,
-                   kv_heads, dim, vdim, unit_eps, q_scale, self.error_word().data_ptr(), _stream())
+                   kv_heads, dim, vdim, unit_eps, q_scale, self.error_word().data_ptr(), wait_cycles, _stream())
         self.launches += 1                                   # what the columns of a tile share, then the scan
         return out
 
