@@ -141,6 +141,21 @@ def test_float32_matrix_product_on_split_operands(ops, m, n, k):
     ops.check_device_errors()
 
 
+@pytest.mark.parametrize("m, n, k", [(16, 2048, 2048), (17, 2048, 2048), (100, 3000, 1024), (530, 64, 65536)])
+def test_float32_matrix_product_repeats_itself(ops, m, n, k):
+    """Operands that one CTA of a pair brings for the other's MMAs: rows one CTA splits by itself, rows split before, more rows than are split at a time."""
+    x, w = rand((m, k), torch.float32, 5).to(DEV), rand((n, k), torch.float32, 6).to(DEV)
+    x[0, 3], x[m - 1, k - 1] = math.inf, math.nan
+    got = ops.linear(x, w)
+    assert torch.equal(got[0].isfinite(), torch.zeros(n, dtype=torch.bool, device=DEV)) and got[m - 1].isnan().all() and got[1:m - 1].isfinite().all()
+    for _ in range(30):
+        assert torch.equal(ops.linear(x, w)[1:m - 1], got[1:m - 1])
+    for a in (1, (m - 13) // 2, m - 14):
+        assert torch.equal(ops.linear(x[a:a + 13].contiguous(), w), got[a:a + 13])
+    torch.cuda.synchronize()
+    ops.check_device_errors()
+
+
 @pytest.mark.parametrize("k", [4, 16, 32, 60, 64, 128, 2048])
 def test_float32_matrix_product_is_no_further_off_than_the_multiply_add_chain(ops, k):
     """The chain takes weights that begin off a 16-byte boundary.  A row of one 1 gives short sums' weights as they are."""

@@ -299,11 +299,6 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
 // the epilogue warps of both.  A cluster barrier after the barriers' initialisation keeps either CTA
 // from signalling a barrier that does not exist yet, another before the tensor memory is given back
 // keeps either from leaving while the other still reads its shared memory.
-__device__ __forceinline__ void tma_load_2d_pair(void* smem, const CUtensorMap* map, uint32_t bar_in_first, int x, int y) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(smem_u32(smem)), "l"(map), "r"(bar_in_first), "r"(x), "r"(y) : "memory");
-}
 __device__ __forceinline__ void umma_pair(uint32_t leader, uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"

@@ -67,7 +67,7 @@ long long sgemm_tcgen05_scratch_floats(int M, int N, int K);
 int sgemm_tcgen05(const float* x, const float* w, float* y, int M, int N, int K, long long ldx, long long ldw, long long ldy,
                   float* scratch, int* error, cudaStream_t stream);
 
-// Floats of scratch `ts_sgemm_nt` may use for rows without gaps (sgemm_tcgen05.cu).
+// Floats of scratch `ts_sgemm_nt` uses for rows without gaps (sgemm_tcgen05.cu), 16-byte aligned.
 TS_API long long ts_sgemm_nt_scratch_floats(int M, int N, int K) {
     return M > 0 && N > 0 && sgemm_tcgen05_supported(nullptr, nullptr, K, K, K) ? sgemm_tcgen05_scratch_floats(M, N, K) : 0;
 }
@@ -80,7 +80,8 @@ TS_API int ts_sgemm_nt(const float* A, const float* B, float* C, int M, int N, i
     TS_REQUIRE(lda >= K && ldb >= K && ldc >= N, "sgemm: row strides smaller than the rows");
     if (M == 0) return 0;
     if (error && sgemm_tcgen05_supported(A, B, K, lda, ldb)) {
-        TS_REQUIRE(scratch_floats >= sgemm_tcgen05_scratch_floats(M, N, K), "sgemm: %lld floats of scratch are too few", scratch_floats);
+        TS_REQUIRE(scratch_floats >= sgemm_tcgen05_scratch_floats(M, N, K) && (uintptr_t)scratch % 16 == 0,
+                   "sgemm: %lld floats of scratch are too few, or not aligned", scratch_floats);
         return sgemm_tcgen05(A, B, C, M, N, K, lda, ldb, ldc, scratch, error, stream);
     }
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);

@@ -11,22 +11,25 @@
 // A row's result does not depend on what else is in the batch: the blocks of k, the segments k is cut into and the order
 // they are added up in follow from N and K alone, and the rows' tile (the MMA's N side) does not enter an element's sum.
 //
-// Two CTAs a tile (`cta_group::2`): 256 rows of W, 128 in each CTA (the MMA's lanes), against BX rows of x, of which each CTA loads and
-// splits half; the first CTA's thread issues the MMAs for both.  Per CTA: warp 0 issues TMA loads into a ring of raw tiles, warp 1 the
-// MMAs, warps 4..11 split (two teams, a block each): a thread puts its row of W into tensor memory as hi and lo (the MMA's A
-// operand, so that neither passes through shared memory again) and its share of x into two swizzled tiles; the warps from 12
-// on add the blocks' sums up.
-// mbarriers: `raw_full` / `raw_empty` TMA <-> split, `ready` / `free` split <-> MMA, `sum_full` / `sum_empty` MMA <-> adders; `ready` and
-// `sum_empty` are the first CTA's, on which both CTAs' warps arrive, `free` and `sum_full` are signalled in both.
+// Two CTAs a tile (`cta_group::2`): 256 rows of W, 128 in each CTA (the MMA's lanes), against BX rows of x, half in each CTA; the first CTA's
+// thread issues the MMAs for both.  x is split into two matrices by a kernel ahead.  Per CTA: warp 0 issues TMA loads into a ring of raw
+// tiles of W, warp 2 those of x's two tiles, warp 1 the MMAs, warps 4..11 split W (two teams, a block each): a thread puts its row into
+// tensor memory as hi and lo (the MMA's A operand, so that neither passes through shared memory again); the warps from 12 on add the blocks'
+// sums up.
+// mbarriers: `raw_full` / `raw_empty` TMA <-> split, `ready` / `free` split and TMA of x <-> MMA, `sum_full` / `sum_empty` MMA <-> adders; `ready`
+// and `sum_empty` are the first CTA's, on which both CTAs' warps arrive, `free` and `sum_full` are signalled in both.
+// Split warps that wrote x's tiles would have to release each block's at cluster scope for MMAs the other CTA issues: 33 -> 50 us in the first
+// row below at 1 row, 45 -> 57 at 100 (released by warps of their own 42 and 53).  Up to 16 rows the first CTA holds all of them, splits them itself, with
+// no such order, and the second one's half is zeros (LOCAL): a kernel less, 2.5 us.
 // K is cut into segments, enough of them that the tiles of W times the segments fill the SMs.  Where there are rows of x enough
 // to fill them anyway a pair takes the segments one after another and adds each one's sum to y; else each segment is a pair's
 // work, its sums go to scratch, and a second kernel adds them up in the same order.
 // Measured on a B200, products with cold weights one after another, us: sgemm.cu, this product with one CTA a tile and the MMAs issued by
 // one lane, and now:
 //   rows of x             1                8               100              300             512             1,024
-//   16,384 x 2,048   192 / 53 / 32   192 / 53 / 32    306 / 63 / 45     - / 170 / 128   - / 222 / 177    - / 405 / 333
-//   2,048 x 8,192                    677 / 29 / 19    636 / 36 / 28     -  / 89 / 65    - / 118 / 90     - / 275 / 177
-//   3,072 x 2,048                                                                     241 /  86 / 46     - / 115 / 91
+//   16,384 x 2,048   192 / 53 / 34   192 / 53 / 35    306 / 63 / 48     - / 170 / 127   - / 222 / 174    - / 405 / 331
+//   2,048 x 8,192                    677 / 29 / 21    636 / 36 / 31     -  / 89 / 70    - / 118 / 96     - / 275 / 186
+//   3,072 x 2,048                                                     241 /  86 / 37     - / 115 / 48
 // A block of k took 0.75 to 0.93 us whatever BX was: 12 MMAs issued by one lane are 58 cycles each at the least (elect_one), and x's
 // tile, loaded and split whole by every CTA, moved more bytes through shared memory than W's.  Now 0.48 (BX 32), 0.57 (64) and 0.68 us
 // (128), of which the MMAs at the tensor cores' rate are 0.1, 0.22 and 0.41; W's stream alone takes 30 us in the first row.  What is left
@@ -38,7 +41,7 @@
 namespace {
 
 constexpr int BW = 128, BK = 32;                     // rows of W a CTA, half of a tile; k a block: 128 bytes, one swizzled row
-constexpr int SPLIT_WARPS = 4, SPLITS_FROM = 4, ADDERS_FROM = SPLITS_FROM + 2 * SPLIT_WARPS;    // two teams of split warps
+constexpr int X_WARP = 2, SPLIT_WARPS = 4, SPLITS_FROM = 4, ADDERS_FROM = SPLITS_FROM + 2 * SPLIT_WARPS;    // two teams of split warps
 __host__ __device__ constexpr int share_of(int bx) { return bx >= 64 ? 4 : 2; }           // adder warps a quarter of the lanes
 __host__ __device__ constexpr int threads_of(int bx) { return 32 * (ADDERS_FROM + 4 * share_of(bx)); }
 constexpr int W_BYTES = BW * BK * 4;
@@ -80,6 +83,11 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
 // the largest number hi is infinite and the rest NaN, and for a NaN the rest is one, so the sum never hides either.
 __device__ __forceinline__ float to_tf32(float v) { return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u); }
 
+__device__ __forceinline__ void split_four(float4 v, float4& hi, float4& lo) {
+    hi = make_float4(to_tf32(v.x), to_tf32(v.y), to_tf32(v.z), to_tf32(v.w));
+    lo = make_float4(v.x - hi.x, v.y - hi.y, v.z - hi.z, v.w - hi.w);
+}
+
 struct Item { int n0, m0, segment, first, count; };    // a pair's piece of work: a tile and the blocks of k it takes
 __device__ __forceinline__ Item item_of(const SgemmParams& p, int item, int bx) {
     const int n_tiles = (p.N + 2 * BW - 1) / (2 * BW), m_tiles = (p.M + bx - 1) / bx;
@@ -94,24 +102,27 @@ __device__ __forceinline__ Item item_of(const SgemmParams& p, int item, int bx) 
 
 // A persistent CTA an SM: the four kinds of warps walk over the same items, each counting blocks (g) over all of them, so that
 // the loads and MMAs of an item run under the sums of the one before.
-template <int BX, int RING, int PAIRS, int SUMS>
+// LOCAL: x's rows (raw, map_hi) fill at most the first CTA's half of the tile, which splits them itself; the second one's half is zeros.
+template <int BX, int RING, int PAIRS, int SUMS, bool LOCAL>
 __global__ void __launch_bounds__(threads_of(BX), 1)
-sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, SgemmParams p) {
-    constexpr int X_BYTES = BX / 2 * BK * 4, RAW_BYTES = W_BYTES + X_BYTES;           // ring of [W | x]; PAIRS of [x hi | x lo]: this CTA's half
+sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
+                     SgemmParams p) {
+    // RING of W (LOCAL: and x); PAIRS of [x hi | x lo], this CTA's half of the rows
+    constexpr int X_BYTES = BX / 2 * BK * 4, RAW_BYTES = W_BYTES + (LOCAL ? X_BYTES : 0);
     constexpr int A_COLS = SUMS * BX, TMEM_USED = A_COLS + PAIRS * 2 * BK;            // PAIRS of [W hi | W lo]
     constexpr int TMEM_COLS = TMEM_USED <= 256 ? 256 : 512;
     static_assert(TMEM_USED <= 512, "tensor memory has 512 columns");
     // a slot's barrier is waited on by one team only: the other could come to it a round early, where the parity it waits
     // for stands for the round before the first
     static_assert(RING % 2 == 0 && PAIRS % 2 == 0, "a ring slot and a pair of operand tiles belong to one team");
-    static_assert(RAW_BYTES % 1024 == 0 && X_BYTES % 1024 == 0, "tiles lie on the swizzle's boundaries");
+    static_assert(W_BYTES % 1024 == 0 && X_BYTES % 1024 == 0, "tiles lie on the swizzle's boundaries");
     constexpr int OWN = BX / share_of(BX);           // columns of an adder
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t raw_full_bar[RING], raw_empty_bar[RING], ready_bar[PAIRS], free_bar[PAIRS], sum_full_bar[SUMS], sum_empty_bar[SUMS];
     __shared__ uint32_t tmem_base_slot;
     __shared__ int failed;
     unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    unsigned char* split = ring + RING * RAW_BYTES;
+    unsigned char* x_tiles = ring + RING * RAW_BYTES;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = (int)pair_rank(), pair = blockIdx.x / 2, pairs = gridDim.x / 2;
 
@@ -121,7 +132,7 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             mbar_init(&raw_empty_bar[s], SPLIT_WARPS);
         }
         for (int b = 0; b < PAIRS; ++b) {
-            mbar_init(&ready_bar[b], 2 * SPLIT_WARPS);
+            mbar_init(&ready_bar[b], 2 * SPLIT_WARPS + (LOCAL ? 0 : 1));          // both CTAs' split warps, and x's bytes
             mbar_init(&free_bar[b], 1);
         }
         for (int b = 0; b < SUMS; ++b) {
@@ -140,9 +151,15 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_slot;
-    pair_sync();                                     // both CTAs' barriers exist
-    chain_wait();
-    chain_release();
+    if (LOCAL && rank) {
+        for (int e = threadIdx.x; e < PAIRS * 2 * X_BYTES / 16; e += threads_of(BX)) reinterpret_cast<float4*>(x_tiles)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    pair_sync();                                     // both CTAs' barriers exist, and the zeros
+    if (LOCAL) {
+        chain_wait();
+        chain_release();
+    }
 
     // The adders' sums want more registers than an even share: the launch's 896 x 72 as 128 x 40 + 256 x 56 + 512 x 88.
     constexpr bool SHARES = threads_of(BX) == 896;
@@ -155,9 +172,27 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                 for (int i = 0; i < it.count; ++i, ++g) {
                     const int s = g % RING;
                     if (!mbar_wait(&raw_empty_bar[s], ((g / RING) & 1) ^ 1, p.error, 21)) { failed = 1; break; }
-                    mbar_expect_tx(&raw_full_bar[s], RAW_BYTES);
+                    mbar_expect_tx(&raw_full_bar[s], LOCAL && rank == 0 ? RAW_BYTES : W_BYTES);
                     tma_load_2d(ring + s * RAW_BYTES, &map_w, &raw_full_bar[s], (it.first + i) * BK, it.n0 + rank * BW);
-                    tma_load_2d(ring + s * RAW_BYTES + W_BYTES, &map_x, &raw_full_bar[s], (it.first + i) * BK, it.m0 + rank * (BX / 2));
+                    if (LOCAL && rank == 0) tma_load_2d(ring + s * RAW_BYTES + W_BYTES, &map_hi, &raw_full_bar[s], (it.first + i) * BK, it.m0);
+                }
+            }
+        } else if (!LOCAL && warp == X_WARP && lane == 0) {
+            // Only x waits for the kernel ahead, which split it: that one has waited for all before it, so W is in memory and nothing reads y
+            // or the scratch any more when this kernel's first CTA starts.
+            chain_wait();
+            chain_release();
+            int g = 0;
+            for (int at = pair; at < p.items && !failed; at += pairs) {
+                const Item it = item_of(p, at, BX);
+                for (int i = 0; i < it.count; ++i, ++g) {
+                    const int a = g % PAIRS;
+                    if (!mbar_wait(&free_bar[a], ((g / PAIRS) & 1) ^ 1, p.error, 27)) { failed = 1; break; }
+                    const uint32_t ready = in_first_cta(&ready_bar[a]);
+                    if (rank == 0) mbar_expect_tx(&ready_bar[a], 4 * X_BYTES);        // of both CTAs
+                    unsigned char* tile = x_tiles + a * 2 * X_BYTES;
+                    tma_load_2d_pair(tile, &map_hi, ready, (it.first + i) * BK, it.m0 + rank * (BX / 2));
+                    tma_load_2d_pair(tile + X_BYTES, &map_lo, ready, (it.first + i) * BK, it.m0 + rank * (BX / 2));
                 }
             }
         } else if (warp == 1 && rank == 0) {
@@ -176,7 +211,7 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                     if (!ok) { failed = 1; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t w_hi = tmem_base + A_COLS + a * 2 * BK, w_lo = w_hi + BK, d = tmem_base + b * BX;
-                    const uint64_t x_hi = smem_desc(split + a * 2 * X_BYTES), x_lo = smem_desc(split + a * 2 * X_BYTES + X_BYTES);
+                    const uint64_t x_hi = smem_desc(x_tiles + a * 2 * X_BYTES), x_lo = smem_desc(x_tiles + a * 2 * X_BYTES + X_BYTES);
 #pragma unroll
                     for (int k = 0; k < BK / 8; ++k) umma_tf32(leader, d, w_hi + 8 * k, x_lo + 2 * k, idesc, k != 0);   // 8 numbers of K: 8 columns, 32 bytes
 #pragma unroll
@@ -221,22 +256,18 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                 tmem_st16(lane_addr + a * 2 * BK + 16 * half, hi);
                 tmem_st16(lane_addr + a * 2 * BK + BK + 16 * half, lo);
             }
-            const float4* raw = reinterpret_cast<const float4*>(ring + s * RAW_BYTES + W_BYTES);
-            float4* x_hi = reinterpret_cast<float4*>(split + a * 2 * X_BYTES);
-            float4* x_lo = reinterpret_cast<float4*>(split + a * 2 * X_BYTES + X_BYTES);
-#pragma unroll 4
-            for (int e = quarter * 32 + lane; e < X_BYTES / 16; e += 32 * SPLIT_WARPS) {
-                const float4 v = raw[e];
-                const float4 h = make_float4(to_tf32(v.x), to_tf32(v.y), to_tf32(v.z), to_tf32(v.w));
-                x_lo[e] = make_float4(v.x - h.x, v.y - h.y, v.z - h.z, v.w - h.w);
-                x_hi[e] = h;
+            if (LOCAL && rank == 0) {
+                const float4* raw = reinterpret_cast<const float4*>(ring + s * RAW_BYTES + W_BYTES);
+                float4* x_hi = reinterpret_cast<float4*>(x_tiles + a * 2 * X_BYTES);
+                for (int e = quarter * 32 + lane; e < X_BYTES / 16; e += 32 * SPLIT_WARPS) split_four(raw[e], x_hi[e], x_hi[X_BYTES / 16 + e]);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");          // the MMAs read x through the async proxy
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");              // the MMAs read x through the async proxy
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive_remote(in_first_cta(&ready_bar[a]));
+                if (rank == 0) mbar_arrive(&ready_bar[a]);
+                else mbar_arrive_remote(in_first_cta(&ready_bar[a]));
                 mbar_arrive(&raw_empty_bar[s]);
             }
         }
@@ -359,13 +390,26 @@ void cut(int N, int K, int* blocks, int* per_segment, int* segments) {
     *segments = (*blocks + *per_segment - 1) / *per_segment;
 }
 
-template <int BX, int RING, int PAIRS, int SUMS>
-int launch(SgemmParams p, int segments, cudaStream_t stream) {
-    CUtensorMap map_w, map_x;
+// x as two TF32 numbers an element, in matrices of their own [M][K].  Its error: to_tf32.
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, long long ldx, float* __restrict__ hi, float* __restrict__ lo, int M, int K) {
+    chain_wait();
+    chain_release();
+    const long long e = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (e >= (long long)M * K) return;
+    split_four(*reinterpret_cast<const float4*>(x + e / K * ldx + e % K), *reinterpret_cast<float4*>(hi + e), *reinterpret_cast<float4*>(lo + e));
+}
+
+// hi, lo: x's pieces in rows of K, or null: LOCAL
+template <int BX, int RING, int PAIRS, int SUMS, bool LOCAL>
+int launch(SgemmParams p, const float* hi, const float* lo, int segments, cudaStream_t stream) {
+    CUtensorMap map_w, map_hi, map_lo;
     if (make_tile_map(&map_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.w, p.N, p.K, p.ldw, BW, "sgemm_tcgen05")) return 1;
-    if (make_tile_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.x, p.M, p.K, p.ldx, BX / 2, "sgemm_tcgen05")) return 1;
-    constexpr size_t smem = (size_t)RING * (W_BYTES + BX / 2 * BK * 4) + PAIRS * BX * BK * 4 + 1024;
-    auto kernel = sgemm_tcgen05_kernel<BX, RING, PAIRS, SUMS>;
+    if (make_tile_map(&map_hi, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, LOCAL ? p.x : hi, p.M, p.K, LOCAL ? p.ldx : p.K, BX / 2, "sgemm_tcgen05")) return 1;
+    if (LOCAL) map_lo = map_hi;                          // not read
+    else if (make_tile_map(&map_lo, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, lo, p.M, p.K, p.K, BX / 2, "sgemm_tcgen05")) return 1;
+    constexpr size_t smem = (size_t)RING * (W_BYTES + (LOCAL ? BX / 2 * BK * 4 : 0)) + PAIRS * BX * BK * 4 + 1024;
+    static_assert(smem <= 226 * 1024, "shared memory of an SM");
+    auto kernel = sgemm_tcgen05_kernel<BX, RING, PAIRS, SUMS, LOCAL>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     p.items = ((p.N + 2 * BW - 1) / (2 * BW)) * ((p.M + BX - 1) / BX) * (p.in_turn ? 1 : segments);
     cudaLaunchConfig_t cfg = {};
@@ -382,7 +426,7 @@ int launch(SgemmParams p, int segments, cudaStream_t stream) {
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ts_chaining_enabled() ? 2 : 1;
-    TS_CHAINED_CHECK("sgemm_tcgen05", cudaLaunchKernelEx(&cfg, kernel, map_w, map_x, p));
+    TS_CHAINED_CHECK("sgemm_tcgen05", cudaLaunchKernelEx(&cfg, kernel, map_w, map_hi, map_lo, p));
     return 0;
 }
 
@@ -420,29 +464,57 @@ bool sgemm_tcgen05_supported(const float* x, const float* w, int K, long long ld
     return K >= MIN_TERMS && K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0;
 }
 
-// Floats of scratch a product of these sizes needs (0: none).
+// Rows of x that the first CTA of a pair splits itself: half of the narrowest tile.
+constexpr int LOCAL_ROWS = 16;
+
+// Rows of x that are split at a time: their pieces stay within MAX_SCRATCH (no fewer than a tile of rows).
+static int rows_at_once(int M, int K) {
+    const long long rows = MAX_SCRATCH / 2 / K / 128 * 128;
+    return rows >= M ? M : rows < 128 ? (M < 128 ? M : 128) : (int)rows;
+}
+
+// Floats of scratch a product of these sizes needs: x's pieces, and the segments' sums where they are apart.
 long long sgemm_tcgen05_scratch_floats(int M, int N, int K) {
     int blocks, per, segments;
     cut(N, K, &blocks, &per, &segments);
-    return segments > 1 && !choose(M, N, blocks, per, segments).in_turn ? (long long)segments * M * N : 0;
+    const int rows = rows_at_once(M, K);
+    long long sums = 0;
+    for (const int m : {rows, M % rows})
+        if (m > 0 && segments > 1 && !choose(m, N, blocks, per, segments).in_turn && (long long)segments * m * N > sums) sums = (long long)segments * m * N;
+    return (M <= LOCAL_ROWS ? 0 : 2ll * rows * K) + sums;
 }
 
-int sgemm_tcgen05(const float* x, const float* w, float* y, int M, int N, int K, long long ldx, long long ldw, long long ldy,
-                  float* scratch, int* error, cudaStream_t stream) {
+static int run_rows(const float* x, const float* w, float* y, int M, int N, int K, long long ldx, long long ldw, long long ldy, float* scratch,
+                    float* sums, int* error, cudaStream_t stream) {
     int blocks, per, segments;
     cut(N, K, &blocks, &per, &segments);
     const Shape shape = choose(M, N, blocks, per, segments);
     const bool parts = segments > 1 && !shape.in_turn;
-    SgemmParams p{parts ? scratch : y, x, w, M, N, K, ldx, ldw, parts ? N : ldy, parts ? (long long)M * N : 0, blocks, per,
+    const bool local = M <= LOCAL_ROWS;
+    float *hi = local ? nullptr : scratch, *lo = local ? nullptr : scratch + (long long)M * K;
+    if (!local) {
+        const long long pieces = (long long)M * K / 4;
+        TS_CHAINED_CHECK("sgemm_tcgen05 (split)", launch_chained(split_rows_kernel, dim3((unsigned)((pieces + 255) / 256)), dim3(256), 0, stream, x, ldx, hi, lo, M, K));
+    }
+    SgemmParams p{parts ? sums : y, x, w, M, N, K, ldx, ldw, parts ? N : ldy, parts ? (long long)M * N : 0, blocks, per,
                   shape.in_turn, 0, error};
-    const int failed = shape.bx == 32 ? launch<32, 10, 4, 4>(p, segments, stream)
-                     : shape.bx == 64 ? launch<64, 8, 4, 4>(p, segments, stream) : launch<128, 6, 4, 2>(p, segments, stream);
+    const int failed = local ? launch<32, 10, 4, 4, true>(p, hi, lo, segments, stream)
+                     : shape.bx == 32 ? launch<32, 10, 6, 4, false>(p, hi, lo, segments, stream)
+                     : shape.bx == 64 ? launch<64, 10, 4, 4, false>(p, hi, lo, segments, stream) : launch<128, 10, 4, 2, false>(p, hi, lo, segments, stream);
     if (failed || !parts) return failed;
-    const bool vec = N % 4 == 0 && ldy % 4 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)scratch % 16 == 0;
+    const bool vec = N % 4 == 0 && ldy % 4 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)sums % 16 == 0;
     const long long items = (long long)M * N / (vec ? 4 : 1);
     auto kernel = vec ? add_segments_kernel<4> : add_segments_kernel<1>;
     TS_CHAINED_CHECK("sgemm_tcgen05 (segments)",
-                     launch_chained(kernel, dim3((unsigned)((items + 255) / 256)), dim3(256), 0, stream, (const float*)scratch, y,
+                     launch_chained(kernel, dim3((unsigned)((items + 255) / 256)), dim3(256), 0, stream, (const float*)sums, y,
                                     segments, (long long)M * N, M, N, ldy));
+    return 0;
+}
+
+int sgemm_tcgen05(const float* x, const float* w, float* y, int M, int N, int K, long long ldx, long long ldw, long long ldy,
+                  float* scratch, int* error, cudaStream_t stream) {
+    const int rows = rows_at_once(M, K);
+    for (int m = 0; m < M; m += rows)
+        if (run_rows(x + m * ldx, w, y + m * ldy, M - m < rows ? M - m : rows, N, K, ldx, ldw, ldy, scratch, scratch + (M <= LOCAL_ROWS ? 0 : 2ll * rows * K), error, stream)) return 1;
     return 0;
 }

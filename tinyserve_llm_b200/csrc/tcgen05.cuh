@@ -77,9 +77,15 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {          // ar
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                  ::"r"(smem_u32(bar)), "h"(both) : "memory");
 }
-// An arrival on the other CTA's barrier for hand-offs to the tensor cores, whose reads and writes are ordered by tcgen05's fences and, in
-// shared memory, by the proxy fence: without an order at cluster scope between this thread's own writes to memory and what the other
-// CTA reads, which costs a microsecond.
+// A load into this CTA's shared memory that is counted on the first CTA's barrier.
+__device__ __forceinline__ void tma_load_2d_pair(void* smem, const CUtensorMap* map, uint32_t bar_in_first, int x, int y) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(smem_u32(smem)), "l"(map), "r"(bar_in_first), "r"(x), "r"(y) : "memory");
+}
+// An arrival on the other CTA's barrier that hands tensor memory over (an accumulator back, an operand on), which tcgen05's fences on both
+// sides order.  It orders none of this thread's writes to shared or global memory for the other CTA: that takes a release at cluster scope,
+// about a microsecond each.  What MMAs of the first CTA read from the second one's shared memory is brought there by TMA.
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t bar_in_cluster) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_in_cluster) : "memory");
 }

@@ -134,6 +134,7 @@ _WAIT_CODES: dict[int, tuple[str, str]] = {
     24: ("sgemm_tcgen05", "MMA issuer waiting for a drained accumulator"),
     25: ("sgemm_tcgen05", "adders waiting for a block's sums"),
     26: ("sgemm_tcgen05", "split warps waiting for free operand tiles"),
+    27: ("sgemm_tcgen05", "TMA producer of x waiting for a free operand tile"),
     31: ("delta_tiles", "warps of the state waiting for a tile"),
     32: ("delta_tiles", "warps of U and the output waiting for a tile"),
 }
