@@ -179,6 +179,31 @@ def test_float32_matrix_product_keeps_infinities_and_nans(ops):
     assert torch.equal(got[got.isinf()], want[want.isinf()])
 
 
+@pytest.mark.parametrize("dtype, out_dtype", [(torch.bfloat16, None), (torch.bfloat16, torch.float32), (torch.float32, None)])
+@pytest.mark.parametrize("columns, offset", [(1, 3), (16, 0), (16, 8), (33, 5), (64, 1), (520, 24)])
+def test_product_of_a_stretch_of_columns(ops, columns, offset, dtype, out_dtype):
+    """Rows around the largest number that the engine's own kernel takes; stretches on and beside 16-byte boundaries, odd ones among them."""
+    n, most = 72, ops.skinny_max_rows
+    from tinyserve_llm_b200.ops.library import KernelError
+    w = rand((n, columns), dtype, 6)
+    for rows in (1, most, most + 1, 3 * most):
+        wide = rand((rows, offset + columns + 7), dtype, 5)
+        x = wide.to(DEV)[:, offset:offset + columns]
+        before = ops.calls.get("library_mm", 0)
+        got = ops.linear_columns(x, w.to(DEV), out_dtype)
+        if dtype == torch.bfloat16 and rows > most and columns > 1:
+            assert ops.calls.get("library_mm", 0) == before + 1
+        want = wide[:, offset:offset + columns].double() @ w.double().T
+        assert got.dtype == (out_dtype or dtype) and got.is_contiguous()
+        # float32 sums of at most `columns` terms, each within 2^-23 of itself, then one rounding to the type, before which the library may
+        # round the sums of pieces of a long K (together no larger than the terms' sizes) to it as well
+        size = wide[:, offset:offset + columns].double().abs() @ w.double().abs().T
+        bound = columns * 2.0 ** -23 * size + (want.abs() * 2.0 ** -8 + size * 2.0 ** -9 * (columns > 256) if got.dtype == torch.bfloat16 else 0)
+        assert bool(((got.cpu().double() - want).abs() <= bound + 1e-30).all())
+    with pytest.raises(KernelError):
+        ops.linear_columns(x, rand((n, columns + 1), dtype, 7).to(DEV))
+
+
 @pytest.mark.parametrize("m, n, k", [(1, 48, 64), (9, 1000, 192), (300, 250, 520)])
 def test_bfloat16_matrix_product(ops, m, n, k):
     x, w = rand((m, k), torch.bfloat16, 5), rand((n, k), torch.bfloat16, 6)

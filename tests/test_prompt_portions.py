@@ -261,7 +261,7 @@ def test_tiles_are_no_further_from_64_bits_than_the_walk(form, tokens, heads):
     assert off[0] <= off[2] and off[1] <= off[3], off
 
 
-def _stretched(dim, vdim, T, plant=None):
+def _stretched(dim, vdim, T, plant=None, name="v"):
     """bfloat16 portions of T, 1 and 130 tokens by stretches: (output, states, what 64 bits give for both)."""
     ops, H, lens = get_ops(), 3, [T, 1, 130]
     g = torch.Generator().manual_seed(dim + vdim)
@@ -271,7 +271,7 @@ def _stretched(dim, vdim, T, plant=None):
     cuts = (0, H * dim, 2 * H * dim, H * (2 * dim + vdim))
     if plant is not None:
         row, column, value = plant
-        y[row, cuts[2] + column] = value
+        (z if name == "z" else y)[row, {"q": 0, "k": cuts[1], "v": cuts[2], "z": 0}[name] + column] = value
     dev, yd = state.cuda(), y.cuda()
     ctx, binding = _step(dev, lens)
     before = ops.calls.get("ts_plain_tiles", 0)
@@ -306,6 +306,25 @@ def test_a_value_that_is_not_finite_stays_in_its_column_by_stretches(value):
     assert torch.equal(got[:201], clean[:201]) and not torch.isfinite(got[201:300, 2 * 40 + 17]).any()
     got[201:300, 2 * 40 + 17] = clean[201:300, 2 * 40 + 17]
     assert torch.equal(got, clean)
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf"), 3.38e38])
+@pytest.mark.parametrize("name", ["q", "k", "z"])
+def test_what_is_not_finite_stays_with_its_head_and_later_tokens_by_stretches(name, value):
+    """In the middle of a tile, a stretch behind it and one before: earlier tokens, other heads and other requests keep their bits, states too."""
+    dim, vdim, token = 64, 40, 201
+    (clean, states, *_), (got, left, *_) = _stretched(dim, vdim, 300), _stretched(dim, vdim, 300, (token, dim + 5, value), name)
+    assert torch.equal(got[:token], clean[:token]) and torch.equal(got[300:], clean[300:])
+    mine = slice(vdim, 2 * vdim)                         # the second head's outputs
+    if name in "qk" and value != 3.38e38:
+        assert not torch.isfinite(got[token, mine]).any()
+    end = token + 1 if name == "q" else 300
+    got[token:end, mine] = clean[token:end, mine]
+    assert torch.equal(got, clean)
+    if name != "q":                                      # the state of that request's head, in the planted channel's row
+        row = states[-1].view(3, dim, vdim)[1, 5].clone()
+        left[-1].view(3, dim, vdim)[1, 5] = row
+    assert torch.equal(left, states)
 
 
 def _recurrence_part(kind, dtype):
@@ -382,6 +401,20 @@ def test_short_portions_walk_token_by_token(kind, entry, tokens):
         assert ops.calls.get(entry, 0) == before + tiles
 
 
+@pytest.mark.parametrize("bound,tiles", [(256, False), (512, True)])
+def test_a_replayed_step_goes_by_its_bound(bound, tiles):
+    """Grids of a replayed step are sized by a power of two: what decides whether its portions go by stretches, however long they are."""
+    ops = get_ops()
+    part, x = _recurrence_part("plain", torch.bfloat16)
+    for longest in (60, 256):
+        ctx = make_ctx([longest, 1], [longest, 1])
+        ctx.prefill_seqs, ctx.replayed, ctx.max_q_len = i32([0, -1]), True, bound
+        state = torch.zeros(2, part.state_bytes(), dtype=torch.uint8, device="cuda")
+        before = ops.calls.get("ts_plain_tiles", 0)
+        part.forward(x[:longest + 1], ctx, EntryBinding(None, None, 0, 0, 16, 0, state=state, state_slots=i32([0, 1])))
+        assert ops.calls.get("ts_plain_tiles", 0) == before + tiles
+
+
 def test_every_tile_of_a_step_has_room_in_the_buffer():
     """The kernels number a request's tiles from cu_q / 16 + its index on; the buffer holds T / 16 + requests + 1."""
     g = torch.Generator().manual_seed(0)
@@ -431,21 +464,26 @@ def test_beside_tiles_only_single_tokens_are_prepared(kind, monkeypatch):
     assert written.nonzero().flatten().tolist() == [300, 341]
 
 
-def _windowed_latent(heads, dim, rot, rank, window, lens, cached, page, plant=None):
+def _windowed_latent(heads, dim, rot, rank, window, lens, cached, page, plant=None, sink=False, gate=False, magnitude=1.0):
     """A windowed latent layer over prompt portions: (output, cache rows written, what 64 bits give).  Pages before a window are given back."""
     from tinyserve_llm_b200.config.spec import InlineRotarySpec, LatentAttentionSpec
     from tinyserve_llm_b200.parts.base import Runtime, part_class
     g = torch.Generator().manual_seed(dim + rank + window)
     W, scale, eps = 96, 2.0 / (dim + rot) ** 0.5, 1e-5
     spec = LatentAttentionSpec(hidden_size=W, num_heads=heads, head_dim=dim, rot_dim=rot, value_dim=dim, q_rank=0, kv_rank=rank, scale=scale, window=window,
-                               norm_eps=eps, position=InlineRotarySpec(dims=rot))
+                               norm_eps=eps, position=InlineRotarySpec(dims=rot), sink=sink, output_gate=gate)
     w = {"q": torch.randn(heads * (dim + rot), W, generator=g) * W ** -0.5, "dkv": torch.randn(rank + rot, W, generator=g) * W ** -0.5,
          "uk": torch.randn(heads * dim, rank, generator=g) * rank ** -0.5, "uv": torch.randn(heads * dim, rank, generator=g) * rank ** -0.5,
          "o": torch.randn(W, heads * dim, generator=g) * (heads * dim) ** -0.5}
     w = {n: t.to(torch.bfloat16) for n, t in w.items()}
     w["dkv.norm"] = 1 + torch.randn(rank, generator=g) * 0.1
+    if sink:
+        w["sink"] = torch.linspace(-2.0, 6.0, heads)
+    if gate:
+        w["g"] = (torch.randn(heads * dim, W, generator=g) * W ** -0.5).to(torch.bfloat16)
     rt = Runtime(dtype=torch.bfloat16, device=torch.device("cuda", 0), ops=get_ops())
     part = part_class("mixer", spec)(spec, w, rt)
+    part.magnitude = magnitude
     x = torch.randn(sum(lens), W, generator=g).to(torch.bfloat16)
     if plant is not None:
         x[plant, 3] = float("nan")
@@ -480,7 +518,7 @@ def _windowed_latent(heads, dim, rot, rank, window, lens, cached, page, plant=No
     def turned(t, positions):                            # [n, k, rot]
         a = positions.double()[:, None, None] * freq
         u, v = t.chunk(2, dim=-1)
-        return torch.cat([u * a.cos() - v * a.sin(), v * a.cos() + u * a.sin()], dim=-1)
+        return torch.cat([u * a.cos() - v * a.sin(), v * a.cos() + u * a.sin()], dim=-1) * magnitude
 
     want, at = [], 0
     for n, c, rows in zip(lens, cached, history):
@@ -494,8 +532,10 @@ def _windowed_latent(heads, dim, rot, rank, window, lens, cached, page, plant=No
         s = torch.einsum("ihd,jhd->hij", q, k) * scale
         j = torch.arange(c + n)[None]
         s = s.masked_fill((j > positions[:, None]) | (j <= positions[:, None] - window), -float("inf"))
-        o = torch.einsum("hij,jhd->ihd", torch.softmax(s, -1), (full[:, :rank] @ d["uv"].t()).view(-1, heads, dim))
-        want.append(o.reshape(n, -1) @ d["o"].t())
+        if sink:                                         # a score without a key or a value
+            s = torch.cat([s, d["sink"][:, None, None].expand(-1, n, 1)], dim=-1)
+        o = torch.einsum("hij,jhd->ihd", torch.softmax(s, -1)[..., :c + n], (full[:, :rank] @ d["uv"].t()).view(-1, heads, dim)).reshape(n, -1)
+        want.append((o * torch.sigmoid(xs @ d["g"].t()) if gate else o) @ d["o"].t())
         at += n
     return got.double().cpu(), torch.cat(want)
 
@@ -510,6 +550,15 @@ def test_windowed_latent_portions_on_keys_and_values_of_their_own(heads, dim, ro
     # single row scores of up to 8 (two is their deviation), off by up to 2^-9 of themselves, move its weights by as much as 8 2^-9 more
     err, off = (got - want).norm(dim=-1) / want.norm(dim=-1), float((got - want).norm() / want.norm())
     assert float(err.max()) < 15 * 2.0 ** -9 and off < 3.5 * 2.0 ** -9, (float(err.max()), off)
+
+
+@pytest.mark.parametrize("heads,dim", [(3, 128), (2, 64)])
+@pytest.mark.parametrize("options", [{"sink": True}, {"gate": True}, {"magnitude": 1.4}, {"sink": True, "gate": True, "magnitude": 0.8}])
+def test_windowed_latent_portions_with_sinks_gates_and_magnitudes(heads, dim, options):
+    """The options of the layers without a window.  Bounds as above; sinks and gates make outputs smaller and round once more."""
+    got, want = _windowed_latent(heads, dim, 32, 128, 90, [200, 1, 150], [0, 70, 333], 64, **options)
+    err, off = (got - want).norm(dim=-1) / want.norm(dim=-1), float((got - want).norm() / want.norm())
+    assert float(err.max()) < 15 * 2.0 ** -9 and off < 4 * 2.0 ** -9, (float(err.max()), off)
 
 
 def test_a_latent_that_is_not_finite_reaches_the_queries_that_see_it_only():
