@@ -141,6 +141,17 @@ def test_float32_matrix_product_on_split_operands(ops, m, n, k):
     ops.check_device_errors()
 
 
+def test_an_error_is_named_whatever_mode_made_the_error_word(ops, monkeypatch):
+    """A word that an engine's step makes, under inference mode, and a caller without one looks at."""
+    from tinyserve_llm_b200.ops.library import KernelError
+    monkeypatch.setattr(ops, "_error_word", None)
+    with torch.inference_mode():
+        ops.error_word()[0] = 23
+    with pytest.raises(KernelError, match="sgemm_tcgen05"):
+        ops.check_device_errors()
+    ops.check_device_errors()
+
+
 @pytest.mark.parametrize("m, n, k", [(16, 2048, 2048), (17, 2048, 2048), (100, 3000, 1024), (530, 64, 65536)])
 def test_float32_matrix_product_repeats_itself(ops, m, n, k):
     """Operands that one CTA of a pair brings for the other's MMAs: rows one CTA splits by itself, rows split before, more rows than are split at a time."""

@@ -272,7 +272,8 @@ class Ops:
         it before every step and names the kernel by the registered code (`register_wait_codes`).
         """
         if self._error_word is None:
-            self._error_word = torch.zeros((1,), dtype=torch.int32).pin_memory()
+            with torch.inference_mode(False):                # `check_device_errors` resets it in whatever mode it is called
+                self._error_word = torch.zeros((1,), dtype=torch.int32).pin_memory()
         return self._error_word
 
     def load_extension(self, name: str, sources: list[str], kernels: dict[str, tuple[str, str]]) -> None:
@@ -895,7 +896,7 @@ class Ops:
             self._check_rows(k_low, "k_low")
             low_cols = (k_low.data_ptr() - k.data_ptr()) // 2
             if k_low.dtype != k.dtype or k_low.shape != k.shape or k_low.stride(0) != k.stride(0) or not 0 < low_cols <= k.stride(0) - k.shape[1]:
-                raise KernelError(f"dense_prompt_attention: second pieces {tuple(k_low.shape)} {k_low.dtype} that are not columns behind k's {tuple(k.shape)}")
+                raise KernelError(f"dense_prompt_attention: second pieces {tuple(k_low.shape)} {k_low.dtype} are not columns behind k's {tuple(k.shape)}")
         if odd_rows is not None:
             self._check(odd_rows, "odd_rows", torch.uint8, 1)
             if odd_rows.shape[0] != k.shape[0]:
