@@ -1,5 +1,5 @@
 // Prefill attention on the fifth-generation tensor cores, head sizes 64 and 128, bfloat16, pages of a
-// multiple of 64 tokens, no window.  A CTA takes 128 consecutive tokens of one request for one query head
+// multiple of 64 tokens; windows in the SIGMOID and BOUNDED forms.  A CTA takes 128 consecutive tokens of one request for one query head
 // (head size 128: rows lie in shared memory as two sub-tiles of 64 dims, key tiles hold 64 keys, so that
 // two CTAs still fit an SM's shared and tensor memory):
 //
@@ -28,12 +28,14 @@
 // row each, into tensor memory as two bfloat16 pieces, x = hi + lo, both A operands against the shared sub-tile.  Behind a window it
 // also takes the heads' own keys and the probabilities as two pieces (PAIR): it stands in for kernels on the latents themselves
 // (attention_latent_mma.cu, attention_latent_tokens.cu), which round neither, and is with them no further from 64 bits than those
-// (relative error of the attention alone, 3 heads of 64 + 32 channels, latent of 256, window 100, scores of deviation 1 / 3 / 6: there 2.45 / 2.81 /
-// 3.23e-3, here 2.32 / 2.34 / 2.32e-3, with keys of one piece 2.62 / 3.35 / 4.02e-3; 2,048 tokens, 16 heads of 128, window 1,024: a layer takes 168 us, 141 with one).
-// With heads of 128 channels one CTA holds an SM.
+// (relative error of the attention alone, 3 heads of 64 + 32 channels, latent of 256, window 100, scores of deviation 1 / 3 / 6: there 2.45 /
+// 2.81 / 3.23e-3, here 2.32 / 2.34 / 2.32e-3, with keys of one piece 2.62 / 3.35 / 4.02e-3; 2,048 tokens, 16 heads of 128, window 1,024: a layer
+// takes 168 us, 141 with one).  With heads of 128 channels one CTA holds an SM: its softmax waits for its own products (issue slots 23 %, tensor
+// cores 26 %).
 //
-// What a tile costs beside its arithmetic (4.5 instructions an element of the scores) is what bounds it: two CTAs an SM issue half of the
-// time, and taking out exponentials, sums or the second product changes little.  So: waits read the clock only where a first look was
+// What bounds it is a tile's chain (scores, wait, softmax, wait, product), which two CTAs an SM do not fill: at 2,048 tokens, 32 heads of 64,
+// issue slots are used to 45 %, the exponentials' unit to 46, the tensor cores to 22, and taking out exponentials, sums or the second product
+// changes little; warps wait for barriers and tensor memory (3.0 of 9.8 cycles an instruction), fixed latencies (1.6) and each other (1.0).  So: waits read the clock only where a first look was
 // not enough and let the hardware choose how long to sleep (a hint of 1 ms cost 3 %), a warp's failure is no vote a tile, the barrier of two warps has its
 // number in a register, and the correction is worked out only where a row's maximum moved.  8,192 tokens, 32 heads, us: 456 -> 412 (head
 // 64), 685 -> 606 (128; 907 TFLOP/s); 2,048 tokens 47.7 -> 44.6 and 60.4 -> 54.7.
@@ -557,7 +559,7 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, ROT, FORM == BOUNDED && RO
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-            if (lane == 0) mbar_arrive(&p_ready);
+                if (lane == 0) mbar_arrive(&p_ready);
             } else {
             if constexpr (LOW) {
                 if (p.cap_pre != 0.f) {              // capped scores: tanh(product * scale / cap); the cap joins the exponent's scale

@@ -644,7 +644,7 @@ __global__ void __launch_bounds__(THREADS) recurrence_tiles_kernel(ScanArgs p) {
 
 // The delta rules' walk.  A CTA owns one request, one head and 16 columns.  Eight warps hold the state's rows.  A tile is a chain: k side
 // against S_0, its sum over the warps, U, the update.  What it does not wait for is beside it: the q side's product runs while two warps
-// without rows make U and two more (P W) (V - R), and those sum up and store the output under the update and the next tile's k side.
+// without rows make U and two more (P W) (V - R), and those sum up and store the output under the update (all meet before the next tile).
 // Packs and coefficients come by bulk copies, two tiles in shared memory.  Every wait for them gives up after about two seconds and says
 // so in an error word; the CTA then stores nothing of that tile and the later ones, leaves the state as it was, waits once more, as long, for
 // the copies on their way (the shared memory they write will be another CTA's) and returns.

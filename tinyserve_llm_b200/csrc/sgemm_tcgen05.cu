@@ -259,7 +259,8 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             if (LOCAL && rank == 0) {
                 const float4* raw = reinterpret_cast<const float4*>(ring + s * RAW_BYTES + W_BYTES);
                 float4* x_hi = reinterpret_cast<float4*>(x_tiles + a * 2 * X_BYTES);
-                for (int e = quarter * 32 + lane; e < X_BYTES / 16; e += 32 * SPLIT_WARPS) split_four(raw[e], x_hi[e], x_hi[X_BYTES / 16 + e]);
+                for (int e = quarter * 32 + lane; e < X_BYTES / 16; e += 32 * SPLIT_WARPS)
+                    split_four(raw[e], x_hi[e], x_hi[X_BYTES / 16 + e]);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");          // the MMAs read x through the async proxy
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -391,7 +392,8 @@ void cut(int N, int K, int* blocks, int* per_segment, int* segments) {
 }
 
 // x as two TF32 numbers an element, in matrices of their own [M][K].  Its error: to_tf32.
-__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, long long ldx, float* __restrict__ hi, float* __restrict__ lo, int M, int K) {
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, long long ldx, float* __restrict__ hi,
+                                                         float* __restrict__ lo, int M, int K) {
     chain_wait();
     chain_release();
     const long long e = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
@@ -479,8 +481,10 @@ long long sgemm_tcgen05_scratch_floats(int M, int N, int K) {
     cut(N, K, &blocks, &per, &segments);
     const int rows = rows_at_once(M, K);
     long long sums = 0;
-    for (const int m : {rows, M % rows})
-        if (m > 0 && segments > 1 && !choose(m, N, blocks, per, segments).in_turn && (long long)segments * m * N > sums) sums = (long long)segments * m * N;
+    for (const int m : {rows, M % rows}) {
+        const long long need = (long long)segments * m * N;
+        if (m > 0 && segments > 1 && !choose(m, N, blocks, per, segments).in_turn && need > sums) sums = need;
+    }
     return (M <= LOCAL_ROWS ? 0 : 2ll * rows * K) + sums;
 }
 
@@ -494,7 +498,8 @@ static int run_rows(const float* x, const float* w, float* y, int M, int N, int 
     float *hi = local ? nullptr : scratch, *lo = local ? nullptr : scratch + (long long)M * K;
     if (!local) {
         const long long pieces = (long long)M * K / 4;
-        TS_CHAINED_CHECK("sgemm_tcgen05 (split)", launch_chained(split_rows_kernel, dim3((unsigned)((pieces + 255) / 256)), dim3(256), 0, stream, x, ldx, hi, lo, M, K));
+        TS_CHAINED_CHECK("sgemm_tcgen05 (split)", launch_chained(split_rows_kernel, dim3((unsigned)((pieces + 255) / 256)), dim3(256), 0,
+                                                                 stream, x, ldx, hi, lo, M, K));
     }
     SgemmParams p{parts ? sums : y, x, w, M, N, K, ldx, ldw, parts ? N : ldy, parts ? (long long)M * N : 0, blocks, per,
                   shape.in_turn, 0, error};
@@ -514,7 +519,8 @@ static int run_rows(const float* x, const float* w, float* y, int M, int N, int 
 int sgemm_tcgen05(const float* x, const float* w, float* y, int M, int N, int K, long long ldx, long long ldw, long long ldy,
                   float* scratch, int* error, cudaStream_t stream) {
     const int rows = rows_at_once(M, K);
+    float* sums = scratch + (M <= LOCAL_ROWS ? 0 : 2ll * rows * K);
     for (int m = 0; m < M; m += rows)
-        if (run_rows(x + m * ldx, w, y + m * ldy, M - m < rows ? M - m : rows, N, K, ldx, ldw, ldy, scratch, scratch + (M <= LOCAL_ROWS ? 0 : 2ll * rows * K), error, stream)) return 1;
+        if (run_rows(x + m * ldx, w, y + m * ldy, M - m < rows ? M - m : rows, N, K, ldx, ldw, ldy, scratch, sums, error, stream)) return 1;
     return 0;
 }
