@@ -156,10 +156,8 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     pair_sync();                                     // both CTAs' barriers exist, and the zeros
-    if (LOCAL) {
-        chain_wait();
-        chain_release();
-    }
+    chain_wait();
+    chain_release();
 
     // The adders' sums want more registers than an even share: the launch's 896 x 72 as 128 x 40 + 256 x 56 + 512 x 88.
     constexpr bool SHARES = threads_of(BX) == 896;
@@ -178,10 +176,6 @@ sgemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                 }
             }
         } else if (!LOCAL && warp == X_WARP && lane == 0) {
-            // Only x waits for the kernel ahead, which split it: that one has waited for all before it, so W is in memory and nothing reads y
-            // or the scratch any more when this kernel's first CTA starts.
-            chain_wait();
-            chain_release();
             int g = 0;
             for (int at = pair; at < p.items && !failed; at += pairs) {
                 const Item it = item_of(p, at, BX);
