@@ -385,7 +385,8 @@ void cut(int N, int K, int* blocks, int* per_segment, int* segments) {
     *segments = (*blocks + *per_segment - 1) / *per_segment;
 }
 
-// x as two TF32 numbers an element, in matrices of their own [M][K].  Its error: to_tf32.
+// x as two TF32 numbers an element, in matrices of their own [M][K].  Its error: to_tf32.  Bound by its launch: 100 to 512 rows of 2,048 take 3.5
+// to 4 us by themselves, 2.5 in a chain.
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, long long ldx, float* __restrict__ hi,
                                                          float* __restrict__ lo, int M, int K) {
     chain_wait();
